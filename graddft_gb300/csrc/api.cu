@@ -4,6 +4,7 @@
 #include <string.h>
 
 #include "common.cuh"
+#include "fx.cuh"
 #include "kernels.cuh"
 #include "mlp.cuh"
 
@@ -107,6 +108,8 @@ WsLayout ws_layout(const gdft_molecule *m) {
   }
   W.off_dpk = off;
   W.off_q = off;
+  W.off_fx = off;
+  if (m->precision == GDFT_FP64) off = align256(off + fx::xc_ws(np, m->n_ao).bytes);
   if (m->precision == GDFT_TF32X3) {
     const size_t ldk = (size_t)round_up(m->n_ao, 128);
     off = align256(off + 2 * ldk * ldk * 2 * sizeof(float));
@@ -327,13 +330,20 @@ static int batch_layout(int n_mol, const gdft_molecule *mols, const gdft_network
   return GDFT_OK;
 }
 
-// Density stage into ws.feat.
-static int run_density(const gdft_molecule *m, const double *rdm1, char *ws, cudaStream_t st) {
+// Density stage into ws.feat.  kin: the Laplacian or tau is read (otherwise the FP64 form leaves both at 0).
+static int run_density(const gdft_molecule *m, const double *rdm1, char *ws, cudaStream_t st, bool kin = true) {
   const WsLayout W = ws_layout(m);
   double *feat = (double *)(ws + W.off_feat);
   if (m->precision == GDFT_FP64) {
     StageTimer tm(GDFT_STAGE_DENSITY, st);
-    return check_cuda(launch_dens_f64(mol_tab(m), m->n_grid_pad, m->ld, m->n_ao, rdm1, feat, st), "dens_f64");
+    const int64_t np = m->n_grid_pad;
+    unsigned char *fw = (unsigned char *)(ws + W.off_fx);
+    int rc = check_cuda(fx::launch_density(mol_tab(m), np, m->ld, m->n_ao, rdm1, kin, feat, fw,
+                                           (int *)(ws + W.off_err), st),
+                        "fx density");
+    if (rc) return rc;
+    const int *bad = fx::bad_word(fw, fx::xc_ws(np, m->n_ao));  // the plain kernel runs for operands that are not finite
+    return check_cuda(launch_dens_f64(mol_tab(m), np, m->ld, m->n_ao, rdm1, feat, bad, st), "dens_f64");
   }
   const int ldk = (int)round_up(m->n_ao, 128);
   float *dpk = (float *)(ws + W.off_dpk);
@@ -352,19 +362,28 @@ static int run_density(const gdft_molecule *m, const double *rdm1, char *ws, cud
 using namespace gdft;
 
 // V_xc contraction of the adjoint coefficients in ws.coef into d_vxc.
-static int run_vxc(const gdft_molecule *mol, const double *coef, double *d_vxc, char *ws, cudaStream_t st) {
+// kin: coef's C_KIN rows may be non-zero.
+static int run_vxc(const gdft_molecule *mol, const double *coef, double *d_vxc, char *ws, cudaStream_t st,
+                   bool kin = true) {
   const WsLayout W = ws_layout(mol);
   int rc;
   double *vpart = (double *)(ws + W.off_vpart);
   if (mol->precision == GDFT_FP64) {
+    const int64_t np = mol->n_grid_pad;
+    unsigned char *fw = (unsigned char *)(ws + W.off_fx);
+    const int *bad = fx::bad_word(fw, fx::xc_ws(np, mol->n_ao));  // as in run_density
     {
       StageTimer tm(GDFT_STAGE_VXC, st);
-      rc = check_cuda(launch_vxc_f64(mol_tab(mol), mol->n_grid_pad, mol->ld, mol->n_ao, coef, W.n_vsplit, vpart, st),
+      if ((rc = check_cuda(fx::launch_vxc(mol_tab(mol), np, mol->ld, mol->n_ao, coef, kin, fw, d_vxc,
+                                          (int *)(ws + W.off_err), st),
+                           "fx vxc")))
+        return rc;
+      rc = check_cuda(launch_vxc_f64(mol_tab(mol), np, mol->ld, mol->n_ao, coef, W.n_vsplit, vpart, bad, st),
                       "vxc_f64");
       if (rc) return rc;
     }
     StageTimer tm(GDFT_STAGE_REDUCE, st);
-    return check_cuda(launch_vxc_reduce(vpart, W.n_vsplit, mol->n_ao, d_vxc, st), "vxc_reduce");
+    return check_cuda(launch_vxc_reduce(vpart, W.n_vsplit, mol->n_ao, d_vxc, bad, st), "vxc_reduce");
   }
   StageTimer tm(GDFT_STAGE_VXC, st);
   return check_cuda(launch_vxc_q_tc(mol_av(mol), mol_af(mol), coef, mol->n_grid_pad, (int)round_up(mol->n_ao, 128),
@@ -616,7 +635,7 @@ int gdft_density(const gdft_molecule *mol, const double *d_rdm1, double *d_rho, 
     return GDFT_ERR_INVALID;
   }
   cudaStream_t st = (cudaStream_t)stream;
-  if ((rc = run_density(mol, d_rdm1, (char *)d_ws, st))) return rc;
+  if ((rc = run_density(mol, d_rdm1, (char *)d_ws, st, d_lapl != nullptr || d_tau != nullptr))) return rc;
   const WsLayout W = ws_layout(mol);
   StageTimer tm(GDFT_STAGE_REDUCE, st);
   return check_cuda(launch_feat_to_reference((const double *)((char *)d_ws + W.off_feat), mol->n_grid,
@@ -642,7 +661,8 @@ static int xc_energy_and_grads(const char *who, const gdft_molecule *mol, const 
   cudaStream_t st = (cudaStream_t)stream;
   char *ws = (char *)d_ws;
   const WsLayout W = ws_layout(mol);
-  if ((rc = run_density(mol, d_rdm1, ws, st))) return rc;
+  const bool kin = xc_reads_kinetic(*fn);
+  if ((rc = run_density(mol, d_rdm1, ws, st, kin))) return rc;
   double *feat = (double *)(ws + W.off_feat);
   double *coef = d_vxc ? (double *)(ws + W.off_coef) : nullptr;
   double *epart = (double *)(ws + W.off_epart);
@@ -658,7 +678,7 @@ static int xc_energy_and_grads(const char *who, const gdft_molecule *mol, const 
     if ((rc = check_cuda(launch_energy_reduce(epart, W.n_eblocks, d_exc, st), "energy_reduce"))) return rc;
   }
   if (d_vxc == nullptr) return GDFT_OK;
-  return run_vxc(mol, coef, d_vxc, ws, st);
+  return run_vxc(mol, coef, d_vxc, ws, st, kin);
 }
 
 int gdft_xc_energy_and_grads(const gdft_molecule *mol, const double *d_rdm1, const gdft_functional *fn,
@@ -716,7 +736,7 @@ static int check_kpts(const gdft_molecule *mols, int32_t n_kpt, const double *h_
 
 // Features summed over k-points into ws + off_fsum.
 static int kpt_density(const gdft_molecule *mols, int32_t K, const double *rdm1c, const double *h_kweights,
-                       char *ws, cudaStream_t st) {
+                       char *ws, cudaStream_t st, bool kin) {
   const WsLayout W = ws_layout(&mols[0]);
   const KptWs KW = kpt_ws(&mols[0]);
   const int n = mols[0].n_ao / 2;
@@ -725,7 +745,7 @@ static int kpt_density(const gdft_molecule *mols, int32_t K, const double *rdm1c
   int rc;
   for (int k = 0; k < K; ++k) {
     if ((rc = check_cuda(launch_kpt_build_m(rdm1c, K, k, n, h_kweights[k], M, st), "kpt_build_m"))) return rc;
-    if ((rc = run_density(&mols[k], M, ws, st))) return rc;
+    if ((rc = run_density(&mols[k], M, ws, st, kin))) return rc;
     if ((rc = check_cuda(launch_feat_add((const double *)(ws + W.off_feat), fsum, nf, k == 0, st), "feat_add")))
       return rc;
   }
@@ -770,7 +790,7 @@ int gdft_kpoint_density(const gdft_molecule *mols, int32_t n_kpt, const double *
   }
   cudaStream_t st = (cudaStream_t)stream;
   char *ws = (char *)d_ws;
-  if ((rc = kpt_density(mols, n_kpt, d_rdm1, h_kweights, ws, st))) return rc;
+  if ((rc = kpt_density(mols, n_kpt, d_rdm1, h_kweights, ws, st, d_lapl != nullptr || d_tau != nullptr))) return rc;
   StageTimer tm(GDFT_STAGE_REDUCE, st);
   return check_cuda(launch_feat_to_reference((const double *)(ws + kpt_ws(&mols[0]).off_fsum), mols[0].n_grid,
                                              mols[0].n_grid_pad, d_rho, d_grad_rho, d_lapl, d_tau, st),
@@ -793,7 +813,8 @@ int gdft_kpoint_xc_energy_and_grads(const gdft_molecule *mols, int32_t n_kpt, co
   char *ws = (char *)d_ws;
   const WsLayout W = ws_layout(&mols[0]);
   const KptWs KW = kpt_ws(&mols[0]);
-  if ((rc = kpt_density(mols, n_kpt, d_rdm1, h_kweights, ws, st))) return rc;
+  const bool kin = xc_reads_kinetic(*fn);
+  if ((rc = kpt_density(mols, n_kpt, d_rdm1, h_kweights, ws, st, kin))) return rc;
   double *coef = d_vxc ? (double *)(ws + W.off_coef) : nullptr;
   double *epart = (double *)(ws + W.off_epart);
   {
@@ -811,7 +832,7 @@ int gdft_kpoint_xc_energy_and_grads(const gdft_molecule *mols, int32_t n_kpt, co
   const int n = mols[0].n_ao / 2;
   double *V = (double *)(ws + KW.off_v);
   for (int k = 0; k < n_kpt; ++k) {
-    if ((rc = run_vxc(&mols[k], coef, V, ws, st))) return rc;
+    if ((rc = run_vxc(&mols[k], coef, V, ws, st, kin))) return rc;
     if ((rc = check_cuda(launch_kpt_vxc(V, n_kpt, k, n, h_kweights[k], d_vxc, st), "kpt_vxc"))) return rc;
   }
   return GDFT_OK;
@@ -1303,7 +1324,7 @@ int gdft_energy_densities(const gdft_molecule *mol, const double *d_rdm1, const 
   cudaStream_t st = (cudaStream_t)stream;
   char *ws = (char *)d_ws;
   const WsLayout W = ws_layout(mol);
-  if ((rc = run_density(mol, d_rdm1, ws, st))) return rc;
+  if ((rc = run_density(mol, d_rdm1, ws, st, xc_reads_kinetic(*fn)))) return rc;
   return check_cuda(launch_xc_point((double *)(ws + W.off_feat), mol_w(mol), mol->n_grid, mol->n_grid_pad, *fn,
                                     d_ehf, n_omega, nullptr, (double *)(ws + W.off_epart), d_dens, st),
                     "xc_point");
@@ -1467,7 +1488,8 @@ static int chunk_pass(const gdft_molecule *m, char *ws, const ChunkWs &C, char *
   int rc;
   // A shorter (last) chunk's layout puts its error word where the full chunks kept other data.
   if ((rc = check_cuda(cudaMemsetAsync(ws + W.off_err, 0, sizeof(int), st), "chunk status clear"))) return rc;
-  if ((rc = run_density(m, rdm1, ws, st))) return rc;
+  const bool kin = net != nullptr || xc_reads_kinetic(*fn);
+  if ((rc = run_density(m, rdm1, ws, st, kin))) return rc;
   const double *ehf_c = nullptr;
   if (ehf != nullptr) {  // this chunk's columns of ehf (omega, spin, grid)
     double *dst = (double *)(base + C.off_ehf);
@@ -1511,7 +1533,7 @@ static int chunk_pass(const gdft_molecule *m, char *ws, const ChunkWs &C, char *
   }
   if (vxc != nullptr) {
     double *v_c = (double *)(base + C.off_v);
-    if ((rc = run_vxc(m, coef, v_c, ws, st))) return rc;
+    if ((rc = run_vxc(m, coef, v_c, ws, st, kin))) return rc;
     StageTimer tm(GDFT_STAGE_REDUCE, st);
     if ((rc = check_cuda(launch_feat_add(v_c, vxc, (size_t)2 * m->n_ao * m->n_ao, first, st), "chunk V")))
       return rc;

@@ -1,4 +1,5 @@
-// dens_f64.cu - plain FP64 form of the density contraction.
+// dens_f64.cu - plain FP64 form of the density contraction: what fx_xc.cu leaves
+// to it (operands that are not finite).
 //
 // For a tile of 32 grid points and each spin it forms X_t = T_t D_sigma for the
 // four AO planes T_t in {phi, d_x phi, d_y phi, d_z phi} (64 output columns at
@@ -23,7 +24,9 @@ constexpr int BK = 16;   // reduction step
 constexpr int NT = 256;  // threads: 32 points x 8 column lanes
 
 __global__ void __launch_bounds__(NT) dens_f64_kernel(const double *__restrict__ tab, int64_t np, int ld, int n,
-                                                      const double *__restrict__ D, double *__restrict__ feat) {
+                                                      const double *__restrict__ D, double *__restrict__ feat,
+                                                      const int *__restrict__ bad) {
+  if (bad != nullptr && *bad == 0) return;
   __shared__ double As[4][BP][BK + 1];
   __shared__ double Bs[BK][BN];
   const size_t pe = (size_t)np * ld;
@@ -118,9 +121,9 @@ __global__ void __launch_bounds__(NT) dens_f64_kernel(const double *__restrict__
 }  // namespace
 
 cudaError_t launch_dens_f64(const double *tab, int64_t np, int ld, int n_ao, const double *rdm1, double *feat,
-                            cudaStream_t st) {
+                            const int *bad, cudaStream_t st) {
   const int64_t blocks = np / BP;
-  dens_f64_kernel<<<(unsigned)blocks, NT, 0, st>>>(tab, np, ld, n_ao, rdm1, feat);
+  dens_f64_kernel<<<(unsigned)blocks, NT, 0, st>>>(tab, np, ld, n_ao, rdm1, feat, bad);
   return cudaGetLastError();
 }
 

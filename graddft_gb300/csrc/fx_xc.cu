@@ -1,0 +1,486 @@
+// fx_xc.cu - the FP64 form's density and V_xc contractions on fx_gemm.cu.
+//
+// Density: X_t = T_t D for the planes t = phi, d_x, d_y, d_z, 128 points x 64
+// columns of both spins per tile, then one pass of row products with the planes
+// (molecule.py:385-502; the sums dens_f64.cu states).  The d_j planes enter only
+// through quadratic forms sum_ab d_j phi_a D_ab d_j phi_b, which need one
+// triangle: column block b takes the row blocks a <= b of U = D + D^T (D itself
+// on the diagonal blocks), (n + 64) / 2n of the products.
+//
+// V_xc: V_s = phi^T Q_s + sum_j d_j phi^T (c_kin,s d_j phi), with
+// Q_s = c_rho phi + sum_j c_gj d_j phi + c_lap lap phi (vxc_f64.cu).  The second
+// sum is symmetric: only tiles that reach the diagonal are formed.
+//
+// Both run over the grid in slabs whose digits and products fit a fixed
+// workspace.  An operand that is not finite (or overflows its bound) sets a
+// word on the device; the plain kernels of dens_f64.cu and vxc_f64.cu then
+// compute the whole result, with IEEE's infinities and NaNs.  This path is the
+// faster one at every size (E_xc + V_xc, B88+LYP, plain kernels -> here: 4 AOs x
+// 128 points 779 -> 294 us, 24 x 3,600 928 -> 397 us, 100 x 10,000 5.4 -> 0.74 ms,
+// 400 x 150,001 827 -> 27.6 ms), and the more accurate one (features at 400 AOs
+// against quadruple precision: 1.4e-16 .. 2.7e-16, before 2.7e-16 .. 6.0e-16).
+#include "common.cuh"
+#include "fx.cuh"
+#include "kernels.cuh"
+
+namespace gdft {
+namespace fx {
+
+namespace {
+
+constexpr size_t kSlabBytes = (size_t)512 << 20;  // workspace of one slab, about
+size_t align256(size_t x) { return (x + 255) / 256 * 256; }
+
+// Digits of D as the B operand: tile nt = columns 64 nt .. of spin 0, then of
+// spin 1; version 0 is D, version 1 the triangle U (chunks 0 .. nt).  A warp
+// takes eight operand rows (columns of D), lane = (row, eight consecutive k).
+__global__ void __launch_bounds__(128) fx_rdm1_kernel(const double *__restrict__ D, int n, int nb, int versions,
+                                                      unsigned char *__restrict__ out, int *__restrict__ exps,
+                                                      int *__restrict__ bad) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = blockIdx.x * 4 + warp;  // group of eight operand rows: 16 per tile
+  if (g >= nb * 16) return;
+  const int version = blockIdx.y;
+  const int nt = g / 16, rt = (g % 16) * 8 + (lane & 7);
+  const int s = rt >> 6, c = nt * 64 + (rt & 63);
+  const double *Ds = D + (size_t)s * n * n;
+  const int chunks = version ? nt + 1 : nb;
+  const int kg = (lane >> 3) * 8;
+  auto value = [&](int k) {
+    if (c >= n || k >= n) return 0.0;
+    const double d = Ds[(size_t)k * n + c];
+    return version && k < nt * 64 ? d + Ds[(size_t)c * n + k] : d;
+  };
+  uint32_t m = 0;
+  for (int k = kg; k < chunks * kChunkK; k += 32)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) m = max(m, (uint32_t)__double2hiint(value(k + j)) & 0x7FFFFFFFu);
+  m = max(m, __shfl_xor_sync(0xffffffffu, m, 8));
+  m = max(m, __shfl_xor_sync(0xffffffffu, m, 16));
+  int emax = exp_field(m);
+  if (emax == 0x7FF) atomicOr(bad, 1);
+  if (emax < 1) emax = 1;
+  if (lane < 8) exps[version * nb * kTile + nt * kTile + rt] = emax;
+  unsigned char *base = out + ((size_t)version * nb + nt) * nb * kSetBytes;
+  for (int k = kg; k < chunks * kChunkK; k += 32) {
+    long long f[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) f[j] = to_fixed(value(k + j), emax);
+    uint4 d[kDigits];
+    digits8(f, d);
+    unsigned char *set = base + (size_t)(k / kChunkK) * kSetBytes + elem_off(rt, k % kChunkK);
+#pragma unroll
+    for (int i = 0; i < kDigits; ++i) *(uint4 *)(set + (size_t)i * kBlockBytes) = d[i];
+  }
+}
+
+// Row products of X with the planes -> feat.  X is [plane][spin][column][slab
+// point], the planes [point][ld]: a block takes 32 points and walks the columns
+// in tiles of 32, the planes' tile through shared memory (rows in, columns out),
+// X directly (lanes are points); both spins share a tile.
+constexpr int kFeatTile = 32;
+__global__ void __launch_bounds__(256) fx_features_kernel(const double *__restrict__ tab, size_t pe, int64_t np, int ld,
+                                                          int64_t p0, int64_t slab, const double *__restrict__ X,
+                                                          int cols, bool kin, double *__restrict__ feat,
+                                                          const int *__restrict__ bad) {
+  if (*bad != 0) return;
+  __shared__ double t[kPlanes][kFeatTile][kFeatTile + 1];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t r0 = (int64_t)blockIdx.x * kFeatTile;
+  const int planes = kin ? kPlanes : 4;
+  const size_t xs = (size_t)slab * cols;
+  double f[2][6];
+#pragma unroll
+  for (int s = 0; s < 2; ++s)
+#pragma unroll
+    for (int k = 0; k < 6; ++k) f[s][k] = 0.0;
+  for (int c0 = 0; c0 < ld; c0 += kFeatTile) {  // ld is a multiple of 32
+    __syncthreads();
+    for (int i = warp; i < planes * kFeatTile; i += 8)
+      t[i / kFeatTile][i % kFeatTile][lane] =
+          tab[(size_t)(i / kFeatTile) * pe + (size_t)(p0 + r0 + i % kFeatTile) * ld + c0 + lane];
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kFeatTile / 8; ++k) {
+      const int c = warp + 8 * k;
+      const double phi = t[T_PHI][lane][c], dx = t[T_DX][lane][c], dy = t[T_DY][lane][c], dz = t[T_DZ][lane][c];
+      const double *x = X + (size_t)(c0 + c) * slab + r0 + lane;
+#pragma unroll
+      for (int s = 0; s < 2; ++s, x += xs) {
+        const double x0 = x[0];
+        f[s][0] = fma(x0, phi, f[s][0]);
+        f[s][1] = fma(x0, dx, f[s][1]);
+        f[s][2] = fma(x0, dy, f[s][2]);
+        f[s][3] = fma(x0, dz, f[s][3]);
+        if (kin) {
+          f[s][4] = fma(x0, t[T_LAP][lane][c], f[s][4]);
+          f[s][5] = fma(x[2 * xs], dx, f[s][5]);
+          f[s][5] = fma(x[4 * xs], dy, f[s][5]);
+          f[s][5] = fma(x[6 * xs], dz, f[s][5]);
+        }
+      }
+    }
+  }
+  __syncthreads();
+  double *red = &t[0][0][0];  // [warp][spin * 6 + feature][point]
+#pragma unroll
+  for (int k = 0; k < 12; ++k) red[(warp * 12 + k) * 32 + lane] = f[k / 6][k % 6];
+  __syncthreads();
+  for (int i = threadIdx.x; i < 12 * 32; i += 256) {
+    double v = 0.0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) v += red[w * 12 * 32 + i];
+    red[i] = v;  // only this thread reads entry i of warp 0's block
+  }
+  __syncthreads();
+  if (warp < 2) {
+    const int64_t p = p0 + r0 + lane;
+    const double *v = red + warp * 6 * 32 + lane;
+    double *fs = feat + (size_t)warp * kFeat * np;
+    fs[F_RHO * np + p] = v[0];
+    fs[F_GX * np + p] = 2.0 * v[32];
+    fs[F_GY * np + p] = 2.0 * v[64];
+    fs[F_GZ * np + p] = 2.0 * v[96];
+    fs[F_LAP * np + p] = 2.0 * v[160] + 2.0 * v[128];
+    fs[F_TAU * np + p] = 0.5 * v[160];
+  }
+}
+
+// ---------------------------------------------------------------- V_xc operands
+// High words add like logarithms: hi(x) + hi(y) - hi(1) is at most the product's
+// and below it by less than 1/8 in the mantissa.  kNone: no value (zero).
+constexpr int kNone = -(1 << 30);
+constexpr int kOneHi = 0x3FF00000;
+__device__ __forceinline__ int hi_of(double x) {
+  const int h = __double2hiint(x) & 0x7FFFFFFF;
+  return h ? h : kNone;
+}
+// Exponent field bound of a sum of `terms` products whose largest has the (approximate) high word m.
+__device__ __forceinline__ int field_of(int m, int octaves) {
+  const int f = m <= 0 ? 1 : ((m + (1 << 18)) >> 20) + octaves;
+  return f < 1 ? 1 : f > 0x7FE ? 0x7FE : f;
+}
+
+// Largest high words over a slab of points: [0] phi, [1] d_j phi (one for the
+// three), [2 + s] the terms of Q_s, [4 + s] c_kin,s d_j phi.  Lanes are AOs, a
+// block takes 32 AOs and `per` points, its warps every eighth point.
+__global__ void __launch_bounds__(256) fx_vmax_kernel(const double *__restrict__ tab, size_t pe, int64_t np, int ld,
+                                                      const double *__restrict__ coef, int64_t p0, int64_t rows,
+                                                      int per, bool kin, int n_max, int *__restrict__ mx,
+                                                      int *__restrict__ bad) {
+  __shared__ int sc[2][kFeat][128];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int a = blockIdx.x * 32 + lane;
+  int m[6] = {kNone, kNone, kNone, kNone, kNone, kNone};
+  const int64_t r_begin = (int64_t)blockIdx.y * per, r_end = r_begin + per < rows ? r_begin + per : rows;
+  for (int64_t q0 = r_begin; q0 < r_end; q0 += 128) {
+    const int cnt = (int)(r_end - q0 < 128 ? r_end - q0 : 128);
+    __syncthreads();
+    for (int i = threadIdx.x; i < 2 * kFeat * 128; i += blockDim.x) {
+      const int p = i % 128;
+      const int h = p < cnt ? hi_of(coef[(size_t)(i / 128) * np + p0 + q0 + p]) : kNone;
+      if (h >= 0x7FF00000) atomicOr(bad, 1);
+      (&sc[0][0][0])[i] = h == kNone ? kNone : h - kOneHi;
+    }
+    __syncthreads();
+    if (a < ld)
+      for (int p = warp; p < cnt; p += 8) {
+        const double *t = tab + (size_t)(p0 + q0 + p) * ld + a;
+        const int phi = hi_of(t[0]), dx = hi_of(t[pe]), dy = hi_of(t[2 * pe]), dz = hi_of(t[3 * pe]),
+                  lp = hi_of(t[4 * pe]);
+        const int dm = max(dx, max(dy, dz));
+        if (max(phi, max(dm, lp)) >= 0x7FF00000) atomicOr(bad, 1);
+        m[0] = max(m[0], phi);
+        m[1] = max(m[1], dm);
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+          int v = sc[s][C_RHO][p] + phi;
+          v = max(v, sc[s][C_GX][p] + dx);
+          v = max(v, sc[s][C_GY][p] + dy);
+          v = max(v, sc[s][C_GZ][p] + dz);
+          v = max(v, sc[s][C_LAP][p] + lp);
+          m[2 + s] = max(m[2 + s], v);
+          if (kin) m[4 + s] = max(m[4 + s], sc[s][C_KIN][p] + dm);
+        }
+      }
+  }
+  if (a < ld) {
+#pragma unroll
+    for (int k = 0; k < 6; ++k) atomicMax(mx + (size_t)k * n_max + a, m[k]);
+  }
+}
+
+// Maxima -> exponent fields of the operand rows: ea [2][128 mt] (phi, kinetic),
+// eb [2][128 nb] (Q, kinetic; tile rows 64 of each spin).
+__global__ void fx_vexp_kernel(const int *__restrict__ mx, int n_max, int n_ao, int mt, int nb, int *__restrict__ ea,
+                               int *__restrict__ eb) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < mt * kTile) {
+    ea[i] = i < n_ao ? max(1, mx[i] >> 20) : 1;
+    ea[mt * kTile + i] = i < n_ao ? max(1, mx[n_max + i] >> 20) : 1;
+  }
+  if (i < nb * kTile) {
+    const int s = (i % kTile) >> 6, b = i / kTile * 64 + (i & 63);
+    eb[i] = b < n_ao ? field_of(mx[(size_t)(2 + s) * n_max + b], 3) : 1;  // five terms
+    eb[nb * kTile + i] = b < n_ao ? field_of(mx[(size_t)(4 + s) * n_max + b], 0) : 1;
+  }
+}
+
+// Digits of both operands for 64 points (one K chunk) and 32 AOs: warp = eight
+// consecutive points, lane = AO.  A sets [mt][4 npc], B sets [nb][4 npc], chunk
+// t npc + pc for plane t.
+__global__ void __launch_bounds__(256) fx_vdigits_kernel(const double *__restrict__ tab, size_t pe, int64_t np, int ld,
+                                                         const double *__restrict__ coef, int64_t p0, int64_t rows,
+                                                         int npc, bool kin, int mt, int nb,
+                                                         const int *__restrict__ ea, const int *__restrict__ eb,
+                                                         unsigned char *__restrict__ va, unsigned char *__restrict__ vb,
+                                                         int *__restrict__ bad) {
+  if (*bad != 0) return;
+  __shared__ double sc[2][kFeat][64];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int pc = blockIdx.y, a = blockIdx.x * 32 + lane;
+  const int64_t q0 = (int64_t)pc * kChunkK;
+  for (int i = threadIdx.x; i < 2 * kFeat * 64; i += blockDim.x) {
+    const int p = i % 64;
+    (&sc[0][0][0])[i] = q0 + p < rows ? coef[(size_t)(i / 64) * np + p0 + q0 + p] : 0.0;
+  }
+  __syncthreads();
+  const int k0 = warp * 8;
+  double v[kPlanes][8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const bool in = a < ld && q0 + k0 + j < rows;
+    const double *t = tab + (size_t)(p0 + q0 + k0 + j) * ld + a;
+#pragma unroll
+    for (int p = 0; p < kPlanes; ++p) v[p][j] = in ? t[(size_t)p * pe] : 0.0;
+  }
+  bool over = false;
+  auto emit = [&](unsigned char *set, int row, const double (&x)[8], int emax) {
+    long long f[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      over = over || exp_field((uint32_t)__double2hiint(x[j])) > emax;
+      f[j] = to_fixed(x[j], emax);
+    }
+    uint4 d[kDigits];
+    digits8(f, d);
+    unsigned char *o = set + elem_off(row, k0);
+#pragma unroll
+    for (int i = 0; i < kDigits; ++i) *(uint4 *)(o + (size_t)i * kBlockBytes) = d[i];
+  };
+  const int planes = kin ? 4 : 1;
+  const size_t chunks = (size_t)planes * npc;
+  if (a < mt * kTile) {
+    unsigned char *A = va + ((size_t)(a / kTile) * chunks + pc) * kSetBytes;
+    emit(A, a % kTile, v[T_PHI], ea[a]);
+    if (kin) {
+      const int e = ea[mt * kTile + a];
+#pragma unroll
+      for (int t = 1; t < 4; ++t) emit(A + (size_t)t * npc * kSetBytes, a % kTile, v[t], e);
+    }
+  }
+  if (a < nb * 64) {
+    unsigned char *B = vb + ((size_t)(a / 64) * chunks + pc) * kSetBytes;
+#pragma unroll 1
+    for (int s = 0; s < 2; ++s) {
+      const int row = s * 64 + a % 64;
+      double q[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const double *c = &sc[s][0][k0 + j];
+        q[j] = c[64 * C_RHO] * v[T_PHI][j] + c[64 * C_GX] * v[T_DX][j] + c[64 * C_GY] * v[T_DY][j] +
+               c[64 * C_GZ] * v[T_DZ][j] + c[64 * C_LAP] * v[T_LAP][j];
+      }
+      emit(B, row, q, eb[a / 64 * kTile + row]);
+      if (kin) {
+        const int e = eb[nb * kTile + a / 64 * kTile + row];
+#pragma unroll
+        for (int t = 1; t < 4; ++t) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) q[j] = sc[s][C_KIN][k0 + j] * v[t][j];
+          emit(B + (size_t)t * npc * kSetBytes, row, q, e);
+        }
+      }
+    }
+  }
+  if (over) atomicOr(bad, 1);
+}
+
+// V[s][a][b] = sum of the phi part's splits at (a, b) and of the kinetic part's
+// at (a, b) or, left of the diagonal tile, (b, a).  part: [split][spin][b][a].
+__global__ void fx_vreduce_kernel(const double *__restrict__ part, int s0, int s1, int n, int rows, int cols,
+                                  double *__restrict__ out, const int *__restrict__ bad) {
+  if (*bad != 0) return;
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= (size_t)2 * n * n) return;
+  const int s = (int)(i / ((size_t)n * n)), a = (int)((i / n) % n), b = (int)(i % n);
+  const size_t split = (size_t)2 * rows * cols, spin = (size_t)s * rows * cols;
+  double v = 0.0;
+  const double *p = part + spin + (size_t)b * rows + a;
+  for (int k = 0; k < s0; ++k) v += p[(size_t)k * split];
+  p = part + (size_t)s0 * split + spin + (b >= a / kTile * kTile ? (size_t)b * rows + a : (size_t)a * rows + b);
+  for (int k = 0; k < s1; ++k) v += p[(size_t)k * split];
+  out[i] = v;
+}
+
+}  // namespace
+
+XcWs xc_ws(int64_t np, int n_ao) {
+  XcWs w{};
+  w.nb = (n_ao + 63) / 64;
+  w.mt = (n_ao + kTile - 1) / kTile;
+  const int64_t n64 = (int64_t)w.nb * 64, n128 = (int64_t)w.mt * kTile;
+  auto slab = [&](int64_t per_point) {
+    int64_t p = (int64_t)kSlabBytes / per_point / 128 * 128;
+    p = p < 1024 ? 1024 : p;
+    return p < np ? p : round_up(np, 128);
+  };
+  w.dens_slab = slab(n64 * (4 * 2 * kDigits + 64));
+  w.v_slab = slab((n128 + n64 * 2) * 4 * 2 * kDigits);
+  // V_xc items: about two rounds of one CTA per SM, at least four chunks each.
+  const int64_t npc = w.v_slab / kChunkK;
+  int64_t upper = 0;
+  for (int m = 0; m < w.mt; ++m) upper += w.nb - 2 * m > 0 ? w.nb - 2 * m : 0;
+  const int64_t work = npc * ((int64_t)w.mt * w.nb + 3 * upper);
+  int64_t per = (work + 2 * 148 - 1) / (2 * 148);
+  per = per < 4 ? 4 : per;
+  w.v_chunks = (int)per;
+  w.s0 = (int)((npc + per - 1) / per);
+  w.s1 = (int)((3 * npc + per - 1) / per);
+  size_t off = 0;
+  w.off_bad = off;
+  off = 256;
+  const size_t shared = off;
+  w.off_dset = off;
+  off = align256(off + (size_t)2 * w.nb * w.nb * kSetBytes);
+  w.off_dexp = off;
+  off = align256(off + (size_t)2 * w.nb * kTile * sizeof(int));
+  w.off_a = off;
+  off = align256(off + (size_t)4 * (w.dens_slab / kTile) * w.nb * kSetBytes);
+  w.off_ea = off;
+  off = align256(off + (size_t)4 * w.dens_slab * sizeof(int));
+  w.off_x = off;
+  off = align256(off + (size_t)8 * w.dens_slab * n64 * sizeof(double));
+  const size_t dens_end = off;
+  off = shared;
+  w.off_va = off;
+  off = align256(off + (size_t)w.mt * 4 * npc * kSetBytes);
+  w.off_vb = off;
+  off = align256(off + (size_t)w.nb * 4 * npc * kSetBytes);
+  w.off_vexp = off;
+  off = align256(off + (size_t)(2 * w.mt * kTile + 2 * w.nb * kTile + 6 * n128) * sizeof(int));
+  w.off_vpart = off;
+  // s0 + s1 is at most this for any grid, so a shorter grid never needs more than a longer one.
+  const int64_t most = 4 * 2 * 148 / ((int64_t)w.mt * w.nb + 3 * upper) + 2;
+  off = align256(off + (size_t)most * 2 * n128 * n64 * sizeof(double));
+  w.bytes = off > dens_end ? off : dens_end;
+  return w;
+}
+
+cudaError_t launch_density(const double *tab, int64_t np, int ld, int n_ao, const double *rdm1, bool kin, double *feat,
+                           unsigned char *ws, int *err, cudaStream_t st) {
+  const XcWs w = xc_ws(np, n_ao);
+  const size_t pe = (size_t)np * ld;
+  int *bad = bad_word(ws, w);
+  unsigned char *dset = ws + w.off_dset;
+  int *dexp = (int *)(ws + w.off_dexp), *ea = (int *)(ws + w.off_ea);
+  double *X = (double *)(ws + w.off_x);
+  cudaError_t e = cudaMemsetAsync(bad, 0, sizeof(int), st);
+  if (e != cudaSuccess) return e;
+  fx_rdm1_kernel<<<dim3((unsigned)(w.nb * 4), kin ? 2 : 1), 128, 0, st>>>(rdm1, n_ao, w.nb, 2, dset, dexp, bad);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  for (int64_t p0 = 0; p0 < np; p0 += w.dens_slab) {
+    const int64_t rows = np - p0 < w.dens_slab ? np - p0 : w.dens_slab;
+    const int planes = kin ? 4 : 1;
+    if ((e = launch_rows(tab + (size_t)p0 * ld, (int64_t)pe, planes, rows, ld, ld, w.nb, ws + w.off_a, ea, bad, st)) !=
+        cudaSuccess)
+      return e;
+    GemmArgs g{};
+    g.a = ws + w.off_a;
+    g.b = dset;
+    g.b1 = dset + (size_t)w.nb * w.nb * kSetBytes;
+    g.ea = ea;
+    g.eb = dexp;
+    g.eb1 = dexp + w.nb * kTile;
+    g.mode = kDensity;
+    g.m_tiles = (int)(rows / kTile);
+    g.n_tiles = w.nb;
+    g.planes = planes;
+    g.chunks = g.a_stride = g.b_stride = w.nb;
+    g.out = X;
+    g.ldc = w.dens_slab;
+    g.half_stride = (int64_t)w.nb * 64 * g.ldc;
+    g.plane_stride = 2 * g.half_stride;
+    g.nt_stride = 64 * g.ldc;
+    g.m_valid = rows;
+    g.bad = bad;
+    g.err = err;
+    if ((e = launch_gemm(g, st)) != cudaSuccess) return e;
+    fx_features_kernel<<<(unsigned)(rows / kFeatTile), 256, 0, st>>>(tab, pe, np, ld, p0, w.dens_slab, X, w.nb * 64, kin,
+                                                                     feat, bad);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
+cudaError_t launch_vxc(const double *tab, int64_t np, int ld, int n_ao, const double *coef, bool kin,
+                       unsigned char *ws, double *vxc, int *err, cudaStream_t st) {
+  const XcWs w = xc_ws(np, n_ao);
+  const size_t pe = (size_t)np * ld;
+  int *bad = bad_word(ws, w);
+  const int n_max = w.mt * kTile;
+  int *ea = (int *)(ws + w.off_vexp), *eb = ea + 2 * n_max, *mx = eb + 2 * w.nb * kTile;
+  unsigned char *va = ws + w.off_va, *vb = ws + w.off_vb;
+  double *part = (double *)(ws + w.off_vpart);
+  cudaError_t e = cudaMemsetAsync(bad, 0, sizeof(int), st);
+  if (e != cudaSuccess) return e;
+  for (int64_t p0 = 0; p0 < np; p0 += w.v_slab) {
+    const int64_t rows = np - p0 < w.v_slab ? np - p0 : w.v_slab;
+    const int npc = (int)((rows + kChunkK - 1) / kChunkK);
+    // 0x80808080 is below every high word.
+    if ((e = cudaMemsetAsync(mx, 0x80, (size_t)6 * n_max * sizeof(int), st)) != cudaSuccess) return e;
+    const int blocks_a = (ld + 31) / 32;
+    int64_t segs = (8 * 148 + blocks_a - 1) / blocks_a;
+    int64_t per = (rows + segs - 1) / segs;
+    per = per < 64 ? 64 : per;
+    segs = (rows + per - 1) / per;
+    fx_vmax_kernel<<<dim3(blocks_a, (unsigned)segs), 256, 0, st>>>(tab, pe, np, ld, coef, p0, rows, (int)per, kin,
+                                                                   n_max, mx, bad);
+    fx_vexp_kernel<<<(w.nb * kTile + 255) / 256, 256, 0, st>>>(mx, n_max, n_ao, w.mt, w.nb, ea, eb);
+    fx_vdigits_kernel<<<dim3(n_max / 32, npc), 256, 0, st>>>(tab, pe, np, ld, coef, p0, rows, npc, kin, w.mt, w.nb, ea,
+                                                             eb, va, vb, bad);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    GemmArgs g{};
+    g.a = va;
+    g.b = g.b1 = vb;
+    g.ea = ea;
+    g.eb = eb;
+    g.eb1 = eb + w.nb * kTile;
+    g.mode = kVxc;
+    g.m_tiles = w.mt;
+    g.n_tiles = w.nb;
+    g.planes = kin ? 2 : 1;
+    g.chunks = npc;
+    g.a_stride = g.b_stride = (kin ? 4 : 1) * npc;
+    g.chunks_per_split = w.v_chunks;
+    g.ldc = n_max;
+    g.half_stride = (int64_t)w.nb * 64 * g.ldc;
+    g.split_stride = 2 * g.half_stride;
+    g.nt_stride = 64 * g.ldc;
+    g.plane_stride = w.s0 * g.split_stride;
+    g.m_valid = n_max;
+    g.out = part;
+    g.accumulate = p0 > 0;
+    g.bad = bad;
+    g.err = err;
+    if ((e = launch_gemm(g, st)) != cudaSuccess) return e;
+  }
+  const size_t total = (size_t)2 * n_ao * n_ao;
+  // The first slab, the longest, writes all s0 + s1 splits.
+  fx_vreduce_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(part, w.s0, kin ? w.s1 : 0, n_ao, n_max, w.nb * 64,
+                                                                     vxc, bad);
+  return cudaGetLastError();
+}
+
+}  // namespace fx
+}  // namespace gdft

@@ -19,13 +19,14 @@ cudaError_t launch_eval_shell_tables(const ShellView &B, const double *coords, c
                                      int64_t np, int ld, double *tab, double *wout, cudaStream_t st);
 
 // dens_f64.cu: FP64 form of the density contraction -> feat[2][6][np].
+// bad (here and below): when given, a device word; the launch does nothing where it is 0.
 cudaError_t launch_dens_f64(const double *tab, int64_t np, int ld, int n_ao, const double *rdm1, double *feat,
-                            cudaStream_t st);
+                            const int *bad, cudaStream_t st);
 
 // vxc_f64.cu: FP64 form of the V_xc contraction -> vpart[nsplit][2][n][n].
 int vxc_f64_splits(int64_t np, int n_ao);
 cudaError_t launch_vxc_f64(const double *tab, int64_t np, int ld, int n_ao, const double *coef, int nsplit,
-                           double *vpart, cudaStream_t st);
+                           double *vpart, const int *bad, cudaStream_t st);
 
 // tc_pack.cu / dens_tc.cu: TF32x3 form.
 cudaError_t launch_pack_tables(const double *ao, const double *grad_ao, const double *grad2_ao, const double *basis,
@@ -69,6 +70,8 @@ cudaError_t launch_kpt_nonxc(const double *rdm1c, const double *h1e, const doubl
                              double e_nuc, double *out, cudaStream_t st);
 
 // xc_point.cu
+// Whether a column of the functional reads the Laplacian or tau.
+bool xc_reads_kinetic(const gdft_functional &fn);
 int xc_point_blocks(int64_t np);
 cudaError_t launch_xc_point(const double *feat, const double *w, int64_t n_grid, int64_t np,
                             const gdft_functional &fn, const double *ehf, int n_omega, double *coef,
@@ -84,7 +87,8 @@ cudaError_t launch_integrate(int64_t n_grid, int n_cols, const gdft_functional &
                              const double *w, double *epart, cudaStream_t st);
 cudaError_t launch_energy_reduce(const double *epart, int n, double *exc, cudaStream_t st);
 cudaError_t launch_err_fold(int *dst, int *src, cudaStream_t st);
-cudaError_t launch_vxc_reduce(const double *vpart, int nsplit, int n_ao, double *vxc, cudaStream_t st);
+cudaError_t launch_vxc_reduce(const double *vpart, int nsplit, int n_ao, double *vxc, const int *bad,
+                              cudaStream_t st);
 cudaError_t launch_feat_to_reference(const double *feat, int64_t n_grid, int64_t np, double *rho, double *grad_rho,
                                      double *lapl, double *tau, cudaStream_t st);
 cudaError_t launch_fock(int n_ao, const double *h1e, const double *vj, const double *vxc, double clip, double *fock,

@@ -28,7 +28,8 @@ __global__ void energy_reduce_kernel(const double *__restrict__ part, int n, dou
 
 // Sum of the split-K partial V tiles in a fixed order (deterministic).
 __global__ void vxc_reduce_kernel(const double *__restrict__ part, int nsplit, size_t total,
-                                  double *__restrict__ out) {
+                                  double *__restrict__ out, const int *__restrict__ bad) {
+  if (bad != nullptr && *bad == 0) return;
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   double s = 0.0;
@@ -175,9 +176,10 @@ cudaError_t launch_energy_reduce(const double *epart, int n, double *exc, cudaSt
   return cudaGetLastError();
 }
 
-cudaError_t launch_vxc_reduce(const double *vpart, int nsplit, int n_ao, double *vxc, cudaStream_t st) {
+cudaError_t launch_vxc_reduce(const double *vpart, int nsplit, int n_ao, double *vxc, const int *bad,
+                              cudaStream_t st) {
   const size_t total = (size_t)2 * n_ao * n_ao;
-  vxc_reduce_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(vpart, nsplit, total, vxc);
+  vxc_reduce_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(vpart, nsplit, total, vxc, bad);
   return cudaGetLastError();
 }
 

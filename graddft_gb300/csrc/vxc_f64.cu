@@ -1,4 +1,5 @@
-// vxc_f64.cu - plain FP64 form of the V_xc contraction.
+// vxc_f64.cu - plain FP64 form of the V_xc contraction: what fx_xc.cu leaves to it
+// (operands that are not finite).
 //
 // V_sigma[a][b] = sum_r phi_ra Qa_sigma[r][b] + sum_j sum_r d_j phi_ra Qk_sigma[r][b] d_j...
 // written as one contraction over the stacked operand pairs
@@ -22,7 +23,8 @@ constexpr int NT = 256;
 
 __global__ void __launch_bounds__(NT) vxc_f64_kernel(const double *__restrict__ tab, int64_t np, int ld, int n,
                                                      const double *__restrict__ coef, int64_t chunk,
-                                                     double *__restrict__ vpart) {
+                                                     double *__restrict__ vpart, const int *__restrict__ bad) {
+  if (bad != nullptr && *bad == 0) return;
   __shared__ double Ps[4][BK][BT];
   __shared__ double Qs[2][4][BK][BT];
   const size_t pe = (size_t)np * ld;
@@ -128,12 +130,12 @@ int vxc_f64_splits(int64_t np, int n_ao) {
 }
 
 cudaError_t launch_vxc_f64(const double *tab, int64_t np, int ld, int n_ao, const double *coef, int nsplit,
-                           double *vpart, cudaStream_t st) {
+                           double *vpart, const int *bad, cudaStream_t st) {
   const int tiles_a = (n_ao + BT - 1) / BT;
   int64_t chunk = (np + nsplit - 1) / nsplit;
   chunk = (chunk + BK - 1) / BK * BK;
   dim3 grid(tiles_a * tiles_a, nsplit);
-  vxc_f64_kernel<<<grid, NT, 0, st>>>(tab, np, ld, n_ao, coef, chunk, vpart);
+  vxc_f64_kernel<<<grid, NT, 0, st>>>(tab, np, ld, n_ao, coef, chunk, vpart, bad);
   return cudaGetLastError();
 }
 

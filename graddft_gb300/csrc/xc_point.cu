@@ -175,6 +175,12 @@ __global__ void __launch_bounds__(kBlock) xc_point_kernel(const double *__restri
 
 int xc_point_blocks(int64_t np) { return (int)((np + kBlock - 1) / kBlock); }
 
+bool xc_reads_kinetic(const gdft_functional &fn) {
+  for (int i = 0; i < fn.n_cols; ++i)
+    if (fn.cols[i] == GDFT_COL_LYP || (is_uw_col(fn.cols[i]) && uw_j(fn.cols[i]) != 0)) return true;
+  return false;
+}
+
 cudaError_t launch_xc_point(const double *feat, const double *w, int64_t n_grid, int64_t np,
                             const gdft_functional &fn, const double *ehf, int n_omega, double *coef,
                             double *epart, double *dens, cudaStream_t st, double *ghf) {

@@ -1,0 +1,132 @@
+"""The FP64 form's contractions on digit products (csrc/fx_*.cu) at the edges of their tiles, against torch float64
+sums on the CPU, and their way to the plain kernels when an operand is not finite.
+
+Bounds, element by element, from the arithmetic.  Digits keep 61 bits of a row's largest value and the products that
+are left out are below 2^-60 of the largest product, so each product of two rows is off by less than 2^-57 of the
+product of their largest values.  What remains are FP64 roundings of 2^-53: one of each X, the n / 8 + 11 additions of
+a feature; for V the additions of at most 320 partial sums.  The CPU sums have their own n (or N) roundings.
+"""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+U = 2.0 ** -53
+
+
+@pytest.fixture(scope="module")
+def E(built_lib):
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from graddft_gb300 import engine
+
+    return engine
+
+
+def _tables(n, N, seed):
+    """Tables with rows and columns of very different sizes (10^-20 .. 10^2), a non-symmetric D."""
+    g = np.random.default_rng(seed)
+    scale = 10.0 ** g.uniform(-3, 2, n)[None, :] * 10.0 ** g.uniform(-17, 0, N)[:, None]
+    ao, g1, g2 = (g.standard_normal((N, n) + s) * (scale if not s else scale[..., None]) for s in ((), (3,), (3,)))
+    ao[g.integers(0, N, max(1, N // 7))] = 0.0
+    return ao, g1, g2, g.standard_normal((2, n, n)), g.standard_normal((2, 6, N)) * 10.0 ** g.uniform(-6, 3, N)
+
+
+def _dot_bound(x, y, k):
+    """(k roundings of sum_c |x| |y|) + what the digits leave out, both times the row maxima."""
+    return k * U * (np.abs(x) * np.abs(y)).sum(-1)
+
+
+def _resident(E, ao, g1, g2):
+    return E.Resident.from_tables(ao, g1, g2, np.ones(ao.shape[0]), "fp64", "cuda:0")
+
+
+SIZES = [(1, 1), (7, 127), (31, 128), (33, 129), (63, 640), (64, 65), (65, 257), (128, 300), (129, 1000), (193, 500),
+         (130, 30001)]  # the last crosses the slabs of both contractions
+
+
+@pytest.mark.parametrize("n,N", SIZES)
+def test_density_features(E, n, N):
+    ao, g1, g2, D, _ = _tables(n, N, 100 * n + N)
+    r = _resident(E, ao, g1, g2)
+    out = {k: v.cpu().numpy() for k, v in r.density(D).items()}
+    r.status()
+    only = {k: v.cpu().numpy() for k, v in r.density(D, want=("rho", "grad_rho")).items() if v is not None}
+    lap = g2.sum(-1)
+    k = n + n / 8 + 14  # the CPU's product and ours
+    for s in range(2):
+        X, aX = ao @ D[s], np.abs(ao) @ np.abs(D[s])
+        # What digits may lose in X: the row's and the column's largest values, n products.
+        lost = 2.0 ** -57 * n * np.abs(ao).max(1)[:, None] * np.abs(D[s]).max(0)[None]
+
+        def check(got, ref, x, y, extra, what):
+            bound = _dot_bound(x, y, k) + extra + 1e-300
+            assert np.all(np.abs(got - ref) <= bound), (what, np.max(np.abs(got - ref) / bound))
+
+        check(out["rho"][:, s], (X * ao).sum(1), aX, ao, (lost * np.abs(ao)).sum(1), "rho")
+        np.testing.assert_array_equal(only["rho"][:, s], out["rho"][:, s])
+        for j in range(3):
+            check(out["grad_rho"][:, s, j] / 2, (X * g1[..., j]).sum(1), aX, g1[..., j],
+                  (lost * np.abs(g1[..., j])).sum(1), "grad")
+            np.testing.assert_array_equal(only["grad_rho"][:, s, j], out["grad_rho"][:, s, j])
+        kin, akin, klost = np.zeros(N), np.zeros(N), np.zeros(N)
+        for j in range(3):
+            kin += ((g1[..., j] @ D[s]) * g1[..., j]).sum(1)
+            akin += ((np.abs(g1[..., j]) @ np.abs(D[s])) * np.abs(g1[..., j])).sum(1)
+            klost += (2.0 ** -56 * n * np.abs(g1[..., j]).max(1) * np.abs(D[s]).max() * np.abs(g1[..., j]).sum(1))
+        kb = (k + 4) * U * akin + klost + 1e-300
+        assert np.all(np.abs(out["tau"][:, s] * 2 - kin) <= kb)
+        lb = 2 * kb + 2 * (_dot_bound(aX, lap, k) + (lost * np.abs(lap)).sum(1))
+        assert np.all(np.abs(out["lapl"][:, s] - 2 * kin - 2 * (X * lap).sum(1)) <= lb)
+
+
+@pytest.mark.parametrize("n,N", SIZES)
+@pytest.mark.parametrize("kinetic", [True, False])
+def test_vxc(E, n, N, kinetic):
+    ao, g1, g2, _, pot = _tables(n, N, 100 * n + N + 1)
+    if not kinetic:
+        pot[:, 5] = 0.0
+    r = _resident(E, ao, g1, g2)
+    got = r.vxc_from_potentials(pot).cpu().numpy()
+    r.status()
+    lap = g2.sum(-1)
+    for s in range(2):
+        c = pot[s][..., None]
+        Q = c[0] * ao + sum(c[1 + j] * g1[..., j] for j in range(3)) + c[4] * lap
+        aQ = np.abs(c[0] * ao) + sum(np.abs(c[1 + j] * g1[..., j]) for j in range(3)) + np.abs(c[4] * lap)
+        ref, size = ao.T @ Q, np.abs(ao).T @ aQ
+        lost = np.abs(ao).max(0)[:, None] * aQ.max(0)[None]
+        for j in range(3):
+            K = c[5] * g1[..., j]
+            ref += g1[..., j].T @ K
+            size += np.abs(g1[..., j]).T @ np.abs(K)
+            lost += np.abs(g1[..., j]).max(0)[:, None] * np.abs(K).max(0)[None]
+        # The kinetic rows share one exponent over the three planes: 10^0.5 at most between them here.
+        bound = (320 + N / 16 + 32) * U * size + N * 2.0 ** -52 * np.maximum(lost, lost.T) + 1e-300
+        assert np.all(np.abs(got[s] - ref) <= bound), np.max(np.abs(got[s] - ref) / bound)
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
+def test_not_finite(E, value):
+    """One bad entry: the plain kernels' (IEEE) pattern, and a following finite call is unaffected."""
+    n, N = 40, 300
+    ao, g1, g2, D, pot = _tables(n, N, 9)
+    r = _resident(E, ao, g1, g2)
+    clean, vclean = r.density(D), r.vxc_from_potentials(pot)
+    bad = D.copy()
+    bad[1, 3, 5] = value
+    out = r.density(bad)
+    assert torch.equal(torch.isfinite(out["rho"][:, 0]), torch.ones(N, dtype=torch.bool, device="cuda"))
+    t = torch.as_tensor(ao)
+    ref = ((t @ torch.as_tensor(bad[1])) * t).sum(1)
+    assert torch.equal(torch.isfinite(out["rho"][:, 1].cpu()), torch.isfinite(ref))
+    badpot = pot.copy()
+    badpot[0, 0, 17] = value
+    v = r.vxc_from_potentials(badpot).cpu().numpy()
+    assert not np.isfinite(v[0]).all() and np.isfinite(v[1]).all()
+    row = ao[17][:, None] * (value * ao[17])[None]
+    assert np.array_equal(np.isnan(v[0]), np.isnan(row) | np.isnan(v[0])) and not np.isfinite(v[0][~np.isfinite(row)]).any()
+    for k, x in r.density(D).items():
+        assert torch.equal(x, clean[k])
+    assert torch.equal(r.vxc_from_potentials(pot), vclean)
