@@ -932,7 +932,7 @@ int gdft_neural_xc_energy_and_grads(const gdft_molecule *mol, const double *d_rd
                       net->clip, ws + W.bytes, d_exc, coef, (int *)(ws + W.off_err), st);
     else
       rc = mlp_run_f64(net_shape(net), d_params, d_dparams, feat, d_ehf, mol_w(mol), mol->n_grid, mol->n_grid_pad,
-                       net->clip, (double *)(ws + W.bytes), d_exc, coef, st);
+                       net->clip, (double *)(ws + W.bytes), d_exc, coef, (int *)(ws + W.off_err), st);
     if (rc) return rc;
   }
   if (d_vxc == nullptr) return GDFT_OK;
@@ -980,7 +980,7 @@ int gdft_neural_xc_hf_grads(const gdft_molecule *mol, const double *d_rdm1, cons
                       net->clip, ws + W.bytes, d_exc, coef, (int *)(ws + W.off_err), st);
     else
       rc = mlp_run_f64(net_shape(net), d_params, nullptr, feat, d_ehf, mol_w(mol), mol->n_grid, mol->n_grid_pad,
-                       net->clip, mws, d_exc, coef, st);
+                       net->clip, mws, d_exc, coef, (int *)(ws + W.off_err), st);
     if (rc) return rc;
   }
   if (net->precision == GDFT_TF32X3) {
@@ -1113,7 +1113,7 @@ int gdft_neural_xc_hvp(const gdft_molecule *mol, const double *d_rdm1, const gdf
                       net->clip, hws, d_value, coef, (int *)(ws + W.off_err), st);
     else
       rc = mlp_hvp_f64(S, d_params, d_hparams, featp, feat, d_ehf, mol_w(mol), mol->n_grid, mol->n_grid_pad,
-                       net->clip, (double *)hws, d_value, coef, st);
+                       net->clip, (double *)hws, d_value, coef, (int *)(ws + W.off_err), st);
     if (rc) return rc;
   }
   if (d_hrdm1 == nullptr) return GDFT_OK;
@@ -1510,7 +1510,7 @@ static int chunk_pass(const gdft_molecule *m, char *ws, const ChunkWs &C, char *
                       ws + W.bytes, e_c, coef, (int *)(ws + W.off_err), st);
     else
       rc = mlp_run_f64(net_shape(net), params, dp_c, feat, ehf_c, mol_w(m), m->n_grid, m->n_grid_pad, net->clip,
-                       (double *)(ws + W.bytes), e_c, coef, st);
+                       (double *)(ws + W.bytes), e_c, coef, (int *)(ws + W.off_err), st);
     if (rc) return rc;
   } else {
     double *epart = (double *)(ws + W.off_epart);

@@ -114,17 +114,29 @@ struct GemmArgs {
   double *out;                 // row r, column c of half h (columns 64 h .. of a tile): out + split_stride split
   int64_t ldc;                 //   + plane_stride plane + half_stride h + nt_stride nt + ldc c + r (lanes are rows)
   int64_t half_stride, nt_stride, split_stride, plane_stride;
-  int64_t m_valid;             // rows written
-  int accumulate;              // add to out
+  int64_t m_valid, n_valid;    // rows and (kFull) columns written
+  const double *add;           // added to the result, laid out like out (may be out itself), or null
   const int *bad;              // non-zero: an operand is not finite, nothing to do
   int *err;
 };
 
 cudaError_t launch_gemm(const GemmArgs &a, cudaStream_t st);
 
-// Row-major FP64 rows (planes of them) -> digit sets [plane][row tile][chunk], exponents [plane][rows].
-cudaError_t launch_rows(const double *src, int64_t plane_elems, int planes, int64_t rows, int ld, int k_valid,
+// Row-major FP64 rows (planes of them, k_valid values each) -> digit sets [plane][row tile][chunk], exponents
+// [plane][rows].  Rows past the last are left as they are: they only reach outputs that are not written.
+cudaError_t launch_rows(const double *src, int64_t plane_elems, int planes, int64_t rows, int64_t ld, int k_valid,
                         int chunks, unsigned char *out, int *exps, int *bad, cudaStream_t st);
+
+// FP64 GEMMs of fx_mat.cu, on row-major operands.  ws: scratch of gemm_rows_bytes / gemm_cols_bytes; err: a device
+// error word or null (an expired wait leaves NaN in the output either way); part: partials of the plain kernel that takes over where an operand is not finite (nsplit x M x N doubles).
+size_t gemm_rows_bytes(int64_t M, int N, int K);
+size_t gemm_cols_bytes(int M, int N, int64_t K);
+// C[m][n] = sum_k A[m][k] B[k][n] (B stored N x K when b_rows) + add[m][n] (laid out like C; null: nothing).
+cudaError_t gemm_rows(int64_t M, int N, int K, const double *A, int64_t lda, const double *B, int64_t ldb, bool b_rows,
+                      double *C, int64_t ldc, const double *add, unsigned char *ws, int *err, cudaStream_t st);
+// C[m][n] = sum_k A[k][m] B[k][n], C contiguous (M x N).
+cudaError_t gemm_cols(int M, int N, int64_t K, const double *A, int64_t lda, const double *B, int64_t ldb, double *C,
+                      unsigned char *ws, int *err, int nsplit, double *part, cudaStream_t st);
 
 // Feature sets of fx_xc.cu: the FP64 form's density and V_xc contractions.
 struct XcWs {

@@ -113,8 +113,8 @@ __device__ __forceinline__ Item item_of(const GemmArgs &A, int upper, int i) {
     t.plane = t.base = 0;
     const int tiles = A.m_tiles * A.n_tiles;
     t.split = i / tiles;
-    t.mt = i % tiles / A.n_tiles;
-    t.nt = i % tiles % A.n_tiles;
+    t.nt = i % tiles / A.m_tiles;
+    t.mt = i % tiles % A.m_tiles;
   }
   t.c0 = t.split * A.chunks_per_split;
   t.c1 = t.c0 + A.chunks_per_split < chunks ? t.c0 + A.chunks_per_split : chunks;
@@ -389,9 +389,11 @@ __global__ void __launch_bounds__(kThreads, 1) fx_gemm_kernel(const GemmArgs A, 
         const int *ea = A.ea + (size_t)t.plane * A.m_tiles * kTile;
         const int *eb = (t.plane ? A.eb1 : A.eb) + (size_t)t.nt * kTile + col;
         const int e0 = (live ? ea[row] : 0) - 2 * 1022 - 14 - 36;
-        double *out = A.out + (int64_t)t.split * A.split_stride + (int64_t)t.plane * A.plane_stride +
-                      (col >> 6) * A.half_stride + (int64_t)t.nt * A.nt_stride + (col & 63) * A.ldc + row;
-        const bool add = A.accumulate || c - t.c0 >= kSumChunks;
+        const int64_t at = (int64_t)t.split * A.split_stride + (int64_t)t.plane * A.plane_stride +
+                           (col >> 6) * A.half_stride + (int64_t)t.nt * A.nt_stride + (col & 63) * A.ldc + row;
+        double *out = A.out + at;
+        const double *add = c - t.c0 >= kSumChunks ? out : A.add != nullptr ? A.add + at : nullptr;
+        const int64_t cols = A.mode == kFull ? A.n_valid - ((int64_t)t.nt * kTile + col) : kCols;  // of these 64
         // 16 columns a turn, the sums moved down by 16 after each: unrolled, the code (some 60 KB, run once an
         // item) is fetched at the pace of instruction-cache misses.
 #pragma unroll 1
@@ -412,19 +414,22 @@ __global__ void __launch_bounds__(kThreads, 1) fx_gemm_kernel(const GemmArgs A, 
             up = up > 0 ? up : 0;
             const float zs = __uint_as_float((uint32_t)(127 + 36 + up) << 23);
             v[k] = fixed_to_double((s << up) + (long long)__float2int_rn(z * zs), e0 - up + __ldg(eb + h + k));
+            if (!ok) v[k] = __longlong_as_double(0x7FF8000000000000ll);
           }
           // Stores apart from the arithmetic: a branch a column would serialise it.
           if (live) {
             double *o = out + (int64_t)h * A.ldc;
-            if (add) {
+            if (add != nullptr) {
+              const double *w = add + (int64_t)h * A.ldc;
               double was[16];
 #pragma unroll
-              for (int k = 0; k < 16; ++k) was[k] = o[(int64_t)k * A.ldc];
+              for (int k = 0; k < 16; ++k) was[k] = h + k < cols ? w[(int64_t)k * A.ldc] : 0.0;
 #pragma unroll
               for (int k = 0; k < 16; ++k) v[k] += was[k];
             }
 #pragma unroll
-            for (int k = 0; k < 16; ++k) o[(int64_t)k * A.ldc] = v[k];
+            for (int k = 0; k < 16; ++k)
+              if (h + k < cols) o[(int64_t)k * A.ldc] = v[k];
           }
 #pragma unroll
           for (int k = 0; k < kCols; ++k) sum[k] = k + 16 < kCols ? sum[k + 16 < kCols ? k + 16 : 0] : 0;
@@ -444,50 +449,54 @@ __global__ void __launch_bounds__(kThreads, 1) fx_gemm_kernel(const GemmArgs A, 
 // Eight rows per warp: lane = (row, eight consecutive k); the row's largest
 // exponent first, then the digits (the second read hits L1).  A warp's store of
 // one digit is 512 contiguous bytes.
+template <bool VEC>
 __global__ void __launch_bounds__(256) fx_rows_kernel(const double *__restrict__ src, int64_t plane_elems, int64_t rows,
-                                                      int ld, int k_valid, int chunks, unsigned char *__restrict__ out,
-                                                      int *__restrict__ exps, int *__restrict__ bad) {
+                                                      int64_t ld, int k_valid, int chunks,
+                                                      unsigned char *__restrict__ out, int *__restrict__ exps,
+                                                      int *__restrict__ bad) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t tiles = rows / kTile;
+  const int64_t tiles = (rows + kTile - 1) / kTile;
   const int64_t r0 = ((int64_t)blockIdx.x * 8 + warp) * 8;
   if (r0 >= rows) return;
   const int plane = blockIdx.y;
   const int64_t row = r0 + (lane & 7);
-  const double *x = src + (size_t)plane * plane_elems + (size_t)row * ld;
+  const bool in = row < rows;
+  const double *x = src + (size_t)plane * plane_elems + (size_t)(in ? row : r0) * ld;
   const int kg = (lane >> 3) * 8;
-  uint32_t m = 0;
-  for (int k = kg; k < k_valid; k += 32) {
-    if (k + 8 <= k_valid) {
+  auto load8 = [&](int k, double (&v)[8]) {
+    if (VEC && k + 8 <= k_valid) {
 #pragma unroll
       for (int j = 0; j < 8; j += 2) {
-        const double2 v = *(const double2 *)(x + k + j);
-        m = max(m, max((uint32_t)__double2hiint(v.x) & 0x7FFFFFFFu, (uint32_t)__double2hiint(v.y) & 0x7FFFFFFFu));
+        const double2 t = *(const double2 *)(x + k + j);
+        v[j] = t.x;
+        v[j + 1] = t.y;
       }
     } else {
-      for (int j = k; j < k_valid; ++j) m = max(m, (uint32_t)__double2hiint(x[j]) & 0x7FFFFFFFu);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = k + j < k_valid ? x[k + j] : 0.0;
     }
+  };
+  uint32_t m = 0;
+  for (int k = kg; k < k_valid; k += 32) {
+    double v[8];
+    load8(k, v);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) m = max(m, (uint32_t)__double2hiint(v[j]) & 0x7FFFFFFFu);
   }
   m = max(m, __shfl_xor_sync(0xffffffffu, m, 8));
   m = max(m, __shfl_xor_sync(0xffffffffu, m, 16));
   int emax = exp_field(m);
   if (emax == 0x7FF) atomicOr(bad, 1);
   if (emax < 1) emax = 1;
-  if (lane < 8) exps[(size_t)plane * rows + row] = emax;
+  if (lane < 8 && in) exps[(size_t)plane * rows + row] = emax;
   unsigned char *base = out + ((size_t)plane * tiles + (size_t)(row / kTile)) * chunks * kSetBytes;
   const int rt = (int)(row % kTile);
   for (int k = kg; k < chunks * kChunkK; k += 32) {
+    double v[8];
+    load8(k, v);
     long long f[8];
-    if (k + 8 <= k_valid) {
 #pragma unroll
-      for (int j = 0; j < 8; j += 2) {
-        const double2 v = *(const double2 *)(x + k + j);
-        f[j] = to_fixed(v.x, emax);
-        f[j + 1] = to_fixed(v.y, emax);
-      }
-    } else {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) f[j] = k + j < k_valid ? to_fixed(x[k + j], emax) : 0;
-    }
+    for (int j = 0; j < 8; ++j) f[j] = to_fixed(v[j], emax);
     uint4 d[kDigits];
     digits8(f, d);
     unsigned char *set = base + (size_t)(k / kChunkK) * kSetBytes + elem_off(rt, k % kChunkK);
@@ -514,11 +523,14 @@ cudaError_t launch_gemm(const GemmArgs &a, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_rows(const double *src, int64_t plane_elems, int planes, int64_t rows, int ld, int k_valid,
+cudaError_t launch_rows(const double *src, int64_t plane_elems, int planes, int64_t rows, int64_t ld, int k_valid,
                         int chunks, unsigned char *out, int *exps, int *bad, cudaStream_t st) {
-  if (rows % kTile != 0 || (ld & 1) != 0) return cudaErrorInvalidValue;
-  const dim3 grid((unsigned)((rows / 8 + 7) / 8), planes);
-  fx_rows_kernel<<<grid, 256, 0, st>>>(src, plane_elems, rows, ld, k_valid, chunks, out, exps, bad);
+  const dim3 grid((unsigned)((rows + 63) / 64), planes);
+  // 16-byte loads where every row starts on a 16-byte boundary.
+  if (((uintptr_t)src & 15) == 0 && (ld & 1) == 0 && (plane_elems & 1) == 0)
+    fx_rows_kernel<true><<<grid, 256, 0, st>>>(src, plane_elems, rows, ld, k_valid, chunks, out, exps, bad);
+  else
+    fx_rows_kernel<false><<<grid, 256, 0, st>>>(src, plane_elems, rows, ld, k_valid, chunks, out, exps, bad);
   return cudaGetLastError();
 }
 

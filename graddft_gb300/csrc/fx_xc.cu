@@ -470,7 +470,7 @@ cudaError_t launch_vxc(const double *tab, int64_t np, int ld, int n_ao, const do
     g.plane_stride = w.s0 * g.split_stride;
     g.m_valid = n_max;
     g.out = part;
-    g.accumulate = p0 > 0;
+    g.add = p0 > 0 ? part : nullptr;
     g.bad = bad;
     g.err = err;
     if ((e = launch_gemm(g, st)) != cudaSuccess) return e;

@@ -7,7 +7,7 @@
 // with g = dE_xc/d ehf.  chi keeps the reference's layout (grid, omega, spin,
 // orbitals).
 //
-// FP64 form: both contractions on the tiled FP64 GEMM: X_s = ao D_s, then a
+// FP64 form: both contractions on digit products (fx_mat.cu): X_s = ao D_s, then a
 // warp per (point, spin) takes the row dot with chi; B_s = -1/2 sum_w g chi,
 // then F_s = ao^T B_s with the grid split over CTAs and the partials summed in
 // a fixed order.
@@ -19,6 +19,7 @@
 // K = grid points split over CTAs, B formed inside its packer (never stored),
 // partials summed in a fixed order.
 #include "common.cuh"
+#include "fx.cuh"
 #include "kernels.cuh"
 #include "mlp_gemm.cuh"
 #include "tc_gemm.cuh"
@@ -224,6 +225,11 @@ int hf_splits(int64_t n_grid) {
   return (int)s;
 }
 
+size_t hf_gemm_off(int64_t n_grid, int n_ao) {
+  return align256((size_t)2 * n_grid * n_ao * sizeof(double)) +
+         align256((size_t)hf_splits(n_grid) * n_ao * n_ao * sizeof(double));
+}
+
 int check_hf_args(const char *who, int form, const void *ao, const void *chi, int64_t n_grid, int n_ao, int n_omega,
                   const void *out, const void *ws, size_t ws_bytes) {
   if (form != GDFT_FP64 && form != GDFT_TF32X3) {
@@ -348,9 +354,9 @@ int gdft_hf_workspace_bytes_form(int64_t n_grid, int32_t n_ao, int32_t n_omega, 
     *bytes = hf_tc_layout(n_grid, n_ao).bytes;
     return GDFT_OK;
   }
-  // X or B: [2][n_grid][n_ao]; split partials of F: [nsplit][n_ao][n_ao].
-  *bytes = align256((size_t)2 * n_grid * n_ao * sizeof(double)) +
-           align256((size_t)hf_splits(n_grid) * n_ao * n_ao * sizeof(double));
+  // X or B: [2][n_grid][n_ao]; split partials of F: [nsplit][n_ao][n_ao]; the GEMMs' scratch.
+  const size_t rows = fx::gemm_rows_bytes(n_grid, n_ao, n_ao), cols = fx::gemm_cols_bytes(n_ao, n_ao, n_grid);
+  *bytes = hf_gemm_off(n_grid, n_ao) + (rows > cols ? rows : cols);
   return GDFT_OK;
 }
 
@@ -372,8 +378,9 @@ int gdft_hf_energy_density_form(const double *d_ao, const double *d_rdm1, const 
                                                        (char *)d_ws, st);
   double *X = (double *)d_ws;
   for (int s = 0; s < 2; ++s)
-    if ((rc = check_cuda(gemm<kNN>((int)n_grid, n_ao, n_ao, d_ao, n_ao, d_rdm1 + (size_t)s * n_ao * n_ao, n_ao,
-                                   X + (size_t)s * n_grid * n_ao, n_ao, 0.0, st),
+    if ((rc = check_cuda(fx::gemm_rows(n_grid, n_ao, n_ao, d_ao, n_ao, d_rdm1 + (size_t)s * n_ao * n_ao, n_ao, false,
+                                       X + (size_t)s * n_grid * n_ao, n_ao, nullptr,
+                                       (unsigned char *)d_ws + hf_gemm_off(n_grid, n_ao), nullptr, st),
                          "hf ao.D")))
       return rc;
   const int64_t threads = 2 * n_grid * 32;
@@ -405,8 +412,9 @@ int gdft_hf_fock_form(const double *d_ao, const double *d_chi, const double *d_g
   if ((rc = check_cuda(cudaGetLastError(), "hf B"))) return rc;
   const int nsplit = hf_splits(n_grid);
   for (int s = 0; s < 2; ++s)
-    if ((rc = check_cuda(gemm_tn_split(n_ao, n_ao, n_grid, d_ao, n_ao, B + (size_t)s * n_grid * n_ao, n_ao,
-                                       d_fock_hf + (size_t)s * n_ao * n_ao, nsplit, part, st),
+    if ((rc = check_cuda(fx::gemm_cols(n_ao, n_ao, n_grid, d_ao, n_ao, B + (size_t)s * n_grid * n_ao, n_ao,
+                                       d_fock_hf + (size_t)s * n_ao * n_ao,
+                                       (unsigned char *)d_ws + hf_gemm_off(n_grid, n_ao), nullptr, nsplit, part, st),
                          "hf ao^T B")))
       return rc;
   return GDFT_OK;

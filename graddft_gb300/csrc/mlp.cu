@@ -20,10 +20,11 @@
 //
 // Data layout: activations row-major [np][width] FP64 per layer; every layer's
 // output h_i and pre-normalisation sum z_i stay resident for the backward.
-// GEMMs are plain tiled FP64; a row of the hidden width is one warp's work.
+// GEMMs run on digit products (fx_mat.cu); a row of the hidden width is one warp's work.
 #include <string.h>
 
 #include "common.cuh"
+#include "fx.cuh"
 #include "kernels.cuh"
 #include "mlp.cuh"
 #include "mlp_gemm.cuh"
@@ -401,6 +402,16 @@ size_t mlp_param_count(const MlpShape &s) {
   return n;
 }
 
+size_t mlp_gemm_bytes(const MlpShape &s, int64_t rows) {
+  const size_t b[] = {fx::gemm_rows_bytes(rows, s.width, s.width), fx::gemm_rows_bytes(rows, s.width, s.n_in),
+                      fx::gemm_rows_bytes(rows, s.n_out, s.width), fx::gemm_rows_bytes(rows, s.n_in, s.width),
+                      fx::gemm_cols_bytes(s.width, s.width, rows), fx::gemm_cols_bytes(s.width, s.n_out, rows),
+                      fx::gemm_cols_bytes(s.n_in, s.width, rows)};
+  size_t most = 0;
+  for (size_t v : b) most = v > most ? v : most;
+  return most;
+}
+
 MlpLayout mlp_layout(const MlpShape &s, int64_t np) {
   MlpLayout L;
   const size_t act = (size_t)np * s.width;
@@ -428,6 +439,7 @@ MlpLayout mlp_layout(const MlpShape &s, int64_t np) {
   L.lnpart = take((size_t)kLnBlocks * 2 * s.width);
   L.colpart = take((size_t)kColBlocks * 2 * s.width);
   L.epart = take((size_t)L.eblocks);
+  L.fx = take((mlp_gemm_bytes(s, np) + 7) / 8);
   L.doubles = off;
   return L;
 }
@@ -439,7 +451,7 @@ size_t layer_offset(const MlpShape &S, int i) {
 }
 
 // u (np x kDm21InPad) -> h_0 .. h_L, z_1 .. z_L and y = h_L W_out (head bias not added).
-int net_forward(const MlpShape &S, const double *params, const MlpLayout &L, double *ws, int64_t np,
+int net_forward(const MlpShape &S, const double *params, const MlpLayout &L, double *ws, int64_t np, int *err,
                 cudaStream_t st) {
   const int Wd = S.width;
   const size_t act = (size_t)np * Wd;
@@ -447,20 +459,22 @@ int net_forward(const MlpShape &S, const double *params, const MlpLayout &L, dou
   const double *W0 = params, *b0 = W0 + (size_t)S.n_in * Wd;
   const double *Wout = params + layer_offset(S, S.n_layers);
   int rc;
-  if ((rc = check_cuda(gemm<kNN>((int)np, Wd, S.n_in, u, kDm21InPad, W0, Wd, h, Wd, 0.0, st), "mlp dense_0")))
-    return rc;
+  auto mul = [&](int N, int K, const double *A, int lda, const double *B, double *C) {  // C = A B, B (K x N)
+    return fx::gemm_rows(np, N, K, A, lda, B, N, false, C, N, nullptr, (unsigned char *)(ws + L.fx), err, st);
+  };
+  if ((rc = check_cuda(mul(Wd, S.n_in, u, kDm21InPad, W0, h), "mlp dense_0"))) return rc;
   tanh_bias_kernel<<<(unsigned)((act + 255) / 256), 256, 0, st>>>(h, b0, act, Wd);
   if ((rc = check_cuda(cudaGetLastError(), "mlp tanh"))) return rc;
   for (int i = 1; i <= S.n_layers; ++i) {
     const double *Wi = params + layer_offset(S, i - 1), *bi = Wi + (size_t)Wd * Wd, *gi = bi + Wd, *bei = gi + Wd;
     const double *hprev = h + (size_t)(i - 1) * act;
     double *hi = h + (size_t)i * act, *zi = z + (size_t)(i - 1) * act;
-    if ((rc = check_cuda(gemm<kNN>((int)np, Wd, Wd, hprev, Wd, Wi, Wd, zi, Wd, 0.0, st), "mlp dense_i"))) return rc;
+    if ((rc = check_cuda(mul(Wd, Wd, hprev, Wd, Wi, zi), "mlp dense_i"))) return rc;
     if ((rc = check_cuda(launch_res_ln_elu_fwd(Wd, zi, bi, hprev, gi, bei, S.ln_eps, np, hi, st), "mlp layernorm")))
       return rc;
   }
   const double *hL = h + (size_t)S.n_layers * act;
-  return check_cuda(gemm<kNN>((int)np, S.n_out, Wd, hL, Wd, Wout, S.n_out, y, S.n_out, 0.0, st), "mlp head");
+  return check_cuda(mul(S.n_out, Wd, hL, Wd, Wout, y), "mlp head");
 }
 
 // u = log(|x| + off) for given network inputs x (rows x n_in).
@@ -507,7 +521,7 @@ int mlp_apply_f64(const MlpShape &S, const double *params, const double *x, int6
   squash_kernel<<<(unsigned)((rows + 255) / 256), 256, 0, st>>>(x, rows, S.n_in, S.squash_offset, ws + L.u);
   int rc = check_cuda(cudaGetLastError(), "mlp squash");
   if (rc) return rc;
-  if ((rc = net_forward(S, params, L, ws, rows, st))) return rc;
+  if ((rc = net_forward(S, params, L, ws, rows, nullptr, st))) return rc;
   const double *bout = params + layer_offset(S, S.n_layers) + (size_t)S.width * S.n_out;
   head_coeff_kernel<<<(unsigned)((rows * S.n_out + 255) / 256), 256, 0, st>>>(ws + L.y, bout, rows, S.n_out,
                                                                              S.sigmoid_scale, c);
@@ -519,7 +533,7 @@ int mlp_apply_f64(const MlpShape &S, const double *params, const double *x, int6
 // Dense_{L+1} (kernel W x n_out, bias n_out).  dparams uses the same order.
 int mlp_run_f64(const MlpShape &S, const double *params, double *dparams, const double *feat, const double *ehf,
                 const double *w, int64_t n_grid, int64_t np, double clip, double *ws, double *exc, double *coef,
-                cudaStream_t st) {
+                int *err, cudaStream_t st) {
   const MlpLayout L = mlp_layout(S, np);
   const int Wd = S.width;
   double *x = ws + L.x, *u = ws + L.u, *e = ws + L.e, *h = ws + L.h, *z = ws + L.z, *y = ws + L.y;
@@ -541,7 +555,7 @@ int mlp_run_f64(const MlpShape &S, const double *params, double *dparams, const 
   // ---- forward ----
   dm21_features_kernel<<<pb, 256, 0, st>>>(feat, ehf, n_grid, np, clip, S.squash_offset, x, u, e);
   GDFT_CK(cudaGetLastError(), "dm21_features");
-  if ((rc = net_forward(S, params, L, ws, np, st)) != GDFT_OK) return rc;
+  if ((rc = net_forward(S, params, L, ws, np, err, st)) != GDFT_OK) return rc;
   head_energy_kernel<<<pb, 256, 0, st>>>(y, bout, e, w, n_grid, np, clip, S.sigmoid_scale, dy, de, epart);
   GDFT_CK(cudaGetLastError(), "mlp head_energy");
   GDFT_CK(launch_energy_reduce(epart, (int)pb, exc, st), "mlp energy_reduce");
@@ -550,7 +564,10 @@ int mlp_run_f64(const MlpShape &S, const double *params, double *dparams, const 
   // ---- backward ----
   const int ns = L.nsplit;
   auto weight_grad = [&](int M, int N, const double *A, int lda, const double *B, int ldb, double *C) {
-    return gemm_tn_split(M, N, np, A, lda, B, ldb, C, ns, kpart, st);
+    return fx::gemm_cols(M, N, np, A, lda, B, ldb, C, (unsigned char *)(ws + L.fx), err, ns, kpart, st);
+  };
+  auto mul_t = [&](int N, int K, const double *A, const double *B, double *C, int ldc, const double *add) {
+    return fx::gemm_rows(np, N, K, A, K, B, K, true, C, ldc, add, (unsigned char *)(ws + L.fx), err, st);
   };
   auto col_sum = [&](const double *X, int64_t rows, int ncols, int ld, double *out) {
     return col_sums(X, rows, ncols, ld, out, colpart, kColBlocks, st);
@@ -560,7 +577,7 @@ int mlp_run_f64(const MlpShape &S, const double *params, double *dparams, const 
     GDFT_CK(weight_grad(Wd, S.n_out, hL, Wd, dy, S.n_out, dparams + head_off), "mlp dW_out");
     GDFT_CK(col_sum(dy, np, S.n_out, S.n_out, dparams + head_off + (size_t)Wd * S.n_out), "mlp db_out");
   }
-  GDFT_CK(gemm<kNT>((int)np, Wd, S.n_out, dy, S.n_out, Wout, S.n_out, d0, Wd, 0.0, st), "mlp dh_L");
+  GDFT_CK(mul_t(Wd, S.n_out, dy, Wout, d0, Wd, nullptr), "mlp dh_L");
   double *dcur = d0, *dnext = d1;
   for (int i = S.n_layers; i >= 1; --i) {
     const double *Wi = params + layer_off(i - 1), *gi = Wi + (size_t)Wd * Wd + Wd, *bei = gi + Wd;
@@ -573,8 +590,7 @@ int mlp_run_f64(const MlpShape &S, const double *params, double *dparams, const 
       GDFT_CK(col_sum(lnpart, kLnBlocks, 2 * Wd, 2 * Wd, dWi + (size_t)Wd * Wd + Wd), "mlp dLN_i");
     }
     // dh_{i-1} = dz (residual) + dz W_i^T.
-    GDFT_CK(cudaMemcpyAsync(dnext, dcur, act * sizeof(double), cudaMemcpyDeviceToDevice, st), "mlp residual");
-    GDFT_CK(gemm<kNT>((int)np, Wd, Wd, dcur, Wd, Wi, Wd, dnext, Wd, 1.0, st), "mlp dh_i");
+    GDFT_CK(mul_t(Wd, Wd, dcur, Wi, dnext, Wd, dcur), "mlp dh_i");
     double *t = dcur;
     dcur = dnext;
     dnext = t;
@@ -587,7 +603,7 @@ int mlp_run_f64(const MlpShape &S, const double *params, double *dparams, const 
     GDFT_CK(col_sum(dcur, np, Wd, Wd, dparams + (size_t)S.n_in * Wd), "mlp db_0");
   }
   if (coef != nullptr) {
-    GDFT_CK(gemm<kNT>((int)np, S.n_in, Wd, dcur, Wd, W0, Wd, du, kDm21InPad, 0.0, st), "mlp du");
+    GDFT_CK(mul_t(S.n_in, Wd, dcur, W0, du, kDm21InPad, nullptr), "mlp du");
     dm21_potentials_kernel<<<pb, 256, 0, st>>>(feat, x, du, de, n_grid, np, clip, S.squash_offset, coef);
     GDFT_CK(cudaGetLastError(), "dm21_potentials");
   }

@@ -25,12 +25,15 @@ struct MlpShape {
 
 // Offsets (in doubles) of the network scratch inside its workspace region.
 struct MlpLayout {
-  size_t x, u, e, h, z, y, dy, de, d0, d1, du, kpart, lnpart, colpart, epart, doubles;
+  size_t x, u, e, h, z, y, dy, de, d0, d1, du, kpart, lnpart, colpart, epart, fx, doubles;  // fx: GEMM scratch
   int nsplit;   // split-K factor of the weight-gradient GEMMs
   int eblocks;  // energy partial sums
 };
 
 size_t mlp_param_count(const MlpShape &s);
+
+// Bytes of the scratch that the FP64 form's GEMMs over `rows` rows need (fx_mat.cu).
+size_t mlp_gemm_bytes(const MlpShape &s, int64_t rows);
 
 // Per-point DM21 inputs x (np x 11), squashed u (np x 16), energy densities e
 // (np x 3); and the V-contraction coefficients from dE/du and dE/de.
@@ -47,7 +50,7 @@ bool mlp_width_supported(int width);
 // dparams = dE/dtheta in the flat parameter order.
 int mlp_run_f64(const MlpShape &S, const double *params, double *dparams, const double *feat, const double *ehf,
                 const double *w, int64_t n_grid, int64_t np, double clip, double *ws, double *exc, double *coef,
-                cudaStream_t st);
+                int *err, cudaStream_t st);
 // After mlp_run_f64 with coef (the backward pass) on the same workspace:
 // g_dens, g_cin (2 omegas, 2 spins, n_grid) = dE/d ehf through the HF
 // energy-density columns and through the HF inputs (either may be null).
@@ -61,7 +64,7 @@ cudaError_t launch_dm21_hf_grads_from(const double *x, const double *du, const d
 // Scratch of the second-order pass (offsets in doubles).  Primal and tangent
 // activations are stacked as [2][np][width] so one GEMM serves both.
 struct MlpHvpLayout {
-  size_t featp, x, xt, u, e, et, h, z, y, gy, ge, d0, d1, gu, kpart, lnpart, colpart, lpart, doubles;
+  size_t featp, x, xt, u, e, et, h, z, y, gy, ge, d0, d1, gu, kpart, lnpart, colpart, lpart, fx, doubles;
   int nsplit;
   int eblocks;
 };
@@ -73,7 +76,7 @@ MlpHvpLayout mlp_hvp_layout(const MlpShape &s, int64_t np);
 // null) and *lval = L (may be null).
 int mlp_hvp_f64(const MlpShape &S, const double *params, double *dparams, const double *featp, const double *featt,
                 const double *ehf, const double *w, int64_t n_grid, int64_t np, double clip, double *ws,
-                double *lval, double *coef, cudaStream_t st);
+                double *lval, double *coef, int *err, cudaStream_t st);
 
 // Mixed (TF32x3 tensor-core) form of mlp_run_f64: FP32 activations, FP64 row
 // statistics, head, features and potentials; widths 128 and 256.

@@ -9,7 +9,10 @@ namespace gdft {
 namespace {
 
 // ----------------------------------------------------------------- GEMM ---
-// C[M x N] = op(A) op(B) (+ beta C); row-major operands with leading dimensions.
+// C[M x N] = op(A) op(B) (+ add, laid out like C); row-major operands with leading
+// dimensions.  bad: when given, a device word; the launch does nothing where it is 0
+// (the network's GEMMs run on digit products, fx_mat.cu, which leaves operands that
+// are not finite to this kernel).
 //   kNN: A (M x K), B (K x N)       kNT: A (M x K), B stored (N x K)
 //   kTN: A stored (K x M), B (K x N); K is split over blockIdx.z, each split
 //        writing its own partial C at C + z * split_stride.
@@ -19,7 +22,9 @@ constexpr int GT = 64, GK = 16, GTH = 256;
 template <int MODE>
 __global__ void __launch_bounds__(GTH) gemm_f64_kernel(int M, int N, int K, const double *__restrict__ A, int lda,
                                                       const double *__restrict__ B, int ldb, double *__restrict__ C,
-                                                      int ldc, double beta, int kchunk, size_t split_stride) {
+                                                      int ldc, const double *__restrict__ add, int kchunk,
+                                                      size_t split_stride, const int *__restrict__ bad) {
+  if (bad != nullptr && *bad == 0) return;
   __shared__ double As[GK][GT + 1];
   __shared__ double Bs[GK][GT + 1];
   const int tid = threadIdx.x, tr = tid >> 4, tc = tid & 15;
@@ -84,13 +89,15 @@ __global__ void __launch_bounds__(GTH) gemm_f64_kernel(int M, int N, int K, cons
       const int m = m0 + tr + 16 * i, n = n0 + tc + 16 * j;
       if (m < M && n < N) {
         double *c = Cz + (size_t)m * ldc + n;
-        *c = beta != 0.0 ? beta * *c + acc[i][j] : acc[i][j];
+        *c = add != nullptr ? add[(size_t)m * ldc + n] + acc[i][j] : acc[i][j];
       }
     }
 }
 
 // C[i] = sum over splits of part[split][i] (fixed order).
-__global__ void sum_splits_kernel(const double *__restrict__ part, int nsplit, size_t total, double *__restrict__ C) {
+__global__ void sum_splits_kernel(const double *__restrict__ part, int nsplit, size_t total, double *__restrict__ C,
+                                  const int *__restrict__ bad) {
+  if (bad != nullptr && *bad == 0) return;
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   double s = 0.0;
@@ -141,24 +148,24 @@ __device__ __forceinline__ double warp_sum(double v) {
 }
 
 template <int MODE>
-cudaError_t gemm(int M, int N, int K, const double *A, int lda, const double *B, int ldb, double *C, int ldc,
-                 double beta, cudaStream_t st) {
+cudaError_t plain_gemm(int M, int N, int K, const double *A, int lda, const double *B, int ldb, double *C, int ldc,
+                       const double *add, const int *bad, cudaStream_t st) {
   dim3 grid((M + GT - 1) / GT, (N + GT - 1) / GT, 1);
-  gemm_f64_kernel<MODE><<<grid, GTH, 0, st>>>(M, N, K, A, lda, B, ldb, C, ldc, beta, K, 0);
+  gemm_f64_kernel<MODE><<<grid, GTH, 0, st>>>(M, N, K, A, lda, B, ldb, C, ldc, add, K, 0, bad);
   return cudaGetLastError();
 }
 
 // Split-K TN GEMM C (M x N) = A^T B over K rows, in nsplit fixed slices whose
 // partials (in part, nsplit x M x N) are summed in slice order.
-inline cudaError_t gemm_tn_split(int M, int N, int64_t K, const double *A, int lda, const double *B, int ldb,
-                                 double *C, int nsplit, double *part, cudaStream_t st) {
+inline cudaError_t plain_gemm_tn_split(int M, int N, int64_t K, const double *A, int lda, const double *B, int ldb,
+                                       double *C, int nsplit, double *part, const int *bad, cudaStream_t st) {
   const int kchunk = (int)(((K + nsplit - 1) / nsplit + GK - 1) / GK * GK);
   dim3 grid((M + GT - 1) / GT, (N + GT - 1) / GT, nsplit);
-  gemm_f64_kernel<kTN><<<grid, GTH, 0, st>>>(M, N, (int)K, A, lda, B, ldb, part, N, 0.0, kchunk, (size_t)M * N);
+  gemm_f64_kernel<kTN><<<grid, GTH, 0, st>>>(M, N, (int)K, A, lda, B, ldb, part, N, nullptr, kchunk, (size_t)M * N, bad);
   cudaError_t r = cudaGetLastError();
   if (r != cudaSuccess) return r;
   const size_t total = (size_t)M * N;
-  sum_splits_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(part, nsplit, total, C);
+  sum_splits_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(part, nsplit, total, C, bad);
   return cudaGetLastError();
 }
 

@@ -15,6 +15,7 @@
 // density.  The result is dL/dtheta and per-point coefficients dL/dF whose V
 // contraction (vxc_*.cu) is dL/dD.
 #include "common.cuh"
+#include "fx.cuh"
 #include "dual.cuh"
 #include "kernels.cuh"
 #include "mlp.cuh"
@@ -485,13 +486,14 @@ MlpHvpLayout mlp_hvp_layout(const MlpShape &s, int64_t np) {
   L.lnpart = take((size_t)kLnBlocks * 2 * s.width);
   L.colpart = take((size_t)kColBlocks * 2 * s.width);
   L.lpart = take((size_t)L.eblocks);
+  L.fx = take((mlp_gemm_bytes(s, 2 * np) + 7) / 8);
   L.doubles = off;
   return L;
 }
 
 int mlp_hvp_f64(const MlpShape &S, const double *params, double *dparams, const double *featp, const double *featt,
                 const double *ehf, const double *w, int64_t n_grid, int64_t np, double clip, double *ws,
-                double *lval, double *coef, cudaStream_t st) {
+                double *lval, double *coef, int *err, cudaStream_t st) {
   const MlpHvpLayout L = mlp_hvp_layout(S, np);
   const int Wd = S.width;
   const size_t act = (size_t)np * Wd, act2 = 2 * act;
@@ -510,28 +512,36 @@ int mlp_hvp_f64(const MlpShape &S, const double *params, double *dparams, const 
     if ((rc = check_cuda((expr), what)) != GDFT_OK) return rc; \
   } while (0)
 
+  unsigned char *fxws = (unsigned char *)(ws + L.fx);
+  auto mul = [&](int N, int K, const double *A, int lda, const double *B, double *C) {  // C = A B, B (K x N)
+    return fx::gemm_rows(rows2, N, K, A, lda, B, N, false, C, N, nullptr, fxws, err, st);
+  };
+  auto mul_t = [&](int N, int K, const double *A, const double *B, double *C, int ldc, const double *add) {
+    return fx::gemm_rows(rows2, N, K, A, K, B, K, true, C, ldc, add, fxws, err, st);
+  };
+
   // ---- tangent-augmented forward ----
   features_tan_kernel<<<pb, 256, 0, st>>>(featp, featt, ehf, n_grid, np, clip, S.squash_offset, x, xt, U, e, et);
   GDFT_CK(cudaGetLastError(), "hvp features");
-  GDFT_CK(gemm<kNN>((int)rows2, Wd, S.n_in, U, kInPad, W0, Wd, Z, Wd, 0.0, st), "hvp dense_0");
+  GDFT_CK(mul(Wd, S.n_in, U, kInPad, W0, Z), "hvp dense_0");
   tanh_tan_kernel<<<(unsigned)((act + 255) / 256), 256, 0, st>>>(Z, b0, act, Wd, H);
   GDFT_CK(cudaGetLastError(), "hvp tanh");
   for (int i = 1; i <= S.n_layers; ++i) {
     const double *Wi = params + hvp_layer_offset(S, i - 1), *bi = Wi + (size_t)Wd * Wd, *gi = bi + Wd,
                  *bei = gi + Wd;
     double *Hp = H + (size_t)(i - 1) * act2, *Hi = H + (size_t)i * act2, *Zi = Z + (size_t)i * act2;
-    GDFT_CK(gemm<kNN>((int)rows2, Wd, Wd, Hp, Wd, Wi, Wd, Zi, Wd, 0.0, st), "hvp dense_i");
+    GDFT_CK(mul(Wd, Wd, Hp, Wd, Wi, Zi), "hvp dense_i");
     GDFT_CK(launch_tan_fwd(Wd, Zi, bi, Hp, gi, bei, S.ln_eps, np, Hi, st), "hvp layernorm");
   }
   double *HL = H + (size_t)S.n_layers * act2;
-  GDFT_CK(gemm<kNN>((int)rows2, S.n_out, Wd, HL, Wd, Wout, S.n_out, Y, S.n_out, 0.0, st), "hvp head");
+  GDFT_CK(mul(S.n_out, Wd, HL, Wd, Wout, Y), "hvp head");
   head_tan_kernel<<<pb, 256, 0, st>>>(Y, bout, e, et, w, n_grid, np, clip, S.sigmoid_scale, GY, GE, lpart);
   GDFT_CK(cudaGetLastError(), "hvp head_tan");
   if (lval) GDFT_CK(launch_energy_reduce(lpart, (int)pb, lval, st), "hvp value");
 
   // ---- reverse of the augmented graph ----
   auto wgrad = [&](int M, int N, const double *A, int lda, const double *B, int ldb, double *C) {
-    return gemm_tn_split(M, N, rows2, A, lda, B, ldb, C, L.nsplit, kpart, st);
+    return fx::gemm_cols(M, N, rows2, A, lda, B, ldb, C, fxws, err, L.nsplit, kpart, st);
   };
   auto csum = [&](const double *X, int64_t rows, int ncols, int ld, double *out) {
     return col_sums(X, rows, ncols, ld, out, colpart, kColBlocks, st);
@@ -540,7 +550,7 @@ int mlp_hvp_f64(const MlpShape &S, const double *params, double *dparams, const 
     GDFT_CK(wgrad(Wd, S.n_out, HL, Wd, GY, S.n_out, dparams + head_off), "hvp dW_out");
     GDFT_CK(csum(GY, np, S.n_out, S.n_out, dparams + head_off + (size_t)Wd * S.n_out), "hvp db_out");
   }
-  GDFT_CK(gemm<kNT>((int)rows2, Wd, S.n_out, GY, S.n_out, Wout, S.n_out, D0, Wd, 0.0, st), "hvp dh_L");
+  GDFT_CK(mul_t(Wd, S.n_out, GY, Wout, D0, Wd, nullptr), "hvp dh_L");
   double *dcur = D0, *dnext = D1;
   for (int i = S.n_layers; i >= 1; --i) {
     const double *Wi = params + hvp_layer_offset(S, i - 1), *gi = Wi + (size_t)Wd * Wd + Wd, *bei = gi + Wd;
@@ -552,8 +562,7 @@ int mlp_hvp_f64(const MlpShape &S, const double *params, double *dparams, const 
       GDFT_CK(csum(dcur, np, Wd, Wd, dWi + (size_t)Wd * Wd), "hvp db_i");
       GDFT_CK(csum(lnpart, kLnBlocks, 2 * Wd, 2 * Wd, dWi + (size_t)Wd * Wd + Wd), "hvp dLN_i");
     }
-    GDFT_CK(cudaMemcpyAsync(dnext, dcur, act2 * sizeof(double), cudaMemcpyDeviceToDevice, st), "hvp residual");
-    GDFT_CK(gemm<kNT>((int)rows2, Wd, Wd, dcur, Wd, Wi, Wd, dnext, Wd, 1.0, st), "hvp dh_i");
+    GDFT_CK(mul_t(Wd, Wd, dcur, Wi, dnext, Wd, dcur), "hvp dh_i");
     double *t = dcur;
     dcur = dnext;
     dnext = t;
@@ -565,7 +574,7 @@ int mlp_hvp_f64(const MlpShape &S, const double *params, double *dparams, const 
     GDFT_CK(csum(dcur, np, Wd, Wd, dparams + (size_t)S.n_in * Wd), "hvp db_0");
   }
   if (coef) {
-    GDFT_CK(gemm<kNT>((int)rows2, S.n_in, Wd, dcur, Wd, W0, Wd, GU, kInPad, 0.0, st), "hvp du");
+    GDFT_CK(mul_t(S.n_in, Wd, dcur, W0, GU, kInPad, nullptr), "hvp du");
     hvp_potentials_kernel<<<pb, 256, 0, st>>>(featp, featt, x, xt, GU, GE, n_grid, np, clip, S.squash_offset, coef);
     GDFT_CK(cudaGetLastError(), "hvp potentials");
   }

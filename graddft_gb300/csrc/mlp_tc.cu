@@ -518,7 +518,7 @@ int run_tc(const MlpShape &S, const double *params, double *dparams, const doubl
     cudaError_t r = launch_tcg(a, ns, st);
     if (r != cudaSuccess) return r;
     const size_t total = (size_t)m_valid * Wd;
-    sum_splits_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(kpart, ns, total, out);
+    sum_splits_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(kpart, ns, total, out, nullptr);
     return cudaGetLastError();
   };
 

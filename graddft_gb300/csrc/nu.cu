@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "fx.cuh"
 #include "mlp_gemm.cuh"
 #include "nu_kernels.cuh"
 
@@ -232,7 +233,7 @@ int make_plan(const gdft_basis *b, PairPlan &plan, const char *who) {
 }
 
 struct NuWs {
-  size_t off_boys, off_pairs, off_pp, off_nu, off_x, bytes;
+  size_t off_boys, off_pairs, off_pp, off_nu, off_x, off_fx, bytes;  // off_fx: scratch of the GEMM X = ao D
 };
 
 NuWs nu_ws(const PairPlan &plan, int n_ao, int64_t chunk, bool want_chi, int n_omega) {
@@ -245,11 +246,13 @@ NuWs nu_ws(const PairPlan &plan, int n_ao, int64_t chunk, bool want_chi, int n_o
   W.off_pp = off;
   off = al256(off + (size_t)n_omega * plan.n_pp * sizeof(double));
   W.off_nu = off;
-  W.off_x = off;
+  W.off_x = W.off_fx = off;
   if (want_chi) {
     off = al256(off + (size_t)n_ao * n_ao * chunk * sizeof(double));
     W.off_x = off;
     off = al256(off + (size_t)2 * chunk * n_ao * sizeof(double));
+    W.off_fx = off;
+    off = al256(off + fx::gemm_rows_bytes(chunk, n_ao, n_ao));
   }
   W.bytes = off;
   return W;
@@ -416,8 +419,9 @@ int gdft_chi(const gdft_basis *basis, const double *d_coords, const double *d_ao
     const int64_t np_ = n_grid - p0 < pc ? n_grid - p0 : pc;
     // X_s = ao[p0 : p0 + np_] D_s, shared by the omegas
     for (int s = 0; s < 2; ++s)
-      if ((rc = check_cuda(gemm<kNN>((int)np_, n, n, d_ao + p0 * n, n, d_rdm1 + (size_t)s * n * n, n,
-                                     X + (size_t)s * pc * n, n, 0.0, st),
+      if ((rc = check_cuda(fx::gemm_rows(np_, n, n, d_ao + p0 * n, n, d_rdm1 + (size_t)s * n * n, n, false,
+                                         X + (size_t)s * pc * n, n, nullptr, (unsigned char *)(ws + W.off_fx), nullptr,
+                                         st),
                            who)))
         return rc;
     for (int w = 0; w < n_omega; ++w) {

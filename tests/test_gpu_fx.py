@@ -130,3 +130,46 @@ def test_not_finite(E, value):
     for k, x in r.density(D).items():
         assert torch.equal(x, clean[k])
     assert torch.equal(r.vxc_from_potentials(pot), vclean)
+
+
+@pytest.mark.parametrize("width", [32, 64, 128, 256])
+@pytest.mark.parametrize("rows", [1, 63, 127, 129, 1000])
+def test_network_layers(E, width, rows):
+    """The coefficient network on given inputs (fx_mat.cu's tall GEMMs, any number of rows) against torch float64.
+
+    A layer's GEMM and its row statistics round at 2^-53 of sums of `width` terms; the sigmoid's input after three
+    layers is of order one, so 1e-13 is some 500 roundings."""
+    import graddft_gb300 as G
+    from graddft_gb300 import synthetic
+    import oracle as O
+
+    f = G.DM21(layer_widths=(width,) * 3)
+    p = synthetic.glorot_params(layer_widths=(width,) * 3, seed=width + rows)
+    x = np.random.default_rng(rows).standard_normal((rows, 11)) * 10.0 ** np.random.default_rng(1).uniform(-8, 2, 11)
+    tp = {"params": {k: {kk: torch.as_tensor(v) for kk, v in d.items()} for k, d in p["params"].items()}}
+    got = f.apply(p, torch.as_tensor(x, device="cuda")).cpu()
+    ref = O.dm21_network(tp, torch.as_tensor(x), n_layers=3)
+    assert got.shape == ref.shape and torch.max(torch.abs(got - ref)) <= 1e-13
+
+
+@pytest.mark.parametrize("n,N", [(1, 1), (13, 65), (64, 128), (65, 129), (130, 1003), (200, 400)])
+def test_exact_exchange(E, n, N):
+    """ehf and the exchange Fock term (fx_mat.cu's two GEMMs) at ragged sizes, element by element as above."""
+    ao, _, _, D, pot = _tables(n, N, 7 * n + N)
+    g = np.random.default_rng(n)
+    chi, w = g.standard_normal((N, 2, 2, n)), pot[:, :2].transpose(1, 0, 2).copy()  # (omega, spin, grid)
+    t = lambda v: torch.as_tensor(v, device="cuda")  # noqa: E731
+    ehf = E.hf_energy_density(t(ao), t(D), t(chi)).cpu().numpy()
+    fock = E.hf_fock(t(ao), t(chi), t(w)).cpu().numpy()
+    for s in range(2):
+        X, aX = ao @ D[s], np.abs(ao) @ np.abs(D[s])
+        lost = 2.0 ** -57 * n * np.abs(ao).max(1)[:, None] * np.abs(D[s]).max(0)[None]
+        for o in range(2):
+            ref = -0.5 * (chi[:, o, s] * X).sum(1)
+            bound = 2 * _dot_bound(aX, chi[:, o, s], 2 * n + 20) + (lost * np.abs(chi[:, o, s])).sum(1) + 1e-300
+            assert np.all(np.abs(ehf[o, s] - ref) <= bound)
+        B = -0.5 * sum(w[o, s][:, None] * chi[:, o, s] for o in range(2))
+        aB = 0.5 * sum(np.abs(w[o, s][:, None] * chi[:, o, s]) for o in range(2))
+        size = np.abs(ao).T @ aB
+        bound = (N + 200) * U * size + N * 2.0 ** -55 * np.abs(ao).max(0)[:, None] * aB.max(0)[None] + 1e-300
+        assert np.all(np.abs(fock[s] - ao.T @ B) <= bound)
