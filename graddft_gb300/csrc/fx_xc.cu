@@ -308,19 +308,30 @@ __global__ void __launch_bounds__(256) fx_vdigits_kernel(const double *__restric
 
 // V[s][a][b] = sum of the phi part's splits at (a, b) and of the kinetic part's
 // at (a, b) or, left of the diagonal tile, (b, a).  part: [split][spin][b][a].
-__global__ void fx_vreduce_kernel(const double *__restrict__ part, int s0, int s1, int n, int rows, int cols,
-                                  double *__restrict__ out, const int *__restrict__ bad) {
+// A block takes one b, 32 a (lanes) and spreads the splits over its eight warps:
+// with few AOs there are hundreds of splits and few elements.
+__global__ void __launch_bounds__(256) fx_vreduce_kernel(const double *__restrict__ part, int s0, int s1, int n,
+                                                         int rows, int cols, double *__restrict__ out,
+                                                         const int *__restrict__ bad) {
   if (*bad != 0) return;
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (size_t)2 * n * n) return;
-  const int s = (int)(i / ((size_t)n * n)), a = (int)((i / n) % n), b = (int)(i % n);
+  __shared__ double sm[8][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int a = blockIdx.x * 32 + lane, b = blockIdx.y, s = blockIdx.z;
   const size_t split = (size_t)2 * rows * cols, spin = (size_t)s * rows * cols;
   double v = 0.0;
-  const double *p = part + spin + (size_t)b * rows + a;
-  for (int k = 0; k < s0; ++k) v += p[(size_t)k * split];
-  p = part + (size_t)s0 * split + spin + (b >= a / kTile * kTile ? (size_t)b * rows + a : (size_t)a * rows + b);
-  for (int k = 0; k < s1; ++k) v += p[(size_t)k * split];
-  out[i] = v;
+  if (a < n) {
+    const double *p = part + spin + (size_t)b * rows + a;
+    for (int k = warp; k < s0; k += 8) v += p[(size_t)k * split];
+    p = part + (size_t)s0 * split + spin + (b >= a / kTile * kTile ? (size_t)b * rows + a : (size_t)a * rows + b);
+    for (int k = warp; k < s1; k += 8) v += p[(size_t)k * split];
+  }
+  sm[warp][lane] = v;
+  __syncthreads();
+  if (warp == 0 && a < n) {
+#pragma unroll
+    for (int w = 1; w < 8; ++w) v += sm[w][lane];
+    out[((size_t)s * n + a) * n + b] = v;
+  }
 }
 
 }  // namespace
@@ -475,9 +486,8 @@ cudaError_t launch_vxc(const double *tab, int64_t np, int ld, int n_ao, const do
     g.err = err;
     if ((e = launch_gemm(g, st)) != cudaSuccess) return e;
   }
-  const size_t total = (size_t)2 * n_ao * n_ao;
   // The first slab, the longest, writes all s0 + s1 splits.
-  fx_vreduce_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(part, w.s0, kin ? w.s1 : 0, n_ao, n_max, w.nb * 64,
+  fx_vreduce_kernel<<<dim3((n_ao + 31) / 32, n_ao, 2), 256, 0, st>>>(part, w.s0, kin ? w.s1 : 0, n_ao, n_max, w.nb * 64,
                                                                      vxc, bad);
   return cudaGetLastError();
 }
