@@ -213,13 +213,14 @@ __device__ __forceinline__ Dual<K> xpow(const Dual<K> &x, double p) {
   return chain(x, pow(x.v, p), p * pow(x.v, p - 1.0));
 }
 // x ** (n/3) with an integer n from CUDA's cube roots (cbrt and rcbrt are
-// within 1 ulp; pow evaluates a logarithm and an exponential): n = -1, -5, 4
-// and 8, the powers of LYP and B88, to within a few ulp (pow for x < 0 or NaN);
-// partial (n/3) f / x (elsewhere than at finite x > 0 the pow form, p x ** (p - 1)).
+// within 1 ulp; pow evaluates a logarithm and an exponential); pow for x < 0 or
+// NaN.  x ** (4/3), the power of the exchange terms: partial (4/3) cbrt(x).
 template <int K>
 __device__ __forceinline__ Dual<K> xpow3(const Dual<K> &x, int n) {
   const double f = xpow3(x.v, n);
-  const double df = x.v > 0.0 && isfinite(f) ? (n / 3.0) * f / x.v : (n / 3.0) * pow(x.v, n / 3.0 - 1.0);
+  const double df = n == 4 && x.v >= 0.0               ? (4.0 / 3.0) * cbrt(x.v)
+                    : x.v > 0.0 && isfinite(f)         ? (n / 3.0) * f / x.v
+                                                       : (n / 3.0) * pow(x.v, n / 3.0 - 1.0);
   return chain(x, f, df);
 }
 // x ** 2 with an integer exponent (jax integer_pow JVP: 2 x).

@@ -2,7 +2,8 @@
 //
 // Each function restates one reference function for a single grid point,
 // keeping its evaluation order, clip and where semantics; it is a template
-// over the scalar type (double for values, Dual<K> for values plus partials).
+// over the scalar type (double for values, Dual<K> for values plus partials),
+// except B88 and LYP, whose partials are written out.
 // Powers of a third come from cube roots (xpow3), within a few ulp of pow, and
 // B88 is evaluated without its logarithms (see b88_x_e).
 // Inputs per point: rho[2], s[2] = |grad rho_sigma|^2, st = |grad rho_a +
@@ -15,12 +16,15 @@ namespace gdft {
 
 constexpr double kPi = 3.14159265358979323846;
 
+// Derivative of xclipmin (jnp.clip's convention at a tie).
+__device__ __forceinline__ double clip_slope(double x, double c) { return x > c ? 1.0 : (x == c ? 0.5 : 0.0); }
+
 // exchange_polarization_correction, functional.py:950-979.
 template <class T>
 __device__ __forceinline__ T exch_pol(const T &e0, const T &e1, const T &r0, const T &r1) {
   const T zeta = (r0 - r1) / (r0 + r1);
   const double den = 2.0 * (pow(2.0, 1.0 / 3.0) - 1.0);
-  const T fz = (xpow(1.0 - zeta, 4.0 / 3.0) + xpow(1.0 + zeta, 4.0 / 3.0) - 2.0) / den;
+  const T fz = (xpow3(1.0 - zeta, 4) + xpow3(1.0 + zeta, 4) - 2.0) / den;
   return e0 + (e1 - e0) * fz;
 }
 
@@ -73,7 +77,7 @@ template <class T>
 __device__ __forceinline__ T lsda_x_e(const T rho_in[2], double clip) {
   const T r0 = xclipmin(rho_in[0], clip);
   const T r1 = xclipmin(rho_in[1], clip);
-  const T s43 = xpow(r0 + r1, 4.0 / 3.0);
+  const T s43 = xpow3(r0 + r1, 4);
   const T e0 = (-3.0 / 4.0 * pow(3.0 / kPi, 1.0 / 3.0)) * s43;
   const T e1 = (-3.0 / 4.0 * pow(6.0 / kPi, 1.0 / 3.0)) * s43;
   return exch_pol(e0, e1, r0, r1);
@@ -86,17 +90,26 @@ __device__ __forceinline__ T lsda_x_e(const T rho_in[2], double clip) {
 // 4/3 log2 rho + 2 log x = log2(g x), the term is beta g x / D with
 // x = g / rho^(4/3): the same function (and the same clips) without the four
 // logarithms and exponentials per spin.
-template <class T>
-__device__ __forceinline__ T b88_x_e(const T rho_in[2], const T s[2], double clip) {
+// Partials by hand, d[0..1] with respect to rho, d[2..3] to s: a spin's term
+// depends on that spin alone, so a dual number over all six variables would
+// carry four zeros through every operation.
+__device__ __forceinline__ double b88_x_e(const double rho_in[2], const double s[2], double clip, double (&d)[4]) {
   const double beta = 0.0042;
-  T out;
+  double out = 0.0;
 #pragma unroll
   for (int sp = 0; sp < 2; ++sp) {
-    const T rho = xclipmin(rho_in[sp], clip);
-    const T g = xsqrt(xclipmin(s[sp], clip));
-    const T x = g / xpow3(xclipmin(rho, clip), 4);
-    const T term = beta * (g * x) / (1.0 + 6.0 * beta * x * xasinh(x));
-    out = sp == 0 ? term : out + term;
+    const double rho = xclipmin(rho_in[sp], clip), sc = xclipmin(s[sp], clip);
+    const double g = sqrt(sc);
+    const double x = g / xpow3(rho, 4);
+    const double as = asinh(x);
+    const double inv = 1.0 / (1.0 + 6.0 * beta * x * as);
+    const double term = beta * (g * x) * inv;
+    // term = beta g x / D; dD/dx = 6 beta (asinh x + x / sqrt(1 + x^2)).
+    const double dx = (beta * g - term * (6.0 * beta * (as + x / sqrt(1.0 + x * x)))) * inv;  // at fixed g
+    const double x_g = x / g;
+    d[sp] = -dx * (-4.0 / 3.0) * x / rho * clip_slope(rho_in[sp], clip);
+    d[2 + sp] = -(dx * x_g + beta * x * inv) * (0.5 / g) * clip_slope(s[sp], clip);
+    out += term;
   }
   return -out;
 }
@@ -156,29 +169,54 @@ __device__ __forceinline__ T vwn_c_e(const T rho_in[2], double clip, unsigned *p
 }
 
 // lyp_c_e, popular_functionals.py:197-269 (original LYP with the Laplacian).
-template <class T>
-__device__ __forceinline__ T lyp_c_e(const T rho_in[2], const T s[2], const T lap[2], double clip) {
+// Partials by hand, d[0..1] with respect to rho, d[2..3] to s, d[4..5] to lap:
+// the terms in s and lap are linear, and what depends on rho alone is shared.
+//   e = -a W (rho + B P),  W = gamma / (1 + d q),  q = rho^(-1/3),
+//   B = 2 b rho^(-5/3) exp(-c q),  P the parenthesis.
+__device__ __forceinline__ double lyp_c_e(const double rho_in[2], const double s[2], const double lap[2], double clip,
+                                          double (&dv)[6]) {
   const double a = 0.04918, b = 0.132, c = 0.2533, d = 0.349;
-  const double CF = (3.0 / 10.0) * pow(3.0 * kPi * kPi, 2.0 / 3.0);
-  const T r0 = xclipmin(rho_in[0], clip);
-  const T r1 = xclipmin(rho_in[1], clip);
-  const T zero = tconst(r0, 0.0);
-  const T t0 = (xwhere(val(r0) > clip, s[0] / r0, zero) - lap[0]) / 8.0;
-  const T t1 = (xwhere(val(r1) > clip, s[1] / r1, zero) - lap[1]) / 8.0;
-  const T rsum = r0 + r1;
-  const bool big = val(rsum) > clip;
-  const T frac = xwhere(big, (xsq(r0) + xsq(r1)) / xsq(rsum), tconst(r0, 1.0));
-  const T gamma = 2.0 * (1.0 - frac);
-  const T rhos_ts = rsum * (t0 + t1);
-  const T rho_t = r0 * t0 + r1 * t1;
-  const T rho_grad2rho = r0 * lap[0] + r1 * lap[1];
-  const T rhom1_3 = xpow3(rsum, -1);
-  const T rho8_3 = xpow3(r0, 8) + xpow3(r1, 8);
-  const T rhom5_3 = xpow3(rsum, -5);
-  const T exp_factor = xwhere(val(rsum) > 0.0, xexp(-c * rhom1_3), zero);
-  const T parenthesis = pow(2.0, 2.0 / 3.0) * CF * rho8_3 - rhos_ts + rho_t / 9.0 + rho_grad2rho / 18.0;
-  const T braket = xwhere(big, 2.0 * b * rhom5_3 * parenthesis * exp_factor, zero);
-  return -a * xwhere(big, gamma / (1.0 + d * rhom1_3) * (rsum + braket), zero);
+  const double CF = (3.0 / 10.0) * pow(3.0 * kPi * kPi, 2.0 / 3.0), K = pow(2.0, 2.0 / 3.0) * CF;
+  const double r[2] = {xclipmin(rho_in[0], clip), xclipmin(rho_in[1], clip)};
+  double t[2], t_r[2], inv[2], r53[2];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const bool on = r[k] > clip;
+    inv[k] = on ? 1.0 / r[k] : 0.0;
+    const double q = on ? s[k] / r[k] : 0.0;
+    t[k] = (q - lap[k]) / 8.0;
+    t_r[k] = on ? -q * inv[k] / 8.0 : 0.0;
+    const double cb = cbrt(r[k]);
+    r53[k] = r[k] * (cb * cb);
+  }
+  const double rho = r[0] + r[1];
+  const bool big = rho > clip;
+  if (!big) {  // every where() takes its other branch (a NaN density too)
+#pragma unroll
+    for (int k = 0; k < 6; ++k) dv[k] = 0.0;
+    return -a * 0.0;
+  }
+  const double irho = 1.0 / rho;
+  const double frac = (r[0] * r[0] + r[1] * r[1]) / (rho * rho);
+  const double gamma = 2.0 * (1.0 - frac);
+  const double q = rcbrt(rho), q_r = q * irho * (-1.0 / 3.0);
+  const double A = 1.0 / (1.0 + d * q), E = exp(-c * q);
+  const double B = 2.0 * b * (q * q * irho) * E;
+  const double B_r = B * (irho * (-5.0 / 3.0) - c * q_r);
+  const double P = K * (r53[0] * r[0] + r53[1] * r[1]) - rho * (t[0] + t[1]) + (r[0] * t[0] + r[1] * t[1]) / 9.0 +
+                   (r[0] * lap[0] + r[1] * lap[1]) / 18.0;
+  const double H = rho + B * P, W = gamma * A;
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const double gamma_r = -4.0 * (r[k] - frac * rho) * (irho * irho);
+    const double lin = r[k] / 9.0 - rho;  // dP/dt_k
+    const double P_r = K * (8.0 / 3.0) * r53[k] - (t[0] + t[1]) + t[k] / 9.0 + lap[k] / 18.0 + lin * t_r[k];
+    const double W_r = gamma_r * A - W * A * d * q_r;
+    dv[k] = -a * (W_r * H + W * (1.0 + B_r * P + B * P_r)) * clip_slope(rho_in[k], clip);
+    dv[2 + k] = -a * W * B * (lin * inv[k] / 8.0);
+    dv[4 + k] = -a * W * B * (r[k] / 18.0 - lin / 8.0);
+  }
+  return -a * (W * H);
 }
 
 // One spin's u^i w^j feature term, 2^(4/3 log rho + i log u + j log w), of
