@@ -78,9 +78,12 @@ __device__ __forceinline__ void digits8(const long long (&f)[8], uint4 (&out)[kD
   }
 }
 
+// Largest exponent field of an operand row: beyond it (2^450, or not finite) the
+// plain kernels take over, which also keeps the products within range.
+constexpr int kMaxField = 1023 + 450;
+
 // v 2^scale as a double, rounded to nearest (halves away from zero), by integer
-// operations: conversions run at the FP64 rate.  Below 2^-1021 the result is 0,
-// from 2^1023 it is infinite.
+// operations: conversions run at the FP64 rate.  Below 2^-1021 the result is 0.
 __device__ __forceinline__ double fixed_to_double(long long v, int scale) {
   const unsigned long long m = v < 0 ? (unsigned long long)(-v) : (unsigned long long)v;
   const int lz = __clzll((long long)m);
@@ -88,7 +91,6 @@ __device__ __forceinline__ double fixed_to_double(long long v, int scale) {
   const unsigned long long r = (n >> 11) + ((n >> 10) & 1);  // 53 bits, may carry to 2^53
   const int e = 63 - lz + scale;                             // exponent of the leading one
   unsigned long long d = ((unsigned long long)(e + 1022) << 52) + r;
-  if (e > 1022) d = 0x7FF0000000000000ull;
   if (e < -1021 || v == 0) d = 0;
   return __longlong_as_double((long long)(d | ((unsigned long long)v & 0x8000000000000000ull)));
 }
@@ -114,7 +116,8 @@ struct GemmArgs {
   double *out;                 // row r, column c of half h (columns 64 h .. of a tile): out + split_stride split
   int64_t ldc;                 //   + plane_stride plane + half_stride h + nt_stride nt + ldc c + r (lanes are rows)
   int64_t half_stride, nt_stride, split_stride, plane_stride;
-  int64_t m_valid, n_valid;    // rows and (kFull) columns written
+  int64_t m_valid, n_valid;    // rows of A and of B (kDensity, kVxc: B's per spin) with values; only their products
+                               // are formed and written, and only their digits need to be there (to a multiple of 8)
   const double *add;           // added to the result, laid out like out (may be out itself), or null
   const int *bad;              // non-zero: an operand is not finite, nothing to do
   int *err;

@@ -17,15 +17,17 @@
 // so a chunk's blocks arrive in five groups.
 //
 // What bounds it: 28 digit pairs take 7,168 clocks a chunk at the dense BF16 rate.
-// Measured with 38,912 rows, K 1,024, N 128 (A read from HBM): 12,400 clocks a
-// chunk, of which the copies' latency takes about 2,000 and the drains 2,300; 49
-// TFLOP/s of FP64 products, where the FP64 pipe gives 1.1.  Error against quadruple
+// Measured with 38,912 rows, K 1,024, N 128 (A read from HBM): 11,300 clocks a
+// chunk (12,400 while the copies were issued in a loop), of which the copies take
+// about 1,500, the drains 1,300 and an item's output 1,200; 54 TFLOP/s of FP64
+// products, where the FP64 pipe gives 1.1.  An item's output costs some 16,000
+// clocks whatever its K.  Error against quadruple
 // precision 4.7e-17 (a sequential FP64 sum: 1.1e-15).
 //
 // Warp roles (384 threads): warp 0 producer (one thread), warp 1 TMEM owner and
 // MMA issuer (one thread), warps 4-11 drains, one per (lane quadrant, 64 columns).
-// A drain thread holds 64 64-bit sums: the two drain warpgroups take 208 registers
-// a thread, the first gives up all but 88 (88 + 2 x 208 = 3 x 168).  Every wait is
+// A drain thread holds 64 64-bit sums: the two drain warpgroups take 216 registers
+// a thread, the first gives up all but 72 (72 + 2 x 216 = 3 x 168).  Every wait is
 // bounded (umma::mbar_wait); on expiry the CTA records an error word, lets its
 // copies and MMAs land and releases TMEM.
 #include "common.cuh"
@@ -121,6 +123,11 @@ __device__ __forceinline__ Item item_of(const GemmArgs &A, int upper, int i) {
   return t;
 }
 
+// Rows of a tile (of `most`) that hold values when `left` are left, to a multiple of 8.
+__device__ __forceinline__ uint32_t valid8(int64_t left, int most) {
+  return left >= most ? (uint32_t)most : (uint32_t)(left + 7) / 8 * 8;
+}
+
 __device__ __forceinline__ void flag(int *err, int code) { atomicCAS(err, 0, code); }
 
 // D (+)= A B^T on BF16 operands, K 16, issued by one thread.  a, b: the low
@@ -159,6 +166,15 @@ __device__ __forceinline__ void add_shifted(long long &sum, int v, int sh, int r
       : "r"(v), "r"(sh), "r"(rsh));
 }
 
+// v 2^e: the conversion, then the exponent field.  e is kept to where the field
+// cannot wrap: products below 2^-1010 come out larger than they are (row exponents
+// are at most 2^kMaxExp, so none is too large).
+__device__ __forceinline__ double scaled(long long v, int e) {
+  const double d = (double)v;
+  const int hi = __double2hiint(d) + (max(e, -1010) << 20);
+  return v == 0 ? 0.0 : __hiloint2double(hi, __double2loint(d));
+}
+
 __global__ void __launch_bounds__(kThreads, 1) fx_gemm_kernel(const GemmArgs A, const int upper) {
   if (A.bad != nullptr && *A.bad != 0) return;
   extern __shared__ unsigned char smem_raw[];
@@ -190,7 +206,7 @@ __global__ void __launch_bounds__(kThreads, 1) fx_gemm_kernel(const GemmArgs A, 
   const uint32_t tbase = tmem_base;
 
   if (warp < 4) {
-  asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
   if (warp == 0) {
     // ------------------------------------------------------------ producer
     if (lane == 0) {
@@ -202,21 +218,41 @@ __global__ void __launch_bounds__(kThreads, 1) fx_gemm_kernel(const GemmArgs A, 
         const int at = A.mode == kDensity ? t.plane * A.m_tiles + t.mt : t.mt;
         const unsigned char *a = A.a + ((size_t)at * A.a_stride + t.base + t.c0) * kSetBytes;
         const unsigned char *b = (t.plane ? A.b1 : A.b) + ((size_t)t.nt * A.b_stride + t.base + t.c0) * kSetBytes;
+        // A block's first rows are its first bytes (128 each): rows without values are not copied.
+        const uint32_t a_bytes = valid8(A.m_valid - (int64_t)t.mt * kTile, kTile) * 128u;
+        const uint32_t b_valid = A.mode == kFull ? valid8(A.n_valid - (int64_t)t.nt * kTile, kTile)
+                                                 : valid8(A.n_valid - (int64_t)t.nt * 64, 64);
+        // Both halves of B in one copy where the first is full.
+        const uint32_t b_bytes = (A.mode == kFull ? b_valid : 2 * b_valid) * 128u;
+        const uint32_t b_first = A.mode != kFull && b_valid < 64 ? b_valid * 128u : b_bytes;
         for (int c = t.c0; c < t.c1 && ok; ++c, a += kSetBytes, b += kSetBytes) {
-#pragma unroll 1
-          for (o = 0; o < kGroups; ++o) {
-            if (!umma::mbar_wait(&empty[o], (chunk & 1) ^ 1)) {
+          // Straight-line code: the issue of a chunk's copies is on the critical path.
+#pragma unroll
+          for (int g = 0; g < kGroups; ++g) {
+            o = g;
+            if (!umma::mbar_wait(&empty[g], (chunk & 1) ^ 1)) {
               flag(A.err, 71);
               ok = false;
               break;
             }
-            umma::mbar_arrive_expect_tx(&full[o], (kGroupAt[o + 1] - kGroupAt[o]) * kBlockBytes);
-            for (int k = kGroupAt[o]; k < kGroupAt[o + 1]; ++k) {
+            uint32_t bytes = 0;
+#pragma unroll
+            for (int k = kGroupAt[g]; k < kGroupAt[g + 1]; ++k) bytes += kGroupOf[k] < kDigits ? a_bytes : b_bytes;
+            umma::mbar_arrive_expect_tx(&full[g], bytes);
+#pragma unroll
+            for (int k = kGroupAt[g]; k < kGroupAt[g + 1]; ++k) {
               const int s = kGroupOf[k];
-              const unsigned char *src = s < kDigits ? a + (size_t)s * kBlockBytes : b + (size_t)(s - kDigits) * kBlockBytes;
-              umma::bulk_g2s(smem + (size_t)s * kBlockBytes, src, kBlockBytes, &full[o]);
+              if (s < kDigits) {
+                umma::bulk_g2s(smem + s * kBlockBytes, a + s * kBlockBytes, a_bytes, &full[g]);
+              } else {
+                umma::bulk_g2s(smem + s * kBlockBytes, b + (s - kDigits) * kBlockBytes, b_first, &full[g]);
+                if (b_first != b_bytes)  // the valid rows of the second half
+                  umma::bulk_g2s(smem + s * kBlockBytes + kBlockBytes / 2,
+                                 b + (s - kDigits) * kBlockBytes + kBlockBytes / 2, b_first, &full[g]);
+              }
             }
           }
+          if (ok) o = kGroups;
           if (ok) ++chunk;
         }
       }
@@ -314,7 +350,7 @@ __global__ void __launch_bounds__(kThreads, 1) fx_gemm_kernel(const GemmArgs A, 
     __syncwarp();
   }
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
     // -------------------------------------------------------------- drains
     const int q = warp & 3, col = ((warp - 4) >> 2) * kCols;
     const uint32_t tl = tbase + ((uint32_t)(q * 32) << 16) + col;
@@ -329,51 +365,60 @@ __global__ void __launch_bounds__(kThreads, 1) fx_gemm_kernel(const GemmArgs A, 
       }
       umma::tc_fence_after();
     };
+    // Columns of accumulator b to `take`; b is free again once the last are in registers.
+    auto drain = [&](int b, int cols, auto &&take) {
+      auto release = [&]() {
+        umma::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) umma::mbar_arrive(&yempty[b]);
+      };
+      if (cols == 0) {
+        release();
+        return;
+      }
+#pragma unroll
+      for (int h = 0; h < kCols; h += 16) {
+        uint32_t y[16];
+        umma::tmem_ld16_nowait(tl + b * 128 + h, y);
+        umma::tmem_ld_wait(y);
+        if (h + 16 == kCols) release();
+#pragma unroll
+        for (int k = 0; k < 16; ++k) take(h + k, y[k]);
+      }
+      __syncwarp();
+    };
     long long sum[kCols];  // orders 0..4 of this thread's row, unit 2^-36 (below 2^59 a chunk)
     for (int i = blockIdx.x; i < items; i += gridDim.x) {
       const Item t = item_of(A, upper, i);
 #pragma unroll
       for (int k = 0; k < kCols; ++k) sum[k] = 0;
       int n = 0;  // chunks in the sums
+      const int *eb = (t.plane ? A.eb1 : A.eb) + (size_t)t.nt * kTile + col;
+      const int eb0 = __ldg(eb + lane), eb1 = __ldg(eb + 32 + lane);  // the columns' exponents, two a lane
+      const int64_t row = (int64_t)t.mt * kTile + q * 32 + lane;
+      // Columns of these 64 that are wanted; none where no row of the warp is.
+      const int64_t left = A.mode == kFull ? A.n_valid - ((int64_t)t.nt * kTile + col) : A.n_valid - (int64_t)t.nt * 64;
+      const int cols = row - lane >= A.m_valid || left <= 0 ? 0 : left < kCols ? (int)left : kCols;
       for (int c = t.c0; c < t.c1; ++c, ++chunk) {
         // Orders 0 and 1 are at most 2^20 and 2^22 units: the integer sits in the mantissa of v + 1.5 2^23 units
-        // (the offsets are taken out below).  The others go through conversions, in one copy of the code:
-        // unrolled, it does not fit the instruction cache.
+        // (the offsets are taken out below).  The others go through conversions, in one copy of the code: the
+        // kernel's loops have to fit the instruction cache.
 #pragma unroll
         for (int d = 0; d < 2; ++d) {
           wait(&yfull[d], (d ? 2 * chunk : 3 * chunk) & 1, 77);
-#pragma unroll
-          for (int h = 0; h < kCols; h += 16) {
-            uint32_t y[16];
-            umma::tmem_ld16_nowait(tl + d * 128 + h, y);
-            umma::tmem_ld_wait(y);
-#pragma unroll
-            for (int k = 0; k < 16; ++k) {
-              const int v = __float_as_int(__uint_as_float(y[k]) + (d ? 24576.0f : 12582912.0f));
-              sum[h + k] += (long long)v << (36 - 9 * d);
-            }
-          }
-          umma::tc_fence_before();
-          __syncwarp();
-          if (lane == 0) umma::mbar_arrive(&yempty[d]);
+          drain(d, cols, [&](int k, uint32_t y) {
+            const int v = __float_as_int(__uint_as_float(y) + (d ? 24576.0f : 12582912.0f));
+            sum[k] += (long long)v << (36 - 9 * d);
+          });
         }
 #pragma unroll 1
         for (int d = 2; d < 5; ++d) {
           const int b = d & 1, sh = 36 - 9 * d;
           const float f = __uint_as_float((uint32_t)(127 + 9 * d) << 23);
           wait(&yfull[b], (b ? 2 * chunk + 1 : 3 * chunk + d / 2) & 1, 77);
-#pragma unroll
-          for (int h = 0; h < kCols; h += 16) {
-            uint32_t y[16];
-            umma::tmem_ld16_nowait(tl + b * 128 + h, y);
-            umma::tmem_ld_wait(y);
-#pragma unroll
-            for (int k = 0; k < 16; ++k)
-              add_shifted(sum[h + k], __float2int_rn(__uint_as_float(y[k]) * f), sh, 32 - sh);
-          }
-          umma::tc_fence_before();
-          __syncwarp();
-          if (lane == 0) umma::mbar_arrive(&yempty[b]);
+          drain(b, cols, [&](int k, uint32_t y) {
+            add_shifted(sum[k], __float2int_rn(__uint_as_float(y) * f), sh, 32 - sh);
+          });
         }
         ++n;
         if (c + 1 < t.c1 && n < kSumChunks) continue;
@@ -384,20 +429,17 @@ __global__ void __launch_bounds__(kThreads, 1) fx_gemm_kernel(const GemmArgs A, 
         const int up_max = 14 - (n > 1 ? 32 - __clz(n - 1) : 0);
         // Offsets of orders 0 and 1: the words of 1.5 2^23 and of 1.5 2^14.
         const long long off = (long long)((unsigned long long)n * ((0x4B400000ull << 36) + (0x46C00000ull << 27)));
-        const int64_t row = (int64_t)t.mt * kTile + q * 32 + lane;
         const bool live = row < A.m_valid;
         const int *ea = A.ea + (size_t)t.plane * A.m_tiles * kTile;
-        const int *eb = (t.plane ? A.eb1 : A.eb) + (size_t)t.nt * kTile + col;
         const int e0 = (live ? ea[row] : 0) - 2 * 1022 - 14 - 36;
         const int64_t at = (int64_t)t.split * A.split_stride + (int64_t)t.plane * A.plane_stride +
                            (col >> 6) * A.half_stride + (int64_t)t.nt * A.nt_stride + (col & 63) * A.ldc + row;
         double *out = A.out + at;
         const double *add = c - t.c0 >= kSumChunks ? out : A.add != nullptr ? A.add + at : nullptr;
-        const int64_t cols = A.mode == kFull ? A.n_valid - ((int64_t)t.nt * kTile + col) : kCols;  // of these 64
         // 16 columns a turn, the sums moved down by 16 after each: unrolled, the code (some 60 KB, run once an
         // item) is fetched at the pace of instruction-cache misses.
 #pragma unroll 1
-        for (int h = 0; h < kCols; h += 16) {
+        for (int h = 0; h < cols; h += 16) {
           uint32_t z5[16], z6[16];
           double v[16];
           __syncwarp();  // per-lane code above, warp-collective loads below
@@ -407,14 +449,19 @@ __global__ void __launch_bounds__(kThreads, 1) fx_gemm_kernel(const GemmArgs A, 
 #pragma unroll
           for (int k = 0; k < 16; ++k) {
             const float z = __uint_as_float(z5[k]) + __uint_as_float(z6[k]);
-            const long long s = sum[k] - off;
-            const int top = (int)(s >> 32);  // up is below 15: the upper word says enough
-            int up = __clz(top ^ (top >> 31)) - 3;
-            up = up < up_max ? up : up_max;
-            up = up > 0 ? up : 0;
+            const long long x = sum[k] - off;
+            const int top = (int)(x >> 32);  // up is below 15: the upper word says enough
+            const int up = max(0, min(up_max, __clz(top ^ (top >> 31)) - 3));
             const float zs = __uint_as_float((uint32_t)(127 + 36 + up) << 23);
-            v[k] = fixed_to_double((s << up) + (long long)__float2int_rn(z * zs), e0 - up + __ldg(eb + h + k));
+            const int e = e0 - up + __shfl_sync(0xffffffffu, h < 32 ? eb0 : eb1, (h & 31) + k);
+            const long long y = (x << up) + (long long)__float2int_rn(z * zs);
+            v[k] = k & 1 ? scaled(y, e) : fixed_to_double(y, e);  // the FP64 pipe takes half of the conversions
             if (!ok) v[k] = __longlong_as_double(0x7FF8000000000000ll);
+          }
+          if (h + 16 >= cols) {  // Z is read
+            umma::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) umma::mbar_arrive(&zempty);
           }
           // Stores apart from the arithmetic: a branch a column would serialise it.
           if (live) {
@@ -434,10 +481,16 @@ __global__ void __launch_bounds__(kThreads, 1) fx_gemm_kernel(const GemmArgs A, 
 #pragma unroll
           for (int k = 0; k < kCols; ++k) sum[k] = k + 16 < kCols ? sum[k + 16 < kCols ? k + 16 : 0] : 0;
         }
+        if (cols <= kCols - 16) {  // turns left out: the sums they would have moved out
+#pragma unroll
+          for (int k = 0; k < kCols; ++k) sum[k] = 0;
+        }
         n = 0;
-        umma::tc_fence_before();
-        __syncwarp();
-        if (lane == 0) umma::mbar_arrive(&zempty);
+        if (cols == 0) {
+          umma::tc_fence_before();
+          __syncwarp();
+          if (lane == 0) umma::mbar_arrive(&zempty);
+        }
       }
     }
   }
@@ -486,7 +539,7 @@ __global__ void __launch_bounds__(256) fx_rows_kernel(const double *__restrict__
   m = max(m, __shfl_xor_sync(0xffffffffu, m, 8));
   m = max(m, __shfl_xor_sync(0xffffffffu, m, 16));
   int emax = exp_field(m);
-  if (emax == 0x7FF) atomicOr(bad, 1);
+  if (emax > kMaxField) atomicOr(bad, 1);
   if (emax < 1) emax = 1;
   if (lane < 8 && in) exps[(size_t)plane * rows + row] = emax;
   unsigned char *base = out + ((size_t)plane * tiles + (size_t)(row / kTile)) * chunks * kSetBytes;

@@ -44,7 +44,7 @@ __global__ void __launch_bounds__(128) fx_short_cols_kernel(const double *__rest
   m = max(m, __shfl_xor_sync(0xffffffffu, m, 8));
   m = max(m, __shfl_xor_sync(0xffffffffu, m, 16));
   int emax = exp_field(m);
-  if (emax == 0x7FF) atomicOr(bad, 1);
+  if (emax > kMaxField) atomicOr(bad, 1);
   if (emax < 1) emax = 1;
   if (lane < 8 && c < cols) exps[c] = emax;
   unsigned char *base = out + (size_t)(c / kTile) * chunks * kSetBytes;
@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(256) fx_tall_cols_kernel(const double *__restr
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int c = blockIdx.y * 32 + lane, chunk = blockIdx.x;
   int emax = c < cols ? exp_field(mx[c]) : 1;
-  if (emax == 0x7FF) atomicOr(bad, 1);
+  if (emax > kMaxField) atomicOr(bad, 1);
   if (emax < 1) emax = 1;
   if (chunk == 0 && warp == 0 && c < cols) exps[c] = emax;
   const int64_t r0 = (int64_t)chunk * kChunkK + warp * 8;

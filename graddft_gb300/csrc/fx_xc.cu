@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(128) fx_rdm1_kernel(const double *__restrict__
   m = max(m, __shfl_xor_sync(0xffffffffu, m, 8));
   m = max(m, __shfl_xor_sync(0xffffffffu, m, 16));
   int emax = exp_field(m);
-  if (emax == 0x7FF) atomicOr(bad, 1);
+  if (emax > kMaxField) atomicOr(bad, 1);
   if (emax < 1) emax = 1;
   if (lane < 8) exps[version * nb * kTile + nt * kTile + rt] = emax;
   unsigned char *base = out + ((size_t)version * nb + nt) * nb * kSetBytes;
@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(256) fx_vmax_kernel(const double *__restrict__
     for (int i = threadIdx.x; i < 2 * kFeat * 128; i += blockDim.x) {
       const int p = i % 128;
       const int h = p < cnt ? hi_of(coef[(size_t)(i / 128) * np + p0 + q0 + p]) : kNone;
-      if (h >= 0x7FF00000) atomicOr(bad, 1);
+      if (h > (kMaxField << 20)) atomicOr(bad, 1);
       (&sc[0][0][0])[i] = h == kNone ? kNone : h - kOneHi;
     }
     __syncthreads();
@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(256) fx_vmax_kernel(const double *__restrict__
         const int phi = hi_of(t[0]), dx = hi_of(t[pe]), dy = hi_of(t[2 * pe]), dz = hi_of(t[3 * pe]),
                   lp = hi_of(t[4 * pe]);
         const int dm = max(dx, max(dy, dz));
-        if (max(phi, max(dm, lp)) >= 0x7FF00000) atomicOr(bad, 1);
+        if (max(phi, max(dm, lp)) > (kMaxField << 20)) atomicOr(bad, 1);
         m[0] = max(m[0], phi);
         m[1] = max(m[1], dm);
 #pragma unroll
@@ -231,7 +231,7 @@ __global__ void fx_vexp_kernel(const int *__restrict__ mx, int n_max, int n_ao, 
 // t npc + pc for plane t.
 __global__ void __launch_bounds__(256) fx_vdigits_kernel(const double *__restrict__ tab, size_t pe, int64_t np, int ld,
                                                          const double *__restrict__ coef, int64_t p0, int64_t rows,
-                                                         int npc, bool kin, int mt, int nb,
+                                                         int npc, bool kin, int mt, int nb, int n8,
                                                          const int *__restrict__ ea, const int *__restrict__ eb,
                                                          unsigned char *__restrict__ va, unsigned char *__restrict__ vb,
                                                          int *__restrict__ bad) {
@@ -256,6 +256,7 @@ __global__ void __launch_bounds__(256) fx_vdigits_kernel(const double *__restric
   }
   bool over = false;
   auto emit = [&](unsigned char *set, int row, const double (&x)[8], int emax) {
+    over = over || emax > kMaxField;
     long long f[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -270,7 +271,7 @@ __global__ void __launch_bounds__(256) fx_vdigits_kernel(const double *__restric
   };
   const int planes = kin ? 4 : 1;
   const size_t chunks = (size_t)planes * npc;
-  if (a < mt * kTile) {
+  if (a < n8) {
     unsigned char *A = va + ((size_t)(a / kTile) * chunks + pc) * kSetBytes;
     emit(A, a % kTile, v[T_PHI], ea[a]);
     if (kin) {
@@ -279,7 +280,7 @@ __global__ void __launch_bounds__(256) fx_vdigits_kernel(const double *__restric
       for (int t = 1; t < 4; ++t) emit(A + (size_t)t * npc * kSetBytes, a % kTile, v[t], e);
     }
   }
-  if (a < nb * 64) {
+  if (a < n8) {
     unsigned char *B = vb + ((size_t)(a / 64) * chunks + pc) * kSetBytes;
 #pragma unroll 1
     for (int s = 0; s < 2; ++s) {
@@ -424,6 +425,7 @@ cudaError_t launch_density(const double *tab, int64_t np, int ld, int n_ao, cons
     g.plane_stride = 2 * g.half_stride;
     g.nt_stride = 64 * g.ldc;
     g.m_valid = rows;
+    g.n_valid = n_ao;
     g.bad = bad;
     g.err = err;
     if ((e = launch_gemm(g, st)) != cudaSuccess) return e;
@@ -458,8 +460,8 @@ cudaError_t launch_vxc(const double *tab, int64_t np, int ld, int n_ao, const do
     fx_vmax_kernel<<<dim3(blocks_a, (unsigned)segs), 256, 0, st>>>(tab, pe, np, ld, coef, p0, rows, (int)per, kin,
                                                                    n_max, mx, bad);
     fx_vexp_kernel<<<(w.nb * kTile + 255) / 256, 256, 0, st>>>(mx, n_max, n_ao, w.mt, w.nb, ea, eb);
-    fx_vdigits_kernel<<<dim3(n_max / 32, npc), 256, 0, st>>>(tab, pe, np, ld, coef, p0, rows, npc, kin, w.mt, w.nb, ea,
-                                                             eb, va, vb, bad);
+    fx_vdigits_kernel<<<dim3(ld / 32, npc), 256, 0, st>>>(tab, pe, np, ld, coef, p0, rows, npc, kin, w.mt, w.nb,
+                                                          (n_ao + 7) / 8 * 8, ea, eb, va, vb, bad);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     GemmArgs g{};
     g.a = va;
@@ -479,7 +481,7 @@ cudaError_t launch_vxc(const double *tab, int64_t np, int ld, int n_ao, const do
     g.split_stride = 2 * g.half_stride;
     g.nt_stride = 64 * g.ldc;
     g.plane_stride = w.s0 * g.split_stride;
-    g.m_valid = n_max;
+    g.m_valid = g.n_valid = n_ao;
     g.out = part;
     g.add = p0 > 0 ? part : nullptr;
     g.bad = bad;

@@ -9,7 +9,7 @@ namespace {
 __device__ __forceinline__ double abs_clip(double x, double t) { return fabs(x) > t ? x : 0.0; }
 
 // Kahan-compensated FP64 sum of the per-block energy partials (functional.py:342):
-// every thread sums its share, then the 1,024 compensated sums are added in a tree
+// every thread sums its share, then the 256 compensated sums are added in a tree
 // of error-free additions (s + e with e the pending error).  The tree replaces one
 // thread's 512 dependent additions, 67 us of every call; now 4 us.
 __device__ __forceinline__ void add_pair(double &s, double &e, double s2, double e2) {
@@ -17,12 +17,12 @@ __device__ __forceinline__ void add_pair(double &s, double &e, double s2, double
   e += e2 + ((s - (t - b)) + (s2 - b));  // TwoSum
   s = t;
 }
-__global__ void __launch_bounds__(1024) energy_reduce_kernel(const double *__restrict__ part, int n,
+__global__ void __launch_bounds__(256) energy_reduce_kernel(const double *__restrict__ part, int n,
                                                             double *__restrict__ out) {
-  __shared__ double hs[32], he[32];
+  __shared__ double hs[8], he[8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   Kahan k{0.0, 0.0};
-  for (int i = threadIdx.x; i < n; i += 1024) k.add(part[i]);
+  for (int i = threadIdx.x; i < n; i += 256) k.add(part[i]);
   double s = k.s, e = -k.c;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1)
@@ -33,10 +33,10 @@ __global__ void __launch_bounds__(1024) energy_reduce_kernel(const double *__res
   }
   __syncthreads();
   if (warp == 0) {
-    s = hs[lane];
-    e = he[lane];
+    s = lane < 8 ? hs[lane] : 0.0;
+    e = lane < 8 ? he[lane] : 0.0;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
+    for (int o = 4; o > 0; o >>= 1)
       add_pair(s, e, __shfl_down_sync(0xffffffffu, s, o), __shfl_down_sync(0xffffffffu, e, o));
     if (lane == 0) out[0] = s + e;
   }
@@ -188,7 +188,7 @@ cudaError_t launch_err_fold(int *dst, int *src, cudaStream_t st) {
 }
 
 cudaError_t launch_energy_reduce(const double *epart, int n, double *exc, cudaStream_t st) {
-  energy_reduce_kernel<<<1, 1024, 0, st>>>(epart, n, exc);
+  energy_reduce_kernel<<<1, 256, 0, st>>>(epart, n, exc);
   return cudaGetLastError();
 }
 
