@@ -25,9 +25,16 @@ namespace gdft {
 
 namespace {
 
-// Points of a block.  One warp: the kernel is bound by the SM's FP64 pipe, so a grid
-// is best spread evenly over the SMs (3,600 points in blocks of 256 use 15 of them).
-constexpr int kBlock = 32;
+// A block takes 32 points (lanes): blocks this small spread a small grid evenly over
+// the SMs (3,600 points in blocks of 256 used 15 of them).  Up to two blocks an SM, a
+// column's dependent operations bound the kernel, and each column has a warp of its
+// own (up to kMaxWarps); beyond that the FP64 pipe does, and warps in different
+// columns only get in each other's way in the instruction cache (B88 + LYP, a warp a
+// column / one warp: 3,600 points 34 / 55 us, 7,500 48 / 60, 10,000 94 / 63, 100,000
+// 504 / 322).
+constexpr int kPoints = 32;
+constexpr int kMaxWarps = 4;
+constexpr int kSplitBlocks = 304;  // two a SM
 
 // Dual variable indices: rho_a, rho_b, |grad rho_a|^2, |grad rho_b|^2, lap_a,
 // lap_b and, for columns that read it (the w powers of the feature columns),
@@ -107,12 +114,57 @@ __device__ __forceinline__ Dual<KV> column(int col, const double rho[2], const d
 }
 
 template <int KV>
-__global__ void __launch_bounds__(kBlock) xc_point_kernel(const double *__restrict__ feat, const double *__restrict__ w,
-                                                          int64_t n_grid, int64_t np, gdft_functional fn,
-                                                          const double *__restrict__ ehf, int n_omega,
-                                                          double *__restrict__ coef, double *__restrict__ epart,
-                                                          double *__restrict__ dens, double *__restrict__ ghf) {
-  const int64_t p = (int64_t)blockIdx.x * kBlock + threadIdx.x;
+__global__ void __launch_bounds__(32 * kMaxWarps) xc_point_kernel(const double *__restrict__ feat,
+                                                                  const double *__restrict__ w, int64_t n_grid,
+                                                                  int64_t np, gdft_functional fn,
+                                                                  const double *__restrict__ ehf, int n_omega,
+                                                                  double *__restrict__ coef, double *__restrict__ epart,
+                                                                  double *__restrict__ dens, double *__restrict__ ghf) {
+  extern __shared__ double cols[];  // [column][1 + KV][point]: value and partials
+  __shared__ unsigned poisoned[kMaxWarps][kPoints];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warps = blockDim.x >> 5;
+  const int64_t p = (int64_t)blockIdx.x * kPoints + lane;
+  const double clip = fn.clip;
+  double f[2][kFeat];
+  unsigned poison = 0;  // spins whose rho gradient is NaN in the reference (see corr_pol)
+  if (p < n_grid) {
+#pragma unroll
+    for (int s = 0; s < 2; ++s)
+#pragma unroll
+      for (int k = 0; k < kFeat; ++k) f[s][k] = feat[((size_t)s * kFeat + k) * np + p];
+    double rho[2], sg[2], lap[2], tau[2];
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      rho[s] = f[s][F_RHO];
+      // jnp.sum(grad_rho**2, axis=-1)
+      sg[s] = (f[s][F_GX] * f[s][F_GX] + f[s][F_GY] * f[s][F_GY]) + f[s][F_GZ] * f[s][F_GZ];
+      lap[s] = f[s][F_LAP];
+      tau[s] = f[s][F_TAU];
+    }
+    double hf = 0.0, hf0 = 0.0, hf1 = 0.0;
+    if (ehf != nullptr) {
+      // ehf layout (omega, spin, grid).
+      for (int o = 0; o < n_omega; ++o) {
+        const double a = ehf[((size_t)o * 2 + 0) * n_grid + p];
+        const double b = ehf[((size_t)o * 2 + 1) * n_grid + p];
+        hf = o == 0 ? (a + b) : hf + (a + b);
+        if (o == 0) hf0 = a + b;
+        if (o == 1) hf1 = a + b;
+      }
+    }
+    for (int i = warp; i < fn.n_cols; i += warps) {
+      const Dual<KV> e = column<KV>(fn.cols[i], rho, sg, lap, tau, hf, hf0, hf1, clip, &poison);
+      if (dens != nullptr) dens[(size_t)p * fn.n_cols + i] = e.v;
+      double *o = cols + (size_t)i * (1 + KV) * kPoints + lane;
+      o[0] = e.v;
+#pragma unroll
+      for (int k = 0; k < KV; ++k) o[(1 + k) * kPoints] = e.d[k];
+    }
+  }
+  poisoned[warp][lane] = poison;
+  __syncthreads();
+  if (warp != 0) return;
   double e_r = 0.0;
   if (p < np) {
     double c[2][kFeat];
@@ -121,45 +173,22 @@ __global__ void __launch_bounds__(kBlock) xc_point_kernel(const double *__restri
 #pragma unroll
       for (int k = 0; k < kFeat; ++k) c[s][k] = 0.0;
     if (p < n_grid) {
-      const double clip = fn.clip;
-      double f[2][kFeat];
-#pragma unroll
-      for (int s = 0; s < 2; ++s)
-#pragma unroll
-        for (int k = 0; k < kFeat; ++k) f[s][k] = feat[((size_t)s * kFeat + k) * np + p];
-      double rho[2], sg[2], lap[2], tau[2];
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        rho[s] = f[s][F_RHO];
-        // jnp.sum(grad_rho**2, axis=-1)
-        sg[s] = (f[s][F_GX] * f[s][F_GX] + f[s][F_GY] * f[s][F_GY]) + f[s][F_GZ] * f[s][F_GZ];
-        lap[s] = f[s][F_LAP];
-        tau[s] = f[s][F_TAU];
-      }
-      double hf = 0.0, hf0 = 0.0, hf1 = 0.0;
-      if (ehf != nullptr) {
-        // ehf layout (omega, spin, grid).
-        for (int o = 0; o < n_omega; ++o) {
-          const double a = ehf[((size_t)o * 2 + 0) * n_grid + p];
-          const double b = ehf[((size_t)o * 2 + 1) * n_grid + p];
-          hf = o == 0 ? (a + b) : hf + (a + b);
-          if (o == 0) hf0 = a + b;
-          if (o == 1) hf1 = a + b;
-        }
-      }
       // Energy density: sum_f c_f * abs_clip(e_f), then abs_clip; weight abs_clip(w).
       Dual<KV> exc = dconst<KV>(0.0);
       double e_raw = 0.0, c_hf = 0.0;  // unclipped columns' sum; coefficient of the HF column
-      unsigned poison = 0;  // spins whose rho gradient is NaN in the reference (see corr_pol)
       for (int i = 0; i < fn.n_cols; ++i) {
-        Dual<KV> e = column<KV>(fn.cols[i], rho, sg, lap, tau, hf, hf0, hf1, clip, &poison);
-        if (dens != nullptr) dens[(size_t)p * fn.n_cols + i] = e.v;
+        const double *o = cols + (size_t)i * (1 + KV) * kPoints + lane;
+        Dual<KV> e;
+        e.v = o[0];
+#pragma unroll
+        for (int k = 0; k < KV; ++k) e.d[k] = o[(1 + k) * kPoints];
         const double ci = fn.n_coeffs == 1 ? fn.coeffs[0] : fn.coeffs[i];
         e_raw += ci * e.v;
         if (fn.cols[i] == GDFT_COL_HF) c_hf += ci;
         if (!(fabs(e.v) > clip)) e = dconst<KV>(0.0);  // abs_clip(densities), functional.py:184
         exc = i == 0 ? ci * e : exc + ci * e;
       }
+      for (int i = 1; i < warps; ++i) poison |= poisoned[i][lane];
       if (!(fabs(exc.v) > clip)) exc = dconst<KV>(0.0);  // functional.py:252 and :342
       const double wr = w[p];
       const double W = fabs(wr) > clip ? wr : 0.0;      // abs_clip(gridweights), functional.py:342
@@ -194,12 +223,12 @@ __global__ void __launch_bounds__(kBlock) xc_point_kernel(const double *__restri
   double v = e_r;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  if (threadIdx.x == 0) epart[blockIdx.x] = v;
+  if (lane == 0) epart[blockIdx.x] = v;
 }
 
 }  // namespace
 
-int xc_point_blocks(int64_t np) { return (int)((np + kBlock - 1) / kBlock); }
+int xc_point_blocks(int64_t np) { return (int)((np + kPoints - 1) / kPoints); }
 
 bool xc_reads_kinetic(const gdft_functional &fn) {
   for (int i = 0; i < fn.n_cols; ++i)
@@ -213,10 +242,12 @@ cudaError_t launch_xc_point(const double *feat, const double *w, int64_t n_grid,
   const int blocks = xc_point_blocks(np);
   bool reads_tau = false;
   for (int i = 0; i < fn.n_cols; ++i) reads_tau |= is_uw_col(fn.cols[i]) && uw_j(fn.cols[i]) != 0;
+  const int warps = blocks > kSplitBlocks ? 1 : fn.n_cols < kMaxWarps ? fn.n_cols : kMaxWarps;
+  const size_t smem = (size_t)fn.n_cols * (1 + (reads_tau ? 8 : 6)) * kPoints * sizeof(double);  // at most 36 KB
   if (reads_tau)
-    xc_point_kernel<8><<<blocks, kBlock, 0, st>>>(feat, w, n_grid, np, fn, ehf, n_omega, coef, epart, dens, ghf);
+    xc_point_kernel<8><<<blocks, 32 * warps, smem, st>>>(feat, w, n_grid, np, fn, ehf, n_omega, coef, epart, dens, ghf);
   else
-    xc_point_kernel<6><<<blocks, kBlock, 0, st>>>(feat, w, n_grid, np, fn, ehf, n_omega, coef, epart, dens, ghf);
+    xc_point_kernel<6><<<blocks, 32 * warps, smem, st>>>(feat, w, n_grid, np, fn, ehf, n_omega, coef, epart, dens, ghf);
   return cudaGetLastError();
 }
 
