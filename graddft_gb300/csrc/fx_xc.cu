@@ -151,6 +151,9 @@ __global__ void __launch_bounds__(256) fx_features_kernel(const double *__restri
 // and below it by less than 1/8 in the mantissa.  kNone: no value (zero).
 constexpr int kNone = -(1 << 30);
 constexpr int kOneHi = 0x3FF00000;
+static_assert((int)T_PHI == (int)C_RHO && (int)T_DX == (int)C_GX && (int)T_DY == (int)C_GY && (int)T_DZ == (int)C_GZ &&
+                  (int)T_LAP == (int)C_LAP,
+              "Q pairs plane p with coefficient p");
 __device__ __forceinline__ int hi_of(double x) {
   const int h = __double2hiint(x) & 0x7FFFFFFF;
   return h ? h : kNone;
@@ -210,51 +213,44 @@ __global__ void __launch_bounds__(256) fx_vmax_kernel(const double *__restrict__
   }
 }
 
-// Maxima -> exponent fields of the operand rows: ea [2][128 mt] (phi, kinetic),
-// eb [2][128 nb] (Q, kinetic; tile rows 64 of each spin).
-__global__ void fx_vexp_kernel(const int *__restrict__ mx, int n_max, int n_ao, int mt, int nb, int *__restrict__ ea,
-                               int *__restrict__ eb) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < mt * kTile) {
-    ea[i] = i < n_ao ? max(1, mx[i] >> 20) : 1;
-    ea[mt * kTile + i] = i < n_ao ? max(1, mx[n_max + i] >> 20) : 1;
-  }
-  if (i < nb * kTile) {
-    const int s = (i % kTile) >> 6, b = i / kTile * 64 + (i & 63);
-    eb[i] = b < n_ao ? field_of(mx[(size_t)(2 + s) * n_max + b], 3) : 1;  // five terms
-    eb[nb * kTile + i] = b < n_ao ? field_of(mx[(size_t)(4 + s) * n_max + b], 0) : 1;
-  }
-}
-
-// Digits of both operands for 64 points (one K chunk) and 32 AOs: warp = eight
-// consecutive points, lane = AO.  A sets [mt][4 npc], B sets [nb][4 npc], chunk
-// t npc + pc for plane t.
-__global__ void __launch_bounds__(256) fx_vdigits_kernel(const double *__restrict__ tab, size_t pe, int64_t np, int ld,
-                                                         const double *__restrict__ coef, int64_t p0, int64_t rows,
-                                                         int npc, bool kin, int mt, int nb, int n8,
-                                                         const int *__restrict__ ea, const int *__restrict__ eb,
-                                                         unsigned char *__restrict__ va, unsigned char *__restrict__ vb,
-                                                         int *__restrict__ bad) {
+// Digits of the operands for 64 points (one K chunk) and 32 AOs: warp = eight
+// consecutive points, lane = AO.  blockIdx.z = 0: A sets [mt][4 npc] (the planes),
+// 1 and 2: B sets [nb][4 npc] of spin 0 and 1 (Q and c_kin d_j phi), chunk t npc + pc
+// for plane t.  One plane's values live at a time (the planes are read again from
+// L1): with all five in registers one block of 168 registers a thread fitted an SM
+// and the kernel ran at 3 TB/s, bound by its latencies (6,800 points x 400 AOs 187 us,
+// now 139: 4.1 TB/s).  The blocks of chunk 0 write
+// the exponent fields of the operand rows: ea [2][128 mt] (phi, kinetic), eb
+// [2][128 nb] (Q, kinetic; tile rows 64 of each spin).
+__global__ void __launch_bounds__(256, 4) fx_vdigits_kernel(const double *__restrict__ tab, size_t pe, int64_t np, int ld,
+                                                            const double *__restrict__ coef, int64_t p0, int64_t rows,
+                                                            int npc, bool kin, int mt, int nb, int n8,
+                                                            const int *__restrict__ mx, int *__restrict__ ea,
+                                                            int *__restrict__ eb, unsigned char *__restrict__ va,
+                                                            unsigned char *__restrict__ vb, int *__restrict__ bad) {
   if (*bad != 0) return;
-  __shared__ double sc[2][kFeat][64];
+  __shared__ double sc[kFeat][64];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int pc = blockIdx.y, a = blockIdx.x * 32 + lane;
+  const int pc = blockIdx.y, a = blockIdx.x * 32 + lane, s = (int)blockIdx.z - 1;
   const int64_t q0 = (int64_t)pc * kChunkK;
-  for (int i = threadIdx.x; i < 2 * kFeat * 64; i += blockDim.x) {
-    const int p = i % 64;
-    (&sc[0][0][0])[i] = q0 + p < rows ? coef[(size_t)(i / 64) * np + p0 + q0 + p] : 0.0;
+  if (s >= 0) {
+    for (int i = threadIdx.x; i < kFeat * 64; i += blockDim.x) {
+      const int p = i % 64;
+      sc[i / 64][p] = q0 + p < rows ? coef[((size_t)s * kFeat + i / 64) * np + p0 + q0 + p] : 0.0;
+    }
+    __syncthreads();
   }
-  __syncthreads();
-  const int k0 = warp * 8;
-  double v[kPlanes][8];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const bool in = a < ld && q0 + k0 + j < rows;
-    const double *t = tab + (size_t)(p0 + q0 + k0 + j) * ld + a;
-#pragma unroll
-    for (int p = 0; p < kPlanes; ++p) v[p][j] = in ? t[(size_t)p * pe] : 0.0;
-  }
+  if (a >= n8) return;  // n8 <= ld
+  const int k0 = warp * 8, n_max = mt * kTile;
+  const int64_t left = rows - q0 - k0;  // points of these eight that there are
+  const double *t0 = tab + (size_t)(p0 + q0 + k0) * ld + a;
+  const size_t chunks = (size_t)(kin ? 4 : 1) * npc;
   bool over = false;
+  auto load = [&](int p, double (&v)[8]) {
+    const double *t = t0 + (size_t)p * pe;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = j < left ? t[(size_t)j * ld] : 0.0;
+  };
   auto emit = [&](unsigned char *set, int row, const double (&x)[8], int emax) {
     over = over || emax > kMaxField;
     long long f[8];
@@ -269,40 +265,46 @@ __global__ void __launch_bounds__(256) fx_vdigits_kernel(const double *__restric
 #pragma unroll
     for (int i = 0; i < kDigits; ++i) *(uint4 *)(o + (size_t)i * kBlockBytes) = d[i];
   };
-  const int planes = kin ? 4 : 1;
-  const size_t chunks = (size_t)planes * npc;
-  if (a < n8) {
+  double v[8];
+  if (s < 0) {
+    const int e0 = max(1, mx[a] >> 20), e1 = max(1, mx[n_max + a] >> 20);
+    if (pc == 0 && warp == 0) {
+      ea[a] = e0;
+      ea[n_max + a] = e1;
+    }
     unsigned char *A = va + ((size_t)(a / kTile) * chunks + pc) * kSetBytes;
-    emit(A, a % kTile, v[T_PHI], ea[a]);
-    if (kin) {
-      const int e = ea[mt * kTile + a];
-#pragma unroll
-      for (int t = 1; t < 4; ++t) emit(A + (size_t)t * npc * kSetBytes, a % kTile, v[t], e);
-    }
-  }
-  if (a < n8) {
-    unsigned char *B = vb + ((size_t)(a / 64) * chunks + pc) * kSetBytes;
 #pragma unroll 1
-    for (int s = 0; s < 2; ++s) {
-      const int row = s * 64 + a % 64;
-      double q[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const double *c = &sc[s][0][k0 + j];
-        q[j] = c[64 * C_RHO] * v[T_PHI][j] + c[64 * C_GX] * v[T_DX][j] + c[64 * C_GY] * v[T_DY][j] +
-               c[64 * C_GZ] * v[T_DZ][j] + c[64 * C_LAP] * v[T_LAP][j];
-      }
-      emit(B, row, q, eb[a / 64 * kTile + row]);
-      if (kin) {
-        const int e = eb[nb * kTile + a / 64 * kTile + row];
-#pragma unroll
-        for (int t = 1; t < 4; ++t) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) q[j] = sc[s][C_KIN][k0 + j] * v[t][j];
-          emit(B + (size_t)t * npc * kSetBytes, row, q, e);
-        }
-      }
+    for (int t = 0; t < (kin ? 4 : 1); ++t) {
+      load(t, v);
+      emit(A + (size_t)t * npc * kSetBytes, a % kTile, v, t ? e1 : e0);
     }
+  } else {
+    const int row = s * 64 + a % 64, at = a / 64 * kTile + row;
+    const int e0 = field_of(mx[(size_t)(2 + s) * n_max + a], 3);  // five terms
+    const int e1 = field_of(mx[(size_t)(4 + s) * n_max + a], 0);
+    if (pc == 0 && warp == 0) {
+      eb[at] = e0;
+      eb[nb * kTile + at] = e1;
+    }
+    unsigned char *B = vb + ((size_t)(a / 64) * chunks + pc) * kSetBytes;
+    double q[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) q[j] = 0.0;
+#pragma unroll 1
+    for (int p = 0; p < kPlanes; ++p) {  // C_RHO phi + C_GX d_x + C_GY d_y + C_GZ d_z + C_LAP lap: same order
+      load(p, v);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) q[j] = fma(sc[p][k0 + j], v[j], q[j]);
+    }
+    emit(B, row, q, e0);
+    if (kin)
+#pragma unroll 1
+      for (int t = 1; t < 4; ++t) {
+        load(t, v);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) q[j] = sc[C_KIN][k0 + j] * v[j];
+        emit(B + (size_t)t * npc * kSetBytes, row, q, e1);
+      }
   }
   if (over) atomicOr(bad, 1);
 }
@@ -459,9 +461,8 @@ cudaError_t launch_vxc(const double *tab, int64_t np, int ld, int n_ao, const do
     segs = (rows + per - 1) / per;
     fx_vmax_kernel<<<dim3(blocks_a, (unsigned)segs), 256, 0, st>>>(tab, pe, np, ld, coef, p0, rows, (int)per, kin,
                                                                    n_max, mx, bad);
-    fx_vexp_kernel<<<(w.nb * kTile + 255) / 256, 256, 0, st>>>(mx, n_max, n_ao, w.mt, w.nb, ea, eb);
-    fx_vdigits_kernel<<<dim3(ld / 32, npc), 256, 0, st>>>(tab, pe, np, ld, coef, p0, rows, npc, kin, w.mt, w.nb,
-                                                          (n_ao + 7) / 8 * 8, ea, eb, va, vb, bad);
+    fx_vdigits_kernel<<<dim3(ld / 32, npc, 3), 256, 0, st>>>(tab, pe, np, ld, coef, p0, rows, npc, kin, w.mt, w.nb,
+                                                             (n_ao + 7) / 8 * 8, mx, ea, eb, va, vb, bad);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     GemmArgs g{};
     g.a = va;
