@@ -19,8 +19,8 @@
 // nograd_* plugin slots make them in the reference (functional.py:176, 203-205).
 //
 // Data layout: activations row-major [np][width] FP64 per layer; every layer's
-// output h_i and pre-normalisation sum z_i stay resident for the backward.
-// GEMMs run on digit products (fx_mat.cu); a row of the hidden width is one warp's work.
+// output h_i and normalised sum stay resident for the backward.  GEMMs run on
+// digit products (fx_mat.cu), the LayerNorm + ELU passes in ln_rows.cu.
 #include <string.h>
 
 #include "common.cuh"
@@ -96,105 +96,6 @@ __global__ void tanh_bias_kernel(double *__restrict__ z, const double *__restric
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   z[i] = tanh(z[i] + b[i % width]);
-}
-
-// z = zW + b + h_prev (stored back into z); a = LayerNorm(z) as flax computes it
-// (var = max(0, E[z^2] - E[z]^2), a = (z - mean) * (rsqrt(var + eps) * scale) + bias);
-// h = elu(a).  One warp per row, PL = width / 32 values per lane.
-template <int PL>
-__global__ void res_ln_elu_fwd_kernel(double *__restrict__ z, const double *__restrict__ b,
-                                      const double *__restrict__ hprev, const double *__restrict__ scale,
-                                      const double *__restrict__ bias, double eps, int64_t rows,
-                                      double *__restrict__ h) {
-  constexpr int W = 32 * PL;
-  const int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (r >= rows) return;
-  double *zr = z + (size_t)r * W;
-  const double *hp = hprev + (size_t)r * W;
-  double v[PL], s1 = 0.0, s2 = 0.0;
-#pragma unroll
-  for (int k = 0; k < PL; ++k) {
-    const int c = lane + 32 * k;
-    v[k] = (zr[c] + b[c]) + hp[c];
-    zr[c] = v[k];
-    s1 += v[k];
-    s2 += v[k] * v[k];
-  }
-  s1 = warp_sum(s1);
-  s2 = warp_sum(s2);
-  const double mean = s1 / W;
-  const double var = fmax(0.0, s2 / W - mean * mean);
-  const double rstd = 1.0 / sqrt(var + eps);
-  double *hr = h + (size_t)r * W;
-#pragma unroll
-  for (int k = 0; k < PL; ++k) {
-    const int c = lane + 32 * k;
-    const double a = (v[k] - mean) * (rstd * scale[c]) + bias[c];
-    hr[c] = a > 0.0 ? a : expm1(a);
-  }
-}
-
-// Backward of res_ln_elu: dh (row) -> dz in place; the LayerNorm parameter
-// gradients accumulate per lane over the rows a warp visits and are summed over
-// the block's warps in warp order into part[block][2][W] (dscale, dbias).
-template <int PL>
-__global__ void __launch_bounds__(256) res_ln_elu_bwd_kernel(double *__restrict__ dh, const double *__restrict__ z,
-                                                             const double *__restrict__ scale,
-                                                             const double *__restrict__ bias, double eps,
-                                                             int64_t rows, double *__restrict__ part) {
-  constexpr int W = 32 * PL;
-  __shared__ double sacc[8][2][W];
-  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double gs[PL], gb[PL];
-#pragma unroll
-  for (int k = 0; k < PL; ++k) gs[k] = gb[k] = 0.0;
-  for (int64_t r = (int64_t)blockIdx.x * 8 + wid; r < rows; r += (int64_t)gridDim.x * 8) {
-    const double *zr = z + (size_t)r * W;
-    double *dr = dh + (size_t)r * W;
-    double zv[PL], s1 = 0.0, s2 = 0.0;
-#pragma unroll
-    for (int k = 0; k < PL; ++k) {
-      zv[k] = zr[lane + 32 * k];
-      s1 += zv[k];
-      s2 += zv[k] * zv[k];
-    }
-    s1 = warp_sum(s1);
-    s2 = warp_sum(s2);
-    const double mean = s1 / W;
-    const double var = fmax(0.0, s2 / W - mean * mean);
-    const double rstd = 1.0 / sqrt(var + eps);
-    double g[PL], xh[PL], m1 = 0.0, m2 = 0.0;
-#pragma unroll
-    for (int k = 0; k < PL; ++k) {
-      const int c = lane + 32 * k;
-      xh[k] = (zv[k] - mean) * rstd;
-      const double a = (zv[k] - mean) * (rstd * scale[c]) + bias[c];
-      const double da = dr[c] * (a > 0.0 ? 1.0 : exp(a));  // elu'(a)
-      gs[k] += da * xh[k];
-      gb[k] += da;
-      g[k] = da * scale[c];
-      m1 += g[k];
-      m2 += g[k] * xh[k];
-    }
-    m1 = warp_sum(m1) / W;
-    m2 = warp_sum(m2) / W;
-#pragma unroll
-    for (int k = 0; k < PL; ++k) dr[lane + 32 * k] = rstd * (g[k] - m1 - xh[k] * m2);
-  }
-#pragma unroll
-  for (int k = 0; k < PL; ++k) {
-    sacc[wid][0][lane + 32 * k] = gs[k];
-    sacc[wid][1][lane + 32 * k] = gb[k];
-  }
-  __syncthreads();
-  double *pb = part + (size_t)blockIdx.x * 2 * W;
-  for (int c = threadIdx.x; c < 2 * W; c += blockDim.x) {
-    const int q = c / W, cc = c % W;
-    double s = 0.0;
-    for (int w8 = 0; w8 < 8; ++w8) s += sacc[w8][q][cc];
-    pb[c] = s;
-  }
 }
 
 // dp0 = dh0 * (1 - h0^2) in place.
@@ -313,32 +214,6 @@ __global__ void dm21_potentials_kernel(const double *__restrict__ feat, const do
     for (int k = 0; k < kFeat; ++k) coef[((size_t)s * kFeat + k) * np + p] = c[s][k];
 }
 
-
-cudaError_t launch_res_ln_elu_fwd(int width, double *z, const double *b, const double *hprev, const double *scale,
-                                  const double *bias, double eps, int64_t rows, double *h, cudaStream_t st) {
-  const unsigned blocks = (unsigned)((rows * 32 + 255) / 256);
-  switch (width) {
-    case 32: res_ln_elu_fwd_kernel<1><<<blocks, 256, 0, st>>>(z, b, hprev, scale, bias, eps, rows, h); break;
-    case 64: res_ln_elu_fwd_kernel<2><<<blocks, 256, 0, st>>>(z, b, hprev, scale, bias, eps, rows, h); break;
-    case 128: res_ln_elu_fwd_kernel<4><<<blocks, 256, 0, st>>>(z, b, hprev, scale, bias, eps, rows, h); break;
-    case 256: res_ln_elu_fwd_kernel<8><<<blocks, 256, 0, st>>>(z, b, hprev, scale, bias, eps, rows, h); break;
-    default: return cudaErrorInvalidValue;
-  }
-  return cudaGetLastError();
-}
-
-cudaError_t launch_res_ln_elu_bwd(int width, double *dh, const double *z, const double *scale, const double *bias,
-                                  double eps, int64_t rows, double *part, cudaStream_t st) {
-  switch (width) {
-    case 32: res_ln_elu_bwd_kernel<1><<<kLnBlocks, 256, 0, st>>>(dh, z, scale, bias, eps, rows, part); break;
-    case 64: res_ln_elu_bwd_kernel<2><<<kLnBlocks, 256, 0, st>>>(dh, z, scale, bias, eps, rows, part); break;
-    case 128: res_ln_elu_bwd_kernel<4><<<kLnBlocks, 256, 0, st>>>(dh, z, scale, bias, eps, rows, part); break;
-    case 256: res_ln_elu_bwd_kernel<8><<<kLnBlocks, 256, 0, st>>>(dh, z, scale, bias, eps, rows, part); break;
-    default: return cudaErrorInvalidValue;
-  }
-  return cudaGetLastError();
-}
-
 }  // namespace
 
 cudaError_t launch_dm21_features(const double *feat, const double *ehf, int64_t n_grid, int64_t np, double clip,
@@ -428,7 +303,8 @@ MlpLayout mlp_layout(const MlpShape &s, int64_t np) {
   L.u = take((size_t)np * kDm21InPad);
   L.e = take((size_t)np * 3);
   L.h = take(act * (s.n_layers + 1));  // h_0 .. h_L
-  L.z = take(act * s.n_layers);        // z_1 .. z_L
+  L.z = take(act * s.n_layers);        // z_1 .. z_L, then their normalised values
+  L.rs = take((size_t)np * s.n_layers);  // 1 / standard deviation of each row
   L.y = take((size_t)np * 3);
   L.dy = take((size_t)np * 3);
   L.de = take((size_t)np * 3);
@@ -436,7 +312,7 @@ MlpLayout mlp_layout(const MlpShape &s, int64_t np) {
   L.d1 = take(act);
   L.du = take((size_t)np * kDm21InPad);
   L.kpart = take((size_t)L.nsplit * s.width * s.width);
-  L.lnpart = take((size_t)kLnBlocks * 2 * s.width);
+  L.lnpart = take((size_t)kLnRowBlocks * 2 * s.width);
   L.colpart = take((size_t)kColBlocks * 2 * s.width);
   L.epart = take((size_t)L.eblocks);
   L.fx = take((mlp_gemm_bytes(s, np) + 7) / 8);
@@ -470,7 +346,8 @@ int net_forward(const MlpShape &S, const double *params, const MlpLayout &L, dou
     const double *hprev = h + (size_t)(i - 1) * act;
     double *hi = h + (size_t)i * act, *zi = z + (size_t)(i - 1) * act;
     if ((rc = check_cuda(mul(Wd, Wd, hprev, Wd, Wi, zi), "mlp dense_i"))) return rc;
-    if ((rc = check_cuda(launch_res_ln_elu_fwd(Wd, zi, bi, hprev, gi, bei, S.ln_eps, np, hi, st), "mlp layernorm")))
+    if ((rc = check_cuda(launch_ln_elu_fwd(Wd, zi, bi, hprev, gi, bei, S.ln_eps, np, hi,
+                                           ws + L.rs + (size_t)(i - 1) * np, st), "mlp layernorm")))
       return rc;
   }
   const double *hL = h + (size_t)S.n_layers * act;
@@ -582,12 +459,12 @@ int mlp_run_f64(const MlpShape &S, const double *params, double *dparams, const 
   for (int i = S.n_layers; i >= 1; --i) {
     const double *Wi = params + layer_off(i - 1), *gi = Wi + (size_t)Wd * Wd + Wd, *bei = gi + Wd;
     const double *hprev = h + (size_t)(i - 1) * act, *zi = z + (size_t)(i - 1) * act;
-    GDFT_CK(launch_res_ln_elu_bwd(Wd, dcur, zi, gi, bei, S.ln_eps, np, lnpart, st), "mlp layernorm bwd");
+    GDFT_CK(launch_ln_elu_bwd(Wd, dcur, zi, ws + L.rs + (size_t)(i - 1) * np, gi, bei, np, lnpart, st), "mlp layernorm bwd");
     if (dparams) {
       double *dWi = dparams + layer_off(i - 1);
       GDFT_CK(weight_grad(Wd, Wd, hprev, Wd, dcur, Wd, dWi), "mlp dW_i");
       GDFT_CK(col_sum(dcur, np, Wd, Wd, dWi + (size_t)Wd * Wd), "mlp db_i");
-      GDFT_CK(col_sum(lnpart, kLnBlocks, 2 * Wd, 2 * Wd, dWi + (size_t)Wd * Wd + Wd), "mlp dLN_i");
+      GDFT_CK(col_sum(lnpart, kLnRowBlocks, 2 * Wd, 2 * Wd, dWi + (size_t)Wd * Wd + Wd), "mlp dLN_i");
     }
     // dh_{i-1} = dz (residual) + dz W_i^T.
     GDFT_CK(mul_t(Wd, Wd, dcur, Wi, dnext, Wd, dcur), "mlp dh_i");

@@ -10,8 +10,10 @@ constexpr int kDm21In = 11;
 // Row stride of the squashed-input matrix u (and of dE/du): padded to 16 doubles.
 constexpr int kDm21InPad = 16;
 constexpr int kDm21Out = 3;
-// Blocks of the LayerNorm backward (per-block parameter-gradient partials).
+// Blocks of the mixed forms' LayerNorm backward (per-block parameter-gradient partials).
 constexpr int kLnBlocks = 592;  // 4 x 148 SMs
+// The same of ln_rows.cu: 3 x 152 SMs, all resident at 168 registers.
+constexpr int kLnRowBlocks = 456;
 // Blocks of the column-sum (bias gradient) first pass.
 constexpr int kColBlocks = 296;
 // Blocks of the head weight-gradient pass of the tensor-core forms (more row
@@ -25,7 +27,7 @@ struct MlpShape {
 
 // Offsets (in doubles) of the network scratch inside its workspace region.
 struct MlpLayout {
-  size_t x, u, e, h, z, y, dy, de, d0, d1, du, kpart, lnpart, colpart, epart, fx, doubles;  // fx: GEMM scratch
+  size_t x, u, e, h, z, rs, y, dy, de, d0, d1, du, kpart, lnpart, colpart, epart, fx, doubles;  // fx: GEMM scratch
   int nsplit;   // split-K factor of the weight-gradient GEMMs
   int eblocks;  // energy partial sums
 };
@@ -64,7 +66,7 @@ cudaError_t launch_dm21_hf_grads_from(const double *x, const double *du, const d
 // Scratch of the second-order pass (offsets in doubles).  Primal and tangent
 // activations are stacked as [2][np][width] so one GEMM serves both.
 struct MlpHvpLayout {
-  size_t featp, x, xt, u, e, et, h, z, y, gy, ge, d0, d1, gu, kpart, lnpart, colpart, lpart, fx, doubles;
+  size_t featp, x, xt, u, e, et, h, z, stat, y, gy, ge, d0, d1, gu, kpart, lnpart, colpart, lpart, fx, doubles;
   int nsplit;
   int eblocks;
 };
@@ -77,6 +79,20 @@ MlpHvpLayout mlp_hvp_layout(const MlpShape &s, int64_t np);
 int mlp_hvp_f64(const MlpShape &S, const double *params, double *dparams, const double *featp, const double *featt,
                 const double *ehf, const double *w, int64_t n_grid, int64_t np, double clip, double *ws,
                 double *lval, double *coef, int *err, cudaStream_t st);
+
+// LayerNorm + ELU passes of the FP64 forms (ln_rows.cu): z (zW + b + h_prev
+// after the call's addition) becomes its normalised value, rs its rows' 1 /
+// standard deviation; the reverse turns dL/dh into dL/dz in place and leaves
+// kLnRowBlocks partials of the parameter gradients.  With tangents, stat is [2][rows].
+cudaError_t launch_ln_elu_fwd(int width, double *z, const double *b, const double *hprev, const double *gam,
+                              const double *bet, double eps, int64_t rows, double *h, double *rs, cudaStream_t st);
+cudaError_t launch_ln_elu_bwd(int width, double *dh, const double *xhat, const double *rs, const double *gam,
+                              const double *bet, int64_t rows, double *part, cudaStream_t st);
+cudaError_t launch_ln_elu_tan_fwd(int width, double *Z, const double *b, const double *Hp, const double *gam,
+                                  const double *bet, double eps, int64_t rows, double *H, double *stat,
+                                  cudaStream_t st);
+cudaError_t launch_ln_elu_tan_bwd(int width, double *D, const double *X, const double *stat, const double *gam,
+                                  const double *bet, int64_t rows, double *part, cudaStream_t st);
 
 // Mixed (TF32x3 tensor-core) form of mlp_run_f64: FP32 activations, FP64 row
 // statistics, head, features and potentials; widths 128 and 256.

@@ -125,58 +125,6 @@ __global__ void tanh_tan_kernel(double *__restrict__ Z, const double *__restrict
   H[act + i] = (1.0 - h * h) * Z[act + i];
 }
 
-// Residual layer, primal and tangent: z = zW + b + h_prev, z~ = z~W + h~_prev
-// (both stored back into Z); a = LayerNorm(z), a~ = gamma * xhat~;
-// h = elu(a), h~ = elu'(a) a~.  One warp per row.
-template <int PL>
-__global__ void res_ln_elu_tan_fwd_kernel(double *__restrict__ Z, const double *__restrict__ b,
-                                          const double *__restrict__ Hp, const double *__restrict__ gam,
-                                          const double *__restrict__ bet, double eps, int64_t rows,
-                                          double *__restrict__ H) {
-  constexpr int W = 32 * PL;
-  const int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (r >= rows) return;
-  const size_t act = (size_t)rows * W;
-  double *z = Z + (size_t)r * W, *zt = Z + act + (size_t)r * W;
-  const double *hp = Hp + (size_t)r * W, *hpt = Hp + act + (size_t)r * W;
-  double v[PL], vt[PL], s1 = 0.0, s2 = 0.0;
-#pragma unroll
-  for (int k = 0; k < PL; ++k) {
-    const int c = lane + 32 * k;
-    v[k] = (z[c] + b[c]) + hp[c];
-    vt[k] = zt[c] + hpt[c];
-    z[c] = v[k];
-    zt[c] = vt[k];
-    s1 += v[k];
-    s2 += v[k] * v[k];
-  }
-  s1 = warp_sum(s1);
-  s2 = warp_sum(s2);
-  const double mean = s1 / W;
-  const double var = fmax(0.0, s2 / W - mean * mean);
-  const double rs = 1.0 / sqrt(var + eps);
-  double m1 = 0.0, m2 = 0.0, xh[PL];
-#pragma unroll
-  for (int k = 0; k < PL; ++k) {
-    xh[k] = (v[k] - mean) * rs;
-    m1 += vt[k];
-    m2 += xh[k] * vt[k];
-  }
-  m1 = warp_sum(m1) / W;
-  m2 = warp_sum(m2) / W;
-  double *h = H + (size_t)r * W, *ht = H + act + (size_t)r * W;
-#pragma unroll
-  for (int k = 0; k < PL; ++k) {
-    const int c = lane + 32 * k;
-    const double a = (v[k] - mean) * (rs * gam[c]) + bet[c];
-    const double at = gam[c] * (rs * (vt[k] - m1 - xh[k] * m2));
-    const double e1 = a > 0.0 ? 1.0 : exp(a);
-    h[c] = a > 0.0 ? a : expm1(a);
-    ht[c] = e1 * at;
-  }
-}
-
 // Head: L_r = m w sum_f (c~_f ec_f + c_f e~'_f) with c = s sigmoid(y/s),
 // c~ = sigmoid' y~; writes G = [dL/dy; dL/dy~], dL/de_0 and dL/de~_0, and
 // block partial sums of L.
@@ -238,96 +186,6 @@ __global__ void __launch_bounds__(256) head_tan_kernel(const double *__restrict_
     v = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0;
     v = warp_sum(v);
     if (threadIdx.x == 0) lpart[blockIdx.x] = v;
-  }
-}
-
-// Reverse of the residual layer: D = [dL/dh; dL/dh~] in, [dL/dz; dL/dz~] out
-// (in place); LayerNorm parameter partials per block:
-// part[block][0][W] = dL/dgamma, part[block][1][W] = dL/dbeta.
-template <int PL>
-__global__ void __launch_bounds__(256) res_ln_elu_tan_bwd_kernel(double *__restrict__ D, const double *__restrict__ Z,
-                                                                 const double *__restrict__ gam,
-                                                                 const double *__restrict__ bet, double eps,
-                                                                 int64_t rows, double *__restrict__ part) {
-  constexpr int W = 32 * PL;
-  __shared__ double sacc[8][2][W];
-  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const size_t act = (size_t)rows * W;
-  double pg[PL], pb[PL];
-#pragma unroll
-  for (int k = 0; k < PL; ++k) pg[k] = pb[k] = 0.0;
-  for (int64_t r = (int64_t)blockIdx.x * 8 + wid; r < rows; r += (int64_t)gridDim.x * 8) {
-    const double *z = Z + (size_t)r * W, *zt = Z + act + (size_t)r * W;
-    double *dh = D + (size_t)r * W, *dht = D + act + (size_t)r * W;
-    double v[PL], vt[PL], s1 = 0.0, s2 = 0.0;
-#pragma unroll
-    for (int k = 0; k < PL; ++k) {
-      v[k] = z[lane + 32 * k];
-      vt[k] = zt[lane + 32 * k];
-      s1 += v[k];
-      s2 += v[k] * v[k];
-    }
-    s1 = warp_sum(s1);
-    s2 = warp_sum(s2);
-    const double mean = s1 / W;
-    const double var = fmax(0.0, s2 / W - mean * mean);
-    const double rs = 1.0 / sqrt(var + eps);
-    double xh[PL], m1 = 0.0, m2 = 0.0;
-#pragma unroll
-    for (int k = 0; k < PL; ++k) {
-      xh[k] = (v[k] - mean) * rs;
-      m1 += vt[k];
-      m2 += xh[k] * vt[k];
-    }
-    m1 = warp_sum(m1) / W;
-    m2 = warp_sum(m2) / W;
-    // g_a, g_a~ -> gp = g_a gamma (primal LN input), gt = g_a~ gamma (tangent).
-    double gp[PL], gt[PL], xht[PL];
-    double sgp = 0.0, sgpx = 0.0, sgt = 0.0, sgtx = 0.0, sgtz = 0.0;
-#pragma unroll
-    for (int k = 0; k < PL; ++k) {
-      const int c = lane + 32 * k;
-      xht[k] = rs * (vt[k] - m1 - xh[k] * m2);
-      const double a = gam[c] * xh[k] + bet[c];
-      const double at = gam[c] * xht[k];
-      const double e1 = a > 0.0 ? 1.0 : exp(a);
-      const double e2 = a > 0.0 ? 0.0 : exp(a);
-      const double gat = dht[c] * e1;
-      const double ga = dh[c] * e1 + dht[c] * at * e2;
-      pg[k] += ga * xh[k] + gat * xht[k];
-      pb[k] += ga;
-      gp[k] = ga * gam[c];
-      gt[k] = gat * gam[c];
-      sgp += gp[k];
-      sgpx += gp[k] * xh[k];
-      sgt += gt[k];
-      sgtx += gt[k] * xh[k];
-      sgtz += gt[k] * vt[k];
-    }
-    const double mgp = warp_sum(sgp) / W, mgpx = warp_sum(sgpx) / W;
-    const double mgt = warp_sum(sgt) / W, mgtx = warp_sum(sgtx) / W, mgtz = warp_sum(sgtz) / W;
-    const double r2 = rs * rs;
-#pragma unroll
-    for (int k = 0; k < PL; ++k) {
-      const int c = lane + 32 * k;
-      const double second =
-          -r2 * (xh[k] * (mgtz - mgt * m1 - 3.0 * m2 * mgtx) + mgtx * (vt[k] - m1) + m2 * (gt[k] - mgt));
-      dh[c] = rs * (gp[k] - mgp - xh[k] * mgpx) + second;
-      dht[c] = rs * (gt[k] - mgt - xh[k] * mgtx);
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < PL; ++k) {
-    sacc[wid][0][lane + 32 * k] = pg[k];
-    sacc[wid][1][lane + 32 * k] = pb[k];
-  }
-  __syncthreads();
-  double *out = part + (size_t)blockIdx.x * 2 * W;
-  for (int c = threadIdx.x; c < 2 * W; c += blockDim.x) {
-    const int q = c / W, cc = c % W;
-    double s = 0.0;
-    for (int w8 = 0; w8 < 8; ++w8) s += sacc[w8][q][cc];
-    out[c] = s;
   }
 }
 
@@ -409,31 +267,6 @@ __global__ void hvp_potentials_kernel(const double *__restrict__ featp, const do
     for (int k = 0; k < kFeat; ++k) coef[((size_t)s * kFeat + k) * np + p] = c[s][k];
 }
 
-cudaError_t launch_tan_fwd(int width, double *Z, const double *b, const double *Hp, const double *gam,
-                           const double *bet, double eps, int64_t rows, double *H, cudaStream_t st) {
-  const unsigned blocks = (unsigned)((rows * 32 + 255) / 256);
-  switch (width) {
-    case 32: res_ln_elu_tan_fwd_kernel<1><<<blocks, 256, 0, st>>>(Z, b, Hp, gam, bet, eps, rows, H); break;
-    case 64: res_ln_elu_tan_fwd_kernel<2><<<blocks, 256, 0, st>>>(Z, b, Hp, gam, bet, eps, rows, H); break;
-    case 128: res_ln_elu_tan_fwd_kernel<4><<<blocks, 256, 0, st>>>(Z, b, Hp, gam, bet, eps, rows, H); break;
-    case 256: res_ln_elu_tan_fwd_kernel<8><<<blocks, 256, 0, st>>>(Z, b, Hp, gam, bet, eps, rows, H); break;
-    default: return cudaErrorInvalidValue;
-  }
-  return cudaGetLastError();
-}
-
-cudaError_t launch_tan_bwd(int width, double *D, const double *Z, const double *gam, const double *bet, double eps,
-                           int64_t rows, double *part, cudaStream_t st) {
-  switch (width) {
-    case 32: res_ln_elu_tan_bwd_kernel<1><<<kLnBlocks, 256, 0, st>>>(D, Z, gam, bet, eps, rows, part); break;
-    case 64: res_ln_elu_tan_bwd_kernel<2><<<kLnBlocks, 256, 0, st>>>(D, Z, gam, bet, eps, rows, part); break;
-    case 128: res_ln_elu_tan_bwd_kernel<4><<<kLnBlocks, 256, 0, st>>>(D, Z, gam, bet, eps, rows, part); break;
-    case 256: res_ln_elu_tan_bwd_kernel<8><<<kLnBlocks, 256, 0, st>>>(D, Z, gam, bet, eps, rows, part); break;
-    default: return cudaErrorInvalidValue;
-  }
-  return cudaGetLastError();
-}
-
 size_t hvp_layer_offset(const MlpShape &S, int i) {
   return (size_t)S.n_in * S.width + S.width + (size_t)i * ((size_t)S.width * S.width + 3 * (size_t)S.width);
 }
@@ -475,7 +308,8 @@ MlpHvpLayout mlp_hvp_layout(const MlpShape &s, int64_t np) {
   L.e = take((size_t)np * 3);
   L.et = take((size_t)np);
   L.h = take(act2 * (s.n_layers + 1));  // [h_i; h~_i], i = 0..L
-  L.z = take(act2 * (s.n_layers + 1));  // [z_i; z~_i], i = 0..L
+  L.z = take(act2 * (s.n_layers + 1));  // [z_i; z~_i], i = 0..L (i > 0: then their normalised values)
+  L.stat = take(2 * (size_t)np * s.n_layers);  // row statistics of the layers (ln_rows.cu)
   L.y = take(2 * (size_t)np * 3);
   L.gy = take(2 * (size_t)np * 3);
   L.ge = take(2 * (size_t)np);
@@ -483,7 +317,7 @@ MlpHvpLayout mlp_hvp_layout(const MlpShape &s, int64_t np) {
   L.d1 = take(act2);
   L.gu = take(2 * (size_t)np * kInPad);
   L.kpart = take((size_t)L.nsplit * s.width * s.width);
-  L.lnpart = take((size_t)kLnBlocks * 2 * s.width);
+  L.lnpart = take((size_t)kLnRowBlocks * 2 * s.width);
   L.colpart = take((size_t)kColBlocks * 2 * s.width);
   L.lpart = take((size_t)L.eblocks);
   L.fx = take((mlp_gemm_bytes(s, 2 * np) + 7) / 8);
@@ -531,7 +365,7 @@ int mlp_hvp_f64(const MlpShape &S, const double *params, double *dparams, const 
                  *bei = gi + Wd;
     double *Hp = H + (size_t)(i - 1) * act2, *Hi = H + (size_t)i * act2, *Zi = Z + (size_t)i * act2;
     GDFT_CK(mul(Wd, Wd, Hp, Wd, Wi, Zi), "hvp dense_i");
-    GDFT_CK(launch_tan_fwd(Wd, Zi, bi, Hp, gi, bei, S.ln_eps, np, Hi, st), "hvp layernorm");
+    GDFT_CK(launch_ln_elu_tan_fwd(Wd, Zi, bi, Hp, gi, bei, S.ln_eps, np, Hi, ws + L.stat + (size_t)(i - 1) * 2 * np, st), "hvp layernorm");
   }
   double *HL = H + (size_t)S.n_layers * act2;
   GDFT_CK(mul(S.n_out, Wd, HL, Wd, Wout, Y), "hvp head");
@@ -555,12 +389,12 @@ int mlp_hvp_f64(const MlpShape &S, const double *params, double *dparams, const 
   for (int i = S.n_layers; i >= 1; --i) {
     const double *Wi = params + hvp_layer_offset(S, i - 1), *gi = Wi + (size_t)Wd * Wd + Wd, *bei = gi + Wd;
     const double *Hp = H + (size_t)(i - 1) * act2, *Zi = Z + (size_t)i * act2;
-    GDFT_CK(launch_tan_bwd(Wd, dcur, Zi, gi, bei, S.ln_eps, np, lnpart, st), "hvp layernorm bwd");
+    GDFT_CK(launch_ln_elu_tan_bwd(Wd, dcur, Zi, ws + L.stat + (size_t)(i - 1) * 2 * np, gi, bei, np, lnpart, st), "hvp layernorm bwd");
     if (dparams) {
       double *dWi = dparams + hvp_layer_offset(S, i - 1);
       GDFT_CK(wgrad(Wd, Wd, Hp, Wd, dcur, Wd, dWi), "hvp dW_i");
       GDFT_CK(csum(dcur, np, Wd, Wd, dWi + (size_t)Wd * Wd), "hvp db_i");
-      GDFT_CK(csum(lnpart, kLnBlocks, 2 * Wd, 2 * Wd, dWi + (size_t)Wd * Wd + Wd), "hvp dLN_i");
+      GDFT_CK(csum(lnpart, kLnRowBlocks, 2 * Wd, 2 * Wd, dWi + (size_t)Wd * Wd + Wd), "hvp dLN_i");
     }
     GDFT_CK(mul_t(Wd, Wd, dcur, Wi, dnext, Wd, dcur), "hvp dh_i");
     double *t = dcur;
