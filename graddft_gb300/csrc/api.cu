@@ -387,8 +387,8 @@ static int run_vxc(const gdft_molecule *mol, const double *coef, double *d_vxc, 
   }
   StageTimer tm(GDFT_STAGE_VXC, st);
   return check_cuda(launch_vxc_q_tc(mol_av(mol), mol_af(mol), coef, mol->n_grid_pad, (int)round_up(mol->n_ao, 128),
-                                    mol->n_ao, (float *)(ws + W.off_q), W.n_vsplit, vpart, d_vxc,
-                                    (int *)(ws + W.off_err), st),
+                                    mol->n_ao, kin, (float *)(ws + W.off_q), vpart, d_vxc, (int *)(ws + W.off_err),
+                                    st),
                     "vxc_q_tc");
 }
 

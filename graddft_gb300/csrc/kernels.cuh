@@ -54,9 +54,8 @@ cudaError_t launch_dens_tc_ragged(const DensMol *mols, int n_mol, void *d_scratc
 // vxc_q.cu: mixed V_xc as Q pre-pass + block-scaled three-slice tensor-core GEMM.
 int vxc_q_splits(int64_t np, int n_ao);
 size_t vxc_q_bytes(int64_t np, int n_ao);
-cudaError_t launch_vxc_q_tc(const float *av, const float *af, const double *coef, int64_t np,
-                            int ldk, int n_ao, float *q, int nsplit, double *vpart, double *vxc, int *err,
-                            cudaStream_t st);
+cudaError_t launch_vxc_q_tc(const float *av, const float *af, const double *coef, int64_t np, int ldk, int n_ao,
+                            bool kin, float *q, double *vpart, double *vxc, int *err, cudaStream_t st);
 
 // kpoint.cu: the doubled real form of a k-point's complex density matrix and gradient.
 cudaError_t launch_kpt_build_m(const double *rdm1c, int K, int k, int n, double wk, double *M, cudaStream_t st);

@@ -463,8 +463,14 @@ __global__ void __launch_bounds__(kThreads, 1) tcg3_kernel(const TcgArgs A) {
   __shared__ uint32_t tmem_base;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int mt = blockIdx.x % A.m_tiles, nt = blockIdx.x / A.m_tiles;
-  const int64_t c0 = (int64_t)blockIdx.y * A.chunks_per_split;
+  int mt = blockIdx.x % A.m_tiles, nt = blockIdx.x / A.m_tiles;
+  if (A.upper > 0) {
+    const int per = A.upper * (A.upper + 1) / 2;
+    int r = blockIdx.x % per;
+    for (mt = 0; r >= A.upper - mt; ++mt) r -= A.upper - mt;
+    nt = (int)(blockIdx.x / per) * A.upper + mt + r;
+  }
+  const int64_t c0 = A.k_first + (int64_t)blockIdx.y * A.chunks_per_split;
   const int64_t c1 = c0 + A.chunks_per_split < A.k_chunks ? c0 + A.chunks_per_split : A.k_chunks;
   const int64_t nst = c1 > c0 ? c1 - c0 : 0;
 
@@ -682,9 +688,11 @@ cudaError_t launch_tcg3(const TcgArgs &a, int nsplit, cudaStream_t st) {
     attr = true;
   }
   if (a.m_tiles <= 0 || a.n_tiles <= 0 || nsplit <= 0 || a.out64 == nullptr || a.out32 != nullptr ||
-      a.k_chunks > a.a_chunks || a.k_chunks > a.b_chunks)
+      a.k_chunks > a.a_chunks || a.k_chunks > a.b_chunks || a.k_first < 0 ||
+      (a.upper > 0 && (a.upper != a.m_tiles || a.n_tiles % a.upper != 0)))
     return cudaErrorInvalidValue;
-  dim3 grid(a.m_tiles * a.n_tiles, nsplit);
+  const int tiles = a.upper > 0 ? a.n_tiles / a.upper * (a.upper * (a.upper + 1) / 2) : a.m_tiles * a.n_tiles;
+  dim3 grid(tiles, nsplit);
   tcg3_kernel<<<grid, kThreads, kSmem3Bytes, st>>>(a);
   return cudaGetLastError();
 }

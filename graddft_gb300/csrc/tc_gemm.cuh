@@ -13,6 +13,11 @@ struct TcgArgs {
   int64_t a_chunks, b_chunks;  // K chunks stored per tile (tile stride)
   int64_t k_chunks;            // K chunks contracted (<= both)
   int64_t chunks_per_split;    // K chunks per blockIdx.y
+  // launch_tcg3 only: the contraction starts at chunk k_first (k_chunks is its
+  // end); with `upper` > 0 only tiles (m, n) with m <= n % upper are formed (B
+  // holds n_tiles / upper operands side by side, each product symmetric).
+  int64_t k_first;
+  int upper;
   float *out32;                // single split: FP32 row-major output, ld ldo
   int ldo;
   double *out64;               // split-K: FP64 partials [split][m_valid][n_valid]

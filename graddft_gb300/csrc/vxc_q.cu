@@ -12,7 +12,11 @@
 // as block-scaled three-slice sets in the AO-major layout of the AO tables; the contraction is then tcg3_kernel with A = the
 // AO-major phi planes (K = 4 planes x grid points), B = Q of both spins
 // (N = 2 x n_ao), split-K over the grid, FP64 partials, and a reduction that
-// also splits the spins.  Both operands' hi slices are quantised per row and
+// also splits the spins.  The three d_j parts are symmetric in (a, b): from two
+// tiles of 128 AOs on only the tiles on and above the diagonal are contracted,
+// in a launch of their own, and the reduction mirrors them (512 AOs x 262,144
+// points: 7.44 -> 5.62 ms); a functional that reads neither the Laplacian nor
+// tau has none.  Both operands' hi slices are quantised per row and
 // 32-point chunk, so each chunk's hi*hi sum is exact in the tensor core's FP32
 // accumulator and only the corrections (below 2^-10 of the terms) meet its
 // truncation.
@@ -25,6 +29,7 @@ namespace gdft {
 
 namespace {
 
+constexpr int kSms = 152;
 constexpr int kBlkF = umma::kBlockBytes / 4;  // floats in one 128 x 32 block
 
 // Double-float values s + c (|c| below an ulp of s, up to rounding).
@@ -74,9 +79,12 @@ __device__ __forceinline__ void df_split3(DF v, umma::Quant u, float &hi, float 
 // quantum needs only the exponent of its largest value: a spin's four plane
 // exponents travel as the bytes of one word (byte max over the thread's two
 // items, then over the four lanes l ^ 8, l ^ 16 that share the row).
+template <bool KIN>
 __global__ void __launch_bounds__(256, 2) build_q_kernel(const float *__restrict__ af,
                                                          const double *__restrict__ coef, int64_t np, int nbt,
                                                          float *__restrict__ q) {
+  constexpr int T = KIN ? 4 : 1;  // planes of Q
+
   __shared__ __align__(16) float sch[2][kFeat][32], scl[2][kFeat][32];  // [spin][coefficient][point] hi, lo
   const int64_t npc = np / 32;
   const int bt = (int)(blockIdx.x / npc);
@@ -100,7 +108,7 @@ __global__ void __launch_bounds__(256, 2) build_q_kernel(const float *__restrict
     for (int h = 0; h < 2; ++h) off[h] = (uint32_t)(64 * g + 32 * h + lane) * 4;  // floats
 #pragma unroll 1
     for (int s = 0; s < 2; ++s) {
-      DF qv[2][4][4];  // [item][plane t][point j]
+      DF qv[2][T][4];  // [item][plane t][point j]
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         // The item's plane values (the second spin re-reads them from L1).
@@ -127,13 +135,13 @@ __global__ void __launch_bounds__(256, 2) build_q_kernel(const float *__restrict
           a = df_add(a, df_mul(ch[32 * C_LAP], cl[32 * C_LAP], th[T_LAP], tl[T_LAP]));
           qv[h][0][j] = df_norm(a);
 #pragma unroll
-          for (int d = 1; d < 4; ++d)
+          for (int d = 1; d < T; ++d)
             qv[h][d][j] = df_norm(df_mul(ch[32 * C_KIN], cl[32 * C_KIN], th[T_PHI + d], tl[T_PHI + d]));
         }
       }
       uint32_t ebw = 0u;  // byte t: exponent field of the largest |Q_t| of the row
 #pragma unroll
-      for (int t = 0; t < 4; ++t) {
+      for (int t = 0; t < T; ++t) {
         float m = 0.0f;
 #pragma unroll
         for (int h = 0; h < 2; ++h)
@@ -144,7 +152,7 @@ __global__ void __launch_bounds__(256, 2) build_q_kernel(const float *__restrict
       ebw = __vmaxu4(ebw, __shfl_xor_sync(0xffffffffu, ebw, 8));
       ebw = __vmaxu4(ebw, __shfl_xor_sync(0xffffffffu, ebw, 16));
 #pragma unroll
-      for (int t = 0; t < 4; ++t) {
+      for (int t = 0; t < T; ++t) {
         const umma::Quant uq = umma::quant_eb((ebw >> (8 * t)) & 0xFFu);
         float *set = q + ((((size_t)s * nbt + bt) * 4 + t) * npc + pc) * 3 * kBlkF;
 #pragma unroll
@@ -163,29 +171,87 @@ __global__ void __launch_bounds__(256, 2) build_q_kernel(const float *__restrict
   }
 }
 
-// V[s][a][b] = sum over splits of part[split][a][s * ldk + b], a, b < n.
-__global__ void vxc_q_reduce_kernel(const double *__restrict__ part, int nsplit, int n, int ldk,
-                                    double *__restrict__ out) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const size_t total = (size_t)2 * n * n;
-  if (i >= total) return;
-  const int s = (int)(i / ((size_t)n * n)), a = (int)((i / n) % n), b = (int)(i % n);
+// The two contractions' tiles and splits: the phi part (all four planes where
+// there is one tile) and the d_j parts' upper tiles.  A CTA fills an SM and all
+// are of equal length, so the splits are the fewest whose last wave leaves less
+// than 3 % of the SMs idle (256 AOs x 131,072 points in one wave each 0.90 ms, in
+// two and four 1.01; 512 x 262,144 in three and two 5.62, in 0.84 of a wave and
+// two 5.87).
+struct Parts {
+  int tiles[2], splits[2];
+  int64_t first[2], end[2];  // K chunks, of 32 points of one plane
+};
+Parts parts_of(int64_t np, int n_ao) {
+  const int nbt = (int)(round_up(n_ao, 128) / 128);
+  const int64_t npc = np / 32;
+  Parts p{};
+  p.tiles[0] = 2 * nbt * nbt;
+  p.end[0] = nbt == 1 ? 4 * npc : npc;
+  p.first[1] = npc;
+  p.tiles[1] = nbt == 1 ? 0 : nbt * (nbt + 1);
+  p.end[1] = 4 * npc;
+  for (int i = 0; i < 2; ++i) {
+    if (p.tiles[i] == 0) continue;
+    const int64_t chunks = p.end[i] - p.first[i];
+    int best = 1;
+    double fill = 0.0;
+    for (int waves = 1; waves <= 4 && fill < 0.97; ++waves) {
+      const int n = waves * kSms / p.tiles[i];
+      const double f = (double)n * p.tiles[i] / (waves * kSms);
+      if (n > 0 && f > fill) {
+        best = n;
+        fill = f;
+      }
+    }
+    p.splits[i] = (int)(best > chunks ? chunks : best);
+  }
+  return p;
+}
+
+// V[s][a][b] = sum over splits of part[split][a][s * ldk + b], a, b < n, and of
+// the same of sym, whose tiles below the diagonal are read mirrored.
+__global__ void __launch_bounds__(256) vxc_q_reduce_kernel(const double *__restrict__ part, int nsplit,
+                                                           const double *__restrict__ sym, int nsym, int n, int ldk,
+                                                           double *__restrict__ out) {
+  __shared__ double m[32][33];
+  const int s = blockIdx.z, a0 = blockIdx.y * 32, b0 = blockIdx.x * 32;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const size_t stride = (size_t)n * 2 * ldk;
-  double acc = 0.0;
-  for (int k = 0; k < nsplit; ++k) acc += part[(size_t)k * stride + (size_t)a * 2 * ldk + (size_t)s * ldk + b];
-  out[i] = acc;
+  const bool mirror = nsym > 0 && a0 / 128 > b0 / 128;
+  if (mirror) {  // sym[b][a] of the block, transposed through shared memory
+#pragma unroll
+    for (int r = ty; r < 32; r += 8) {
+      double acc = 0.0;
+      if (b0 + r < n)
+#pragma unroll 8
+        for (int k = 0; k < nsym; ++k) acc += sym[(size_t)k * stride + (size_t)(b0 + r) * 2 * ldk + (size_t)s * ldk + a0 + tx];
+      m[r][tx] = acc;
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int r = ty; r < 32; r += 8) {
+    const int a = a0 + r, b = b0 + tx;
+    if (a >= n || b >= n) continue;
+    const size_t at = (size_t)a * 2 * ldk + (size_t)s * ldk + b;
+    double acc = 0.0;
+#pragma unroll 8
+    for (int k = 0; k < nsplit; ++k) acc += part[(size_t)k * stride + at];
+    if (mirror)
+      acc += m[tx][r];
+    else
+#pragma unroll 8
+      for (int k = 0; k < nsym; ++k) acc += sym[(size_t)k * stride + at];
+    out[((size_t)s * n + a) * n + b] = acc;
+  }
 }
 
 }  // namespace
 
-// Split-K factor: about four waves of CTAs over the (a tile, b tile of both spins) grid.
+// Partial results of both contractions.
 int vxc_q_splits(int64_t np, int n_ao) {
-  const int nbt = (int)(round_up(n_ao, 128) / 128);
-  const int tiles = nbt * 2 * nbt;
-  const int64_t kch = 4 * (np / 32);
-  int s = (4 * 148 + tiles - 1) / tiles;
-  if (s > kch) s = (int)kch;
-  return s < 1 ? 1 : s;
+  const Parts p = parts_of(np, n_ao);
+  return p.splits[0] + p.splits[1];
 }
 
 size_t vxc_q_bytes(int64_t np, int n_ao) {
@@ -193,28 +259,46 @@ size_t vxc_q_bytes(int64_t np, int n_ao) {
   return (size_t)2 * 4 * np * ldk * 3 * sizeof(float);
 }
 
-cudaError_t launch_vxc_q_tc(const float *av, const float *af, const double *coef, int64_t np,
-                            int ldk, int n_ao, float *q, int nsplit, double *vpart, double *vxc, int *err,
-                            cudaStream_t st) {
+cudaError_t launch_vxc_q_tc(const float *av, const float *af, const double *coef, int64_t np, int ldk, int n_ao,
+                            bool kin, float *q, double *vpart, double *vxc, int *err, cudaStream_t st) {
   const int nbt = ldk / 128;
   const int64_t npc = np / 32;
-  build_q_kernel<<<(unsigned)(nbt * npc), 256, 0, st>>>(af, coef, np, nbt, q);
+  if (kin)
+    build_q_kernel<true><<<(unsigned)(nbt * npc), 256, 0, st>>>(af, coef, np, nbt, q);
+  else
+    build_q_kernel<false><<<(unsigned)(nbt * npc), 256, 0, st>>>(af, coef, np, nbt, q);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  TcgArgs a{};
-  a.a = av;
-  a.b = q;
-  a.m_tiles = nbt;
-  a.n_tiles = 2 * nbt;
-  a.a_chunks = a.b_chunks = a.k_chunks = 4 * npc;
-  a.chunks_per_split = (a.k_chunks + nsplit - 1) / nsplit;
-  a.out64 = vpart;
-  a.m_valid = n_ao;
-  a.n_valid = 2 * ldk;
-  a.err = err;
-  if ((e = launch_tcg3(a, nsplit, st)) != cudaSuccess) return e;
-  const size_t total = (size_t)2 * n_ao * n_ao;
-  vxc_q_reduce_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(vpart, nsplit, n_ao, ldk, vxc);
+  Parts p = parts_of(np, n_ao);
+  if (!kin) {
+    if (p.end[0] > npc) {
+      p.end[0] = npc;
+      if (p.splits[0] > npc) p.splits[0] = (int)npc;
+    }
+    p.splits[1] = 0;
+  }
+  const size_t stride = (size_t)n_ao * 2 * ldk;
+  for (int i = 0; i < 2; ++i) {
+    if (p.splits[i] == 0) continue;
+    TcgArgs a{};
+    a.a = av;
+    a.b = q;
+    a.m_tiles = nbt;
+    a.n_tiles = 2 * nbt;
+    a.a_chunks = a.b_chunks = 4 * npc;
+    a.k_first = p.first[i];
+    a.k_chunks = p.end[i];
+    a.chunks_per_split = (p.end[i] - p.first[i] + p.splits[i] - 1) / p.splits[i];
+    a.upper = i == 1 ? nbt : 0;
+    a.out64 = vpart + (i == 1 ? p.splits[0] * stride : 0);
+    a.m_valid = n_ao;
+    a.n_valid = 2 * ldk;
+    a.err = err;
+    if ((e = launch_tcg3(a, p.splits[i], st)) != cudaSuccess) return e;
+  }
+  const unsigned b = (unsigned)((n_ao + 31) / 32);
+  vxc_q_reduce_kernel<<<dim3(b, b, 2), 256, 0, st>>>(vpart, p.splits[0], vpart + p.splits[0] * stride, p.splits[1],
+                                                     n_ao, ldk, vxc);
   return cudaGetLastError();
 }
 
