@@ -15,12 +15,15 @@
 // exponent omega^2, whose convolution with the product Gaussian is a Gaussian of
 // exponent mu.  R^n_000 = (-2 mu)^n F_n(mu |P - C|^2) and
 //   R^n_(t+1)uv = t R^(n+1)_(t-1)uv + X_PC R^(n+1)_tuv  (likewise in u and v).
-// The Boys function F_n(T) = int_0^1 u^(2n) exp(-T u^2) du comes from a table of
-// F_n on T = 0, 0.1, ..., 60 filled on the device from the positive series
-// F_n(T) = exp(-T) sum_k (2T)^k / ((2n+1)(2n+3)...(2n+2k+1)), a 9-term Taylor
-// expansion about the nearest tabulated T (F_n' = -F_(n+1)) for the highest n,
-// and the downward recursion F_n = (2T F_(n+1) + exp(-T)) / (2n+1); beyond T = 60,
-// F_0 = sqrt(pi/T)/2 and F_(n+1) = (2n+1) F_n / (2T).
+// The Boys function F_n(T) = int_0^1 u^(2n) exp(-T u^2) du comes from a table on
+// T = 0, 1/16, ..., 60 filled on the device (below 16 from the positive series
+// F_n(T) = exp(-T) sum_k (2T)^k / ((2n+1)(2n+3)...(2n+2k+1)), then from F_0 =
+// sqrt(pi/T) erf(sqrt T)/2 by F_(n+1) = ((2n+1) F_n - exp(-T)) / (2T)), an 8-term
+// Taylor expansion about the nearest tabulated T (F_n' = -F_(n+1)) for the
+// highest n, and the downward recursion F_n = (2T F_(n+1) + exp(-T)) / (2n+1);
+// beyond T = 60, F_0 = sqrt(pi/T)/2 and F_(n+1) = (2n+1) F_n / (2T).  Error against
+// quad precision below 60: 0.8 to 1.4 ulp rms for L up to 3 (3.1 to 3.3 with a
+// table of step 0.1 from the series in its natural order).
 //
 // Work layout: one warp per shell pair and 32 grid points (lanes = points), so the
 // shell pair's primitive data (set up once per pair and omega by
@@ -38,28 +41,39 @@ namespace {
 
 using namespace nu_detail;
 
+// One thread per T_i and n: F_n(T_i) to every series that has it as a term.
 __global__ void boys_table_kernel(double *__restrict__ tab) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= kBoysPts * kBoysN) return;
   const int pt = i / kBoysN, n = i % kBoysN;
-  const double T = pt * kBoysStep;
-  double term = 1.0 / (2 * n + 1), sum = term;
-  for (int k = 1; k < 1000; ++k) {
-    term *= 2.0 * T / (2 * n + 2 * k + 1);
-    sum += term;
-    if (term < 1e-18 * sum) break;
+  const double T = pt / kBoysInv;
+  const double e = exp(-T);
+  double c;
+  if (T < 16.0) {
+    // The series from its end, where each step's rounding is damped by the later ones.
+    double sum = 1.0;
+#pragma unroll 4  // the quotients do not wait for one another
+    for (int k = 24 + (int)(2.6 * T); k >= 1; --k) sum = fma(sum, 2.0 * T / (2 * n + 2 * k + 1), 1.0);
+    c = e * sum / (2 * n + 1);
+  } else {  // F_0 from the error function, upwards: exp(-T) is small beside (2k+1) F_k
+    c = 0.5 * sqrt(kPi / T) * erf(sqrt(T));
+    for (int k = 0; k < n; ++k) c = ((2 * k + 1) * c - e) * (0.5 / T);
   }
-  tab[i] = exp(-T) * sum;
+  for (int k = 0; k < kBoysTerms && k <= n; ++k) {
+    if (k > 1) c /= k;
+    if (n - k < kBoysL) tab[((size_t)(n - k) * kBoysPts + pt) * kBoysTerms + k] = c;
+  }
+  if (n == 0) tab[kBoysExp + pt] = e;
 }
 
-// One thread per shell pair: the primitive-pair records.  Besides mu and P,
+// One warp per shell pair, a lane per pair of primitives: their records.  Besides mu and P,
 // a record holds, for every pair of cartesian components (qa, qb) in PySCF's
 // order and every (t, u, v) with t <= ia + ib, u <= ka + kb, v <= ma + mb, the
 // product pref * E^x_t E^y_u E^z_v (pref = (2 pi / p) sqrt(mu / p)): the same for
 // all grid points, so the per-point work is one FMA per term.
 __global__ void nu_pair_setup_kernel(ShellView B, const int32_t *__restrict__ pairs, int n_pairs, double omega,
                                      double *__restrict__ pp, int64_t n_pp) {
-  const int ip = blockIdx.x * blockDim.x + threadIdx.x;
+  const int ip = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (ip >= n_pairs) return;
   const int s1 = pairs[4 * ip], s2 = pairs[4 * ip + 1];
   const int64_t off = pairs[4 * ip + 2];
@@ -69,53 +83,52 @@ __global__ void nu_pair_setup_kernel(ShellView B, const int32_t *__restrict__ pa
   const int len = rec_len(r1.l, r2.l);
   if (off < 0 || off + (int64_t)r1.np * r2.np * len > n_pp) return;
   const double *A = B.centre + 3 * s1, *Bc = B.centre + 3 * s2;
-  for (int i1 = 0; i1 < r1.np; ++i1) {
-    for (int i2 = 0; i2 < r2.np; ++i2) {
-      double *rec = pp + off + ((int64_t)i1 * r2.np + i2) * len;
-      const double a = B.exps[r1.poff + i1], b = B.exps[r2.poff + i2];
-      const double p = a + b, ip2 = 0.5 / p;
-      const double mu = omega == 0.0 ? p : p * omega * omega / (p + omega * omega);
-      const double pref = (2.0 * kPi / p) * sqrt(mu / p);
-      rec[0] = mu;
-      rec[5] = p;
-      double E[3][kETab];
-      for (int d = 0; d < 3; ++d) {
-        const double P = (a * A[d] + b * Bc[d]) / p;
-        rec[2 + d] = P;
-        const double xab = A[d] - Bc[d], xpa = P - A[d], xpb = P - Bc[d];
-        for (int q = 0; q < kETab; ++q) E[d][q] = 0.0;
-        E[d][e_idx(0, 0, 0)] = exp(-a * b / p * xab * xab);
-        for (int i = 0; i < r1.l; ++i)
-          for (int t = 0; t <= i + 1; ++t)
-            E[d][e_idx(i + 1, 0, t)] = (t > 0 ? ip2 * E[d][e_idx(i, 0, t - 1)] : 0.0) + xpa * E[d][e_idx(i, 0, t)] +
-                                       (t + 1 <= i ? (t + 1) * E[d][e_idx(i, 0, t + 1)] : 0.0);
-        for (int j = 0; j < r2.l; ++j)
-          for (int i = 0; i <= r1.l; ++i)
-            for (int t = 0; t <= i + j + 1; ++t)
-              E[d][e_idx(i, j + 1, t)] = (t > 0 ? ip2 * E[d][e_idx(i, j, t - 1)] : 0.0) +
-                                         xpb * E[d][e_idx(i, j, t)] +
-                                         (t + 1 <= i + j ? (t + 1) * E[d][e_idx(i, j, t + 1)] : 0.0);
-      }
-      // screening: a Gaussian product of overlap prefactor below 1e-30 contributes
-      // nothing at double precision to any point's integrals (the Hermite integrals
-      // grow at most like (2 mu)^(L/2), far from closing the gap for l <= 3)
-      rec[1] = E[0][0] * E[1][0] * E[2][0] < kScreen ? 1.0 : 0.0;
-      double *E3 = rec + 8;
-      int idx = 0;
-      for (int ia = r1.l; ia >= 0; --ia)
-        for (int ka = r1.l - ia; ka >= 0; --ka) {
-          const int ma = r1.l - ia - ka;
-          for (int ib = r2.l; ib >= 0; --ib)
-            for (int kb = r2.l - ib; kb >= 0; --kb) {
-              const int mb = r2.l - ib - kb;
-              for (int t = 0; t <= ia + ib; ++t)
-                for (int u = 0; u <= ka + kb; ++u)
-                  for (int v = 0; v <= ma + mb; ++v)
-                    if (idx < len - 8)
-                      E3[idx++] = pref * E[0][e_idx(ia, ib, t)] * E[1][e_idx(ka, kb, u)] * E[2][e_idx(ma, mb, v)];
-            }
-        }
+  for (int64_t ij = threadIdx.x & 31; ij < (int64_t)r1.np * r2.np; ij += 32) {
+    const int i1 = (int)(ij / r2.np), i2 = (int)(ij % r2.np);
+    double *rec = pp + off + ij * len;
+    const double a = B.exps[r1.poff + i1], b = B.exps[r2.poff + i2];
+    const double p = a + b, ip2 = 0.5 / p;
+    const double mu = omega == 0.0 ? p : p * omega * omega / (p + omega * omega);
+    const double pref = (2.0 * kPi / p) * sqrt(mu / p);
+    rec[0] = mu;
+    rec[5] = p;
+    double E[3][kETab];
+    for (int d = 0; d < 3; ++d) {
+      const double P = (a * A[d] + b * Bc[d]) / p;
+      rec[2 + d] = P;
+      const double xab = A[d] - Bc[d], xpa = P - A[d], xpb = P - Bc[d];
+      for (int q = 0; q < kETab; ++q) E[d][q] = 0.0;
+      E[d][e_idx(0, 0, 0)] = exp(-a * b / p * xab * xab);
+      for (int i = 0; i < r1.l; ++i)
+        for (int t = 0; t <= i + 1; ++t)
+          E[d][e_idx(i + 1, 0, t)] = (t > 0 ? ip2 * E[d][e_idx(i, 0, t - 1)] : 0.0) + xpa * E[d][e_idx(i, 0, t)] +
+                                     (t + 1 <= i ? (t + 1) * E[d][e_idx(i, 0, t + 1)] : 0.0);
+      for (int j = 0; j < r2.l; ++j)
+        for (int i = 0; i <= r1.l; ++i)
+          for (int t = 0; t <= i + j + 1; ++t)
+            E[d][e_idx(i, j + 1, t)] = (t > 0 ? ip2 * E[d][e_idx(i, j, t - 1)] : 0.0) +
+                                       xpb * E[d][e_idx(i, j, t)] +
+                                       (t + 1 <= i + j ? (t + 1) * E[d][e_idx(i, j, t + 1)] : 0.0);
     }
+    // screening: a Gaussian product of overlap prefactor below 1e-30 contributes
+    // nothing at double precision to any point's integrals (the Hermite integrals
+    // grow at most like (2 mu)^(L/2), far from closing the gap for l <= 3)
+    rec[1] = E[0][0] * E[1][0] * E[2][0] < kScreen ? 1.0 : 0.0;
+    double *E3 = rec + 8;
+    int idx = 0;
+    for (int ia = r1.l; ia >= 0; --ia)
+      for (int ka = r1.l - ia; ka >= 0; --ka) {
+        const int ma = r1.l - ia - ka;
+        for (int ib = r2.l; ib >= 0; --ib)
+          for (int kb = r2.l - ib; kb >= 0; --kb) {
+            const int mb = r2.l - ib - kb;
+            for (int t = 0; t <= ia + ib; ++t)
+              for (int u = 0; u <= ka + kb; ++u)
+                for (int v = 0; v <= ma + mb; ++v)
+                  if (idx < len - 8)
+                    E3[idx++] = pref * E[0][e_idx(ia, ib, t)] * E[1][e_idx(ka, kb, u)] * E[2][e_idx(ma, mb, v)];
+          }
+      }
   }
 }
 
@@ -240,7 +253,7 @@ NuWs nu_ws(const PairPlan &plan, int n_ao, int64_t chunk, bool want_chi, int n_o
   NuWs W;
   size_t off = 0;
   W.off_boys = off;
-  off = al256(off + (size_t)kBoysPts * kBoysN * sizeof(double));
+  off = al256(off + kBoysLen * sizeof(double));
   W.off_pairs = off;
   off = al256(off + plan.pairs.size() * sizeof(int32_t));
   W.off_pp = off;
@@ -309,7 +322,7 @@ int setup_nu(const ShellView &B, const PairPlan &plan, const NuWs &W, char *ws, 
              const char *who, cudaStream_t st) {
   int rc;
   if (first) {
-    boys_table_kernel<<<(kBoysPts * kBoysN + 255) / 256, 256, 0, st>>>((double *)(ws + W.off_boys));
+    boys_table_kernel<<<(kBoysPts * kBoysN + 31) / 32, 32, 0, st>>>((double *)(ws + W.off_boys));
     if ((rc = check_cuda(cudaGetLastError(), who))) return rc;
     if ((rc = check_cuda(cudaMemcpyAsync(ws + W.off_pairs, plan.pairs.data(), plan.pairs.size() * sizeof(int32_t),
                                          cudaMemcpyHostToDevice, st),
@@ -317,7 +330,7 @@ int setup_nu(const ShellView &B, const PairPlan &plan, const NuWs &W, char *ws, 
       return rc;
   }
   const int np = (int)(plan.pairs.size() / 4);
-  nu_pair_setup_kernel<<<(np + 127) / 128, 128, 0, st>>>(
+  nu_pair_setup_kernel<<<(np + 3) / 4, 128, 0, st>>>(
       B, (const int32_t *)(ws + W.off_pairs), np, omega,
       (double *)(ws + W.off_pp) + (size_t)w * plan.n_pp, plan.n_pp);
   return check_cuda(cudaGetLastError(), who);

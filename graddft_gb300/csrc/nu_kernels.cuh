@@ -11,10 +11,15 @@ namespace nu_detail {
 
 constexpr int kNuMaxL = 3;                 // shells up to f
 constexpr int kMaxOmega = 8;               // omegas of one gdft_chi call
-constexpr int kBoysN = 17;                 // F_0 .. F_16 tabulated
-constexpr int kBoysPts = 601;              // T = 0, 0.1, ..., 60
-constexpr double kBoysStep = 0.1;
-constexpr double kBoysTMax = 60.0;
+// Boys table: for each L <= 2 kNuMaxL and each T_i = 0, 1/16, ..., 60 the eight
+// Taylor coefficients F_(L+k)(T_i) / k!, then exp(-T_i).
+constexpr int kBoysTerms = 8;
+constexpr int kBoysL = 2 * kNuMaxL + 1;
+constexpr int kBoysN = kBoysL - 1 + kBoysTerms;  // F_0 .. F_13 are tabulated
+constexpr int kBoysPts = 961;
+constexpr double kBoysInv = 16.0;                // 1 / step
+constexpr size_t kBoysExp = (size_t)kBoysL * kBoysPts * kBoysTerms;  // offset of the exponentials
+constexpr size_t kBoysLen = kBoysExp + kBoysPts;
 constexpr int kETab = 4 * 4 * 7;           // E[i][j][t], i, j <= 3, t <= 6 (per dimension)
 
 // Hermite products pref * E^x_t E^y_u E^z_v of a primitive pair of angular momenta
@@ -32,30 +37,51 @@ __host__ __device__ constexpr int rec_len(int la, int lb) { return 8 + nprod(la,
 constexpr double kPi = 3.14159265358979323846;
 constexpr double kScreen = 1e-30;          // product-overlap prefactor below which a primitive pair is skipped
 
-// F_0 .. F_L at T.
+// F_0 .. F_L at T >= 0.  The pair kernels are bound by the FP64 pipe, so the
+// count of operations decides: with the coefficients tabulated as the series
+// needs them F_L takes 7 (8 terms; the next is below 2^-58 of F_L), and so does
+// F_0 where it is the only other one; from L = 2 on the downward recursion needs
+// exp(-T) = exp(-T_i) exp(T_i - T), 8 more.  Beyond 60, one reciprocal root.
 template <int L>
 __device__ __forceinline__ void boys(const double *__restrict__ tab, double T, double F[L + 1]) {
-  if (T < kBoysTMax) {
-    const int i = (int)(T * (1.0 / kBoysStep) + 0.5);
-    const double md = i * kBoysStep - T;  // -(T - T_i)
-    const double *row = tab + i * kBoysN + L;
-    // sum_k F_(L+k)(T_i) (-(T - T_i))^k / k!, Horner from k = 8
-    constexpr double inv_fact[9] = {1.0, 1.0, 1.0 / 2, 1.0 / 6, 1.0 / 24, 1.0 / 120, 1.0 / 720, 1.0 / 5040,
-                                    1.0 / 40320};
-    double acc = row[8] * inv_fact[8];
+  const unsigned top = (unsigned)__double2hiint(T);
+  if (top < 0x404E0000u) {  // T < 60
+    constexpr double kMagic = 6755399441055744.0;   // 1.5 2^52: the sum's low word is the rounded integer
+    const double s = fma(T, kBoysInv, kMagic);
+    const int i = __double2loint(s);
+    const double md = fma(s - kMagic, 1.0 / kBoysInv, -T);  // T_i - T
+    auto series = [&](int l) {
+      const double2 *row = (const double2 *)(tab + ((size_t)l * kBoysPts + i) * kBoysTerms);
+      double acc = 0.0;
 #pragma unroll
-    for (int k = 7; k >= 0; --k) acc = fma(acc, md, row[k] * inv_fact[k]);
-    F[L] = acc;
-    if (L > 0) {
-      const double e = exp(-T);
+      for (int k = kBoysTerms / 2 - 1; k >= 0; --k) {
+        const double2 c = __ldg(row + k);
+        acc = k == kBoysTerms / 2 - 1 ? c.y : fma(acc, md, c.y);
+        acc = fma(acc, md, c.x);
+      }
+      return acc;
+    };
+    F[L] = series(L);
+    if (L == 1) F[0] = series(0);
+    if (L > 1) {
+      double e = 1.0 / 5040;
+      constexpr double inv_fact[7] = {1.0, 1.0, 1.0 / 2, 1.0 / 6, 1.0 / 24, 1.0 / 120, 1.0 / 720};
 #pragma unroll
-      for (int n = L - 1; n >= 0; --n) F[n] = fma(2.0 * T, F[n + 1], e) * (1.0 / (2 * n + 1));
+      for (int k = 6; k >= 0; --k) e = fma(e, md, inv_fact[k]);
+      e *= __ldg(tab + kBoysExp + i);
+      const double T2 = T + T;
+#pragma unroll
+      for (int n = L - 1; n >= 0; --n) F[n] = fma(T2, F[n + 1], e) * (1.0 / (2 * n + 1));
     }
   } else {
-    F[0] = 0.5 * sqrt(kPi / T);
-    const double h = 0.5 / T;
+    const double y = rsqrt(T);
+    F[0] = 0.88622692545275801365 * y;  // sqrt(pi) / 2
+    if (L > 0) {
+      double h = 0.5 * y * y;
+      if (top < 0x7FD00000u) h = fma(h, fma(-2.0 * T, h, 1.0), h);  // 1 / (2 T); past 2^1022, 0 as it is
 #pragma unroll
-    for (int n = 0; n < L; ++n) F[n + 1] = F[n] * ((2 * n + 1) * h);
+      for (int n = 0; n < L; ++n) F[n + 1] = F[n] * ((2 * n + 1) * h);
+    }
   }
 }
 
@@ -86,15 +112,12 @@ struct CartPow {
   static __device__ __forceinline__ constexpr int z(int q) { return L - x(q) - y(q); }
 };
 
-// Hermite Coulomb integrals R^0_tuv, t + u + v <= L.
+// Hermite Coulomb integrals R^0_tuv, t + u + v <= L, from G_n = c (-2 mu)^n F_n (times c).
 template <int L>
-__device__ __forceinline__ void hermite_r(const double F[L + 1], double mu, double X, double Y, double Z,
+__device__ __forceinline__ void hermite_r(const double G[L + 1], double X, double Y, double Z,
                                           double R[L + 1][L + 1][L + 1]) {
   double nxt[L + 1][L + 1][L + 1];
-  double m2 = 1.0;
-#pragma unroll
-  for (int n = 0; n < L; ++n) m2 *= -2.0 * mu;
-  nxt[0][0][0] = m2 * F[L];
+  nxt[0][0][0] = G[L];
 #pragma unroll
   for (int n = L - 1; n >= 0; --n) {
     double cur[L + 1][L + 1][L + 1];
@@ -113,12 +136,8 @@ __device__ __forceinline__ void hermite_r(const double F[L + 1], double mu, doub
             val = (u > 1 ? (u - 1) * nxt[0][u > 1 ? u - 2 : 0][v] : 0.0) + Y * nxt[0][u - 1][v];
           else if (v > 0)
             val = (v > 1 ? (v - 1) * nxt[0][0][v > 1 ? v - 2 : 0] : 0.0) + Z * nxt[0][0][v - 1];
-          else {
-            double m = 1.0;
-#pragma unroll
-            for (int k = 0; k < n; ++k) m *= -2.0 * mu;
-            val = m * F[n];
-          }
+          else
+            val = G[n];
           cur[t][u][v] = val;
         }
 #pragma unroll
@@ -144,7 +163,13 @@ struct NuOut {
   int n;
 };
 
-// One warp per shell pair of class (LA, LB), lanes = 32 points from p0.
+// One warp per shell pair of class (LA, LB), lanes = 32 points from p0.  Bound by
+// the FP64 pipe: 22 operations a primitive pair and point for s-s, 39 for p-s, 525
+// for d-d (336 of them the Hermite sums).  115 AOs x 4,096 points, 4 + 3 + 2
+// primitives: s-s 841 -> 522 us, p-s 1,649 -> 1,001, p-p 890 -> 650, d-s 1,182 -> 870,
+// d-p 1,499 -> 1,221, d-d 915 -> 819 (with a Boys function of twice the operations
+// and the contraction coefficient at each component sum).  Leaving out the zeros
+// of the angular rows at the end gained nothing.
 template <int LA, int LB>
 __global__ void __launch_bounds__(256) nu_kernel(ShellView B, const int32_t *__restrict__ pairs, int pair_lo,
                                                  int pair_hi, const double *__restrict__ pp, int64_t n_pp,
@@ -189,8 +214,17 @@ __global__ void __launch_bounds__(256) nu_kernel(ShellView B, const int32_t *__r
           const double X = rec[2] - Cx, Y = rec[3] - Cy, Z = rec[4] - Cz;
           double F[L + 1];
           boys<L>(boys_tab, mu * (X * X + Y * Y + Z * Z), F);
+          // The contraction coefficient goes into the L + 1 Boys values, so that the
+          // component sums below are the contraction's own.
+          double f = cc;
+          F[0] *= f;
+#pragma unroll
+          for (int n = 1; n <= L; ++n) {
+            f *= -2.0 * mu;
+            F[n] *= f;
+          }
           double R[L + 1][L + 1][L + 1];
-          hermite_r<L>(F, mu, X, Y, Z, R);
+          hermite_r<L>(F, X, Y, Z, R);
           const double *E3 = rec + 8;
           int idx = 0;
 #pragma unroll
@@ -199,7 +233,6 @@ __global__ void __launch_bounds__(256) nu_kernel(ShellView B, const int32_t *__r
 #pragma unroll
             for (int qb = 0; qb < NB; ++qb) {
               const int ib = CartPow<LB>::x(qb), kb = CartPow<LB>::y(qb), mb = CartPow<LB>::z(qb);
-              double s = 0.0;
 #pragma unroll
               for (int t = 0; t <= L; ++t) {
                 if (t > ia + ib) continue;
@@ -209,12 +242,11 @@ __global__ void __launch_bounds__(256) nu_kernel(ShellView B, const int32_t *__r
 #pragma unroll
                   for (int v = 0; v <= L; ++v) {
                     if (v > ma + mb) continue;
-                    s = fma(E3[idx], R[t][u][v], s);
+                    cart[qa][qb] = fma(E3[idx], R[t][u][v], cart[qa][qb]);
                     ++idx;
                   }
                 }
               }
-              cart[qa][qb] = fma(cc, s, cart[qa][qb]);
             }
           }
         }
