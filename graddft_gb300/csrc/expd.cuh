@@ -7,7 +7,7 @@
 // exp(a) = 2^k T_j (1 + p(r)), T_j = 2^(j/256) to twice FP64, p the Taylor
 // polynomial of degree 5 (the next term is below 2^-57 of r): 11 operations for
 // exp and 12 for expm1, the exponent and index work in integers.  Errors over
-// [-699, 0] against quad precision: exp 0.502 ulp at most, expm1 1.28 (1.0 below -ln 2).
+// [-707, 0] against quad precision: exp 0.502 ulp at most, expm1 1.40 (1.0 below -ln 2).
 #pragma once
 
 namespace gdft {
@@ -59,7 +59,7 @@ __device__ __forceinline__ double2 table_entry(int j) {
   const double p = h1 * h2;
   const double l = fma(h1, h2, -p) + fma(h1, l2, l1 * h2);
   const double t = p + l;
-  return make_double2(t, (l - (t - p)) / t);
+  return make_double2(t, (double)((float)(l - (t - p)) / (float)t));  // 24 of the bits past 2^-53 are plenty
 }
 
 // By all threads of a block, which then synchronises.
@@ -67,7 +67,7 @@ __device__ __forceinline__ void build_table(double2 *tab) {
   for (int j = threadIdx.x; j < kTable; j += blockDim.x) tab[j] = table_entry(j);
 }
 
-// exp(a) = t (1 + r + tail) for -700 < a <= 0; r is exact, tail carries what the
+// exp(a) = t (1 + r + tail) for |a| < 708; r is exact, tail carries what the
 // reduction and the table left over and the polynomial from its square on.
 struct Parts {
   double t, r, tail;
@@ -95,9 +95,9 @@ __device__ __forceinline__ double expm1_of(const Parts &e) {
   return fma(e.t, half ? e.tail : e.r + e.tail, half ? fma(e.t, e.r, w) : w);
 }
 
-// Arguments at or below -700, infinities and NaN go to the library.
+// Arguments from 708 on (2^k would not be a normal number), infinities and NaN: the caller's.
 __device__ __forceinline__ bool tabled(double a) {
-  return (unsigned)(__double2hiint(a) & 0x7fffffff) < 0x4085E000u;
+  return (unsigned)(__double2hiint(a) & 0x7fffffff) < 0x40862000u;
 }
 // True for 0 < a < infinity, by the high word (a denormal may read as zero).
 __device__ __forceinline__ bool positive(double a) { return (unsigned)(__double2hiint(a) - 1) < 0x7fefffffu; }

@@ -7,23 +7,31 @@
 //   A(d) = sum_(i,j,k) t_ijk x^i y^j z^k  (the component's row of cartesian coefficients, degree l),
 // so that d_x phi = A_x E0 + A x E1 and d_xx phi = A_xx E0 + 2 A_x x E1 + A (E1 + x^2 E2).
 //
-// Work layout: a CTA evaluates a tile of 32 grid points x 64 AOs into shared
+// Work layout: a CTA evaluates a tile of 32 grid points x 32 AOs into shared
 // memory, then a sink writes the tile to its destination with the AO index
 // fastest (coalesced).  In the evaluation phase the lanes of a warp are the 32
-// points and each warp takes whole shells, so the angular momentum and the
-// primitive count are uniform across the warp (no divergence) and each
+// points and each warp takes the next whole shell, so the angular momentum and
+// the primitive count are uniform across the warp (no divergence) and each
 // exponential is computed once per point and shell, shared by all of the
 // shell's contractions and components.
+//
+// What bounds it is the FP64 pipe (16 clocks a warp operation): s, p and d
+// shells have their own angular forms, sharing P E1 and P E2 between the seven
+// values, and the exponential is taken by table (expd.cuh).  Three tiles of 32
+// AOs share an SM, so that one's output runs beside the others' evaluation (of
+// 64 AOs only one fits with second derivatives).
+// 506 AOs (s, p, d of 4, 3, 2 primitives) x 20,001 points: 2.66 -> 1.28 ms.
 #pragma once
 
 #include "common.cuh"
+#include "expd.cuh"
 
 namespace gdft {
 
 constexpr int kMaxShellL = 6;
 constexpr int kShellCols = 8;  // l, nprim, exp offset, coef offset, first AO, ncomp, nctr, row offset
 constexpr int kTilePts = 32;
-constexpr int kTileAo = 64;
+constexpr int kTileAo = 32;
 constexpr int kTileLd = kTileAo + 1;  // padded row: lanes (points) land in different banks
 constexpr int kTileThreads = 256;
 constexpr int kCtrGroup = 4;  // contractions whose radial sums are carried together
@@ -85,15 +93,118 @@ __device__ __forceinline__ void poly(const double *__restrict__ t, double x, dou
   }
 }
 
-__device__ __forceinline__ void poly_l(int l, const double *t, double x, double y, double z, double P[7]) {
-  switch (l) {
-    case 0: poly<0>(t, x, y, z, P); break;
-    case 1: poly<1>(t, x, y, z, P); break;
-    case 2: poly<2>(t, x, y, z, P); break;
-    case 3: poly<3>(t, x, y, z, P); break;
-    case 4: poly<4>(t, x, y, z, P); break;
-    case 5: poly<5>(t, x, y, z, P); break;
-    default: poly<6>(t, x, y, z, P); break;
+// exp(a) for the radial sums, a = -alpha r^2, by a whole warp: by table; where a
+// lane is below -708, from a + 64 ln 2 and scaled back (denormal results), and
+// zero below -745.25.  Only infinities and NaN reach the library: at many points
+// some lane of a warp is that far out.
+__device__ __forceinline__ double radial_exp(double a, const double2 *tab) {
+  if (!__any_sync(0xffffffffu, !expd::tabled(a))) return expd::exp_of(expd::parts(a, tab));
+  const unsigned hi = (unsigned)__double2hiint(a);
+  const bool zero = hi >= 0xC0874A00u && hi < 0xFFF00000u, deep = hi >= 0xC0862000u && hi < 0xC0874A00u;
+  double b = zero ? -1.0 : a;
+  if (deep) b += 0x1.62e42fefa39efp+5;
+  if (!expd::tabled(b)) return exp(a);
+  double e = expd::exp_of(expd::parts(b, tab));
+  if (deep) e *= 0x1p-64;
+  return zero ? 0.0 : e;
+}
+
+// Radial sums at a point and what of them the components share.
+struct Radial {
+  double E0, E1, E2;
+};
+
+// The sums of N contractions from c on.  N is a constant (not a bound under which
+// four are predicated): left-out FP64 operations take their slots too.
+template <int N>
+__device__ __forceinline__ void radial_sums(const double *__restrict__ exps, const double *__restrict__ coef, int np,
+                                            double r2, const double2 *tab, Radial *E) {
+#pragma unroll
+  for (int j = 0; j < N; ++j) E[j].E0 = E[j].E1 = E[j].E2 = 0.0;
+  for (int q = 0; q < np; ++q) {
+    const double al = exps[q];
+    const double e = radial_exp(-al * r2, tab);
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      const double ce = coef[(int64_t)j * np + q] * e, ae = al * ce;
+      E[j].E0 += ce;
+      E[j].E1 += ae;
+      E[j].E2 = fma(al, ae, E[j].E2);
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    E[j].E1 *= -2.0;
+    E[j].E2 *= 4.0;
+  }
+}
+
+// The seven values of the component with angular row t at d = (x, y, z).  q: the
+// squares x^2, y^2, z^2.  A row's zeros are the same for the whole warp and are
+// left out (solid harmonics are mostly zeros).
+__device__ __forceinline__ bool nonzero(double t) { return (__double_as_longlong(t) << 1) != 0; }
+
+// From the polynomial P[0] and its derivatives: first P[1..3], diagonal second P[4..6].
+template <bool SECOND>
+__device__ __forceinline__ void combine(const double P[7], const double d[3], const Radial &r, double v[7]) {
+  const double g1 = P[0] * r.E1, g2 = P[0] * r.E2, e1 = r.E1 + r.E1;
+  v[0] = P[0] * r.E0;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    v[1 + i] = fma(g1, d[i], P[1 + i] * r.E0);
+    v[4 + i] = fma(d[i], fma(g2, d[i], P[1 + i] * e1), g1);
+    if (SECOND) v[4 + i] = fma(P[4 + i], r.E0, v[4 + i]);
+  }
+}
+
+__device__ __forceinline__ void component(int l, const double *__restrict__ t, const double d[3], const double q[3],
+                                          const Radial &r, double v[7]) {
+  double P[7];
+  if (l == 0) {
+    const double c = t[0], e0 = c * r.E0, e1 = c * r.E1, e2 = c * r.E2;
+    v[0] = e0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      v[1 + i] = e1 * d[i];
+      v[4 + i] = fma(q[i], e2, e1);
+    }
+  } else if (l == 1) {
+    P[0] = 0.0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      P[1 + i] = t[i];
+      if (nonzero(t[i])) P[0] = fma(t[i], d[i], P[0]);
+    }
+    combine<false>(P, d, r, v);
+  } else if (l == 2) {
+#pragma unroll
+    for (int k = 0; k < 7; ++k) P[k] = 0.0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int j = i; j < 3; ++j) {  // xx, xy, xz, yy, yz, zz
+        const double c = t[i == 0 ? j : i + j + 1];
+        if (!nonzero(c)) continue;
+        if (i == j) {
+          P[0] = fma(c, q[i], P[0]);
+          P[4 + i] = c + c;
+          P[1 + i] = fma(c + c, d[i], P[1 + i]);
+        } else {
+          const double cj = c * d[j];
+          P[0] = fma(cj, d[i], P[0]);
+          P[1 + i] += cj;
+          P[1 + j] = fma(c, d[i], P[1 + j]);
+        }
+      }
+    combine<true>(P, d, r, v);
+  } else {
+    switch (l) {
+      case 3: poly<3>(t, d[0], d[1], d[2], P); break;
+      case 4: poly<4>(t, d[0], d[1], d[2], P); break;
+      case 5: poly<5>(t, d[0], d[1], d[2], P); break;
+      default: poly<6>(t, d[0], d[1], d[2], P); break;
+    }
+    combine<true>(P, d, r, v);
   }
 }
 
@@ -123,7 +234,8 @@ __device__ __forceinline__ bool load_shell(const ShellView &B, int s, ShellRec &
 
 }  // namespace shells_detail
 
-// Evaluation phase: the tile [kVals][kTilePts][kTileLd] of AOs [a0, a0 + kTileAo)
+// Evaluation phase, by all threads of the block (the caller synchronises): the tile
+// [kVals][kTilePts][kTileLd] of AOs [a0, a0 + kTileAo)
 // at points [p0, p0 + 32).  kVals = 7 keeps the three diagonal second
 // derivatives, kVals = 5 their sum (the Laplacian).  Entries no shell covers
 // stay NaN; AOs at or beyond n_ao stay NaN too (sinks write zero padding there).
@@ -131,11 +243,16 @@ template <int kVals>
 __device__ __forceinline__ void eval_tile(const ShellView &B, const double *__restrict__ coords, int64_t n_grid,
                                           int64_t p0, int a0, double *tile) {
   using namespace shells_detail;
+  __shared__ double2 tab[expd::kTable];
+  __shared__ int next;  // the next shell that a warp takes
+  expd::build_table(tab);
   for (int i = threadIdx.x; i < kVals * kTilePts * kTileLd; i += blockDim.x) tile[i] = nan_value();
-  __syncthreads();
-  if (a0 >= B.n_ao) return;
   const int a1 = min(a0 + kTileAo, B.n_ao);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const int s_lo = a0 < B.n_ao ? B.ao[4 * a0] : 0, s_hi = a0 < B.n_ao ? B.ao[4 * (a1 - 1)] : -1;
+  if (threadIdx.x == 0) next = s_lo;
+  __syncthreads();
+  if (s_lo < 0 || s_hi >= B.n_shell || s_hi < s_lo) return;
+  const int lane = threadIdx.x & 31;
   const int64_t p = p0 + lane;
   double px = 0.0, py = 0.0, pz = 0.0;
   if (p < n_grid) {
@@ -143,56 +260,36 @@ __device__ __forceinline__ void eval_tile(const ShellView &B, const double *__re
     py = coords[3 * p + 1];
     pz = coords[3 * p + 2];
   }
-  const int s_lo = B.ao[4 * a0], s_hi = B.ao[4 * (a1 - 1)];
-  if (s_lo < 0 || s_hi >= B.n_shell || s_hi < s_lo) return;
-  for (int s = s_lo + warp; s <= s_hi; s += nwarps) {
+  for (;;) {
+    int s = lane == 0 ? atomicAdd(&next, 1) : 0;
+    s = __shfl_sync(0xffffffffu, s, 0);
+    if (s > s_hi) break;
     ShellRec r;
     if (!load_shell(B, s, r)) continue;
     const int lo = max(a0, r.aoff), hi = min(a1, r.aoff + r.nctr * r.ncomp);
     if (lo >= hi) continue;
-    const double x = px - B.centre[3 * s + 0];
-    const double y = py - B.centre[3 * s + 1];
-    const double z = pz - B.centre[3 * s + 2];
-    const double r2 = x * x + y * y + z * z;
-    const double d[3] = {x, y, z};
+    const double d[3] = {px - B.centre[3 * s + 0], py - B.centre[3 * s + 1], pz - B.centre[3 * s + 2]};
+    const double sq[3] = {d[0] * d[0], d[1] * d[1], d[2] * d[2]};
+    const double r2 = sq[0] + sq[1] + sq[2];
     const int c_lo = (lo - r.aoff) / r.ncomp, c_hi = (hi - 1 - r.aoff) / r.ncomp;
     for (int cg = c_lo; cg <= c_hi; cg += kCtrGroup) {
       const int nc = min(kCtrGroup, c_hi - cg + 1);
-      double E0[kCtrGroup], E1[kCtrGroup], E2[kCtrGroup];
-#pragma unroll
-      for (int j = 0; j < kCtrGroup; ++j) E0[j] = E1[j] = E2[j] = 0.0;
-      for (int q = 0; q < r.np; ++q) {
-        const double al = B.exps[r.poff + q];
-        const double e = exp(-al * r2);
-        const double m1 = -2.0 * al;
-#pragma unroll
-        for (int j = 0; j < kCtrGroup; ++j) {
-          if (j < nc) {
-            const double ce = B.coef[r.coff + (int64_t)(cg + j) * r.np + q] * e;
-            E0[j] += ce;
-            E1[j] = fma(m1, ce, E1[j]);
-            E2[j] = fma(m1 * m1, ce, E2[j]);
-          }
-        }
+      Radial E[kCtrGroup];
+      const double *exps = B.exps + r.poff, *coef = B.coef + r.coff + (int64_t)cg * r.np;
+      switch (nc) {
+        case 1: radial_sums<1>(exps, coef, r.np, r2, tab, E); break;
+        case 2: radial_sums<2>(exps, coef, r.np, r2, tab, E); break;
+        case 3: radial_sums<3>(exps, coef, r.np, r2, tab, E); break;
+        default: radial_sums<kCtrGroup>(exps, coef, r.np, r2, tab, E);
       }
-      for (int k = 0; k < r.ncomp; ++k) {
-        double P[7];
-        bool have = false;
 #pragma unroll
-        for (int j = 0; j < kCtrGroup; ++j) {
+      for (int j = 0; j < kCtrGroup; ++j) {
+        if (j >= nc) break;
+        for (int k = 0; k < r.ncomp; ++k) {
           const int a = r.aoff + (cg + j) * r.ncomp + k;
-          if (j >= nc || a < lo || a >= hi) continue;
-          if (!have) {
-            poly_l(r.l, B.trans + r.toff + (int64_t)k * r.ncart, x, y, z, P);
-            have = true;
-          }
+          if (a < lo || a >= hi) continue;
           double v[7];
-          v[0] = P[0] * E0[j];
-#pragma unroll
-          for (int i = 0; i < 3; ++i) {
-            v[1 + i] = fma(P[0] * d[i], E1[j], P[1 + i] * E0[j]);
-            v[4 + i] = P[4 + i] * E0[j] + 2.0 * P[1 + i] * d[i] * E1[j] + P[0] * fma(d[i] * d[i], E2[j], E1[j]);
-          }
+          component(r.l, B.trans + r.toff + (int64_t)k * r.ncart, d, sq, E[j], v);
           double *t = tile + (size_t)lane * kTileLd + (a - a0);
 #pragma unroll
           for (int q = 0; q < 4; ++q) t[q * kTilePts * kTileLd] = v[q];
@@ -208,10 +305,10 @@ __device__ __forceinline__ void eval_tile(const ShellView &B, const double *__re
   }
 }
 
-// One tile per CTA: blockIdx.x = 32-point group, blockIdx.y = 64-AO chunk of
+// One tile per CTA: blockIdx.x = 32-point group, blockIdx.y = 32-AO chunk of
 // the sink's AO extent.  The sink is called after the whole tile is written.
 template <int kVals, class Sink>
-__global__ void __launch_bounds__(kTileThreads) eval_shells_tile_kernel(ShellView B, const double *__restrict__ coords,
+__global__ void __launch_bounds__(kTileThreads, 3) eval_shells_tile_kernel(ShellView B, const double *__restrict__ coords,
                                                                         int64_t n_grid, Sink sink) {
   extern __shared__ double tile[];
   const int64_t p0 = (int64_t)blockIdx.x * kTilePts;
@@ -226,7 +323,7 @@ __global__ void __launch_bounds__(kTileThreads) eval_shells_tile_kernel(ShellVie
 
 constexpr size_t tile_smem_bytes(int vals) { return (size_t)vals * kTilePts * kTileLd * sizeof(double); }
 
-// Launch over (points rounded to 32) x (AO extent rounded to 64).
+// Launch over (points rounded to 32) x (AO extent rounded to 32).
 template <int kVals, class Sink>
 cudaError_t launch_shell_tiles(const ShellView &B, const double *coords, int64_t n_grid, int64_t n_points,
                                int ao_extent, const Sink &sink, cudaStream_t st) {
