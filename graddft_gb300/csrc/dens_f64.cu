@@ -26,6 +26,7 @@ constexpr int NT = 256;  // threads: 32 points x 8 column lanes
 __global__ void __launch_bounds__(NT) dens_f64_kernel(const double *__restrict__ tab, int64_t np, int ld, int n,
                                                       const double *__restrict__ D, double *__restrict__ feat,
                                                       const int *__restrict__ bad) {
+  previous_done();
   if (bad != nullptr && *bad == 0) return;
   __shared__ double As[4][BP][BK + 1];
   __shared__ double Bs[BK][BN];
@@ -123,7 +124,7 @@ __global__ void __launch_bounds__(NT) dens_f64_kernel(const double *__restrict__
 cudaError_t launch_dens_f64(const double *tab, int64_t np, int ld, int n_ao, const double *rdm1, double *feat,
                             const int *bad, cudaStream_t st) {
   const int64_t blocks = np / BP;
-  dens_f64_kernel<<<(unsigned)blocks, NT, 0, st>>>(tab, np, ld, n_ao, rdm1, feat, bad);
+  launch_next(dens_f64_kernel, (unsigned)blocks, NT, 0, st, tab, np, ld, n_ao, rdm1, feat, bad);
   return cudaGetLastError();
 }
 

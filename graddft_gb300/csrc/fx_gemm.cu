@@ -176,6 +176,7 @@ __device__ __forceinline__ double scaled(long long v, int e) {
 }
 
 __global__ void __launch_bounds__(kThreads, 1) fx_gemm_kernel(const GemmArgs A, const int upper) {
+  previous_done();
   if (A.bad != nullptr && *A.bad != 0) return;
   extern __shared__ unsigned char smem_raw[];
   unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -507,6 +508,7 @@ __global__ void __launch_bounds__(256) fx_rows_kernel(const double *__restrict__
                                                       int64_t ld, int k_valid, int chunks,
                                                       unsigned char *__restrict__ out, int *__restrict__ exps,
                                                       int *__restrict__ bad) {
+  previous_done();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t tiles = (rows + kTile - 1) / kTile;
   const int64_t r0 = ((int64_t)blockIdx.x * 8 + warp) * 8;
@@ -572,7 +574,7 @@ cudaError_t launch_gemm(const GemmArgs &a, cudaStream_t st) {
   if (items < 1) return cudaSuccess;
   if (items > 0x3FFFFFFF) return cudaErrorInvalidValue;
   const unsigned grid = (unsigned)(items < sms ? items : sms);
-  fx_gemm_kernel<<<grid, kThreads, kSmemBytes, st>>>(a, upper);
+  launch_next(fx_gemm_kernel, grid, kThreads, kSmemBytes, st, a, upper);
   return cudaGetLastError();
 }
 
@@ -581,9 +583,9 @@ cudaError_t launch_rows(const double *src, int64_t plane_elems, int planes, int6
   const dim3 grid((unsigned)((rows + 63) / 64), planes);
   // 16-byte loads where every row starts on a 16-byte boundary.
   if (((uintptr_t)src & 15) == 0 && (ld & 1) == 0 && (plane_elems & 1) == 0)
-    fx_rows_kernel<true><<<grid, 256, 0, st>>>(src, plane_elems, rows, ld, k_valid, chunks, out, exps, bad);
+    launch_next(fx_rows_kernel<true>, grid, 256, 0, st, src, plane_elems, rows, ld, k_valid, chunks, out, exps, bad);
   else
-    fx_rows_kernel<false><<<grid, 256, 0, st>>>(src, plane_elems, rows, ld, k_valid, chunks, out, exps, bad);
+    launch_next(fx_rows_kernel<false>, grid, 256, 0, st, src, plane_elems, rows, ld, k_valid, chunks, out, exps, bad);
   return cudaGetLastError();
 }
 

@@ -32,6 +32,7 @@ constexpr int64_t chunks_of(int64_t k) { return (k + kChunkK - 1) / kChunkK; }
 __global__ void __launch_bounds__(128) fx_short_cols_kernel(const double *__restrict__ X, int k_rows, int cols,
                                                             int64_t ld, int chunks, unsigned char *__restrict__ out,
                                                             int *__restrict__ exps, int *__restrict__ bad) {
+  previous_done();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int c0 = (blockIdx.x * 4 + warp) * 8;
   if (c0 >= cols) return;
@@ -64,6 +65,7 @@ __global__ void __launch_bounds__(128) fx_short_cols_kernel(const double *__rest
 // takes 32 of them and `per` rows.
 __global__ void __launch_bounds__(256) fx_colmax_kernel(const double *__restrict__ X, int64_t rows, int cols,
                                                         int64_t ld, int64_t per, uint32_t *__restrict__ mx) {
+  previous_done();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int c = blockIdx.x * 32 + lane;
   const int64_t r0 = (int64_t)blockIdx.y * per, r1 = r0 + per < rows ? r0 + per : rows;
@@ -86,6 +88,7 @@ __global__ void __launch_bounds__(256) fx_tall_cols_kernel(const double *__restr
                                                            int64_t ld, int chunks, const uint32_t *__restrict__ mx,
                                                            unsigned char *__restrict__ out, int *__restrict__ exps,
                                                            int *__restrict__ bad) {
+  previous_done();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int c = blockIdx.y * 32 + lane, chunk = blockIdx.x;
   int emax = c < cols ? exp_field(mx[c]) : 1;
@@ -106,6 +109,7 @@ __global__ void __launch_bounds__(256) fx_tall_cols_kernel(const double *__restr
 // C[i] = sum over splits of part[split][i].
 __global__ void fx_sum_kernel(const double *__restrict__ part, int nsplit, size_t total, size_t stride,
                               double *__restrict__ C, const int *__restrict__ bad) {
+  previous_done();
   if (*bad != 0) return;
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
@@ -191,7 +195,7 @@ cudaError_t gemm_rows(int64_t M, int N, int K, const double *A, int64_t lda, con
     if (b_rows)
       e = launch_rows(B, 0, 1, N, ldb, K, ch, sw, ew, bad, st);
     else {
-      fx_short_cols_kernel<<<(N + 31) / 32, 128, 0, st>>>(B, K, N, ldb, ch, sw, ew, bad);
+      launch_next(fx_short_cols_kernel, (N + 31) / 32, 128, 0, st, B, K, N, ldb, ch, sw, ew, bad);
       e = cudaGetLastError();
     }
     if (e != cudaSuccess) return e;
@@ -244,8 +248,8 @@ cudaError_t gemm_cols(int M, int N, int64_t K, const double *A, int64_t lda, con
       int64_t segs = (4 * 148 + bc - 1) / bc, per = (rows + segs - 1) / segs;
       per = per < 64 ? 64 : per;
       segs = (rows + per - 1) / per;
-      fx_colmax_kernel<<<dim3(bc, (unsigned)segs), 256, 0, st>>>(X + k0 * ld, rows, cols, ld, per, mx);
-      fx_tall_cols_kernel<<<dim3(ch, bc), 256, 0, st>>>(X + k0 * ld, rows, cols, ld, ch, mx, set, exps, bad);
+      launch_next(fx_colmax_kernel, dim3(bc, (unsigned)segs), 256, 0, st, X + k0 * ld, rows, cols, ld, per, mx);
+      launch_next(fx_tall_cols_kernel, dim3(ch, bc), 256, 0, st, X + k0 * ld, rows, cols, ld, ch, mx, set, exps, bad);
       return cudaGetLastError();
     };
     if ((e = digits(A, lda, M, ma, ws + w.off_a, ea)) != cudaSuccess) return e;
@@ -274,7 +278,7 @@ cudaError_t gemm_cols(int M, int N, int64_t K, const double *A, int64_t lda, con
     if ((e = launch_gemm(g, st)) != cudaSuccess) return e;
   }
   const size_t total = (size_t)M * N;
-  fx_sum_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(fpart, w.splits, total, total, C, bad);
+  launch_next(fx_sum_kernel, (unsigned)((total + 255) / 256), 256, 0, st, fpart, w.splits, total, total, C, bad);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   return plain_gemm_tn_split(M, N, K, A, (int)lda, B, (int)ldb, C, nsplit, part, bad, st);
 }

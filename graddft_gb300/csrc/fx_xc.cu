@@ -37,6 +37,7 @@ size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 __global__ void __launch_bounds__(128) fx_rdm1_kernel(const double *__restrict__ D, int n, int nb, int versions,
                                                       unsigned char *__restrict__ out, int *__restrict__ exps,
                                                       int *__restrict__ bad) {
+  previous_done();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = blockIdx.x * 4 + warp;  // group of eight operand rows: 16 per tile
   if (g >= nb * 16) return;
@@ -83,6 +84,7 @@ __global__ void __launch_bounds__(256) fx_features_kernel(const double *__restri
                                                           int64_t p0, int64_t slab, const double *__restrict__ X,
                                                           int cols, bool kin, double *__restrict__ feat,
                                                           const int *__restrict__ bad) {
+  previous_done();
   if (*bad != 0) return;
   __shared__ double t[kPlanes][kFeatTile][kFeatTile + 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -164,6 +166,15 @@ __device__ __forceinline__ int field_of(int m, int octaves) {
   return f < 1 ? 1 : f > 0x7FE ? 0x7FE : f;
 }
 
+// The non-finite word, and n maxima below every high word (a kernel, not a
+// memset: launches before and after it stay chained).
+__global__ void fx_clear_kernel(int *bad, int *mx, int n) {
+  previous_done();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0 && bad != nullptr) *bad = 0;
+  if (i < n) mx[i] = kNone;
+}
+
 // Largest high words over a slab of points: [0] phi, [1] d_j phi (one for the
 // three), [2 + s] the terms of Q_s, [4 + s] c_kin,s d_j phi.  Lanes are AOs, a
 // block takes 32 AOs and `per` points, its warps every eighth point.
@@ -171,6 +182,7 @@ __global__ void __launch_bounds__(256) fx_vmax_kernel(const double *__restrict__
                                                       const double *__restrict__ coef, int64_t p0, int64_t rows,
                                                       int per, bool kin, int n_max, int *__restrict__ mx,
                                                       int *__restrict__ bad) {
+  previous_done();
   __shared__ int sc[2][kFeat][128];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int a = blockIdx.x * 32 + lane;
@@ -228,6 +240,7 @@ __global__ void __launch_bounds__(256, 4) fx_vdigits_kernel(const double *__rest
                                                             const int *__restrict__ mx, int *__restrict__ ea,
                                                             int *__restrict__ eb, unsigned char *__restrict__ va,
                                                             unsigned char *__restrict__ vb, int *__restrict__ bad) {
+  previous_done();
   if (*bad != 0) return;
   __shared__ double sc[kFeat][64];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -316,6 +329,7 @@ __global__ void __launch_bounds__(256, 4) fx_vdigits_kernel(const double *__rest
 __global__ void __launch_bounds__(256) fx_vreduce_kernel(const double *__restrict__ part, int s0, int s1, int n,
                                                          int rows, int cols, double *__restrict__ out,
                                                          const int *__restrict__ bad) {
+  previous_done();
   if (*bad != 0) return;
   __shared__ double sm[8][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -399,9 +413,10 @@ cudaError_t launch_density(const double *tab, int64_t np, int ld, int n_ao, cons
   unsigned char *dset = ws + w.off_dset;
   int *dexp = (int *)(ws + w.off_dexp), *ea = (int *)(ws + w.off_ea);
   double *X = (double *)(ws + w.off_x);
-  cudaError_t e = cudaMemsetAsync(bad, 0, sizeof(int), st);
-  if (e != cudaSuccess) return e;
-  fx_rdm1_kernel<<<dim3((unsigned)(w.nb * 4), kin ? 2 : 1), 128, 0, st>>>(rdm1, n_ao, w.nb, 2, dset, dexp, bad);
+  cudaError_t e;
+  launch_next(fx_clear_kernel, 1, 32, 0, st, bad, nullptr, 0);
+  launch_next(fx_rdm1_kernel, dim3((unsigned)(w.nb * 4), kin ? 2 : 1), 128, 0, st, rdm1, n_ao, w.nb, 2, dset, dexp,
+              bad);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   for (int64_t p0 = 0; p0 < np; p0 += w.dens_slab) {
     const int64_t rows = np - p0 < w.dens_slab ? np - p0 : w.dens_slab;
@@ -431,6 +446,8 @@ cudaError_t launch_density(const double *tab, int64_t np, int ld, int n_ao, cons
     g.bad = bad;
     g.err = err;
     if ((e = launch_gemm(g, st)) != cudaSuccess) return e;
+    // Not chained: its blocks would be placed while the GEMM still holds most SMs, and crowd on the rest (24 AOs x
+    // 3,600 points: 8 us, chained 24).
     fx_features_kernel<<<(unsigned)(rows / kFeatTile), 256, 0, st>>>(tab, pe, np, ld, p0, w.dens_slab, X, w.nb * 64, kin,
                                                                      feat, bad);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
@@ -447,22 +464,20 @@ cudaError_t launch_vxc(const double *tab, int64_t np, int ld, int n_ao, const do
   int *ea = (int *)(ws + w.off_vexp), *eb = ea + 2 * n_max, *mx = eb + 2 * w.nb * kTile;
   unsigned char *va = ws + w.off_va, *vb = ws + w.off_vb;
   double *part = (double *)(ws + w.off_vpart);
-  cudaError_t e = cudaMemsetAsync(bad, 0, sizeof(int), st);
-  if (e != cudaSuccess) return e;
+  cudaError_t e;
   for (int64_t p0 = 0; p0 < np; p0 += w.v_slab) {
     const int64_t rows = np - p0 < w.v_slab ? np - p0 : w.v_slab;
     const int npc = (int)((rows + kChunkK - 1) / kChunkK);
-    // 0x80808080 is below every high word.
-    if ((e = cudaMemsetAsync(mx, 0x80, (size_t)6 * n_max * sizeof(int), st)) != cudaSuccess) return e;
+    launch_next(fx_clear_kernel, (6 * n_max + 255) / 256, 256, 0, st, p0 == 0 ? bad : nullptr, mx, 6 * n_max);
     const int blocks_a = (ld + 31) / 32;
     int64_t segs = (8 * 148 + blocks_a - 1) / blocks_a;
     int64_t per = (rows + segs - 1) / segs;
     per = per < 64 ? 64 : per;
     segs = (rows + per - 1) / per;
-    fx_vmax_kernel<<<dim3(blocks_a, (unsigned)segs), 256, 0, st>>>(tab, pe, np, ld, coef, p0, rows, (int)per, kin,
-                                                                   n_max, mx, bad);
-    fx_vdigits_kernel<<<dim3(ld / 32, npc, 3), 256, 0, st>>>(tab, pe, np, ld, coef, p0, rows, npc, kin, w.mt, w.nb,
-                                                             (n_ao + 7) / 8 * 8, mx, ea, eb, va, vb, bad);
+    launch_next(fx_vmax_kernel, dim3(blocks_a, (unsigned)segs), 256, 0, st, tab, pe, np, ld, coef, p0, rows, (int)per,
+                kin, n_max, mx, bad);
+    launch_next(fx_vdigits_kernel, dim3(ld / 32, npc, 3), 256, 0, st, tab, pe, np, ld, coef, p0, rows, npc, kin, w.mt,
+                w.nb, (n_ao + 7) / 8 * 8, mx, ea, eb, va, vb, bad);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     GemmArgs g{};
     g.a = va;
@@ -490,8 +505,8 @@ cudaError_t launch_vxc(const double *tab, int64_t np, int ld, int n_ao, const do
     if ((e = launch_gemm(g, st)) != cudaSuccess) return e;
   }
   // The first slab, the longest, writes all s0 + s1 splits.
-  fx_vreduce_kernel<<<dim3((n_ao + 31) / 32, n_ao, 2), 256, 0, st>>>(part, w.s0, kin ? w.s1 : 0, n_ao, n_max, w.nb * 64,
-                                                                     vxc, bad);
+  launch_next(fx_vreduce_kernel, dim3((n_ao + 31) / 32, n_ao, 2), 256, 0, st, part, w.s0, kin ? w.s1 : 0, n_ao, n_max,
+              w.nb * 64, vxc, bad);
   return cudaGetLastError();
 }
 

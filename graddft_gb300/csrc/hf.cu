@@ -33,6 +33,7 @@ namespace {
 // X[s * spin_stride + r * ld + c].
 __global__ void hf_rowdot_kernel(const double *__restrict__ chi, const double *__restrict__ X, int64_t n_grid, int n,
                                  int n_omega, int64_t ld, int64_t spin_stride, double *__restrict__ ehf) {
+  previous_done();
   const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (gw >= 2 * n_grid) return;  // whole warps leave together
@@ -52,6 +53,7 @@ __global__ void hf_rowdot_kernel(const double *__restrict__ chi, const double *_
 // B[s][r][b] = -1/2 sum_w g[w][s][r] chi[r][w][s][b].
 __global__ void hf_bmat_kernel(const double *__restrict__ chi, const double *__restrict__ g, int64_t n_grid, int n,
                                int n_omega, double *__restrict__ B) {
+  previous_done();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t per_spin = (size_t)n_grid * n;
   if (i >= 2 * per_spin) return;
@@ -66,6 +68,7 @@ __global__ void hf_bmat_kernel(const double *__restrict__ chi, const double *__r
 
 // fock[s] = abs_clip(fock[s] + F[s] + F[s]^T)  (train.py:200-210).
 __global__ void fock_add_hf_kernel(double *__restrict__ fock, const double *__restrict__ F, int n, double clip) {
+  previous_done();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t nn = (size_t)n * n;
   if (i >= 2 * nn) return;
@@ -153,6 +156,7 @@ __device__ __forceinline__ void store_row3_scaled(float *blk3, int row, const do
 template <class Fetch>
 __global__ void __launch_bounds__(128) hf_pack3_kernel(Fetch f, int64_t rows, int64_t kdim, int64_t kchunks,
                                                        float scale, float *__restrict__ out) {
+  previous_done();
   const int64_t t = blockIdx.x / kchunks, kc = blockIdx.x % kchunks;
   const int64_t m = t * 128 + threadIdx.x;
   double v[32];
@@ -166,6 +170,7 @@ __global__ void __launch_bounds__(128) hf_pack3_kernel(Fetch f, int64_t rows, in
 
 // F[s][a][b] = sum_z part[z][a][s n + b], the splits in order.
 __global__ void hf_fock_reduce_kernel(const double *__restrict__ part, int nsplit, int n, double *__restrict__ F) {
+  previous_done();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t nn = (size_t)n * n;
   if (i >= 2 * nn) return;
@@ -283,10 +288,10 @@ int hf_energy_density_tc(const double *ao, const double *rdm1, const double *chi
   float *pa = (float *)(ws + L.off_pa), *pb = (float *)(ws + L.off_pb);
   double *X = (double *)(ws + L.off_x);
   if ((rc = check_cuda(cudaMemsetAsync(err, 0, sizeof(int), st), "hf err clear"))) return rc;
-  hf_pack3_kernel<FetchRows><<<(unsigned)(L.tiles_g * L.kc_ao), 128, 0, st>>>(FetchRows{ao, n}, n_grid, n, L.kc_ao,
-                                                                               1.0f, pa);
-  hf_pack3_kernel<FetchDensity><<<(unsigned)(L.tiles_j * L.kc_ao), 128, 0, st>>>(FetchDensity{rdm1, n}, 2 * n, n,
-                                                                                  L.kc_ao, 1.0f, pb);
+  launch_next(hf_pack3_kernel<FetchRows>, (unsigned)(L.tiles_g * L.kc_ao), 128, 0, st, FetchRows{ao, n}, n_grid, n,
+              L.kc_ao, 1.0f, pa);
+  launch_next(hf_pack3_kernel<FetchDensity>, (unsigned)(L.tiles_j * L.kc_ao), 128, 0, st, FetchDensity{rdm1, n}, 2 * n,
+              n, L.kc_ao, 1.0f, pb);
   if ((rc = check_cuda(cudaGetLastError(), "hf pack ao, D"))) return rc;
   TcgArgs a{};
   a.a = pa;
@@ -300,8 +305,8 @@ int hf_energy_density_tc(const double *ao, const double *rdm1, const double *chi
   a.err = err;
   if ((rc = check_cuda(launch_tcg3(a, 1, st), "hf ao.[D0|D1]"))) return rc;
   const int64_t threads = 2 * n_grid * 32;
-  hf_rowdot_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(chi, X, n_grid, n, n_omega, 2 * (int64_t)n, n,
-                                                                       ehf);
+  launch_next(hf_rowdot_kernel, (unsigned)((threads + 255) / 256), 256, 0, st, chi, X, n_grid, n, n_omega,
+              2 * (int64_t)n, n, ehf);
   return check_cuda(cudaGetLastError(), "hf rowdot");
 }
 
@@ -314,10 +319,10 @@ int hf_fock_tc(const double *ao, const double *chi, const double *g, int64_t n_g
   float *fa = (float *)(ws + L.off_fa), *fb = (float *)(ws + L.off_fb);
   double *part = (double *)(ws + L.off_part);
   if ((rc = check_cuda(cudaMemsetAsync(err, 0, sizeof(int), st), "hf err clear"))) return rc;
-  hf_pack3_kernel<FetchCols><<<(unsigned)(L.tiles_ao * L.rchunks), 128, 0, st>>>(FetchCols{ao, n}, n, n_grid,
-                                                                                  L.rchunks, 1.0f, fa);
-  hf_pack3_kernel<FetchHfB><<<(unsigned)(L.tiles_j * L.rchunks), 128, 0, st>>>(
-      FetchHfB{chi, g, n_grid, n, n_omega}, 2 * n, n_grid, L.rchunks, -0.5f, fb);
+  launch_next(hf_pack3_kernel<FetchCols>, (unsigned)(L.tiles_ao * L.rchunks), 128, 0, st, FetchCols{ao, n}, n, n_grid,
+              L.rchunks, 1.0f, fa);
+  launch_next(hf_pack3_kernel<FetchHfB>, (unsigned)(L.tiles_j * L.rchunks), 128, 0, st, FetchHfB{chi, g, n_grid, n,
+              n_omega}, 2 * n, n_grid, L.rchunks, -0.5f, fb);
   if ((rc = check_cuda(cudaGetLastError(), "hf pack ao^T, B"))) return rc;
   TcgArgs a{};
   a.a = fa;
@@ -332,7 +337,7 @@ int hf_fock_tc(const double *ao, const double *chi, const double *g, int64_t n_g
   a.err = err;
   if ((rc = check_cuda(launch_tcg3(a, L.nsplit, st), "hf ao^T [B0|B1]"))) return rc;
   const size_t total = (size_t)2 * n * n;
-  hf_fock_reduce_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(part, L.nsplit, n, F);
+  launch_next(hf_fock_reduce_kernel, (unsigned)((total + 255) / 256), 256, 0, st, part, L.nsplit, n, F);
   return check_cuda(cudaGetLastError(), "hf fock reduce");
 }
 
@@ -384,8 +389,8 @@ int gdft_hf_energy_density_form(const double *d_ao, const double *d_rdm1, const 
                          "hf ao.D")))
       return rc;
   const int64_t threads = 2 * n_grid * 32;
-  hf_rowdot_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(d_chi, X, n_grid, n_ao, n_omega, n_ao,
-                                                                       n_grid * n_ao, d_ehf);
+  launch_next(hf_rowdot_kernel, (unsigned)((threads + 255) / 256), 256, 0, st, d_chi, X, n_grid, n_ao, n_omega, n_ao,
+              n_grid * n_ao, d_ehf);
   return check_cuda(cudaGetLastError(), "hf rowdot");
 }
 
@@ -408,7 +413,7 @@ int gdft_hf_fock_form(const double *d_ao, const double *d_chi, const double *d_g
   double *B = (double *)d_ws;
   double *part = (double *)((char *)d_ws + align256((size_t)2 * n_grid * n_ao * sizeof(double)));
   const size_t total = (size_t)2 * n_grid * n_ao;
-  hf_bmat_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(d_chi, d_g, n_grid, n_ao, n_omega, B);
+  launch_next(hf_bmat_kernel, (unsigned)((total + 255) / 256), 256, 0, st, d_chi, d_g, n_grid, n_ao, n_omega, B);
   if ((rc = check_cuda(cudaGetLastError(), "hf B"))) return rc;
   const int nsplit = hf_splits(n_grid);
   for (int s = 0; s < 2; ++s)
@@ -450,8 +455,8 @@ int gdft_fock_add_hf(double *d_fock, const double *d_fock_hf, int32_t n_ao, doub
     return GDFT_ERR_INVALID;
   }
   const size_t total = (size_t)2 * n_ao * n_ao;
-  fock_add_hf_kernel<<<(unsigned)((total + 255) / 256), 256, 0, (cudaStream_t)stream>>>(d_fock, d_fock_hf, n_ao,
-                                                                                       clip);
+  launch_next(fock_add_hf_kernel, (unsigned)((total + 255) / 256), 256, 0, (cudaStream_t)stream, d_fock, d_fock_hf,
+              n_ao, clip);
   return check_cuda(cudaGetLastError(), "fock_add_hf");
 }
 

@@ -92,6 +92,7 @@ __global__ void __launch_bounds__(32 * kWarps, 4)
     ln_elu_fwd_kernel(double *__restrict__ z, const double *__restrict__ b, const double *__restrict__ hprev,
                       const double *__restrict__ gam, const double *__restrict__ bet, double eps, int64_t rows,
                       double *__restrict__ h, double *__restrict__ rs) {
+  previous_done();
   constexpr int W = 32 * PL, E = R * PL;
   __shared__ double2 tab[expd::kTable];
   __shared__ Rows<E, 1> work[kWarps];
@@ -173,6 +174,7 @@ __global__ void __launch_bounds__(32 * kWarps, 3)
     ln_elu_bwd_kernel(double *__restrict__ dh, const double *__restrict__ xhat, const double *__restrict__ rs,
                       const double *__restrict__ gam, const double *__restrict__ bet, int64_t rows,
                       double *__restrict__ part) {
+  previous_done();
   constexpr int W = 32 * PL, E = R * PL;
   __shared__ double2 tab[expd::kTable];
   __shared__ union {
@@ -244,6 +246,7 @@ __global__ void __launch_bounds__(32 * kWarps, 4)
     ln_elu_tan_fwd_kernel(double *__restrict__ Z, const double *__restrict__ b, const double *__restrict__ Hp,
                           const double *__restrict__ gam, const double *__restrict__ bet, double eps, int64_t rows,
                           double *__restrict__ H, double *__restrict__ stat) {
+  previous_done();
   constexpr int W = 32 * PL, E = R * PL;
   __shared__ double2 tab[expd::kTable];
   __shared__ Rows<E, 2> work[kWarps];
@@ -337,6 +340,7 @@ __global__ void __launch_bounds__(32 * kWarps, 3)
     ln_elu_tan_bwd_kernel(double *__restrict__ D, const double *__restrict__ X, const double *__restrict__ stat,
                           const double *__restrict__ gam, const double *__restrict__ bet, int64_t rows,
                           double *__restrict__ part) {
+  previous_done();
   constexpr int W = 32 * PL;
   __shared__ double2 tab[expd::kTable];
   __shared__ union {
@@ -421,7 +425,8 @@ unsigned blocks_for(int64_t rows, int group) {  // a block for every group of ro
 cudaError_t launch_ln_elu_fwd(int width, double *z, const double *b, const double *hprev, const double *gam,
                               const double *bet, double eps, int64_t rows, double *h, double *rs, cudaStream_t st) {
 #define GDFT_FWD(PL) \
-  ln_elu_fwd_kernel<PL, 4><<<blocks_for(rows, 4), 32 * kWarps, 0, st>>>(z, b, hprev, gam, bet, eps, rows, h, rs)
+  launch_next(ln_elu_fwd_kernel<PL, 4>, blocks_for(rows, 4), 32 * kWarps, 0, st, z, b, hprev, gam, bet, eps, rows, h, \
+              rs)
   GDFT_WIDTHS(GDFT_FWD);
 #undef GDFT_FWD
 }
@@ -429,7 +434,7 @@ cudaError_t launch_ln_elu_fwd(int width, double *z, const double *b, const doubl
 cudaError_t launch_ln_elu_bwd(int width, double *dh, const double *xhat, const double *rs, const double *gam,
                               const double *bet, int64_t rows, double *part, cudaStream_t st) {
 #define GDFT_BWD(PL) \
-  ln_elu_bwd_kernel<PL, 2><<<kLnRowBlocks, 32 * kWarps, 0, st>>>(dh, xhat, rs, gam, bet, rows, part)
+  launch_next(ln_elu_bwd_kernel<PL, 2>, kLnRowBlocks, 32 * kWarps, 0, st, dh, xhat, rs, gam, bet, rows, part)
   GDFT_WIDTHS(GDFT_BWD);
 #undef GDFT_BWD
 }
@@ -438,14 +443,16 @@ cudaError_t launch_ln_elu_tan_fwd(int width, double *Z, const double *b, const d
                                   const double *bet, double eps, int64_t rows, double *H, double *stat,
                                   cudaStream_t st) {
 #define GDFT_FWD(PL) \
-  ln_elu_tan_fwd_kernel<PL, 2><<<blocks_for(rows, 2), 32 * kWarps, 0, st>>>(Z, b, Hp, gam, bet, eps, rows, H, stat)
+  launch_next(ln_elu_tan_fwd_kernel<PL, 2>, blocks_for(rows, 2), 32 * kWarps, 0, st, Z, b, Hp, gam, bet, eps, rows, H, \
+              stat)
   GDFT_WIDTHS(GDFT_FWD);
 #undef GDFT_FWD
 }
 
 cudaError_t launch_ln_elu_tan_bwd(int width, double *D, const double *X, const double *stat, const double *gam,
                                   const double *bet, int64_t rows, double *part, cudaStream_t st) {
-#define GDFT_BWD(PL) ln_elu_tan_bwd_kernel<PL><<<kLnRowBlocks, 32 * kWarps, 0, st>>>(D, X, stat, gam, bet, rows, part)
+#define GDFT_BWD(PL) \
+  launch_next(ln_elu_tan_bwd_kernel<PL>, kLnRowBlocks, 32 * kWarps, 0, st, D, X, stat, gam, bet, rows, part)
   GDFT_WIDTHS(GDFT_BWD);
 #undef GDFT_BWD
 }

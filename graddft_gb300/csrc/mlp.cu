@@ -39,6 +39,7 @@ namespace {
 __global__ void dm21_features_kernel(const double *__restrict__ feat, const double *__restrict__ ehf,
                                      int64_t n_grid, int64_t np, double clip, double off, double *__restrict__ x,
                                      double *__restrict__ u, double *__restrict__ e) {
+  previous_done();
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= np) return;
   double xv[kDm21In];
@@ -93,6 +94,7 @@ __global__ void dm21_features_kernel(const double *__restrict__ feat, const doub
 
 // h0 = tanh(z + b0) in place.
 __global__ void tanh_bias_kernel(double *__restrict__ z, const double *__restrict__ b, size_t total, int width) {
+  previous_done();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   z[i] = tanh(z[i] + b[i % width]);
@@ -100,6 +102,7 @@ __global__ void tanh_bias_kernel(double *__restrict__ z, const double *__restric
 
 // dp0 = dh0 * (1 - h0^2) in place.
 __global__ void tanh_bwd_kernel(double *__restrict__ dh, const double *__restrict__ h, size_t total) {
+  previous_done();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < total) dh[i] *= 1.0 - h[i] * h[i];
 }
@@ -112,6 +115,7 @@ __global__ void __launch_bounds__(256) head_energy_kernel(const double *__restri
                                                           const double *__restrict__ w, int64_t n_grid, int64_t np,
                                                           double clip, double sscale, double *__restrict__ dy,
                                                           double *__restrict__ de, double *__restrict__ epart) {
+  previous_done();
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   double e_r = 0.0;
   if (p < np) {
@@ -162,6 +166,7 @@ __global__ void __launch_bounds__(256) head_energy_kernel(const double *__restri
 __global__ void dm21_potentials_kernel(const double *__restrict__ feat, const double *__restrict__ x,
                                        const double *__restrict__ du, const double *__restrict__ de, int64_t n_grid,
                                        int64_t np, double clip, double off, double *__restrict__ coef) {
+  previous_done();
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= np) return;
   double c[2][kFeat];
@@ -218,7 +223,8 @@ __global__ void dm21_potentials_kernel(const double *__restrict__ feat, const do
 
 cudaError_t launch_dm21_features(const double *feat, const double *ehf, int64_t n_grid, int64_t np, double clip,
                                  double off, double *x, double *u, double *e, cudaStream_t st) {
-  dm21_features_kernel<<<(unsigned)((np + 255) / 256), 256, 0, st>>>(feat, ehf, n_grid, np, clip, off, x, u, e);
+  launch_next(dm21_features_kernel, (unsigned)((np + 255) / 256), 256, 0, st, feat, ehf, n_grid, np, clip, off, x, u,
+              e);
   return cudaGetLastError();
 }
 
@@ -231,6 +237,7 @@ cudaError_t launch_dm21_features(const double *feat, const double *ehf, int64_t 
 __global__ void dm21_hf_grads_kernel(const double *__restrict__ x, const double *__restrict__ du,
                                      const double *__restrict__ de, int64_t n_grid, double off,
                                      double *__restrict__ g_dens, double *__restrict__ g_cin) {
+  previous_done();
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n_grid) return;
 #pragma unroll
@@ -255,16 +262,16 @@ cudaError_t launch_dm21_hf_grads(const MlpShape &S, int64_t n_grid, int64_t np, 
 
 cudaError_t launch_dm21_hf_grads_from(const double *x, const double *du, const double *de, int64_t n_grid,
                                       double squash_offset, double *g_dens, double *g_cin, cudaStream_t st) {
-  dm21_hf_grads_kernel<<<(unsigned)((n_grid + 255) / 256), 256, 0, st>>>(x, du, de, n_grid, squash_offset, g_dens,
-                                                                          g_cin);
+  launch_next(dm21_hf_grads_kernel, (unsigned)((n_grid + 255) / 256), 256, 0, st, x, du, de, n_grid, squash_offset,
+              g_dens, g_cin);
   return cudaGetLastError();
 }
 
 cudaError_t launch_dm21_potentials(const double *feat, const double *x, const double *du, const double *de,
                                    int64_t n_grid, int64_t np, double clip, double off, double *coef,
                                    cudaStream_t st) {
-  dm21_potentials_kernel<<<(unsigned)((np + 255) / 256), 256, 0, st>>>(feat, x, du, de, n_grid, np, clip, off,
-                                                                      coef);
+  launch_next(dm21_potentials_kernel, (unsigned)((np + 255) / 256), 256, 0, st, feat, x, du, de, n_grid, np, clip, off,
+              coef);
   return cudaGetLastError();
 }
 
@@ -339,7 +346,7 @@ int net_forward(const MlpShape &S, const double *params, const MlpLayout &L, dou
     return fx::gemm_rows(np, N, K, A, lda, B, N, false, C, N, nullptr, (unsigned char *)(ws + L.fx), err, st);
   };
   if ((rc = check_cuda(mul(Wd, S.n_in, u, kDm21InPad, W0, h), "mlp dense_0"))) return rc;
-  tanh_bias_kernel<<<(unsigned)((act + 255) / 256), 256, 0, st>>>(h, b0, act, Wd);
+  launch_next(tanh_bias_kernel, (unsigned)((act + 255) / 256), 256, 0, st, h, b0, act, Wd);
   if ((rc = check_cuda(cudaGetLastError(), "mlp tanh"))) return rc;
   for (int i = 1; i <= S.n_layers; ++i) {
     const double *Wi = params + layer_offset(S, i - 1), *bi = Wi + (size_t)Wd * Wd, *gi = bi + Wd, *bei = gi + Wd;
@@ -357,6 +364,7 @@ int net_forward(const MlpShape &S, const double *params, const MlpLayout &L, dou
 // u = log(|x| + off) for given network inputs x (rows x n_in).
 __global__ void squash_kernel(const double *__restrict__ x, int64_t rows, int n_in, double off,
                               double *__restrict__ u) {
+  previous_done();
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= rows) return;
   for (int k = 0; k < kDm21InPad; ++k) u[(size_t)p * kDm21InPad + k] = k < n_in ? log(fabs(x[(size_t)p * n_in + k]) + off) : 0.0;
@@ -365,6 +373,7 @@ __global__ void squash_kernel(const double *__restrict__ x, int64_t rows, int n_
 // c = s * sigmoid((y + b) / s), written (rows x n_out).
 __global__ void head_coeff_kernel(const double *__restrict__ y, const double *__restrict__ bout, int64_t rows,
                                   int n_out, double sscale, double *__restrict__ c) {
+  previous_done();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= rows * n_out) return;
   const double yv = y[i] + bout[i % n_out];
@@ -376,8 +385,8 @@ __global__ void head_coeff_kernel(const double *__restrict__ y, const double *__
 int mlp_inputs_f64(const MlpShape &S, const double *feat, const double *ehf, int64_t n_grid, int64_t np,
                    double clip, double *ws, double *x_out, double *e_out, cudaStream_t st) {
   const MlpLayout L = mlp_layout(S, np);
-  dm21_features_kernel<<<(unsigned)L.eblocks, 256, 0, st>>>(feat, ehf, n_grid, np, clip, S.squash_offset, ws + L.x,
-                                                            ws + L.u, ws + L.e);
+  launch_next(dm21_features_kernel, (unsigned)L.eblocks, 256, 0, st, feat, ehf, n_grid, np, clip, S.squash_offset,
+              ws + L.x, ws + L.u, ws + L.e);
   int rc = check_cuda(cudaGetLastError(), "dm21_features");
   if (rc) return rc;
   if (x_out &&
@@ -395,13 +404,13 @@ int mlp_inputs_f64(const MlpShape &S, const double *feat, const double *ehf, int
 int mlp_apply_f64(const MlpShape &S, const double *params, const double *x, int64_t rows, double *ws, double *c,
                   cudaStream_t st) {
   const MlpLayout L = mlp_layout(S, rows);
-  squash_kernel<<<(unsigned)((rows + 255) / 256), 256, 0, st>>>(x, rows, S.n_in, S.squash_offset, ws + L.u);
+  launch_next(squash_kernel, (unsigned)((rows + 255) / 256), 256, 0, st, x, rows, S.n_in, S.squash_offset, ws + L.u);
   int rc = check_cuda(cudaGetLastError(), "mlp squash");
   if (rc) return rc;
   if ((rc = net_forward(S, params, L, ws, rows, nullptr, st))) return rc;
   const double *bout = params + layer_offset(S, S.n_layers) + (size_t)S.width * S.n_out;
-  head_coeff_kernel<<<(unsigned)((rows * S.n_out + 255) / 256), 256, 0, st>>>(ws + L.y, bout, rows, S.n_out,
-                                                                             S.sigmoid_scale, c);
+  launch_next(head_coeff_kernel, (unsigned)((rows * S.n_out + 255) / 256), 256, 0, st, ws + L.y, bout, rows, S.n_out,
+              S.sigmoid_scale, c);
   return check_cuda(cudaGetLastError(), "mlp head_coeff");
 }
 
@@ -430,10 +439,10 @@ int mlp_run_f64(const MlpShape &S, const double *params, double *dparams, const 
   } while (0)
 
   // ---- forward ----
-  dm21_features_kernel<<<pb, 256, 0, st>>>(feat, ehf, n_grid, np, clip, S.squash_offset, x, u, e);
+  launch_next(dm21_features_kernel, pb, 256, 0, st, feat, ehf, n_grid, np, clip, S.squash_offset, x, u, e);
   GDFT_CK(cudaGetLastError(), "dm21_features");
   if ((rc = net_forward(S, params, L, ws, np, err, st)) != GDFT_OK) return rc;
-  head_energy_kernel<<<pb, 256, 0, st>>>(y, bout, e, w, n_grid, np, clip, S.sigmoid_scale, dy, de, epart);
+  launch_next(head_energy_kernel, pb, 256, 0, st, y, bout, e, w, n_grid, np, clip, S.sigmoid_scale, dy, de, epart);
   GDFT_CK(cudaGetLastError(), "mlp head_energy");
   GDFT_CK(launch_energy_reduce(epart, (int)pb, exc, st), "mlp energy_reduce");
   if (coef == nullptr && dparams == nullptr) return GDFT_OK;
@@ -473,7 +482,7 @@ int mlp_run_f64(const MlpShape &S, const double *params, double *dparams, const 
     dnext = t;
   }
   // Layer 0: dp0 = dh0 (1 - h0^2); dW0 = u^T dp0; db0 = sum_r dp0; du = dp0 W0^T.
-  tanh_bwd_kernel<<<(unsigned)((act + 255) / 256), 256, 0, st>>>(dcur, h, act);
+  launch_next(tanh_bwd_kernel, (unsigned)((act + 255) / 256), 256, 0, st, dcur, h, act);
   GDFT_CK(cudaGetLastError(), "mlp tanh bwd");
   if (dparams) {
     GDFT_CK(weight_grad(S.n_in, Wd, u, kDm21InPad, dcur, Wd, dparams), "mlp dW_0");
@@ -481,7 +490,7 @@ int mlp_run_f64(const MlpShape &S, const double *params, double *dparams, const 
   }
   if (coef != nullptr) {
     GDFT_CK(mul_t(S.n_in, Wd, dcur, W0, du, kDm21InPad, nullptr), "mlp du");
-    dm21_potentials_kernel<<<pb, 256, 0, st>>>(feat, x, du, de, n_grid, np, clip, S.squash_offset, coef);
+    launch_next(dm21_potentials_kernel, pb, 256, 0, st, feat, x, du, de, n_grid, np, clip, S.squash_offset, coef);
     GDFT_CK(cudaGetLastError(), "dm21_potentials");
   }
 #undef GDFT_CK

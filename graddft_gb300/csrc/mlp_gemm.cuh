@@ -24,6 +24,7 @@ __global__ void __launch_bounds__(GTH) gemm_f64_kernel(int M, int N, int K, cons
                                                       const double *__restrict__ B, int ldb, double *__restrict__ C,
                                                       int ldc, const double *__restrict__ add, int kchunk,
                                                       size_t split_stride, const int *__restrict__ bad) {
+  previous_done();
   if (bad != nullptr && *bad == 0) return;
   __shared__ double As[GK][GT + 1];
   __shared__ double Bs[GK][GT + 1];
@@ -97,6 +98,7 @@ __global__ void __launch_bounds__(GTH) gemm_f64_kernel(int M, int N, int K, cons
 // C[i] = sum over splits of part[split][i] (fixed order).
 __global__ void sum_splits_kernel(const double *__restrict__ part, int nsplit, size_t total, double *__restrict__ C,
                                   const int *__restrict__ bad) {
+  previous_done();
   if (bad != nullptr && *bad == 0) return;
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
@@ -109,6 +111,7 @@ __global__ void sum_splits_kernel(const double *__restrict__ part, int nsplit, s
 // range into part[b][ncols]; second pass sums the partials in block order.
 __global__ void colsum_part_kernel(const double *__restrict__ X, int64_t rows, int ncols, int ld,
                                    double *__restrict__ part) {
+  previous_done();
   const int64_t chunk = (rows + gridDim.x - 1) / gridDim.x;
   const int64_t r0 = (int64_t)blockIdx.x * chunk, r1 = r0 + chunk < rows ? r0 + chunk : rows;
   for (int c = threadIdx.x; c < ncols; c += blockDim.x) {
@@ -122,6 +125,7 @@ __global__ void colsum_part_kernel(const double *__restrict__ X, int64_t rows, i
 // warp sums an interleaved slice of the parts, warp 0 adds the eight in order.
 __global__ void __launch_bounds__(256) colsum_final_kernel(const double *__restrict__ part, int nparts, int ncols,
                                                            double *__restrict__ out) {
+  previous_done();
   __shared__ double ws[8][32];
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int c = blockIdx.x * 32 + lane;
@@ -138,7 +142,7 @@ __global__ void __launch_bounds__(256) colsum_final_kernel(const double *__restr
   }
 }
 inline void launch_colsum_final(const double *part, int nparts, int ncols, double *out, cudaStream_t st) {
-  colsum_final_kernel<<<(ncols + 31) / 32, 256, 0, st>>>(part, nparts, ncols, out);
+  launch_next(colsum_final_kernel, (ncols + 31) / 32, 256, 0, st, part, nparts, ncols, out);
 }
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -151,7 +155,7 @@ template <int MODE>
 cudaError_t plain_gemm(int M, int N, int K, const double *A, int lda, const double *B, int ldb, double *C, int ldc,
                        const double *add, const int *bad, cudaStream_t st) {
   dim3 grid((M + GT - 1) / GT, (N + GT - 1) / GT, 1);
-  gemm_f64_kernel<MODE><<<grid, GTH, 0, st>>>(M, N, K, A, lda, B, ldb, C, ldc, add, K, 0, bad);
+  launch_next(gemm_f64_kernel<MODE>, grid, GTH, 0, st, M, N, K, A, lda, B, ldb, C, ldc, add, K, 0, bad);
   return cudaGetLastError();
 }
 
@@ -161,18 +165,19 @@ inline cudaError_t plain_gemm_tn_split(int M, int N, int64_t K, const double *A,
                                        double *C, int nsplit, double *part, const int *bad, cudaStream_t st) {
   const int kchunk = (int)(((K + nsplit - 1) / nsplit + GK - 1) / GK * GK);
   dim3 grid((M + GT - 1) / GT, (N + GT - 1) / GT, nsplit);
-  gemm_f64_kernel<kTN><<<grid, GTH, 0, st>>>(M, N, (int)K, A, lda, B, ldb, part, N, nullptr, kchunk, (size_t)M * N, bad);
+  launch_next(gemm_f64_kernel<kTN>, grid, GTH, 0, st, M, N, (int)K, A, lda, B, ldb, part, N, nullptr, kchunk,
+              (size_t)M * N, bad);
   cudaError_t r = cudaGetLastError();
   if (r != cudaSuccess) return r;
   const size_t total = (size_t)M * N;
-  sum_splits_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(part, nsplit, total, C, bad);
+  launch_next(sum_splits_kernel, (unsigned)((total + 255) / 256), 256, 0, st, part, nsplit, total, C, bad);
   return cudaGetLastError();
 }
 
 // Column sums of X (rows x ncols, stride ld) into out, in a fixed order.
 inline cudaError_t col_sums(const double *X, int64_t rows, int ncols, int ld, double *out, double *part, int nparts,
                             cudaStream_t st) {
-  colsum_part_kernel<<<nparts, 256, 0, st>>>(X, rows, ncols, ld, part);
+  launch_next(colsum_part_kernel, nparts, 256, 0, st, X, rows, ncols, ld, part);
   launch_colsum_final(part, nparts, ncols, out, st);
   return cudaGetLastError();
 }
@@ -188,6 +193,7 @@ __device__ __forceinline__ float warp_sumf(float v) {
 }
 
 __global__ void to_f32_kernel(const double *__restrict__ x, size_t n, float *__restrict__ y) {
+  previous_done();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) y[i] = (float)x[i];
 }
@@ -198,6 +204,7 @@ __global__ void to_f32_kernel(const double *__restrict__ x, size_t n, float *__r
 __global__ void head_wgrad_part_kernel(const float *__restrict__ H, const float *__restrict__ dyf,
                                        const double *__restrict__ dy, int64_t rows, int64_t rows_bias, int width,
                                        double *__restrict__ part) {
+  previous_done();
   const int64_t chunk = (rows + gridDim.x - 1) / gridDim.x;
   const int64_t r0 = (int64_t)blockIdx.x * chunk, r1 = r0 + chunk < rows ? r0 + chunk : rows;
   double *pb = part + (size_t)blockIdx.x * (3 * width + 3);

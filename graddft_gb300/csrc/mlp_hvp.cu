@@ -36,6 +36,7 @@ __global__ void features_tan_kernel(const double *__restrict__ featp, const doub
                                     const double *__restrict__ ehf, int64_t n_grid, int64_t np, double clip,
                                     double off, double *__restrict__ x, double *__restrict__ xt,
                                     double *__restrict__ u, double *__restrict__ e, double *__restrict__ et) {
+  previous_done();
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= np) return;
   double xv[kIn], xd[kIn];
@@ -116,6 +117,7 @@ __global__ void features_tan_kernel(const double *__restrict__ featp, const doub
 // added in place), H = [h; h~].
 __global__ void tanh_tan_kernel(double *__restrict__ Z, const double *__restrict__ b, size_t act, int width,
                                 double *__restrict__ H) {
+  previous_done();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= act) return;
   const double z = Z[i] + b[i % width];
@@ -133,6 +135,7 @@ __global__ void __launch_bounds__(256) head_tan_kernel(const double *__restrict_
                                                        const double *__restrict__ w, int64_t n_grid, int64_t np,
                                                        double clip, double sscale, double *__restrict__ GY,
                                                        double *__restrict__ ge, double *__restrict__ lpart) {
+  previous_done();
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   double l_r = 0.0;
   if (p < np) {
@@ -192,6 +195,7 @@ __global__ void __launch_bounds__(256) head_tan_kernel(const double *__restrict_
 // Reverse of layer 0: D = [dL/dh0; dL/dh0~] -> [dL/dz0; dL/dz0~] in place.
 __global__ void tanh_tan_bwd_kernel(double *__restrict__ D, const double *__restrict__ H,
                                     const double *__restrict__ Z, size_t act) {
+  previous_done();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= act) return;
   const double h = H[i], s = 1.0 - h * h;
@@ -205,6 +209,7 @@ __global__ void hvp_potentials_kernel(const double *__restrict__ featp, const do
                                       const double *__restrict__ x, const double *__restrict__ xt,
                                       const double *__restrict__ GU, const double *__restrict__ ge, int64_t n_grid,
                                       int64_t np, double clip, double off, double *__restrict__ coef) {
+  previous_done();
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= np) return;
   double c[2][kFeat];
@@ -276,16 +281,16 @@ size_t hvp_layer_offset(const MlpShape &S, int i) {
 cudaError_t launch_features_tan(const double *featp, const double *featt, const double *ehf, int64_t n_grid,
                                 int64_t np, double clip, double off, double *x, double *xt, double *u, double *e,
                                 double *et, cudaStream_t st) {
-  features_tan_kernel<<<(unsigned)((np + 255) / 256), 256, 0, st>>>(featp, featt, ehf, n_grid, np, clip, off, x, xt,
-                                                                   u, e, et);
+  launch_next(features_tan_kernel, (unsigned)((np + 255) / 256), 256, 0, st, featp, featt, ehf, n_grid, np, clip, off,
+              x, xt, u, e, et);
   return cudaGetLastError();
 }
 
 cudaError_t launch_hvp_potentials(const double *featp, const double *featt, const double *x, const double *xt,
                                   const double *GU, const double *ge, int64_t n_grid, int64_t np, double clip,
                                   double off, double *coef, cudaStream_t st) {
-  hvp_potentials_kernel<<<(unsigned)((np + 255) / 256), 256, 0, st>>>(featp, featt, x, xt, GU, ge, n_grid, np, clip,
-                                                                     off, coef);
+  launch_next(hvp_potentials_kernel, (unsigned)((np + 255) / 256), 256, 0, st, featp, featt, x, xt, GU, ge, n_grid, np,
+              clip, off, coef);
   return cudaGetLastError();
 }
 
@@ -355,10 +360,11 @@ int mlp_hvp_f64(const MlpShape &S, const double *params, double *dparams, const 
   };
 
   // ---- tangent-augmented forward ----
-  features_tan_kernel<<<pb, 256, 0, st>>>(featp, featt, ehf, n_grid, np, clip, S.squash_offset, x, xt, U, e, et);
+  launch_next(features_tan_kernel, pb, 256, 0, st, featp, featt, ehf, n_grid, np, clip, S.squash_offset, x, xt, U, e,
+              et);
   GDFT_CK(cudaGetLastError(), "hvp features");
   GDFT_CK(mul(Wd, S.n_in, U, kInPad, W0, Z), "hvp dense_0");
-  tanh_tan_kernel<<<(unsigned)((act + 255) / 256), 256, 0, st>>>(Z, b0, act, Wd, H);
+  launch_next(tanh_tan_kernel, (unsigned)((act + 255) / 256), 256, 0, st, Z, b0, act, Wd, H);
   GDFT_CK(cudaGetLastError(), "hvp tanh");
   for (int i = 1; i <= S.n_layers; ++i) {
     const double *Wi = params + hvp_layer_offset(S, i - 1), *bi = Wi + (size_t)Wd * Wd, *gi = bi + Wd,
@@ -369,7 +375,7 @@ int mlp_hvp_f64(const MlpShape &S, const double *params, double *dparams, const 
   }
   double *HL = H + (size_t)S.n_layers * act2;
   GDFT_CK(mul(S.n_out, Wd, HL, Wd, Wout, Y), "hvp head");
-  head_tan_kernel<<<pb, 256, 0, st>>>(Y, bout, e, et, w, n_grid, np, clip, S.sigmoid_scale, GY, GE, lpart);
+  launch_next(head_tan_kernel, pb, 256, 0, st, Y, bout, e, et, w, n_grid, np, clip, S.sigmoid_scale, GY, GE, lpart);
   GDFT_CK(cudaGetLastError(), "hvp head_tan");
   if (lval) GDFT_CK(launch_energy_reduce(lpart, (int)pb, lval, st), "hvp value");
 
@@ -401,7 +407,7 @@ int mlp_hvp_f64(const MlpShape &S, const double *params, double *dparams, const 
     dcur = dnext;
     dnext = t;
   }
-  tanh_tan_bwd_kernel<<<(unsigned)((act + 255) / 256), 256, 0, st>>>(dcur, H, Z, act);
+  launch_next(tanh_tan_bwd_kernel, (unsigned)((act + 255) / 256), 256, 0, st, dcur, H, Z, act);
   GDFT_CK(cudaGetLastError(), "hvp tanh bwd");
   if (dparams) {
     GDFT_CK(wgrad(S.n_in, Wd, U, kInPad, dcur, Wd, dparams), "hvp dW_0");
@@ -409,7 +415,8 @@ int mlp_hvp_f64(const MlpShape &S, const double *params, double *dparams, const 
   }
   if (coef) {
     GDFT_CK(mul_t(S.n_in, Wd, dcur, W0, GU, kInPad, nullptr), "hvp du");
-    hvp_potentials_kernel<<<pb, 256, 0, st>>>(featp, featt, x, xt, GU, GE, n_grid, np, clip, S.squash_offset, coef);
+    launch_next(hvp_potentials_kernel, pb, 256, 0, st, featp, featt, x, xt, GU, GE, n_grid, np, clip, S.squash_offset,
+                coef);
     GDFT_CK(cudaGetLastError(), "hvp potentials");
   }
 #undef GDFT_CK

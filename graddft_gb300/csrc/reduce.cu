@@ -19,6 +19,7 @@ __device__ __forceinline__ void add_pair(double &s, double &e, double s2, double
 }
 __global__ void __launch_bounds__(256) energy_reduce_kernel(const double *__restrict__ part, int n,
                                                             double *__restrict__ out) {
+  previous_done();
   __shared__ double hs[8], he[8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   Kahan k{0.0, 0.0};
@@ -45,6 +46,7 @@ __global__ void __launch_bounds__(256) energy_reduce_kernel(const double *__rest
 // Sum of the split-K partial V tiles in a fixed order (deterministic).
 __global__ void vxc_reduce_kernel(const double *__restrict__ part, int nsplit, size_t total,
                                   double *__restrict__ out, const int *__restrict__ bad) {
+  previous_done();
   if (bad != nullptr && *bad == 0) return;
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
@@ -55,6 +57,7 @@ __global__ void vxc_reduce_kernel(const double *__restrict__ part, int nsplit, s
 
 __global__ void feat_to_ref_kernel(const double *__restrict__ feat, int64_t n_grid, int64_t np, double *rho,
                                    double *grad_rho, double *lapl, double *tau) {
+  previous_done();
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n_grid) return;
 #pragma unroll
@@ -74,6 +77,7 @@ __global__ void feat_to_ref_kernel(const double *__restrict__ feat, int64_t n_gr
 // predict's Fock assembly (train.py:147-163).
 __global__ void fock_kernel(int n, const double *__restrict__ h1e, const double *__restrict__ vj,
                             const double *__restrict__ vxc, double clip, double *__restrict__ fock) {
+  previous_done();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t nn = (size_t)n * n;
   if (i >= 2 * nn) return;
@@ -87,6 +91,7 @@ __global__ void fock_kernel(int n, const double *__restrict__ h1e, const double 
 // J_pq = sum_rt (pq|rt) (D_a + D_b)_rt, one warp per (p, q) (molecule.py:783-811).
 __global__ void coulomb_kernel(int n, const double *__restrict__ eri, const double *__restrict__ rdm1,
                                double *__restrict__ vj) {
+  previous_done();
   const size_t warp = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const size_t nn = (size_t)n * n;
@@ -102,6 +107,7 @@ __global__ void coulomb_kernel(int n, const double *__restrict__ eri, const doub
 // E_nuc + tr(D h1e) + 1/2 tr(D J) (molecule.py:694-781).
 __global__ void nonxc_kernel(int n, const double *__restrict__ rdm1, const double *__restrict__ h1e,
                              const double *__restrict__ vj, double enuc, double *__restrict__ out) {
+  previous_done();
   __shared__ double sh[256], sj[256];
   const size_t nn = (size_t)n * n;
   double a = 0.0, b = 0.0;
@@ -126,6 +132,7 @@ __global__ void nonxc_kernel(int n, const double *__restrict__ rdm1, const doubl
 // Functional.xc_energy on given densities (functional.py:219-253, :316-342).
 __global__ void integrate_kernel(int64_t n_grid, int n_cols, gdft_functional fn, const double *__restrict__ dens,
                                  const double *__restrict__ w, double *__restrict__ part) {
+  previous_done();
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   double e_r = 0.0;
   if (p < n_grid) {
@@ -154,6 +161,7 @@ __global__ void integrate_kernel(int64_t n_grid, int n_cols, gdft_functional fn,
 // (2, 6, n_grid) -> [2][6][np] (padded points get zero potentials).
 __global__ void pad_potentials_kernel(const double *__restrict__ pot, int64_t n_grid, int64_t np,
                                       double *__restrict__ coef) {
+  previous_done();
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= np) return;
 #pragma unroll
@@ -163,7 +171,7 @@ __global__ void pad_potentials_kernel(const double *__restrict__ pot, int64_t n_
 }  // namespace
 
 cudaError_t launch_pad_potentials(const double *pot, int64_t n_grid, int64_t np, double *coef, cudaStream_t st) {
-  pad_potentials_kernel<<<(unsigned)((np + 255) / 256), 256, 0, st>>>(pot, n_grid, np, coef);
+  launch_next(pad_potentials_kernel, (unsigned)((np + 255) / 256), 256, 0, st, pot, n_grid, np, coef);
   return cudaGetLastError();
 }
 
@@ -171,54 +179,56 @@ int integrate_blocks(int64_t n_grid) { return (int)((n_grid + 255) / 256); }
 
 cudaError_t launch_integrate(int64_t n_grid, int n_cols, const gdft_functional &fn, const double *dens,
                              const double *w, double *epart, cudaStream_t st) {
-  integrate_kernel<<<integrate_blocks(n_grid), 256, 0, st>>>(n_grid, n_cols, fn, dens, w, epart);
+  launch_next(integrate_kernel, integrate_blocks(n_grid), 256, 0, st, n_grid, n_cols, fn, dens, w, epart);
   return cudaGetLastError();
 }
 
 // Move a per-call error word into a persistent one (the first code recorded wins) and clear it.
 __global__ void err_fold_kernel(int *__restrict__ dst, int *__restrict__ src) {
+  previous_done();
   const int e = *src;
   if (e != 0) atomicCAS(dst, 0, e);
   *src = 0;
 }
 
 cudaError_t launch_err_fold(int *dst, int *src, cudaStream_t st) {
-  err_fold_kernel<<<1, 1, 0, st>>>(dst, src);
+  launch_next(err_fold_kernel, 1, 1, 0, st, dst, src);
   return cudaGetLastError();
 }
 
 cudaError_t launch_energy_reduce(const double *epart, int n, double *exc, cudaStream_t st) {
-  energy_reduce_kernel<<<1, 256, 0, st>>>(epart, n, exc);
+  launch_next(energy_reduce_kernel, 1, 256, 0, st, epart, n, exc);
   return cudaGetLastError();
 }
 
 cudaError_t launch_vxc_reduce(const double *vpart, int nsplit, int n_ao, double *vxc, const int *bad,
                               cudaStream_t st) {
   const size_t total = (size_t)2 * n_ao * n_ao;
-  vxc_reduce_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(vpart, nsplit, total, vxc, bad);
+  launch_next(vxc_reduce_kernel, (unsigned)((total + 255) / 256), 256, 0, st, vpart, nsplit, total, vxc, bad);
   return cudaGetLastError();
 }
 
 cudaError_t launch_feat_to_reference(const double *feat, int64_t n_grid, int64_t np, double *rho, double *grad_rho,
                                      double *lapl, double *tau, cudaStream_t st) {
-  feat_to_ref_kernel<<<(unsigned)((n_grid + 255) / 256), 256, 0, st>>>(feat, n_grid, np, rho, grad_rho, lapl, tau);
+  launch_next(feat_to_ref_kernel, (unsigned)((n_grid + 255) / 256), 256, 0, st, feat, n_grid, np, rho, grad_rho, lapl,
+              tau);
   return cudaGetLastError();
 }
 
 cudaError_t launch_fock(int n_ao, const double *h1e, const double *vj, const double *vxc, double clip, double *fock,
                         cudaStream_t st) {
   const size_t total = (size_t)2 * n_ao * n_ao;
-  fock_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(n_ao, h1e, vj, vxc, clip, fock);
+  launch_next(fock_kernel, (unsigned)((total + 255) / 256), 256, 0, st, n_ao, h1e, vj, vxc, clip, fock);
   return cudaGetLastError();
 }
 
 cudaError_t launch_coulomb(int n_ao, const double *eri, const double *rdm1, const double *h1e, double enuc,
                            double *vj, double *enonxc, cudaStream_t st) {
   const size_t nn = (size_t)n_ao * n_ao;
-  coulomb_kernel<<<(unsigned)((nn * 32 + 255) / 256), 256, 0, st>>>(n_ao, eri, rdm1, vj);
+  launch_next(coulomb_kernel, (unsigned)((nn * 32 + 255) / 256), 256, 0, st, n_ao, eri, rdm1, vj);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  if (enonxc != nullptr) nonxc_kernel<<<1, 256, 0, st>>>(n_ao, rdm1, h1e, vj, enuc, enonxc);
+  if (enonxc != nullptr) launch_next(nonxc_kernel, 1, 256, 0, st, n_ao, rdm1, h1e, vj, enuc, enonxc);
   return cudaGetLastError();
 }
 

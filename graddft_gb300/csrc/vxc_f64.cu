@@ -24,6 +24,7 @@ constexpr int NT = 256;
 __global__ void __launch_bounds__(NT) vxc_f64_kernel(const double *__restrict__ tab, int64_t np, int ld, int n,
                                                      const double *__restrict__ coef, int64_t chunk,
                                                      double *__restrict__ vpart, const int *__restrict__ bad) {
+  previous_done();
   if (bad != nullptr && *bad == 0) return;
   __shared__ double Ps[4][BK][BT];
   __shared__ double Qs[2][4][BK][BT];
@@ -135,7 +136,7 @@ cudaError_t launch_vxc_f64(const double *tab, int64_t np, int ld, int n_ao, cons
   int64_t chunk = (np + nsplit - 1) / nsplit;
   chunk = (chunk + BK - 1) / BK * BK;
   dim3 grid(tiles_a * tiles_a, nsplit);
-  vxc_f64_kernel<<<grid, NT, 0, st>>>(tab, np, ld, n_ao, coef, chunk, vpart, bad);
+  launch_next(vxc_f64_kernel, grid, NT, 0, st, tab, np, ld, n_ao, coef, chunk, vpart, bad);
   return cudaGetLastError();
 }
 

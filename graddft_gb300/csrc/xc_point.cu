@@ -120,6 +120,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps) xc_point_kernel(const double *
                                                                   const double *__restrict__ ehf, int n_omega,
                                                                   double *__restrict__ coef, double *__restrict__ epart,
                                                                   double *__restrict__ dens, double *__restrict__ ghf) {
+  previous_done();
   extern __shared__ double cols[];  // [column][1 + KV][point]: value and partials
   __shared__ unsigned poisoned[kMaxWarps][kPoints];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -244,6 +245,8 @@ cudaError_t launch_xc_point(const double *feat, const double *w, int64_t n_grid,
   for (int i = 0; i < fn.n_cols; ++i) reads_tau |= is_uw_col(fn.cols[i]) && uw_j(fn.cols[i]) != 0;
   const int warps = blocks > kSplitBlocks ? 1 : fn.n_cols < kMaxWarps ? fn.n_cols : kMaxWarps;
   const size_t smem = (size_t)fn.n_cols * (1 + (reads_tau ? 8 : 6)) * kPoints * sizeof(double);  // at most 36 KB
+  // Not chained to the kernel before it: its blocks would be placed before that one leaves the SMs, and crowd on some
+  // of them (24 AOs x 3,600 points, BLYP: 161 us a call, chained 173).
   if (reads_tau)
     xc_point_kernel<8><<<blocks, 32 * warps, smem, st>>>(feat, w, n_grid, np, fn, ehf, n_omega, coef, epart, dens, ghf);
   else
