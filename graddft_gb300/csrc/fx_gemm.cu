@@ -574,7 +574,14 @@ cudaError_t launch_gemm(const GemmArgs &a, cudaStream_t st) {
   if (items < 1) return cudaSuccess;
   if (items > 0x3FFFFFFF) return cudaErrorInvalidValue;
   const unsigned grid = (unsigned)(items < sms ? items : sms);
-  launch_next(fx_gemm_kernel, grid, kThreads, kSmemBytes, st, a, upper);
+  // Chained (common.cuh) where few CTAs share an operand tile.  CTAs placed as SMs fall free do not start side by side,
+  // and with more tiles in both directions those on one tile then miss each other in L2 (BLYP 400 x 150,001, 4 x 7 and
+  // 74 x 7 tiles, 24.8 ms, chained 25.6; features of 187 AOs x 100,003 2.59 and 2.73; B88 115 x 65,536, two tiles, 1,191 us and
+  // 1,177).
+  if (a.m_tiles <= 2 || a.n_tiles <= 2)
+    launch_next(fx_gemm_kernel, grid, kThreads, kSmemBytes, st, a, upper);
+  else
+    fx_gemm_kernel<<<grid, kThreads, kSmemBytes, st>>>(a, upper);
   return cudaGetLastError();
 }
 
