@@ -173,18 +173,6 @@ __device__ __forceinline__ void tmem_ld_wait(uint32_t (&a)[16], uint32_t (&b)[16
   for (int i = 0; i < 16; ++i) asm volatile("" : "+r"(a[i]), "+r"(b[i]));
 }
 
-// 8 consecutive 32-bit TMEM columns of this thread's lane, without waiting.
-__device__ __forceinline__ void tmem_ld8_nowait(uint32_t taddr, uint32_t (&r)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-               : "r"(taddr));
-}
-__device__ __forceinline__ void tmem_ld_wait(uint32_t (&a)[8], uint32_t (&b)[8]) {
-  tmem_ld_wait();
-#pragma unroll
-  for (int i = 0; i < 8; ++i) asm volatile("" : "+r"(a[i]), "+r"(b[i]));
-}
-
 // Store 32 consecutive 32-bit TMEM columns of this thread's lane (warp-collective).
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const float (&v)[32]) {
   asm volatile(
