@@ -13,13 +13,15 @@
 // The products of orders 5 and 6 are issued between those of L and H, which gives
 // a drain about 1,300 clocks (float-to-integer conversions run at 16 per clock:
 // 1,024 for one order), and in an order that frees the digits a chunk starts with
-// six pairs before its end.  Few barriers: a wait costs the issuer some 150 clocks,
-// so a chunk's blocks arrive in five groups.
+// six pairs before its end.  Few waits: each leaves the tensor core idle for some 110
+// clocks, so a chunk's blocks arrive in four groups and the drains' releases count
+// towards two of them.
 //
 // What bounds it: 28 digit pairs take 7,168 clocks a chunk at the dense BF16 rate.
-// Measured with 38,912 rows, K 1,024, N 128 (A read from HBM): 11,300 clocks a
-// chunk (12,400 while the copies were issued in a loop), of which the copies take
-// about 1,500, the drains 1,300 and an item's output 1,200; 54 TFLOP/s of FP64
+// Measured with 38,912 rows, K 1,024, N 128 (A read from HBM): 11,020 clocks a
+// chunk (12,400 while the copies were issued in a loop, 11,200 with eight waits a
+// chunk instead of five), of which the copies take
+// about 1,500, the drains 1,300 and an item's output 1,200; 55 TFLOP/s of FP64
 // products, where the FP64 pipe gives 1.1.  An item's output costs some 16,000
 // clocks whatever its K.  Error against quadruple
 // precision 4.7e-17 (a sequential FP64 sum: 1.1e-15).
@@ -50,9 +52,9 @@ constexpr int kSumChunks = 16;  // chunks of one 64-bit sum, then it is added to
 
 // A chunk's blocks (0-6: A's digits, 7-13: B's) arrive in groups, in the order in
 // which they are first read; a group's slots are free again together.
-constexpr int kGroups = 5;
+constexpr int kGroups = 4;
 __device__ constexpr int kGroupOf[2 * kDigits] = {0, 7, 8, 1, 5, 6, 12, 13, 9, 10, 2, 3, 4, 11};
-__device__ constexpr int kGroupAt[kGroups + 1] = {0, 3, 4, 8, 11, 14};
+__device__ constexpr int kGroupAt[kGroups + 1] = {0, 4, 8, 11, 14};
 
 struct Item {
   int plane, mt, nt, c0, c1, split, base;  // base: set of chunk 0 within the tile's sets
@@ -181,7 +183,7 @@ __global__ void __launch_bounds__(kThreads, 1) fx_gemm_kernel(const GemmArgs A, 
   if (A.bad != nullptr && *A.bad != 0) return;
   extern __shared__ unsigned char smem_raw[];
   unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  __shared__ __align__(8) uint64_t full[kGroups], empty[kGroups], yfull[2], yempty[2], zfull, zempty, drain;
+  __shared__ __align__(8) uint64_t full[kGroups], empty[kGroups], yfull[2], yempty, zfull, zempty, drain;
   __shared__ uint32_t tmem_base;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -189,13 +191,11 @@ __global__ void __launch_bounds__(kThreads, 1) fx_gemm_kernel(const GemmArgs A, 
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kGroups; ++s) {
-      umma::mbar_init(&full[s], 1);
+      umma::mbar_init(&full[s], s == 0 || s == 2 ? 1 + kDrains : 1);  // the copies, and accumulators drained
       umma::mbar_init(&empty[s], 1);
     }
-    for (int b = 0; b < 2; ++b) {
-      umma::mbar_init(&yfull[b], 1);
-      umma::mbar_init(&yempty[b], kDrains);
-    }
+    for (int b = 0; b < 2; ++b) umma::mbar_init(&yfull[b], 1);
+    umma::mbar_init(&yempty, kDrains);
     umma::mbar_init(&zfull, 1);
     umma::mbar_init(&zempty, kDrains);
     umma::mbar_init(&drain, 1);
@@ -281,8 +281,6 @@ __global__ void __launch_bounds__(kThreads, 1) fx_gemm_kernel(const GemmArgs A, 
       };
       auto ready = [&](int g) { check(umma::mbar_wait(&full[g], chunk & 1), 73); };
       auto done = [&](int g) { umma::mma_commit(&empty[g]); };
-      // The drains are done with fill `fills - 1` of accumulator b.
-      auto free_y = [&](int b, uint32_t fills) { check(umma::mbar_wait(&yempty[b], (fills & 1) ^ 1), 74); };
       // Digit i of A times digit j of B (n 128) or digits j and j + 1 (n 256) into TMEM columns d.
       auto mul = [&](uint32_t d, int n, int i, int j, bool first) {
         const uint32_t a = d0 + i * (kBlockBytes >> 4), b = d0 + (kDigits + j) * (kBlockBytes >> 4);
@@ -296,50 +294,46 @@ __global__ void __launch_bounds__(kThreads, 1) fx_gemm_kernel(const GemmArgs A, 
         for (int c = t.c0; c < t.c1 && ok; ++c, ++chunk) {
           const bool zfirst = (c - t.c0) % kSumChunks == 0;
           const bool zlast = (c - t.c0) % kSumChunks == kSumChunks - 1 || c + 1 == t.c1;
-          // L is filled three times a chunk (orders 0, 2, 4), H twice (1, 3); the drains take them in order, so
-          // the last one needed stands for both.
+          // L is filled three times a chunk (orders 0, 2, 4), H twice (1, 3).  The drains take them in order, so the
+          // last one needed stands for both; the release of order 4 counts towards the next chunk's group 0, that of
+          // order 1 towards group 2: one wait for both.
           ready(0);
-          free_y(0, 3 * chunk);
           if (!ok) break;
           mul(l, 256, 0, 0, true);
           umma::mma_commit(&yfull[0]);
-          ready(1);
-          if (!ok) break;
           mul(h, 128, 1, 0, false);
           umma::mma_commit(&yfull[1]);
-          ready(2);
+          ready(1);
           if (zfirst) check(umma::mbar_wait(&zempty, (group & 1) ^ 1), 75);
           if (!ok) break;
           mul(z5, 256, 5, 0, zfirst);
           mul(z6, 128, 6, 0, false);
           mul(z5, 256, 0, 5, false);
-          ready(3);
-          free_y(1, 2 * chunk + 1);
+          ready(2);
           if (!ok) break;
           mul(l, 256, 0, 2, true);
           mul(l, 256, 1, 1, false);
           mul(l, 256, 2, 0, false);
           umma::mma_commit(&yfull[0]);
-          ready(4);
+          ready(3);
           if (!ok) break;
           mul(h, 128, 3, 0, false);
           umma::mma_commit(&yfull[1]);
           mul(z5, 256, 4, 1, false);
           mul(z5, 256, 1, 4, false);
-          done(2);
-          free_y(0, 3 * chunk + 2);
+          done(1);
+          check(umma::mbar_wait(&yempty, chunk & 1), 74);  // order 2 is drained
           if (!ok) break;
           mul(l, 128, 0, 4, true);
           mul(l, 128, 4, 0, false);
           mul(l, 128, 3, 1, false);
-          done(0);
           mul(l, 128, 1, 3, false);
-          done(1);
+          done(0);
           mul(l, 128, 2, 2, false);
           umma::mma_commit(&yfull[0]);
           mul(z5, 256, 2, 3, false);
           mul(z5, 256, 3, 2, false);
-          done(3), done(4);
+          done(2), done(3);
           if (zlast) {
             umma::mma_commit(&zfull);
             ++group;
@@ -367,12 +361,12 @@ __global__ void __launch_bounds__(kThreads, 1) fx_gemm_kernel(const GemmArgs A, 
       }
       umma::tc_fence_after();
     };
-    // Columns of accumulator b to `take`; b is free again once the last are in registers.
-    auto drain = [&](int b, int cols, auto &&take) {
+    // Columns of accumulator b to `take`; once the last are in registers, `freed` (if any) hears of it.
+    auto drain = [&](int b, int cols, uint64_t *freed, auto &&take) {
       auto release = [&]() {
         umma::tc_fence_before();
         __syncwarp();
-        if (lane == 0) umma::mbar_arrive(&yempty[b]);
+        if (lane == 0 && freed != nullptr) umma::mbar_arrive(freed);
       };
       if (cols == 0) {
         release();
@@ -389,6 +383,7 @@ __global__ void __launch_bounds__(kThreads, 1) fx_gemm_kernel(const GemmArgs A, 
       }
       __syncwarp();
     };
+    if (lane == 0) umma::mbar_arrive(&full[0]);  // L and H are free
     long long sum[kCols];  // orders 0..4 of this thread's row, unit 2^-36 (below 2^59 a chunk)
     for (int i = blockIdx.x; i < items; i += gridDim.x) {
       const Item t = item_of(A, upper, i);
@@ -408,7 +403,7 @@ __global__ void __launch_bounds__(kThreads, 1) fx_gemm_kernel(const GemmArgs A, 
 #pragma unroll
         for (int d = 0; d < 2; ++d) {
           wait(&yfull[d], (d ? 2 * chunk : 3 * chunk) & 1, 77);
-          drain(d, cols, [&](int k, uint32_t y) {
+          drain(d, cols, d ? &full[2] : nullptr, [&](int k, uint32_t y) {
             const int v = __float_as_int(__uint_as_float(y) + (d ? 24576.0f : 12582912.0f));
             sum[k] += (long long)v << (36 - 9 * d);
           });
@@ -418,7 +413,7 @@ __global__ void __launch_bounds__(kThreads, 1) fx_gemm_kernel(const GemmArgs A, 
           const int b = d & 1, sh = 36 - 9 * d;
           const float f = __uint_as_float((uint32_t)(127 + 9 * d) << 23);
           wait(&yfull[b], (b ? 2 * chunk + 1 : 3 * chunk + d / 2) & 1, 77);
-          drain(b, cols, [&](int k, uint32_t y) {
+          drain(b, cols, d == 2 ? &yempty : d == 4 ? &full[0] : nullptr, [&](int k, uint32_t y) {
             add_shifted(sum[k], __float2int_rn(__uint_as_float(y) * f), sh, 32 - sh);
           });
         }
