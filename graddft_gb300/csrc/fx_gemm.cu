@@ -14,13 +14,13 @@
 // a drain about 1,300 clocks (float-to-integer conversions run at 16 per clock:
 // 1,024 for one order), and in an order that frees the digits a chunk starts with
 // six pairs before its end.  Few waits: each leaves the tensor core idle for some 110
-// clocks, so a chunk's blocks arrive in four groups and the drains' releases count
+// clocks, so a chunk's blocks arrive in three groups and the drains' releases count
 // towards two of them.
 //
 // What bounds it: 28 digit pairs take 7,168 clocks a chunk at the dense BF16 rate.
 // Measured with 38,912 rows, K 1,024, N 128 (A read from HBM): 11,020 clocks a
 // chunk (12,400 while the copies were issued in a loop, 11,200 with eight waits a
-// chunk instead of five), of which the copies take
+// chunk instead of four), of which the copies take
 // about 1,500, the drains 1,300 and an item's output 1,200; 55 TFLOP/s of FP64
 // products, where the FP64 pipe gives 1.1.  An item's output costs some 16,000
 // clocks whatever its K.  Error against quadruple
@@ -52,9 +52,9 @@ constexpr int kSumChunks = 16;  // chunks of one 64-bit sum, then it is added to
 
 // A chunk's blocks (0-6: A's digits, 7-13: B's) arrive in groups, in the order in
 // which they are first read; a group's slots are free again together.
-constexpr int kGroups = 4;
+constexpr int kGroups = 3;
 __device__ constexpr int kGroupOf[2 * kDigits] = {0, 7, 8, 1, 5, 6, 12, 13, 9, 10, 2, 3, 4, 11};
-__device__ constexpr int kGroupAt[kGroups + 1] = {0, 4, 8, 11, 14};
+__device__ constexpr int kGroupAt[kGroups + 1] = {0, 4, 8, 14};
 
 struct Item {
   int plane, mt, nt, c0, c1, split, base;  // base: set of chunk 0 within the tile's sets
@@ -315,8 +315,6 @@ __global__ void __launch_bounds__(kThreads, 1) fx_gemm_kernel(const GemmArgs A, 
           mul(l, 256, 1, 1, false);
           mul(l, 256, 2, 0, false);
           umma::mma_commit(&yfull[0]);
-          ready(3);
-          if (!ok) break;
           mul(h, 128, 3, 0, false);
           umma::mma_commit(&yfull[1]);
           mul(z5, 256, 4, 1, false);
@@ -333,7 +331,7 @@ __global__ void __launch_bounds__(kThreads, 1) fx_gemm_kernel(const GemmArgs A, 
           umma::mma_commit(&yfull[0]);
           mul(z5, 256, 2, 3, false);
           mul(z5, 256, 3, 2, false);
-          done(2), done(3);
+          done(2);
           if (zlast) {
             umma::mma_commit(&zfull);
             ++group;
