@@ -78,16 +78,21 @@ __global__ void __launch_bounds__(128) fx_rdm1_kernel(const double *__restrict__
 
 // Row products of X with the planes -> feat.  X is [plane][spin][column][slab
 // point], the planes [point][ld]: a block takes 32 points and walks the columns
-// in tiles of 32, the planes' tile through shared memory (rows in, columns out),
-// X directly (lanes are points); both spins share a tile.
-constexpr int kFeatTile = 32;
-__global__ void __launch_bounds__(256) fx_features_kernel(const double *__restrict__ tab, size_t pe, int64_t np, int ld,
+// in tiles of 16, the planes' tile through shared memory (rows in, columns out),
+// X directly (lanes are points); both spins share a tile.  Bound by the FP64 pipe
+// (16 FMA per point and column); the next tile is copied asynchronously while one
+// is used, and at 43 KB four blocks share an SM: 9,376 x 400 148 -> 130 us (one tile
+// of 32 at a time; two of 32 127, but 79.5 against 75.9 at 33,920 x 43), where the
+// pipe needs 108.
+constexpr int kFeatTile = 32;  // points
+constexpr int kFeatCols = 16;
+__global__ void __launch_bounds__(256, 4) fx_features_kernel(const double *__restrict__ tab, size_t pe, int64_t np, int ld,
                                                           int64_t p0, int64_t slab, const double *__restrict__ X,
                                                           int cols, bool kin, double *__restrict__ feat,
                                                           const int *__restrict__ bad) {
   previous_done();
   if (*bad != 0) return;
-  __shared__ double t[kPlanes][kFeatTile][kFeatTile + 1];
+  __shared__ double tile[2][kPlanes][kFeatTile][kFeatCols + 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t r0 = (int64_t)blockIdx.x * kFeatTile;
   const int planes = kin ? kPlanes : 4;
@@ -97,14 +102,27 @@ __global__ void __launch_bounds__(256) fx_features_kernel(const double *__restri
   for (int s = 0; s < 2; ++s)
 #pragma unroll
     for (int k = 0; k < 6; ++k) f[s][k] = 0.0;
-  for (int c0 = 0; c0 < ld; c0 += kFeatTile) {  // ld is a multiple of 32
+  auto fetch = [&](int c0, int b) {  // the planes' columns c0 .. c0 + 15, 16 lanes a point
+    const int l = threadIdx.x % kFeatCols;
+    for (int i = threadIdx.x / kFeatCols; i < planes * kFeatTile; i += 256 / kFeatCols) {
+      const unsigned dst = (unsigned)__cvta_generic_to_shared(&tile[b][i / kFeatTile][i % kFeatTile][l]);
+      const double *src = tab + (size_t)(i / kFeatTile) * pe + (size_t)(p0 + r0 + i % kFeatTile) * ld + c0 + l;
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  fetch(0, 0);
+  for (int c0 = 0, b = 0; c0 < ld; c0 += kFeatCols, b ^= 1) {  // ld is a multiple of 32
+    if (c0 + kFeatCols < ld) {
+      fetch(c0 + kFeatCols, b ^ 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
     __syncthreads();
-    for (int i = warp; i < planes * kFeatTile; i += 8)
-      t[i / kFeatTile][i % kFeatTile][lane] =
-          tab[(size_t)(i / kFeatTile) * pe + (size_t)(p0 + r0 + i % kFeatTile) * ld + c0 + lane];
-    __syncthreads();
+    const auto &t = tile[b];
 #pragma unroll
-    for (int k = 0; k < kFeatTile / 8; ++k) {
+    for (int k = 0; k < kFeatCols / 8; ++k) {
       const int c = warp + 8 * k;
       const double phi = t[T_PHI][lane][c], dx = t[T_DX][lane][c], dy = t[T_DY][lane][c], dz = t[T_DZ][lane][c];
       const double *x = X + (size_t)(c0 + c) * slab + r0 + lane;
@@ -123,9 +141,9 @@ __global__ void __launch_bounds__(256) fx_features_kernel(const double *__restri
         }
       }
     }
+    __syncthreads();
   }
-  __syncthreads();
-  double *red = &t[0][0][0];  // [warp][spin * 6 + feature][point]
+  double *red = &tile[0][0][0][0];  // [warp][spin * 6 + feature][point]
 #pragma unroll
   for (int k = 0; k < 12; ++k) red[(warp * 12 + k) * 32 + lane] = f[k / 6][k % 6];
   __syncthreads();
