@@ -245,12 +245,13 @@ __global__ void __launch_bounds__(256) fx_vmax_kernel(const double *__restrict__
 }
 
 // Digits of the operands for 64 points (one K chunk) and 32 AOs: warp = eight
-// consecutive points, lane = AO.  blockIdx.z = 0: A sets [mt][4 npc] (the planes),
+// consecutive points, lane = AO.  blockIdx.x = 0: A sets [mt][4 npc] (the planes),
 // 1 and 2: B sets [nb][4 npc] of spin 0 and 1 (Q and c_kin d_j phi), chunk t npc + pc
 // for plane t.  One plane's values live at a time (the planes are read again from
 // L1): with all five in registers one block of 168 registers a thread fitted an SM
 // and the kernel ran at 3 TB/s, bound by its latencies (6,800 points x 400 AOs 187 us,
-// now 139: 4.1 TB/s).  The blocks of chunk 0 write
+// then 139).  The three blocks of a tile are neighbours in the launch, so that its
+// planes come from HBM once (128 us).  The blocks of chunk 0 write
 // the exponent fields of the operand rows: ea [2][128 mt] (phi, kinetic), eb
 // [2][128 nb] (Q, kinetic; tile rows 64 of each spin).
 __global__ void __launch_bounds__(256, 4) fx_vdigits_kernel(const double *__restrict__ tab, size_t pe, int64_t np, int ld,
@@ -263,7 +264,7 @@ __global__ void __launch_bounds__(256, 4) fx_vdigits_kernel(const double *__rest
   if (*bad != 0) return;
   __shared__ double sc[kFeat][64];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int pc = blockIdx.y, a = blockIdx.x * 32 + lane, s = (int)blockIdx.z - 1;
+  const int pc = blockIdx.z, a = blockIdx.y * 32 + lane, s = (int)blockIdx.x - 1;
   const int64_t q0 = (int64_t)pc * kChunkK;
   if (s >= 0) {
     for (int i = threadIdx.x; i < kFeat * 64; i += blockDim.x) {
@@ -495,7 +496,7 @@ cudaError_t launch_vxc(const double *tab, int64_t np, int ld, int n_ao, const do
     segs = (rows + per - 1) / per;
     launch_next(fx_vmax_kernel, dim3(blocks_a, (unsigned)segs), 256, 0, st, tab, pe, np, ld, coef, p0, rows, (int)per,
                 kin, n_max, mx, bad);
-    launch_next(fx_vdigits_kernel, dim3(ld / 32, npc, 3), 256, 0, st, tab, pe, np, ld, coef, p0, rows, npc, kin, w.mt,
+    launch_next(fx_vdigits_kernel, dim3(3, ld / 32, npc), 256, 0, st, tab, pe, np, ld, coef, p0, rows, npc, kin, w.mt,
                 w.nb, (n_ao + 7) / 8 * 8, mx, ea, eb, va, vb, bad);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     GemmArgs g{};
