@@ -175,8 +175,8 @@ NEURAL_WORKLOAD = ("synthetic neural functional (DM21-style network, 6 x 256, 11
 
 def _neural_launches(n_layers: int) -> int:
     """Kernels one mixed neural step launches (the sequence in mlp_tc.cu plus the two contractions):
-    weight packing 2 + 2n, forward 6 + 2n, backward 5 + 5n, density 2 and V_xc 3."""
-    return (2 + 2 * n_layers) + (6 + 2 * n_layers) + (5 + 5 * n_layers) + 5
+    weight packing 2 + 2n, forward 6 + 2n, backward 5 + 5n, density 2 and V_xc 4."""
+    return (2 + 2 * n_layers) + (6 + 2 * n_layers) + (5 + 5 * n_layers) + 6
 
 
 def run_neural(args):
@@ -1135,9 +1135,11 @@ def main():
         _lib.check(lib.gdft_profile_read(sid, ctypes.byref(t), ctypes.byref(n)))
         stage[name] = (t.value, n.value)
     # Kernels per step of the library's XC call (the stage timers count regions, some of which hold
-    # several kernels): mixed pack_rdm1, dens_tc, xc_point, energy_reduce, build_q, tcg3, vxc_q_reduce;
-    # FP64 dens_f64, xc_point, energy_reduce, vxc_f64, vxc_reduce.
-    launches = (7 if form == "tf32x3" else 5) * args.steps
+    # several kernels): mixed pack_rdm1, dens_tc, xc_point, energy_reduce, build_q, tcg3 (twice from
+    # two tiles of 128 AOs on), vxc_q_reduce; FP64, with one slab of the grid (more slabs launch
+    # more): fx clear, rdm1, rows, gemm, features, dens_f64, xc_point, energy_reduce, clear, vmax,
+    # vdigits, gemm, vreduce, vxc_f64, vxc_reduce.
+    launches = ((8 if args.n_ao > 128 else 7) if form == "tf32x3" else 15) * args.steps
     if world > 1:
         import torch.distributed as dist
 

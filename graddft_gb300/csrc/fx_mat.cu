@@ -10,7 +10,7 @@
 // Measured (plain FP64 GEMM -> here, with the digits' kernels): a layer of the
 // network, 16,512 x 256 x 256, 1,430 -> 95 us; its weight gradient (K 16,512),
 // which ran on 16 CTAs, 17,800 -> 95 us.  A DM21 training step on 16,400 points:
-// 177.3 -> 7.9 ms, the second-order pass on 8,192: 260 -> 11.6 ms (5.6 and 8.4
+// 177.3 -> 7.9 ms, the second-order pass on 8,192: 260 -> 11.6 ms (5.6 and 8.3
 // with the row passes of ln_rows.cu and chained launches).
 #include "common.cuh"
 #include "fx.cuh"

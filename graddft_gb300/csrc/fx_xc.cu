@@ -18,7 +18,7 @@
 // faster one at every size (E_xc + V_xc, B88+LYP, plain kernels -> here: 4 AOs x
 // 128 points 779 -> 294 us, 24 x 3,600 928 -> 397 us, 100 x 10,000 5.4 -> 0.74 ms,
 // 400 x 150,001 827 -> 27.6 ms; with the point kernel's and launches' later forms 24 x
-// 3,600 147 us, 400 x 150,001 24.6 ms), and the more accurate one (features at 400 AOs
+// 3,600 147 us, 400 x 150,001 23.7 ms), and the more accurate one (features at 400 AOs
 // against quadruple precision: 1.4e-16 .. 2.7e-16, before 2.7e-16 .. 6.0e-16).
 #include "common.cuh"
 #include "fx.cuh"
