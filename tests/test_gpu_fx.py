@@ -43,7 +43,7 @@ def _resident(E, ao, g1, g2):
 
 
 SIZES = [(1, 1), (7, 127), (31, 128), (33, 129), (63, 640), (64, 65), (65, 257), (128, 300), (129, 1000), (193, 500),
-         (130, 30001)]  # the last crosses the slabs of both contractions
+         (130, 30001), (7, 300001)]  # the last crosses the slabs of both contractions
 
 
 @pytest.mark.parametrize("n,N", SIZES)
