@@ -18,7 +18,7 @@
 // faster one at every size (E_xc + V_xc, B88+LYP, plain kernels -> here: 4 AOs x
 // 128 points 779 -> 294 us, 24 x 3,600 928 -> 397 us, 100 x 10,000 5.4 -> 0.74 ms,
 // 400 x 150,001 827 -> 27.6 ms; with the point kernel's and launches' later forms 24 x
-// 3,600 147 us, 400 x 150,001 22.0 ms), and the more accurate one (features at 400 AOs
+// 3,600 147 us, 400 x 150,001 22.6 ms), and the more accurate one (features at 400 AOs
 // against quadruple precision: 1.4e-16 .. 2.7e-16, before 2.7e-16 .. 6.0e-16).
 #include "common.cuh"
 #include "fx.cuh"
@@ -32,9 +32,9 @@ namespace {
 // Workspace of one slab, about.  A slab's GEMM ends in a wave that is not full and
 // its sums are added to the slab before's, so few and large ones are faster (B88 115 x
 // 65,536 at 512 MB, 1, 2 and 4 GB: 1,128, 1,108, 971, 971 us; BLYP 400 x 150,001 23.7,
-// 22.4, 21.9, 21.7 ms); 2 GB are 0.7 % of the memory, and no more than the grid needs is
-// asked for.
-constexpr size_t kSlabBytes = (size_t)2 << 30;
+// 22.4, 21.9, 21.7 ms); but every resident molecule holds its workspace, and a set of
+// them should not take several times the memory of its tables.
+constexpr size_t kSlabBytes = (size_t)1 << 30;
 size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 
 // Digits of D as the B operand: tile nt = columns 64 nt .. of spin 0, then of
