@@ -92,9 +92,9 @@ __global__ void __launch_bounds__(128) fx_rdm1_kernel(const double *__restrict__
 constexpr int kFeatTile = 32;  // points
 constexpr int kFeatCols = 16;
 __global__ void __launch_bounds__(256, 4) fx_features_kernel(const double *__restrict__ tab, size_t pe, int64_t np, int ld,
-                                                          int64_t p0, int64_t slab, const double *__restrict__ X,
-                                                          int cols, bool kin, double *__restrict__ feat,
-                                                          const int *__restrict__ bad) {
+                                                          int n, int64_t p0, int64_t slab,
+                                                          const double *__restrict__ X, int cols, bool kin,
+                                                          double *__restrict__ feat, const int *__restrict__ bad) {
   previous_done();
   if (*bad != 0) return;
   __shared__ double tile[2][kPlanes][kFeatTile][kFeatCols + 1];
@@ -117,8 +117,8 @@ __global__ void __launch_bounds__(256, 4) fx_features_kernel(const double *__res
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
   fetch(0, 0);
-  for (int c0 = 0, b = 0; c0 < ld; c0 += kFeatCols, b ^= 1) {  // ld is a multiple of 32
-    if (c0 + kFeatCols < ld) {
+  for (int c0 = 0, b = 0; c0 < n; c0 += kFeatCols, b ^= 1) {  // ld, a multiple of 32, holds the last tile
+    if (c0 + kFeatCols < n) {
       fetch(c0 + kFeatCols, b ^ 1);
       asm volatile("cp.async.wait_group 1;" ::: "memory");
     } else {
@@ -129,6 +129,7 @@ __global__ void __launch_bounds__(256, 4) fx_features_kernel(const double *__res
 #pragma unroll
     for (int k = 0; k < kFeatCols / 8; ++k) {
       const int c = warp + 8 * k;
+      if (c0 + c >= n) break;  // X has no columns from n on: whatever memory holds there times the planes' zeros
       const double phi = t[T_PHI][lane][c], dx = t[T_DX][lane][c], dy = t[T_DY][lane][c], dz = t[T_DZ][lane][c];
       const double *x = X + (size_t)(c0 + c) * slab + r0 + lane;
 #pragma unroll
@@ -473,8 +474,8 @@ cudaError_t launch_density(const double *tab, int64_t np, int ld, int n_ao, cons
     if ((e = launch_gemm(g, st)) != cudaSuccess) return e;
     // Not chained: its blocks would be placed while the GEMM still holds most SMs, and crowd on the rest (24 AOs x
     // 3,600 points: 8 us, chained 24).
-    fx_features_kernel<<<(unsigned)(rows / kFeatTile), 256, 0, st>>>(tab, pe, np, ld, p0, w.dens_slab, X, w.nb * 64, kin,
-                                                                     feat, bad);
+    fx_features_kernel<<<(unsigned)(rows / kFeatTile), 256, 0, st>>>(tab, pe, np, ld, n_ao, p0, w.dens_slab, X,
+                                                                     w.nb * 64, kin, feat, bad);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
   return cudaSuccess;
