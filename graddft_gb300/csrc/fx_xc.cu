@@ -9,7 +9,17 @@
 //
 // V_xc: V_s = phi^T Q_s + sum_j d_j phi^T (c_kin,s d_j phi), with
 // Q_s = c_rho phi + sum_j c_gj d_j phi + c_lap lap phi (vxc_f64.cu).  The second
-// sum is symmetric: only tiles that reach the diagonal are formed.
+// sum is symmetric: only tiles that reach the diagonal are formed.  A row of this
+// contraction is one AO over the points of a slab, in fixed point on its largest
+// value, and phi and Q are graded against one another: a steep function is large
+// where the weights, and so Q, are small.  Both are therefore taken times a power
+// of two for each point that shares the coefficients out evenly (phi 2^t and
+// Q 2^-t, t half the exponent of the point's largest coefficient; exact): rows are then
+// like sqrt(|c|) phi, square-integrable, and the error is relative to the product of
+// two such maxima instead of max |phi_a| max |Q_b|.  s functions of exponents A and 0.15
+// on one centre, 300 radial points, error relative to sum |phi_a Q_b|: A = 6,665
+// 8e-13 -> 2e-15, 1e6 3e-10 -> 3e-14, 1e8 1e-6 -> 5e-13 (an FP64 sum 7e-16).  What is left of
+// the grading, and AOs that hardly meet (distant centres), are held to 2^-58 of that product.
 //
 // Both run over the grid in slabs whose digits and products fit a fixed
 // workspace.  An operand that is not finite (or overflows its bound) sets a
@@ -185,11 +195,18 @@ __device__ __forceinline__ int hi_of(double x) {
   const int h = __double2hiint(x) & 0x7FFFFFFF;
   return h ? h : kNone;
 }
+// Exponent field of a row's largest high word m, negative where the octaves have moved it there; 1 for a row without
+// values (kNone, or a little above it).
+constexpr int kNoRow = -(600 << 20);
+__device__ __forceinline__ int field_at(int m) { return m < kNoRow ? 1 : m >> 20; }
 // Exponent field bound of a sum of `terms` products whose largest has the (approximate) high word m.
 __device__ __forceinline__ int field_of(int m, int octaves) {
-  const int f = m <= 0 ? 1 : ((m + (1 << 18)) >> 20) + octaves;
-  return f < 1 ? 1 : f > 0x7FE ? 0x7FE : f;
+  if (m < kNoRow) return 1;
+  const int f = ((m + (1 << 18)) >> 20) + octaves;
+  return f > 0x7FE ? 0x7FE : f;
 }
+// Octaves t of a point without coefficients: phi 2^t has no digits, and Q is zero.
+constexpr int kDead = -(1 << 14);
 
 // The non-finite word, and n maxima below every high word (a kernel, not a
 // memset: launches before and after it stay chained).
@@ -201,14 +218,16 @@ __global__ void fx_clear_kernel(int *bad, int *mx, int n) {
 }
 
 // Largest high words over a slab of points: [0] phi, [1] d_j phi (one for the
-// three), [2 + s] the terms of Q_s, [4 + s] c_kin,s d_j phi.  Lanes are AOs, a
-// block takes 32 AOs and `per` points, its warps every eighth point.
+// three), [2 + s] the terms of Q_s, [4 + s] c_kin,s d_j phi, each with its point's
+// octaves, which go to oct[2][oct_stride] (phi's and Q's, then the kinetic part's).
+// Lanes are AOs, a block takes 32 AOs and `per` points, its warps every eighth point.
 __global__ void __launch_bounds__(256) fx_vmax_kernel(const double *__restrict__ tab, size_t pe, int64_t np, int ld,
                                                       const double *__restrict__ coef, int64_t p0, int64_t rows,
                                                       int per, bool kin, int n_max, int *__restrict__ mx,
+                                                      int *__restrict__ oct, int64_t oct_stride,
                                                       int *__restrict__ bad) {
   previous_done();
-  __shared__ int sc[2][kFeat][128];
+  __shared__ int sc[2][kFeat][128], so[2][128];  // high words over 1 (2^-t, for the octaves), octaves
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int a = blockIdx.x * 32 + lane;
   int m[6] = {kNone, kNone, kNone, kNone, kNone, kNone};
@@ -223,6 +242,19 @@ __global__ void __launch_bounds__(256) fx_vmax_kernel(const double *__restrict__
       (&sc[0][0][0])[i] = h == kNone ? kNone : h - kOneHi;
     }
     __syncthreads();
+    {
+      const int p = threadIdx.x % 128, part = threadIdx.x / 128;  // part 1: the kinetic rows
+      const int k0 = part ? C_KIN : 0, k1 = part ? C_KIN + 1 : C_KIN;
+      int m = kNone;
+      for (int k = k0; k < k1; ++k) m = max(m, max(sc[0][k][p], sc[1][k][p]));
+      const int t = m == kNone ? kDead : m >> 21;
+      so[part][p] = t;
+      for (int k = k0; k < k1; ++k)
+        for (int s = 0; s < 2; ++s)  // kept at or above kNone: two of them still add without overflow
+          if (sc[s][k][p] != kNone) sc[s][k][p] = max(sc[s][k][p] - (t << 20), kNone);
+      if (blockIdx.x == 0 && p < cnt) oct[part * oct_stride + q0 + p] = t;
+    }
+    __syncthreads();
     if (a < ld)
       for (int p = warp; p < cnt; p += 8) {
         const double *t = tab + (size_t)(p0 + q0 + p) * ld + a;
@@ -230,8 +262,8 @@ __global__ void __launch_bounds__(256) fx_vmax_kernel(const double *__restrict__
                   lp = hi_of(t[4 * pe]);
         const int dm = max(dx, max(dy, dz));
         if (max(phi, max(dm, lp)) > (kMaxField << 20)) atomicOr(bad, 1);
-        m[0] = max(m[0], phi);
-        m[1] = max(m[1], dm);
+        if (so[0][p] != kDead) m[0] = max(m[0], phi + (so[0][p] << 20));
+        if (so[1][p] != kDead) m[1] = max(m[1], dm + (so[1][p] << 20));
 #pragma unroll
         for (int s = 0; s < 2; ++s) {
           int v = sc[s][C_RHO][p] + phi;
@@ -263,12 +295,15 @@ __global__ void __launch_bounds__(256) fx_vmax_kernel(const double *__restrict__
 __global__ void __launch_bounds__(256, 4) fx_vdigits_kernel(const double *__restrict__ tab, size_t pe, int64_t np, int ld,
                                                             const double *__restrict__ coef, int64_t p0, int64_t rows,
                                                             int npc, bool kin, int mt, int nb, int n8,
-                                                            const int *__restrict__ mx, int *__restrict__ ea,
-                                                            int *__restrict__ eb, unsigned char *__restrict__ va,
+                                                            const int *__restrict__ mx,
+                                                            const int *__restrict__ oct, int64_t oct_stride,
+                                                            int *__restrict__ ea, int *__restrict__ eb,
+                                                            unsigned char *__restrict__ va,
                                                             unsigned char *__restrict__ vb, int *__restrict__ bad) {
   previous_done();
   if (*bad != 0) return;
   __shared__ double sc[kFeat][64];
+  __shared__ int so[2][64];  // the points' octaves, for B with the other sign
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int pc = blockIdx.z, a = blockIdx.y * 32 + lane, s = (int)blockIdx.x - 1;
   const int64_t q0 = (int64_t)pc * kChunkK;
@@ -277,8 +312,12 @@ __global__ void __launch_bounds__(256, 4) fx_vdigits_kernel(const double *__rest
       const int p = i % 64;
       sc[i / 64][p] = q0 + p < rows ? coef[((size_t)s * kFeat + i / 64) * np + p0 + q0 + p] : 0.0;
     }
-    __syncthreads();
   }
+  if (threadIdx.x < 128) {
+    const int p = threadIdx.x % 64, t = q0 + p < rows ? oct[threadIdx.x / 64 * oct_stride + q0 + p] : 0;
+    so[threadIdx.x / 64][p] = s < 0 ? t : -t;
+  }
+  __syncthreads();
   if (a >= n8) return;  // n8 <= ld
   const int k0 = warp * 8, n_max = mt * kTile;
   const int64_t left = rows - q0 - k0;  // points of these eight that there are
@@ -290,13 +329,17 @@ __global__ void __launch_bounds__(256, 4) fx_vdigits_kernel(const double *__rest
 #pragma unroll
     for (int j = 0; j < 8; ++j) v[j] = j < left ? t[(size_t)j * ld] : 0.0;
   };
-  auto emit = [&](unsigned char *set, int row, const double (&x)[8], int emax) {
+  auto emit = [&](unsigned char *set, int row, const double (&x)[8], int emax, const int *octaves) {
     over = over || emax > kMaxField;
     long long f[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      over = over || exp_field((uint32_t)__double2hiint(x[j])) > emax;
-      f[j] = to_fixed(x[j], emax);
+      const int e = emax - octaves[k0 + j];
+      if (s >= 0) {  // A's maxima are exact, and have been looked at
+        const int ef = exp_field((uint32_t)__double2hiint(x[j]));
+        over = over || (ef != 0 && ef > e);
+      }
+      f[j] = to_fixed(x[j], e);
     }
     uint4 d[kDigits];
     digits8(f, d);
@@ -306,7 +349,7 @@ __global__ void __launch_bounds__(256, 4) fx_vdigits_kernel(const double *__rest
   };
   double v[8];
   if (s < 0) {
-    const int e0 = max(1, mx[a] >> 20), e1 = max(1, mx[n_max + a] >> 20);
+    const int e0 = field_at(mx[a]), e1 = field_at(mx[n_max + a]);
     if (pc == 0 && warp == 0) {
       ea[a] = e0;
       ea[n_max + a] = e1;
@@ -315,7 +358,7 @@ __global__ void __launch_bounds__(256, 4) fx_vdigits_kernel(const double *__rest
 #pragma unroll 1
     for (int t = 0; t < (kin ? 4 : 1); ++t) {
       load(t, v);
-      emit(A + (size_t)t * npc * kSetBytes, a % kTile, v, t ? e1 : e0);
+      emit(A + (size_t)t * npc * kSetBytes, a % kTile, v, t ? e1 : e0, so[t ? 1 : 0]);
     }
   } else {
     const int row = s * 64 + a % 64, at = a / 64 * kTile + row;
@@ -335,14 +378,14 @@ __global__ void __launch_bounds__(256, 4) fx_vdigits_kernel(const double *__rest
 #pragma unroll
       for (int j = 0; j < 8; ++j) q[j] = fma(sc[p][k0 + j], v[j], q[j]);
     }
-    emit(B, row, q, e0);
+    emit(B, row, q, e0, so[0]);
     if (kin)
 #pragma unroll 1
       for (int t = 1; t < 4; ++t) {
         load(t, v);
 #pragma unroll
         for (int j = 0; j < 8; ++j) q[j] = sc[C_KIN][k0 + j] * v[j];
-        emit(B + (size_t)t * npc * kSetBytes, row, q, e1);
+        emit(B + (size_t)t * npc * kSetBytes, row, q, e1, so[1]);
       }
   }
   if (over) atomicOr(bad, 1);
@@ -422,7 +465,7 @@ XcWs xc_ws(int64_t np, int n_ao) {
   w.off_vb = off;
   off = align256(off + (size_t)w.nb * 4 * npc * kSetBytes);
   w.off_vexp = off;
-  off = align256(off + (size_t)(2 * w.mt * kTile + 2 * w.nb * kTile + 6 * n128) * sizeof(int));
+  off = align256(off + (size_t)(2 * w.mt * kTile + 2 * w.nb * kTile + 6 * n128 + 2 * w.v_slab) * sizeof(int));
   w.off_vpart = off;
   // s0 + s1 is at most this for any grid, so a shorter grid never needs more than a longer one.
   const int64_t most = 4 * 2 * 148 / ((int64_t)w.mt * w.nb + 3 * upper) + 2;
@@ -487,7 +530,7 @@ cudaError_t launch_vxc(const double *tab, int64_t np, int ld, int n_ao, const do
   const size_t pe = (size_t)np * ld;
   int *bad = bad_word(ws, w);
   const int n_max = w.mt * kTile;
-  int *ea = (int *)(ws + w.off_vexp), *eb = ea + 2 * n_max, *mx = eb + 2 * w.nb * kTile;
+  int *ea = (int *)(ws + w.off_vexp), *eb = ea + 2 * n_max, *mx = eb + 2 * w.nb * kTile, *oct = mx + 6 * n_max;
   unsigned char *va = ws + w.off_va, *vb = ws + w.off_vb;
   double *part = (double *)(ws + w.off_vpart);
   cudaError_t e;
@@ -501,9 +544,9 @@ cudaError_t launch_vxc(const double *tab, int64_t np, int ld, int n_ao, const do
     per = per < 64 ? 64 : per;
     segs = (rows + per - 1) / per;
     launch_next(fx_vmax_kernel, dim3(blocks_a, (unsigned)segs), 256, 0, st, tab, pe, np, ld, coef, p0, rows, (int)per,
-                kin, n_max, mx, bad);
+                kin, n_max, mx, oct, w.v_slab, bad);
     launch_next(fx_vdigits_kernel, dim3(3, ld / 32, npc), 256, 0, st, tab, pe, np, ld, coef, p0, rows, npc, kin, w.mt,
-                w.nb, (n_ao + 7) / 8 * 8, mx, ea, eb, va, vb, bad);
+                w.nb, (n_ao + 7) / 8 * 8, mx, oct, w.v_slab, ea, eb, va, vb, bad);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     GemmArgs g{};
     g.a = va;

@@ -1,0 +1,70 @@
+"""The FP64 form's contractions over grid points where their operands are graded against one another: steep functions,
+largest where the integration weights are smallest, beside diffuse ones.
+
+Bound, element by element.  A row is fixed point on its largest value after each point's power of two (half the
+exponent of the point's largest coefficient), 61 bits, and the products left out are below 2^-58 of the product of the
+rows' powers of two.  Those are at most twice the largest phi 2^t and 2^5 times the largest term of Q 2^-t (three
+octaves for the sum of five terms, a quarter for the approximate product, one for the mantissa), so 2^-52 of the
+product of these maxima for each point.  Without the octaves the maxima are those of phi and Q themselves, thousands
+of times the bound for the steepest pair.  What remains are FP64 roundings: of the five terms, of at most 320 partial
+sums, and the CPU's N."""
+import numpy as np
+import pytest
+import torch
+
+from test_gpu_fx import E, U  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+ALPHAS = np.array([1e10, 1e8, 1e6, 6665.0, 30.0, 1.0, 0.15])
+
+
+def _octaves(c):
+    """2^t, t half the exponent of the largest |c| of a point (floor), c (k, N)."""
+    return 2.0 ** ((np.frexp(np.abs(c).max(0))[1] - 1) // 2)
+
+
+def _tables(N, seed):
+    """s functions on one centre, on a logarithmic radial grid with its weights."""
+    g = np.random.default_rng(seed)
+    r = np.exp(np.linspace(np.log(1e-7), np.log(12.0), N))
+    u = g.standard_normal((N, 3))
+    x = r[:, None] * u / np.linalg.norm(u, axis=1, keepdims=True)
+    w = 4 * np.pi * r ** 3 * np.log(12.0 / 1e-7) / N
+    phi = (2 * ALPHAS / np.pi) ** 0.75 * np.exp(-ALPHAS * r[:, None] ** 2)
+    g1 = -2 * ALPHAS[None, :, None] * x[:, None] * phi[..., None]
+    g2 = (4 * ALPHAS[None, :, None] ** 2 * x[:, None] ** 2 - 2 * ALPHAS[None, :, None]) * phi[..., None]
+    v = (50 * np.exp(-16 * r) + 0.5 * np.exp(-2 * r)) ** (1 / 3)
+    return phi, g1, g2, x, w, v
+
+
+@pytest.mark.parametrize("terms", ["rho", "gradient", "all"])
+def test_vxc(E, terms):  # noqa: F811
+    N = 300
+    phi, g1, g2, x, w, v = _tables(N, 1)
+    n = len(ALPHAS)
+    pot = np.zeros((2, 6, N))
+    pot[:, 0] = -w * v
+    if terms != "rho":
+        pot[:, 1:4] = 0.1 * (w * v)[None, None] * x.T[None]
+    if terms == "all":
+        pot[:, 4], pot[:, 5] = 1e-3 * w * v, 0.02 * w * v
+    pot[1] *= 0.7
+    r = E.Resident.from_tables(phi, g1, g2, np.ones(N), "fp64", "cuda:0")
+    got = r.vxc_from_potentials(pot).cpu().numpy()
+    assert r.status() == 0
+    lap = g2.sum(-1)
+    t0, t1 = _octaves(pot[:, :5].reshape(-1, N))[:, None], _octaves(np.maximum(pot[:, 5], 1e-300))[:, None]
+    for s in range(2):
+        c = pot[s][..., None]
+        each = [c[0] * phi, *(c[1 + j] * g1[..., j] for j in range(3)), c[4] * lap]
+        ref, size = phi.T @ sum(each), np.abs(phi).T @ sum(np.abs(t) for t in each)
+        lost = np.abs(phi * t0).max(0)[:, None] * np.max([np.abs(t / t0) for t in each], (0, 1))[None]
+        kin = np.zeros((n, n))
+        for j in range(3):
+            ref += g1[..., j].T @ (c[5] * g1[..., j])
+            size += np.abs(g1[..., j]).T @ np.abs(c[5] * g1[..., j])
+        if pot[s, 5].any():
+            kin = np.abs(g1 * t1[..., None]).max((0, 2))[:, None] * np.abs(c[5][..., None] * g1 / t1[..., None]).max((0, 2))
+        bound = (320 + N + 10) * U * size + N * 2.0 ** -52 * (lost + 3 * np.maximum(kin, kin.T))
+        assert np.all(np.abs(got[s] - ref) <= bound), np.max(np.abs(got[s] - ref) / bound)
