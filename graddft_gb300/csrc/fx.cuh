@@ -50,6 +50,9 @@ __device__ __forceinline__ long long to_fixed(double x, int emax) {
   return b < 0 ? -(long long)m : (long long)m;
 }
 
+// Octaves t of a term k that is taken as (a_k 2^t)(b_k 2^-t), where b_k is zero: a_k 2^t has no digits.
+constexpr int kDead = -(1 << 14);
+
 // The digits of a row's fixed-point values, eight consecutive k at a time:
 // out[i] holds digit i times 2^(-9i) of the eight values as BF16.
 __device__ __forceinline__ void digits8(const long long (&f)[8], uint4 (&out)[kDigits]) {
@@ -137,9 +140,11 @@ size_t gemm_cols_bytes(int M, int N, int64_t K);
 // C[m][n] = sum_k A[m][k] B[k][n] (B stored N x K when b_rows) + add[m][n] (laid out like C; null: nothing).
 cudaError_t gemm_rows(int64_t M, int N, int K, const double *A, int64_t lda, const double *B, int64_t ldb, bool b_rows,
                       double *C, int64_t ldc, const double *add, unsigned char *ws, int *err, cudaStream_t st);
-// C[m][n] = sum_k A[k][m] B[k][n], C contiguous (M x N).
-cudaError_t gemm_cols(int M, int N, int64_t K, const double *A, int64_t lda, const double *B, int64_t ldb, double *C,
-                      unsigned char *ws, int *err, int nsplit, double *part, cudaStream_t st);
+// C[m][n] = sum_k A[k][m] B[k][n], C contiguous (M x N).  oct, or null: K octaves t; A's rows are taken times 2^t and
+// B's times 2^-t, for operands that are graded against one another (fx_xc.cu).
+cudaError_t gemm_cols(int M, int N, int64_t K, const double *A, int64_t lda, const double *B, int64_t ldb,
+                      const int *oct, double *C, unsigned char *ws, int *err, int nsplit, double *part,
+                      cudaStream_t st);
 
 // Feature sets of fx_xc.cu: the FP64 form's density and V_xc contractions.
 struct XcWs {

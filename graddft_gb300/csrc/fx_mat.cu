@@ -23,6 +23,7 @@ namespace fx {
 namespace {
 
 constexpr size_t kSlabBytes = (size_t)512 << 20;  // digits held at a time, about
+constexpr uint32_t kInfHi = 0x7FF00000u;  // high word of an infinity
 constexpr size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 constexpr int64_t tiles_of(int64_t n) { return (n + kTile - 1) / kTile; }
 constexpr int64_t chunks_of(int64_t k) { return (k + kChunkK - 1) / kChunkK; }
@@ -62,17 +63,27 @@ __global__ void __launch_bounds__(128) fx_short_cols_kernel(const double *__rest
   }
 }
 
-// Largest high words of the columns of X [rows][cols]: lanes are columns, a block
-// takes 32 of them and `per` rows.
+// Largest high words of the columns of X [rows][cols], with OCT those of row r times 2^(sign oct[r]): lanes are
+// columns, a block takes 32 of them and `per` rows.
+template <bool OCT>
 __global__ void __launch_bounds__(256) fx_colmax_kernel(const double *__restrict__ X, int64_t rows, int cols,
-                                                        int64_t ld, int64_t per, uint32_t *__restrict__ mx) {
+                                                        int64_t ld, int64_t per, const int *__restrict__ oct, int sign,
+                                                        uint32_t *__restrict__ mx) {
   previous_done();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int c = blockIdx.x * 32 + lane;
   const int64_t r0 = (int64_t)blockIdx.y * per, r1 = r0 + per < rows ? r0 + per : rows;
   uint32_t m = 0;
   if (c < cols)
-    for (int64_t r = r0 + warp; r < r1; r += 8) m = max(m, (uint32_t)__double2hiint(X[(size_t)r * ld + c]) & 0x7FFFFFFFu);
+    for (int64_t r = r0 + warp; r < r1; r += 8) {
+      uint32_t h = (uint32_t)__double2hiint(X[(size_t)r * ld + c]) & 0x7FFFFFFFu;
+      if (OCT && h < kInfHi && h != 0) {  // infinities and NaN stay what they are
+        const int t = oct[r];
+        const long long v = t == kDead ? 0 : (long long)h + (long long)(sign * t) * (1 << 20);
+        h = v < 0 ? 0u : v > kInfHi ? kInfHi : (uint32_t)v;
+      }
+      m = max(m, h);
+    }
   __shared__ uint32_t sm[8][32];
   sm[warp][lane] = m;
   __syncthreads();
@@ -83,10 +94,12 @@ __global__ void __launch_bounds__(256) fx_colmax_kernel(const double *__restrict
   }
 }
 
-// Columns of a tall X as operand rows, K = its rows: a block takes 64 rows (one
-// chunk) and 32 columns, a warp eight consecutive rows.
+// Columns of a tall X as operand rows, K = its rows (times 2^(sign oct)): a block takes 64
+// rows (one chunk) and 32 columns, a warp eight consecutive rows.
+template <bool OCT>
 __global__ void __launch_bounds__(256) fx_tall_cols_kernel(const double *__restrict__ X, int64_t rows, int cols,
-                                                           int64_t ld, int chunks, const uint32_t *__restrict__ mx,
+                                                           int64_t ld, int chunks, const int *__restrict__ oct,
+                                                           int sign, const uint32_t *__restrict__ mx,
                                                            unsigned char *__restrict__ out, int *__restrict__ exps,
                                                            int *__restrict__ bad) {
   previous_done();
@@ -99,7 +112,10 @@ __global__ void __launch_bounds__(256) fx_tall_cols_kernel(const double *__restr
   const int64_t r0 = (int64_t)chunk * kChunkK + warp * 8;
   long long f[8];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) f[j] = c < cols && r0 + j < rows ? to_fixed(X[(size_t)(r0 + j) * ld + c], emax) : 0;
+  for (int j = 0; j < 8; ++j)
+    f[j] = c < cols && r0 + j < rows
+               ? to_fixed(X[(size_t)(r0 + j) * ld + c], OCT ? emax - sign * oct[r0 + j] : emax)
+               : 0;
   uint4 d[kDigits];
   digits8(f, d);
   unsigned char *set = out + ((size_t)(c / kTile) * chunks + chunk) * kSetBytes + elem_off(c % kTile, warp * 8);
@@ -230,8 +246,9 @@ cudaError_t gemm_rows(int64_t M, int N, int K, const double *A, int64_t lda, con
   return cudaSuccess;
 }
 
-cudaError_t gemm_cols(int M, int N, int64_t K, const double *A, int64_t lda, const double *B, int64_t ldb, double *C,
-                      unsigned char *ws, int *err, int nsplit, double *part, cudaStream_t st) {
+cudaError_t gemm_cols(int M, int N, int64_t K, const double *A, int64_t lda, const double *B, int64_t ldb,
+                      const int *oct, double *C, unsigned char *ws, int *err, int nsplit, double *part,
+                      cudaStream_t st) {
   const ColsWs w = cols_ws(M, N, K);
   const int64_t tm = tiles_of(M), tn = tiles_of(N);
   ws = aligned(ws);
@@ -244,17 +261,20 @@ cudaError_t gemm_cols(int M, int N, int64_t K, const double *A, int64_t lda, con
     const int64_t rows = K - k0 < w.slab ? K - k0 : w.slab;
     const int ch = (int)chunks_of(rows);
     if ((e = cudaMemsetAsync(ma, 0, (size_t)(tm + tn) * kTile * sizeof(uint32_t), st)) != cudaSuccess) return e;
-    auto digits = [&](const double *X, int64_t ld, int cols, uint32_t *mx, unsigned char *set, int *exps) {
+    const int *o = oct != nullptr ? oct + k0 : nullptr;
+    auto digits = [&](const double *X, int64_t ld, int cols, int sign, uint32_t *mx, unsigned char *set, int *exps) {
       const int bc = (cols + 31) / 32;
       int64_t segs = (4 * 148 + bc - 1) / bc, per = (rows + segs - 1) / segs;
       per = per < 64 ? 64 : per;
       segs = (rows + per - 1) / per;
-      launch_next(fx_colmax_kernel, dim3(bc, (unsigned)segs), 256, 0, st, X + k0 * ld, rows, cols, ld, per, mx);
-      launch_next(fx_tall_cols_kernel, dim3(ch, bc), 256, 0, st, X + k0 * ld, rows, cols, ld, ch, mx, set, exps, bad);
+      launch_next(o != nullptr ? fx_colmax_kernel<true> : fx_colmax_kernel<false>, dim3(bc, (unsigned)segs), 256, 0,
+                  st, X + k0 * ld, rows, cols, ld, per, o, sign, mx);
+      launch_next(o != nullptr ? fx_tall_cols_kernel<true> : fx_tall_cols_kernel<false>, dim3(ch, bc), 256, 0, st,
+                  X + k0 * ld, rows, cols, ld, ch, o, sign, mx, set, exps, bad);
       return cudaGetLastError();
     };
-    if ((e = digits(A, lda, M, ma, ws + w.off_a, ea)) != cudaSuccess) return e;
-    if ((e = digits(B, ldb, N, mb, ws + w.off_b, eb)) != cudaSuccess) return e;
+    if ((e = digits(A, lda, M, 1, ma, ws + w.off_a, ea)) != cudaSuccess) return e;
+    if ((e = digits(B, ldb, N, -1, mb, ws + w.off_b, eb)) != cudaSuccess) return e;
     GemmArgs g{};  // rows of the tiles: columns n of B (consecutive in C); columns: m
     g.a = ws + w.off_b;
     g.b = g.b1 = ws + w.off_a;

@@ -205,8 +205,6 @@ __device__ __forceinline__ int field_of(int m, int octaves) {
   const int f = ((m + (1 << 18)) >> 20) + octaves;
   return f > 0x7FE ? 0x7FE : f;
 }
-// Octaves t of a point without coefficients: phi 2^t has no digits, and Q is zero.
-constexpr int kDead = -(1 << 14);
 
 // The non-finite word, and n maxima below every high word (a kernel, not a
 // memset: launches before and after it stay chained).

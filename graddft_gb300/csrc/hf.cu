@@ -10,7 +10,8 @@
 // FP64 form: both contractions on digit products (fx_mat.cu): X_s = ao D_s, then a
 // warp per (point, spin) takes the row dot with chi; B_s = -1/2 sum_w g chi,
 // then F_s = ao^T B_s with the grid split over CTAs and the partials summed in
-// a fixed order.
+// a fixed order.  g carries the integration weights, smallest where the steepest AOs are
+// largest: ao and B share its exponent at each point (fx_xc.cu says why).
 //
 // Mixed (TF32x3) form: the same two contractions on the block-scaled
 // three-slice tcgen05 GEMM (tcg3: exact hi*hi chunk sums, compensated FP32
@@ -64,6 +65,16 @@ __global__ void hf_bmat_kernel(const double *__restrict__ chi, const double *__r
   for (int w = 0; w < n_omega; ++w)
     acc = fma(g[((size_t)w * 2 + s) * n_grid + r], chi[(((size_t)r * n_omega + w) * 2 + s) * n + b], acc);
   B[i] = -0.5 * acc;
+}
+
+// Octaves of a point for ao^T B: half the exponent of its largest |g|.
+__global__ void hf_octaves_kernel(const double *__restrict__ g, int64_t n_grid, int n_rows, int *__restrict__ oct) {
+  previous_done();
+  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= n_grid) return;
+  int m = 0;
+  for (int k = 0; k < n_rows; ++k) m = max(m, __double2hiint(g[(size_t)k * n_grid + r]) & 0x7FFFFFFF);
+  oct[r] = m == 0 ? fx::kDead : ((m >> 20) - 1023) >> 1;
 }
 
 // fock[s] = abs_clip(fock[s] + F[s] + F[s]^T)  (train.py:200-210).
@@ -359,8 +370,9 @@ int gdft_hf_workspace_bytes_form(int64_t n_grid, int32_t n_ao, int32_t n_omega, 
     *bytes = hf_tc_layout(n_grid, n_ao).bytes;
     return GDFT_OK;
   }
-  // X or B: [2][n_grid][n_ao]; split partials of F: [nsplit][n_ao][n_ao]; the GEMMs' scratch.
-  const size_t rows = fx::gemm_rows_bytes(n_grid, n_ao, n_ao), cols = fx::gemm_cols_bytes(n_ao, n_ao, n_grid);
+  // X or B: [2][n_grid][n_ao]; split partials of F: [nsplit][n_ao][n_ao]; the GEMMs' scratch (F's: with the octaves).
+  const size_t rows = fx::gemm_rows_bytes(n_grid, n_ao, n_ao);
+  const size_t cols = align256((size_t)n_grid * sizeof(int)) + fx::gemm_cols_bytes(n_ao, n_ao, n_grid);
   *bytes = hf_gemm_off(n_grid, n_ao) + (rows > cols ? rows : cols);
   return GDFT_OK;
 }
@@ -414,12 +426,14 @@ int gdft_hf_fock_form(const double *d_ao, const double *d_chi, const double *d_g
   double *part = (double *)((char *)d_ws + align256((size_t)2 * n_grid * n_ao * sizeof(double)));
   const size_t total = (size_t)2 * n_grid * n_ao;
   launch_next(hf_bmat_kernel, (unsigned)((total + 255) / 256), 256, 0, st, d_chi, d_g, n_grid, n_ao, n_omega, B);
+  int *oct = (int *)((char *)d_ws + hf_gemm_off(n_grid, n_ao));
+  unsigned char *gws = (unsigned char *)oct + align256((size_t)n_grid * sizeof(int));
+  launch_next(hf_octaves_kernel, (unsigned)((n_grid + 255) / 256), 256, 0, st, d_g, n_grid, 2 * n_omega, oct);
   if ((rc = check_cuda(cudaGetLastError(), "hf B"))) return rc;
   const int nsplit = hf_splits(n_grid);
   for (int s = 0; s < 2; ++s)
     if ((rc = check_cuda(fx::gemm_cols(n_ao, n_ao, n_grid, d_ao, n_ao, B + (size_t)s * n_grid * n_ao, n_ao,
-                                       d_fock_hf + (size_t)s * n_ao * n_ao,
-                                       (unsigned char *)d_ws + hf_gemm_off(n_grid, n_ao), nullptr, nsplit, part, st),
+                                       oct, d_fock_hf + (size_t)s * n_ao * n_ao, gws, nullptr, nsplit, part, st),
                          "hf ao^T B")))
       return rc;
   return GDFT_OK;

@@ -450,7 +450,7 @@ int mlp_run_f64(const MlpShape &S, const double *params, double *dparams, const 
   // ---- backward ----
   const int ns = L.nsplit;
   auto weight_grad = [&](int M, int N, const double *A, int lda, const double *B, int ldb, double *C) {
-    return fx::gemm_cols(M, N, np, A, lda, B, ldb, C, (unsigned char *)(ws + L.fx), err, ns, kpart, st);
+    return fx::gemm_cols(M, N, np, A, lda, B, ldb, nullptr, C, (unsigned char *)(ws + L.fx), err, ns, kpart, st);
   };
   auto mul_t = [&](int N, int K, const double *A, const double *B, double *C, int ldc, const double *add) {
     return fx::gemm_rows(np, N, K, A, K, B, K, true, C, ldc, add, (unsigned char *)(ws + L.fx), err, st);

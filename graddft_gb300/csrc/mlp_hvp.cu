@@ -381,7 +381,7 @@ int mlp_hvp_f64(const MlpShape &S, const double *params, double *dparams, const 
 
   // ---- reverse of the augmented graph ----
   auto wgrad = [&](int M, int N, const double *A, int lda, const double *B, int ldb, double *C) {
-    return fx::gemm_cols(M, N, rows2, A, lda, B, ldb, C, fxws, err, L.nsplit, kpart, st);
+    return fx::gemm_cols(M, N, rows2, A, lda, B, ldb, nullptr, C, fxws, err, L.nsplit, kpart, st);
   };
   auto csum = [&](const double *X, int64_t rows, int ncols, int ld, double *out) {
     return col_sums(X, rows, ncols, ld, out, colpart, kColBlocks, st);

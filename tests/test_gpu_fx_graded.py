@@ -68,3 +68,20 @@ def test_vxc(E, terms):  # noqa: F811
             kin = np.abs(g1 * t1[..., None]).max((0, 2))[:, None] * np.abs(c[5][..., None] * g1 / t1[..., None]).max((0, 2))
         bound = (320 + N + 10) * U * size + N * 2.0 ** -52 * (lost + 3 * np.maximum(kin, kin.T))
         assert np.all(np.abs(got[s] - ref) <= bound), np.max(np.abs(got[s] - ref) / bound)
+
+
+def test_exact_exchange_fock(E):  # noqa: F811
+    """F = ao^T B with B = -1/2 sum_w g chi: the octaves are those of g, and both rows' powers of two are at most twice
+    their largest values, 2^-56 of whose product is lost for each point."""
+    N, n = 300, len(ALPHAS)
+    phi, _, _, _, w, v = _tables(N, 2)
+    chi = phi[:, None, None] * np.random.default_rng(3).uniform(0.5, 1.0, (N, 2, 2, 1))
+    g = -(w * v)[None, None] * np.array([1.0, 0.6])[:, None, None] * np.array([1.0, 0.7])[None, :, None]
+    c = lambda x: torch.as_tensor(x, device="cuda")  # noqa: E731
+    got = E.hf_fock(c(phi), c(chi), c(g)).cpu().numpy()
+    t = _octaves(g.reshape(-1, N))[:, None]
+    for s in range(2):
+        B = -0.5 * sum(g[o, s][:, None] * chi[:, o, s] for o in range(2))
+        size = np.abs(phi).T @ np.abs(B)
+        bound = (N + 200) * U * size + N * 2.0 ** -56 * np.abs(phi * t).max(0)[:, None] * np.abs(B / t).max(0)
+        assert np.all(np.abs(got[s] - phi.T @ B) <= bound), np.max(np.abs(got[s] - phi.T @ B) / bound)
