@@ -86,7 +86,7 @@ __device__ __forceinline__ void digits8(const long long (&f)[8], uint4 (&out)[kD
 constexpr int kMaxField = 1023 + 450;
 
 // v 2^scale as a double, rounded to nearest (halves away from zero), by integer
-// operations: conversions run at the FP64 rate.  Below 2^-1021 the result is 0.
+// operations: conversions run at the FP64 rate.  Below 2^-1022 the result is 0.
 __device__ __forceinline__ double fixed_to_double(long long v, int scale) {
   const unsigned long long m = v < 0 ? (unsigned long long)(-v) : (unsigned long long)v;
   const int lz = __clzll((long long)m);
@@ -94,7 +94,7 @@ __device__ __forceinline__ double fixed_to_double(long long v, int scale) {
   const unsigned long long r = (n >> 11) + ((n >> 10) & 1);  // 53 bits, may carry to 2^53
   const int e = 63 - lz + scale;                             // exponent of the leading one
   unsigned long long d = ((unsigned long long)(e + 1022) << 52) + r;
-  if (e < -1021 || v == 0) d = 0;
+  if (e < -1022 || v == 0) return 0.0;
   return __longlong_as_double((long long)(d | ((unsigned long long)v & 0x8000000000000000ull)));
 }
 

@@ -169,13 +169,12 @@ __device__ __forceinline__ void add_shifted(long long &sum, int v, int sh, int r
       : "r"(v), "r"(sh), "r"(rsh));
 }
 
-// v 2^e: the conversion, then the exponent field.  e is kept to where the field
-// cannot wrap: products below 2^-1010 come out larger than they are (row exponents
-// are at most 2^kMaxExp, so none is too large).
+// v 2^e: the conversion, then the exponent field.  Below 2^-1022 the result is 0, as
+// fixed_to_double's (kMaxField keeps products from the other end).
 __device__ __forceinline__ double scaled(long long v, int e) {
   const double d = (double)v;
-  const int hi = __double2hiint(d) + (max(e, -1010) << 20);
-  return v == 0 ? 0.0 : __hiloint2double(hi, __double2loint(d));
+  const int hi = __double2hiint(d);
+  return exp_field((uint32_t)hi) + e < 1 || v == 0 ? 0.0 : __hiloint2double(hi + e * (1 << 20), __double2loint(d));
 }
 
 __global__ void __launch_bounds__(kThreads, 1) fx_gemm_kernel(const GemmArgs A, const int upper) {

@@ -173,3 +173,18 @@ def test_exact_exchange(E, n, N):
         size = np.abs(ao).T @ aB
         bound = (N + 200) * U * size + N * 2.0 ** -55 * np.abs(ao).max(0)[:, None] * aB.max(0)[None] + 1e-300
         assert np.all(np.abs(fock[s] - ao.T @ B) <= bound)
+
+
+def test_tiny_products(E):
+    """Products down to the smallest normal numbers, in every column alike: off by the digits' 2^-57 and FP64 roundings
+    as above, and by 2^-1022 for each product that FP64 would have kept as a denormal number."""
+    n, N = 70, 200
+    g = np.random.default_rng(5)
+    ao = g.uniform(1, 2, (N, n)) * 10.0 ** g.uniform(-308, -280, N)[:, None]
+    D, chi = g.standard_normal((2, n, n)), g.standard_normal((N, 1, 2, n))
+    ehf = E.hf_energy_density(*(torch.as_tensor(v, device="cuda") for v in (ao, D, chi))).cpu().numpy()
+    for s in range(2):
+        aX = np.abs(ao) @ np.abs(D[s])
+        bound = 2 * _dot_bound(aX, chi[:, 0, s], 2 * n + 20) + n * (2.0 ** -57 * np.abs(ao).max(1) * np.abs(
+            D[s]).max() + 2.0 ** -1022) * np.abs(chi[:, 0, s]).sum(1)
+        assert np.all(np.abs(ehf[0, s] + 0.5 * (chi[:, 0, s] * (ao @ D[s])).sum(1)) <= bound)
