@@ -129,9 +129,10 @@ struct GemmArgs {
 cudaError_t launch_gemm(const GemmArgs &a, cudaStream_t st);
 
 // Row-major FP64 rows (planes of them, k_valid values each) -> digit sets [plane][row tile][chunk], exponents
-// [plane][rows].  Rows past the last are left as they are: they only reach outputs that are not written.
+// [plane][rows].  Rows past the last are left as they are: they only reach outputs that are not written.  oct, or
+// null: 64 chunks octaves t, aligned to 16 bytes; column k is taken times 2^t.
 cudaError_t launch_rows(const double *src, int64_t plane_elems, int planes, int64_t rows, int64_t ld, int k_valid,
-                        int chunks, unsigned char *out, int *exps, int *bad, cudaStream_t st);
+                        int chunks, const int *oct, unsigned char *out, int *exps, int *bad, cudaStream_t st);
 
 // FP64 GEMMs of fx_mat.cu, on row-major operands.  ws: scratch of gemm_rows_bytes / gemm_cols_bytes; err: a device
 // error word or null (an expired wait leaves NaN in the output either way); part: partials of the plain kernel that takes over where an operand is not finite (nsplit x M x N doubles).
@@ -152,8 +153,8 @@ struct XcWs {
   int64_t dens_slab, v_slab;  // grid points per pass (multiples of 128)
   int v_chunks;            // K chunks of one V_xc item
   int s0, s1;              // splits of the phi and kinetic parts of a full slab
-  size_t off_bad, off_dset, off_dexp, off_a, off_ea, off_x;          // density
-  size_t off_va, off_vb, off_vexp, off_vpart;                                        // V_xc
+  size_t off_bad, off_dset, off_dexp, off_doct, off_a, off_ea, off_x;  // density
+  size_t off_va, off_vb, off_vexp, off_vpart;                          // V_xc
   size_t bytes;
 };
 XcWs xc_ws(int64_t np, int n_ao);

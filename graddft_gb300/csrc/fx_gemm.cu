@@ -500,11 +500,11 @@ __global__ void __launch_bounds__(kThreads, 1) fx_gemm_kernel(const GemmArgs A, 
 // loads, so that no sector is asked for twice (L1 was busy for 75 % of the time).
 // 9,376 x 400, four planes: 96 -> 77 us.
 enum Load { kScalar, k16, k32 };  // bytes of a load
-template <Load LOAD>
+template <Load LOAD, bool OCT>
 __global__ void __launch_bounds__(256) fx_rows_kernel(const double *__restrict__ src, int64_t plane_elems, int64_t rows,
                                                       int64_t ld, int k_valid, int chunks,
-                                                      unsigned char *__restrict__ out, int *__restrict__ exps,
-                                                      int *__restrict__ bad) {
+                                                      const int *__restrict__ oct, unsigned char *__restrict__ out,
+                                                      int *__restrict__ exps, int *__restrict__ bad) {
   previous_done();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t tiles = (rows + kTile - 1) / kTile;
@@ -536,27 +536,48 @@ __global__ void __launch_bounds__(256) fx_rows_kernel(const double *__restrict__
       for (int j = 0; j < 8; ++j) v[j] = k + j < k_valid ? x[k + j] : 0.0;
     }
   };
+  auto load_octaves = [&](int k, int (&t)[8]) {
+    const int4 a = *(const int4 *)(oct + k), b = *(const int4 *)(oct + k + 4);
+    t[0] = a.x, t[1] = a.y, t[2] = a.z, t[3] = a.w, t[4] = b.x, t[5] = b.y, t[6] = b.z, t[7] = b.w;
+  };
   uint32_t m = 0;
+  int mt = -(1 << 30);  // with the octaves; a zero counts as 2^(t - 1023)
   for (int k = kg; k < k_valid; k += kChunkK) {
     double v[8];
+    int t[8];
     load8(k, v);
+    if (OCT) load_octaves(k, t);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) m = max(m, (uint32_t)__double2hiint(v[j]) & 0x7FFFFFFFu);
+    for (int j = 0; j < 8; ++j) {
+      const uint32_t h = (uint32_t)__double2hiint(v[j]) & 0x7FFFFFFFu;
+      m = max(m, h);
+      if (OCT) mt = max(mt, (int)min(h, 0x7FF00000u - (450u << 20)) + t[j] * (1 << 20));
+    }
   }
 #pragma unroll
-  for (int o = kRowsPerWarp; o < 32; o *= 2) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+  for (int o = kRowsPerWarp; o < 32; o *= 2) {
+    m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (OCT) mt = max(mt, __shfl_xor_sync(0xffffffffu, mt, o));
+  }
   int emax = exp_field(m);
-  if (emax > kMaxField) atomicOr(bad, 1);
-  if (emax < 1) emax = 1;
+  if (OCT) {
+    if (max(emax, mt >> 20) > kMaxField) atomicOr(bad, 1);
+    emax = mt >> 20;
+  } else {
+    if (emax > kMaxField) atomicOr(bad, 1);
+    if (emax < 1) emax = 1;
+  }
   if (lane < kRowsPerWarp && in) exps[(size_t)plane * rows + row] = emax;
   unsigned char *set = out + ((size_t)plane * tiles + (size_t)(row / kTile)) * chunks * kSetBytes +
                        elem_off((int)(row % kTile), kg);
   for (int k = kg; k < chunks * kChunkK; k += kChunkK, set += kSetBytes) {
     double v[8];
+    int t[8];
     load8(k, v);
+    if (OCT) load_octaves(k, t);
     long long f[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) f[j] = to_fixed(v[j], emax);
+    for (int j = 0; j < 8; ++j) f[j] = to_fixed(v[j], OCT ? emax - t[j] : emax);
     uint4 d[kDigits];
     digits8(f, d);
 #pragma unroll
@@ -590,12 +611,14 @@ cudaError_t launch_gemm(const GemmArgs &a, cudaStream_t st) {
 }
 
 cudaError_t launch_rows(const double *src, int64_t plane_elems, int planes, int64_t rows, int64_t ld, int k_valid,
-                        int chunks, unsigned char *out, int *exps, int *bad, cudaStream_t st) {
+                        int chunks, const int *oct, unsigned char *out, int *exps, int *bad, cudaStream_t st) {
   const dim3 grid((unsigned)((rows + 8 * kRowsPerWarp - 1) / (8 * kRowsPerWarp)), planes);
   // The widest load that every row and plane starts on a boundary of.
   const uintptr_t at = (uintptr_t)src | (uintptr_t)(ld * sizeof(double)) | (uintptr_t)(plane_elems * sizeof(double));
-  auto kernel = at % 32 == 0 ? fx_rows_kernel<k32> : at % 16 == 0 ? fx_rows_kernel<k16> : fx_rows_kernel<kScalar>;
-  launch_next(kernel, grid, 256, 0, st, src, plane_elems, rows, ld, k_valid, chunks, out, exps, bad);
+  auto kernel = at % 32 == 0   ? oct != nullptr ? fx_rows_kernel<k32, true> : fx_rows_kernel<k32, false>
+                : at % 16 == 0 ? oct != nullptr ? fx_rows_kernel<k16, true> : fx_rows_kernel<k16, false>
+                               : oct != nullptr ? fx_rows_kernel<kScalar, true> : fx_rows_kernel<kScalar, false>;
+  launch_next(kernel, grid, 256, 0, st, src, plane_elems, rows, ld, k_valid, chunks, oct, out, exps, bad);
   return cudaGetLastError();
 }
 

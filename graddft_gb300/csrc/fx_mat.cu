@@ -210,13 +210,13 @@ cudaError_t gemm_rows(int64_t M, int N, int K, const double *A, int64_t lda, con
     const int64_t rows = M - m0 < w.slab ? M - m0 : w.slab;
     if ((e = cudaMemsetAsync(bad, 0, 2 * sizeof(int), st)) != cudaSuccess) return e;
     if (b_rows)
-      e = launch_rows(B, 0, 1, N, ldb, K, ch, sw, ew, bad, st);
+      e = launch_rows(B, 0, 1, N, ldb, K, ch, nullptr, sw, ew, bad, st);
     else {
       launch_next(fx_short_cols_kernel, (N + 31) / 32, 128, 0, st, B, K, N, ldb, ch, sw, ew, bad);
       e = cudaGetLastError();
     }
     if (e != cudaSuccess) return e;
-    if ((e = launch_rows(A + m0 * lda, 0, 1, rows, lda, K, ch, sx, ex, bad, st)) != cudaSuccess) return e;
+    if ((e = launch_rows(A + m0 * lda, 0, 1, rows, lda, K, ch, nullptr, sx, ex, bad, st)) != cudaSuccess) return e;
     GemmArgs g{};
     g.a = sw;
     g.b = g.b1 = sx;

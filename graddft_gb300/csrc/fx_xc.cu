@@ -5,7 +5,12 @@
 // (molecule.py:385-502; the sums dens_f64.cu states).  The d_j planes enter only
 // through quadratic forms sum_ab d_j phi_a D_ab d_j phi_b, which need one
 // triangle: column block b takes the row blocks a <= b of U = D + D^T (D itself
-// on the diagonal blocks), (n + 64) / 2n of the products.
+// on the diagonal blocks), (n + 64) / 2n of the products.  A point's row of AOs is fixed
+// point on the largest, which may be one that D hardly occupies (a steep function near its
+// nucleus): phi_a is taken times 2^t and D_ab times 2^-t, t half the exponent of the
+// largest entry of D in row or column a (exact), so that rows are like phi_a sqrt(D_aa).
+// s functions up to exponent 1e10, the two steepest not in D, errors relative to the sums of
+// the terms' sizes: rho 5e-15 -> 3e-16, tau 8e-11 -> 4e-16.
 //
 // V_xc: V_s = phi^T Q_s + sum_j d_j phi^T (c_kin,s d_j phi), with
 // Q_s = c_rho phi + sum_j c_gj d_j phi + c_lap lap phi (vxc_f64.cu).  The second
@@ -47,12 +52,45 @@ namespace {
 constexpr size_t kSlabBytes = (size_t)1 << 30;
 size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 
+// High word of |x|, kNone for a zero.
+constexpr int kNone = -(1 << 30);
+__device__ __forceinline__ int hi_of(double x) {
+  const int h = __double2hiint(x) & 0x7FFFFFFF;
+  return h ? h : kNone;
+}
+// Exponent field of a row's largest high word m, negative where the octaves have moved it there; 1 for a row without
+// values (kNone, or a little above it).
+constexpr int kNoRow = -(600 << 20);
+__device__ __forceinline__ int field_at(int m) { return m < kNoRow ? 1 : m >> 20; }
+
+// Octaves of the AOs, a warp each: half the exponent of the largest entry of either
+// spin's D in row or column a; also clears the non-finite word.  kEmpty where there is
+// none (and past the last AO): the AO's digits are then below all others.
+constexpr int kEmpty = -1200;
+__global__ void __launch_bounds__(256) fx_octaves_kernel(const double *__restrict__ D, int n, int n_pad,
+                                                         int *__restrict__ oct, int *__restrict__ bad) {
+  previous_done();
+  if (blockIdx.x == 0 && threadIdx.x == 0) *bad = 0;
+  const int a = (blockIdx.x * 256 + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (a >= n_pad) return;
+  int m = kNone;
+  for (int b = lane; a < n && b < n; b += 32)
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      const double *Ds = D + (size_t)s * n * n;
+      m = max(m, max(hi_of(Ds[(size_t)a * n + b]), hi_of(Ds[(size_t)b * n + a])));
+    }
+#pragma unroll
+  for (int o = 16; o > 0; o /= 2) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if (lane == 0) oct[a] = m == kNone ? kEmpty : ((m >> 20) - 1023) >> 1;
+}
+
 // Digits of D as the B operand: tile nt = columns 64 nt .. of spin 0, then of
 // spin 1; version 0 is D, version 1 the triangle U (chunks 0 .. nt).  A warp
 // takes eight operand rows (columns of D), lane = (row, eight consecutive k).
-__global__ void __launch_bounds__(128) fx_rdm1_kernel(const double *__restrict__ D, int n, int nb, int versions,
-                                                      unsigned char *__restrict__ out, int *__restrict__ exps,
-                                                      int *__restrict__ bad) {
+__global__ void __launch_bounds__(128) fx_rdm1_kernel(const double *__restrict__ D, int n, int nb,
+                                                      const int *__restrict__ oct, unsigned char *__restrict__ out,
+                                                      int *__restrict__ exps, int *__restrict__ bad) {
   previous_done();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = blockIdx.x * 4 + warp;  // group of eight operand rows: 16 per tile
@@ -68,21 +106,23 @@ __global__ void __launch_bounds__(128) fx_rdm1_kernel(const double *__restrict__
     const double d = Ds[(size_t)k * n + c];
     return version && k < nt * 64 ? d + Ds[(size_t)c * n + k] : d;
   };
-  uint32_t m = 0;
+  int m = kNone;
   for (int k = kg; k < chunks * kChunkK; k += 32)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) m = max(m, (uint32_t)__double2hiint(value(k + j)) & 0x7FFFFFFFu);
+    for (int j = 0; j < 8; ++j) {
+      const int h = hi_of(value(k + j));
+      if (h != kNone) m = max(m, h - oct[k + j] * (1 << 20));
+    }
   m = max(m, __shfl_xor_sync(0xffffffffu, m, 8));
   m = max(m, __shfl_xor_sync(0xffffffffu, m, 16));
-  int emax = exp_field(m);
+  const int emax = field_at(m);
   if (emax > kMaxField) atomicOr(bad, 1);
-  if (emax < 1) emax = 1;
   if (lane < 8) exps[version * nb * kTile + nt * kTile + rt] = emax;
   unsigned char *base = out + ((size_t)version * nb + nt) * nb * kSetBytes;
   for (int k = kg; k < chunks * kChunkK; k += 32) {
     long long f[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) f[j] = to_fixed(value(k + j), emax);
+    for (int j = 0; j < 8; ++j) f[j] = to_fixed(value(k + j), emax + oct[k + j]);
     uint4 d[kDigits];
     digits8(f, d);
     unsigned char *set = base + (size_t)(k / kChunkK) * kSetBytes + elem_off(rt, k % kChunkK);
@@ -185,20 +225,11 @@ __global__ void __launch_bounds__(256, 4) fx_features_kernel(const double *__res
 
 // ---------------------------------------------------------------- V_xc operands
 // High words add like logarithms: hi(x) + hi(y) - hi(1) is at most the product's
-// and below it by less than 1/8 in the mantissa.  kNone: no value (zero).
-constexpr int kNone = -(1 << 30);
+// and below it by less than 1/8 in the mantissa. 
 constexpr int kOneHi = 0x3FF00000;
 static_assert((int)T_PHI == (int)C_RHO && (int)T_DX == (int)C_GX && (int)T_DY == (int)C_GY && (int)T_DZ == (int)C_GZ &&
                   (int)T_LAP == (int)C_LAP,
               "Q pairs plane p with coefficient p");
-__device__ __forceinline__ int hi_of(double x) {
-  const int h = __double2hiint(x) & 0x7FFFFFFF;
-  return h ? h : kNone;
-}
-// Exponent field of a row's largest high word m, negative where the octaves have moved it there; 1 for a row without
-// values (kNone, or a little above it).
-constexpr int kNoRow = -(600 << 20);
-__device__ __forceinline__ int field_at(int m) { return m < kNoRow ? 1 : m >> 20; }
 // Exponent field bound of a sum of `terms` products whose largest has the (approximate) high word m.
 __device__ __forceinline__ int field_of(int m, int octaves) {
   if (m < kNoRow) return 1;
@@ -450,6 +481,8 @@ XcWs xc_ws(int64_t np, int n_ao) {
   off = align256(off + (size_t)2 * w.nb * w.nb * kSetBytes);
   w.off_dexp = off;
   off = align256(off + (size_t)2 * w.nb * kTile * sizeof(int));
+  w.off_doct = off;
+  off = align256(off + (size_t)w.nb * 64 * sizeof(int));
   w.off_a = off;
   off = align256(off + (size_t)4 * (w.dens_slab / kTile) * w.nb * kSetBytes);
   w.off_ea = off;
@@ -478,17 +511,18 @@ cudaError_t launch_density(const double *tab, int64_t np, int ld, int n_ao, cons
   const size_t pe = (size_t)np * ld;
   int *bad = bad_word(ws, w);
   unsigned char *dset = ws + w.off_dset;
-  int *dexp = (int *)(ws + w.off_dexp), *ea = (int *)(ws + w.off_ea);
+  int *dexp = (int *)(ws + w.off_dexp), *ea = (int *)(ws + w.off_ea), *oct = (int *)(ws + w.off_doct);
   double *X = (double *)(ws + w.off_x);
   cudaError_t e;
-  launch_next(fx_clear_kernel, 1, 32, 0, st, bad, nullptr, 0);
-  launch_next(fx_rdm1_kernel, dim3((unsigned)(w.nb * 4), kin ? 2 : 1), 128, 0, st, rdm1, n_ao, w.nb, 2, dset, dexp,
+  launch_next(fx_octaves_kernel, w.nb * 8, 256, 0, st, rdm1, n_ao, w.nb * 64, oct, bad);
+  launch_next(fx_rdm1_kernel, dim3((unsigned)(w.nb * 4), kin ? 2 : 1), 128, 0, st, rdm1, n_ao, w.nb, oct, dset, dexp,
               bad);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   for (int64_t p0 = 0; p0 < np; p0 += w.dens_slab) {
     const int64_t rows = np - p0 < w.dens_slab ? np - p0 : w.dens_slab;
     const int planes = kin ? 4 : 1;
-    if ((e = launch_rows(tab + (size_t)p0 * ld, (int64_t)pe, planes, rows, ld, ld, w.nb, ws + w.off_a, ea, bad, st)) !=
+    if ((e = launch_rows(tab + (size_t)p0 * ld, (int64_t)pe, planes, rows, ld, ld, w.nb, oct, ws + w.off_a, ea, bad,
+                         st)) !=
         cudaSuccess)
       return e;
     GemmArgs g{};

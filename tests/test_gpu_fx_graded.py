@@ -85,3 +85,46 @@ def test_exact_exchange_fock(E):  # noqa: F811
         size = np.abs(phi).T @ np.abs(B)
         bound = (N + 200) * U * size + N * 2.0 ** -56 * np.abs(phi * t).max(0)[:, None] * np.abs(B / t).max(0)
         assert np.all(np.abs(got[s] - phi.T @ B) <= bound), np.max(np.abs(got[s] - phi.T @ B) / bound)
+
+
+@pytest.mark.parametrize("faint", [0.0, 1e-9, 1.0])
+def test_density(E, faint):  # noqa: F811
+    """Features of density matrices that hold little of the two steepest functions.  phi_a is taken times 2^t, D_ab
+    times 2^-t, t half the exponent of D's largest entry in row or column a: X is off by 2^-56 of the product of these
+    rows' largest values for each of n products (2^-55 where D + D^T is contracted), tau by such sums over d_j phi."""
+    N = 300
+    phi, g1, g2, *_ = _tables(N, 4)
+    n = len(ALPHAS)
+    scale = np.where(np.arange(n) < 2, faint, 1.0)
+    D = []
+    for s in range(2):
+        q = np.linalg.qr(np.random.default_rng(s).standard_normal((n, n)))[0][:, :3] * scale[:, None]
+        D.append(q @ q.T)
+    D = np.array(D)
+    r = E.Resident.from_tables(phi, g1, g2, np.ones(N), "fp64", "cuda:0")
+    out = {k: v.cpu().numpy() for k, v in r.density(D).items()}
+    assert r.status() == 0
+    big = np.abs(D).max((0, 1))
+    t = np.where(big > 0, 2.0 ** ((np.frexp(np.maximum(big, 1e-300))[1] - 1) // 2), 0.0)
+    lap, k = g2.sum(-1), 2 * n + 20
+    for s in range(2):
+        X, aX = phi @ D[s], np.abs(phi) @ np.abs(D[s])
+        scaled = np.divide(np.abs(D[s]), t[:, None], out=np.zeros((n, n)), where=t[:, None] > 0).max(0)
+        lost = lambda a, eps: n * 2.0 ** eps * (np.abs(a) * t).max(1)[:, None] * scaled  # noqa: E731
+
+        def check(got, ref, size, extra):
+            bound = k * U * size + extra + 1e-290
+            assert np.all(np.abs(got - ref) <= bound), np.max(np.abs(got - ref) / bound)
+
+        check(out["rho"][:, s], (X * phi).sum(1), (aX * np.abs(phi)).sum(1), (lost(phi, -56) * np.abs(phi)).sum(1))
+        kin, akin, klost = np.zeros(N), np.zeros(N), np.zeros(N)
+        for j in range(3):
+            g = g1[..., j]
+            check(out["grad_rho"][:, s, j], 2 * (X * g).sum(1), 2 * (aX * np.abs(g)).sum(1),
+                  2 * (lost(phi, -56) * np.abs(g)).sum(1))
+            kin += ((g @ D[s]) * g).sum(1)
+            akin += ((np.abs(g) @ np.abs(D[s])) * np.abs(g)).sum(1)
+            klost += (lost(g, -55) * np.abs(g)).sum(1)
+        check(out["tau"][:, s], kin / 2, akin / 2, klost / 2)
+        check(out["lapl"][:, s], 2 * kin + 2 * (X * lap).sum(1), 2 * akin + 2 * (aX * np.abs(lap)).sum(1),
+              2 * klost + 2 * (lost(phi, -56) * np.abs(lap)).sum(1))
