@@ -138,14 +138,21 @@ cudaError_t launch_rows(const double *src, int64_t plane_elems, int planes, int6
 // error word or null (an expired wait leaves NaN in the output either way); part: partials of the plain kernel that takes over where an operand is not finite (nsplit x M x N doubles).
 size_t gemm_rows_bytes(int64_t M, int N, int K);
 size_t gemm_cols_bytes(int M, int N, int64_t K);
-// C[m][n] = sum_k A[m][k] B[k][n] (B stored N x K when b_rows) + add[m][n] (laid out like C; null: nothing).
+// C[m][n] = sum_k A[m][k] B[k][n] (B stored N x K when b_rows) + add[m][n] (laid out like C; null: nothing).  oct, or
+// null (it has to be with b_rows): octaves_len(K) octaves t, aligned to 16 bytes; A's columns are taken times 2^t, B's
+// rows times 2^-t.
 cudaError_t gemm_rows(int64_t M, int N, int K, const double *A, int64_t lda, const double *B, int64_t ldb, bool b_rows,
-                      double *C, int64_t ldc, const double *add, unsigned char *ws, int *err, cudaStream_t st);
+                      const int *oct, double *C, int64_t ldc, const double *add, unsigned char *ws, int *err, cudaStream_t st);
 // C[m][n] = sum_k A[k][m] B[k][n], C contiguous (M x N).  oct, or null: K octaves t; A's rows are taken times 2^t and
 // B's times 2^-t, for operands that are graded against one another (fx_xc.cu).
 cudaError_t gemm_cols(int M, int N, int64_t K, const double *A, int64_t lda, const double *B, int64_t ldb,
                       const int *oct, double *C, unsigned char *ws, int *err, int nsplit, double *part,
                       cudaStream_t st);
+
+// Octaves of the AOs for products of AO values with D (2, n, n), fx_xc.cu: octaves_len(n) of them.  bad: a word to clear,
+// or null.
+inline int octaves_len(int n) { return (n + 63) / 64 * 64; }
+cudaError_t launch_octaves(const double *D, int n, int *oct, int *bad, cudaStream_t st);
 
 // Feature sets of fx_xc.cu: the FP64 form's density and V_xc contractions.
 struct XcWs {

@@ -29,24 +29,28 @@ constexpr int64_t tiles_of(int64_t n) { return (n + kTile - 1) / kTile; }
 constexpr int64_t chunks_of(int64_t k) { return (k + kChunkK - 1) / kChunkK; }
 
 // Columns of a short row-major matrix X [k_rows][cols] as operand rows (weights,
-// density matrices): a warp takes eight columns, lane = (column, eight k), both
-// passes over k in one kernel.
+// density matrices), with oct row k times 2^-oct[k]: a warp takes eight columns, lane =
+// (column, eight k), both passes over k in one kernel.
 __global__ void __launch_bounds__(128) fx_short_cols_kernel(const double *__restrict__ X, int k_rows, int cols,
-                                                            int64_t ld, int chunks, unsigned char *__restrict__ out,
-                                                            int *__restrict__ exps, int *__restrict__ bad) {
+                                                            int64_t ld, int chunks, const int *__restrict__ oct,
+                                                            unsigned char *__restrict__ out, int *__restrict__ exps,
+                                                            int *__restrict__ bad) {
   previous_done();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int c0 = (blockIdx.x * 4 + warp) * 8;
   if (c0 >= cols) return;
   const int c = c0 + (lane & 7), kg = (lane >> 3) * 8;
   auto value = [&](int k) { return c < cols && k < k_rows ? X[(size_t)k * ld + c] : 0.0; };
-  uint32_t m = 0;
+  int m = 0;
   for (int k = kg; k < k_rows; k += 32)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) m = max(m, (uint32_t)__double2hiint(value(k + j)) & 0x7FFFFFFFu);
+    for (int j = 0; j < 8; ++j) {
+      const int h = __double2hiint(value(k + j)) & 0x7FFFFFFF;
+      if (h != 0) m = max(m, oct != nullptr ? h - oct[k + j] * (1 << 20) : h);
+    }
   m = max(m, __shfl_xor_sync(0xffffffffu, m, 8));
   m = max(m, __shfl_xor_sync(0xffffffffu, m, 16));
-  int emax = exp_field(m);
+  int emax = m >> 20;
   if (emax > kMaxField) atomicOr(bad, 1);
   if (emax < 1) emax = 1;
   if (lane < 8 && c < cols) exps[c] = emax;
@@ -54,7 +58,7 @@ __global__ void __launch_bounds__(128) fx_short_cols_kernel(const double *__rest
   for (int k = kg; k < chunks * kChunkK; k += 32) {
     long long f[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) f[j] = to_fixed(value(k + j), emax);
+    for (int j = 0; j < 8; ++j) f[j] = to_fixed(value(k + j), oct != nullptr ? emax + oct[k + j] : emax);
     uint4 d[kDigits];
     digits8(f, d);
     unsigned char *set = base + (size_t)(k / kChunkK) * kSetBytes + elem_off(c % kTile, k % kChunkK);
@@ -199,7 +203,9 @@ size_t gemm_rows_bytes(int64_t M, int N, int K) { return rows_ws(M, N, K).bytes 
 size_t gemm_cols_bytes(int M, int N, int64_t K) { return cols_ws(M, N, K).bytes + 256; }
 
 cudaError_t gemm_rows(int64_t M, int N, int K, const double *A, int64_t lda, const double *B, int64_t ldb, bool b_rows,
-                      double *C, int64_t ldc, const double *add, unsigned char *ws, int *err, cudaStream_t st) {
+                      const int *oct, double *C, int64_t ldc, const double *add, unsigned char *ws, int *err,
+                      cudaStream_t st) {
+  if (b_rows && oct != nullptr) return cudaErrorInvalidValue;
   const RowsWs w = rows_ws(M, N, K);
   const int ch = (int)chunks_of(K);
   ws = aligned(ws);
@@ -212,11 +218,11 @@ cudaError_t gemm_rows(int64_t M, int N, int K, const double *A, int64_t lda, con
     if (b_rows)
       e = launch_rows(B, 0, 1, N, ldb, K, ch, nullptr, sw, ew, bad, st);
     else {
-      launch_next(fx_short_cols_kernel, (N + 31) / 32, 128, 0, st, B, K, N, ldb, ch, sw, ew, bad);
+      launch_next(fx_short_cols_kernel, (N + 31) / 32, 128, 0, st, B, K, N, ldb, ch, oct, sw, ew, bad);
       e = cudaGetLastError();
     }
     if (e != cudaSuccess) return e;
-    if ((e = launch_rows(A + m0 * lda, 0, 1, rows, lda, K, ch, nullptr, sx, ex, bad, st)) != cudaSuccess) return e;
+    if ((e = launch_rows(A + m0 * lda, 0, 1, rows, lda, K, ch, oct, sx, ex, bad, st)) != cudaSuccess) return e;
     GemmArgs g{};
     g.a = sw;
     g.b = g.b1 = sx;

@@ -64,13 +64,13 @@ constexpr int kNoRow = -(600 << 20);
 __device__ __forceinline__ int field_at(int m) { return m < kNoRow ? 1 : m >> 20; }
 
 // Octaves of the AOs, a warp each: half the exponent of the largest entry of either
-// spin's D in row or column a; also clears the non-finite word.  kEmpty where there is
+// spin's D in row or column a; also clears the non-finite word, if any.  kEmpty where there is
 // none (and past the last AO): the AO's digits are then below all others.
 constexpr int kEmpty = -1200;
 __global__ void __launch_bounds__(256) fx_octaves_kernel(const double *__restrict__ D, int n, int n_pad,
                                                          int *__restrict__ oct, int *__restrict__ bad) {
   previous_done();
-  if (blockIdx.x == 0 && threadIdx.x == 0) *bad = 0;
+  if (blockIdx.x == 0 && threadIdx.x == 0 && bad != nullptr) *bad = 0;
   const int a = (blockIdx.x * 256 + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (a >= n_pad) return;
   int m = kNone;
@@ -482,7 +482,7 @@ XcWs xc_ws(int64_t np, int n_ao) {
   w.off_dexp = off;
   off = align256(off + (size_t)2 * w.nb * kTile * sizeof(int));
   w.off_doct = off;
-  off = align256(off + (size_t)w.nb * 64 * sizeof(int));
+  off = align256(off + (size_t)octaves_len(n_ao) * sizeof(int));
   w.off_a = off;
   off = align256(off + (size_t)4 * (w.dens_slab / kTile) * w.nb * kSetBytes);
   w.off_ea = off;
@@ -505,6 +505,12 @@ XcWs xc_ws(int64_t np, int n_ao) {
   return w;
 }
 
+cudaError_t launch_octaves(const double *D, int n, int *oct, int *bad, cudaStream_t st) {
+  const int len = octaves_len(n);
+  launch_next(fx_octaves_kernel, len / 8, 256, 0, st, D, n, len, oct, bad);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_density(const double *tab, int64_t np, int ld, int n_ao, const double *rdm1, bool kin, double *feat,
                            unsigned char *ws, int *err, cudaStream_t st) {
   const XcWs w = xc_ws(np, n_ao);
@@ -514,7 +520,7 @@ cudaError_t launch_density(const double *tab, int64_t np, int ld, int n_ao, cons
   int *dexp = (int *)(ws + w.off_dexp), *ea = (int *)(ws + w.off_ea), *oct = (int *)(ws + w.off_doct);
   double *X = (double *)(ws + w.off_x);
   cudaError_t e;
-  launch_next(fx_octaves_kernel, w.nb * 8, 256, 0, st, rdm1, n_ao, w.nb * 64, oct, bad);
+  if ((e = launch_octaves(rdm1, n_ao, oct, bad, st)) != cudaSuccess) return e;
   launch_next(fx_rdm1_kernel, dim3((unsigned)(w.nb * 4), kin ? 2 : 1), 128, 0, st, rdm1, n_ao, w.nb, oct, dset, dexp,
               bad);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;

@@ -11,7 +11,8 @@
 // warp per (point, spin) takes the row dot with chi; B_s = -1/2 sum_w g chi,
 // then F_s = ao^T B_s with the grid split over CTAs and the partials summed in
 // a fixed order.  g carries the integration weights, smallest where the steepest AOs are
-// largest: ao and B share its exponent at each point (fx_xc.cu says why).
+// largest: ao and B share its exponent at each point, and ao and D those of D's rows
+// (fx_xc.cu says why).
 //
 // Mixed (TF32x3) form: the same two contractions on the block-scaled
 // three-slice tcgen05 GEMM (tcg3: exact hi*hi chunk sums, compensated FP32
@@ -245,6 +246,11 @@ size_t hf_gemm_off(int64_t n_grid, int n_ao) {
   return align256((size_t)2 * n_grid * n_ao * sizeof(double)) +
          align256((size_t)hf_splits(n_grid) * n_ao * n_ao * sizeof(double));
 }
+// The octaves of an FP64 call (the workspace itself may be aligned to 8 bytes only); `len` of them, then the scratch.
+int *hf_octaves(void *ws, int64_t n_grid, int n_ao) {
+  return (int *)(((uintptr_t)ws + hf_gemm_off(n_grid, n_ao) + 255) & ~(uintptr_t)255);
+}
+unsigned char *hf_scratch(int *oct, int64_t len) { return (unsigned char *)oct + align256((size_t)len * sizeof(int)); }
 
 int check_hf_args(const char *who, int form, const void *ao, const void *chi, int64_t n_grid, int n_ao, int n_omega,
                   const void *out, const void *ws, size_t ws_bytes) {
@@ -370,10 +376,10 @@ int gdft_hf_workspace_bytes_form(int64_t n_grid, int32_t n_ao, int32_t n_omega, 
     *bytes = hf_tc_layout(n_grid, n_ao).bytes;
     return GDFT_OK;
   }
-  // X or B: [2][n_grid][n_ao]; split partials of F: [nsplit][n_ao][n_ao]; the GEMMs' scratch (F's: with the octaves).
-  const size_t rows = fx::gemm_rows_bytes(n_grid, n_ao, n_ao);
+  // X or B: [2][n_grid][n_ao]; split partials of F: [nsplit][n_ao][n_ao]; the GEMMs' octaves and scratch, aligned.
+  const size_t rows = align256((size_t)fx::octaves_len(n_ao) * sizeof(int)) + fx::gemm_rows_bytes(n_grid, n_ao, n_ao);
   const size_t cols = align256((size_t)n_grid * sizeof(int)) + fx::gemm_cols_bytes(n_ao, n_ao, n_grid);
-  *bytes = hf_gemm_off(n_grid, n_ao) + (rows > cols ? rows : cols);
+  *bytes = hf_gemm_off(n_grid, n_ao) + 256 + (rows > cols ? rows : cols);
   return GDFT_OK;
 }
 
@@ -394,10 +400,12 @@ int gdft_hf_energy_density_form(const double *d_ao, const double *d_rdm1, const 
   if (form == GDFT_TF32X3) return hf_energy_density_tc(d_ao, d_rdm1, d_chi, n_grid, n_ao, n_omega, d_ehf,
                                                        (char *)d_ws, st);
   double *X = (double *)d_ws;
+  int *oct = hf_octaves(d_ws, n_grid, n_ao);
+  if ((rc = check_cuda(fx::launch_octaves(d_rdm1, n_ao, oct, nullptr, st), "hf octaves"))) return rc;
   for (int s = 0; s < 2; ++s)
     if ((rc = check_cuda(fx::gemm_rows(n_grid, n_ao, n_ao, d_ao, n_ao, d_rdm1 + (size_t)s * n_ao * n_ao, n_ao, false,
-                                       X + (size_t)s * n_grid * n_ao, n_ao, nullptr,
-                                       (unsigned char *)d_ws + hf_gemm_off(n_grid, n_ao), nullptr, st),
+                                       oct, X + (size_t)s * n_grid * n_ao, n_ao, nullptr,
+                                       hf_scratch(oct, fx::octaves_len(n_ao)), nullptr, st),
                          "hf ao.D")))
       return rc;
   const int64_t threads = 2 * n_grid * 32;
@@ -426,14 +434,14 @@ int gdft_hf_fock_form(const double *d_ao, const double *d_chi, const double *d_g
   double *part = (double *)((char *)d_ws + align256((size_t)2 * n_grid * n_ao * sizeof(double)));
   const size_t total = (size_t)2 * n_grid * n_ao;
   launch_next(hf_bmat_kernel, (unsigned)((total + 255) / 256), 256, 0, st, d_chi, d_g, n_grid, n_ao, n_omega, B);
-  int *oct = (int *)((char *)d_ws + hf_gemm_off(n_grid, n_ao));
-  unsigned char *gws = (unsigned char *)oct + align256((size_t)n_grid * sizeof(int));
+  int *oct = hf_octaves(d_ws, n_grid, n_ao);
   launch_next(hf_octaves_kernel, (unsigned)((n_grid + 255) / 256), 256, 0, st, d_g, n_grid, 2 * n_omega, oct);
   if ((rc = check_cuda(cudaGetLastError(), "hf B"))) return rc;
   const int nsplit = hf_splits(n_grid);
   for (int s = 0; s < 2; ++s)
     if ((rc = check_cuda(fx::gemm_cols(n_ao, n_ao, n_grid, d_ao, n_ao, B + (size_t)s * n_grid * n_ao, n_ao,
-                                       oct, d_fock_hf + (size_t)s * n_ao * n_ao, gws, nullptr, nsplit, part, st),
+                                       oct, d_fock_hf + (size_t)s * n_ao * n_ao, hf_scratch(oct, n_grid), nullptr, nsplit,
+                                       part, st),
                          "hf ao^T B")))
       return rc;
   return GDFT_OK;

@@ -343,7 +343,7 @@ int net_forward(const MlpShape &S, const double *params, const MlpLayout &L, dou
   const double *Wout = params + layer_offset(S, S.n_layers);
   int rc;
   auto mul = [&](int N, int K, const double *A, int lda, const double *B, double *C) {  // C = A B, B (K x N)
-    return fx::gemm_rows(np, N, K, A, lda, B, N, false, C, N, nullptr, (unsigned char *)(ws + L.fx), err, st);
+    return fx::gemm_rows(np, N, K, A, lda, B, N, false, nullptr, C, N, nullptr, (unsigned char *)(ws + L.fx), err, st);
   };
   if ((rc = check_cuda(mul(Wd, S.n_in, u, kDm21InPad, W0, h), "mlp dense_0"))) return rc;
   launch_next(tanh_bias_kernel, (unsigned)((act + 255) / 256), 256, 0, st, h, b0, act, Wd);
@@ -453,7 +453,7 @@ int mlp_run_f64(const MlpShape &S, const double *params, double *dparams, const 
     return fx::gemm_cols(M, N, np, A, lda, B, ldb, nullptr, C, (unsigned char *)(ws + L.fx), err, ns, kpart, st);
   };
   auto mul_t = [&](int N, int K, const double *A, const double *B, double *C, int ldc, const double *add) {
-    return fx::gemm_rows(np, N, K, A, K, B, K, true, C, ldc, add, (unsigned char *)(ws + L.fx), err, st);
+    return fx::gemm_rows(np, N, K, A, K, B, K, true, nullptr, C, ldc, add, (unsigned char *)(ws + L.fx), err, st);
   };
   auto col_sum = [&](const double *X, int64_t rows, int ncols, int ld, double *out) {
     return col_sums(X, rows, ncols, ld, out, colpart, kColBlocks, st);

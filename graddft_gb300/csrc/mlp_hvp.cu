@@ -353,10 +353,10 @@ int mlp_hvp_f64(const MlpShape &S, const double *params, double *dparams, const 
 
   unsigned char *fxws = (unsigned char *)(ws + L.fx);
   auto mul = [&](int N, int K, const double *A, int lda, const double *B, double *C) {  // C = A B, B (K x N)
-    return fx::gemm_rows(rows2, N, K, A, lda, B, N, false, C, N, nullptr, fxws, err, st);
+    return fx::gemm_rows(rows2, N, K, A, lda, B, N, false, nullptr, C, N, nullptr, fxws, err, st);
   };
   auto mul_t = [&](int N, int K, const double *A, const double *B, double *C, int ldc, const double *add) {
-    return fx::gemm_rows(rows2, N, K, A, K, B, K, true, C, ldc, add, fxws, err, st);
+    return fx::gemm_rows(rows2, N, K, A, K, B, K, true, nullptr, C, ldc, add, fxws, err, st);
   };
 
   // ---- tangent-augmented forward ----

@@ -246,7 +246,7 @@ int make_plan(const gdft_basis *b, PairPlan &plan, const char *who) {
 }
 
 struct NuWs {
-  size_t off_boys, off_pairs, off_pp, off_nu, off_x, off_fx, bytes;  // off_fx: scratch of the GEMM X = ao D
+  size_t off_boys, off_pairs, off_pp, off_nu, off_x, off_oct, off_fx, bytes;  // off_oct, off_fx: of the GEMM X = ao D
 };
 
 NuWs nu_ws(const PairPlan &plan, int n_ao, int64_t chunk, bool want_chi, int n_omega) {
@@ -259,11 +259,13 @@ NuWs nu_ws(const PairPlan &plan, int n_ao, int64_t chunk, bool want_chi, int n_o
   W.off_pp = off;
   off = al256(off + (size_t)n_omega * plan.n_pp * sizeof(double));
   W.off_nu = off;
-  W.off_x = W.off_fx = off;
+  W.off_x = W.off_oct = W.off_fx = off;
   if (want_chi) {
     off = al256(off + (size_t)n_ao * n_ao * chunk * sizeof(double));
     W.off_x = off;
     off = al256(off + (size_t)2 * chunk * n_ao * sizeof(double));
+    W.off_oct = off;
+    off = al256(off + (size_t)fx::octaves_len(n_ao) * sizeof(int));
     W.off_fx = off;
     off = al256(off + fx::gemm_rows_bytes(chunk, n_ao, n_ao));
   }
@@ -426,6 +428,8 @@ int gdft_chi(const gdft_basis *basis, const double *d_coords, const double *d_ao
   char *ws = (char *)d_ws;
   double *nu = (double *)(ws + W.off_nu);
   double *X = (double *)(ws + W.off_x);
+  int *oct = (int *)(ws + W.off_oct);
+  if ((rc = check_cuda(fx::launch_octaves(d_rdm1, n, oct, nullptr, st), who))) return rc;
   for (int w = 0; w < n_omega; ++w)
     if ((rc = setup_nu(B, plan, W, ws, w, h_omegas[w], w == 0, who, st))) return rc;
   for (int64_t p0 = 0; p0 < n_grid; p0 += pc) {
@@ -433,7 +437,7 @@ int gdft_chi(const gdft_basis *basis, const double *d_coords, const double *d_ao
     // X_s = ao[p0 : p0 + np_] D_s, shared by the omegas
     for (int s = 0; s < 2; ++s)
       if ((rc = check_cuda(fx::gemm_rows(np_, n, n, d_ao + p0 * n, n, d_rdm1 + (size_t)s * n * n, n, false,
-                                         X + (size_t)s * pc * n, n, nullptr, (unsigned char *)(ws + W.off_fx), nullptr,
+                                         oct, X + (size_t)s * pc * n, n, nullptr, (unsigned char *)(ws + W.off_fx), nullptr,
                                          st),
                            who)))
         return rc;

@@ -128,3 +128,21 @@ def test_density(E, faint):  # noqa: F811
         check(out["tau"][:, s], kin / 2, akin / 2, klost / 2)
         check(out["lapl"][:, s], 2 * kin + 2 * (X * lap).sum(1), 2 * akin + 2 * (aX * np.abs(lap)).sum(1),
               2 * klost + 2 * (lost(phi, -56) * np.abs(lap)).sum(1))
+
+
+def test_exact_exchange_energy(E):  # noqa: F811
+    """ehf = -1/2 sum_b chi_b X_b with X = ao D as in the density, D holding nothing of the four steepest functions."""
+    N, n = 300, len(ALPHAS)
+    phi, *_ = _tables(N, 5)
+    chi = np.random.default_rng(6).standard_normal((N, 1, 2, n))
+    D = np.random.default_rng(7).standard_normal((2, n, n))
+    D[:, :4] = D[:, :, :4] = 0.0
+    got = E.hf_energy_density(*(torch.as_tensor(x, device="cuda") for x in (phi, D, chi))).cpu().numpy()
+    big = np.maximum(np.abs(D).max((0, 1)), np.abs(D).max((0, 2)))[4:]
+    t = np.r_[np.zeros(4), 2.0 ** ((np.frexp(big)[1] - 1) // 2)]
+    for s in range(2):
+        c = np.abs(chi[:, 0, s])
+        scaled = (np.abs(D[s, 4:]) / t[4:, None]).max(0)
+        bound = (2 * n + 20) * U * (np.abs(phi) @ np.abs(D[s]) * c).sum(1)
+        bound += n * 2.0 ** -56 * (np.abs(phi) * t).max(1) * (scaled * c).sum(1)
+        assert np.all(np.abs(got[0, s] + 0.5 * (chi[:, 0, s] * (phi @ D[s])).sum(1)) <= bound)
