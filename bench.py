@@ -583,7 +583,7 @@ def run_stream(args):
         "data": "synthetic (seeded Gaussian basis, evaluated per chunk on the device)",
         "config": {"workload": _workload(args.n_grid, args.n_ao) + ", AO tables recomputed per chunk",
                    "n_ao": args.n_ao, "n_grid": args.n_grid, "chunk": c.chunk, "form": form},
-        "device_bytes": {"chunked_workspace": c.nbytes, "resident_tables": mol_bytes.value},
+        "device_bytes": {"chunked_workspace": c.workspace_bytes(c.chunk), "resident_tables": mol_bytes.value},
         "stage_ms_per_step": stage, "clocks": clk.summary(),
         "e_xc": float(exc),
     }

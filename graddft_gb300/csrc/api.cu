@@ -84,6 +84,8 @@ MolLayout mol_layout(int64_t n_grid, int n_ao, int precision) {
     L.off_af = off;
     off = align256(off + kPlanes * 2 * plane);
   }
+  L.off_err = off;
+  off = align256(off + sizeof(int));
   L.bytes = off;
   return L;
 }
@@ -116,8 +118,6 @@ WsLayout ws_layout(const gdft_molecule *m) {
     W.off_q = off;
     off = align256(off + vxc_q_bytes(np, m->n_ao));
   }
-  W.off_err = off;
-  off = align256(off + 64);
   W.bytes = off;
   return W;
 }
@@ -191,6 +191,10 @@ static const double *mol_tab(const gdft_molecule *m) {
 }
 static const double *mol_w(const gdft_molecule *m) {
   return (const double *)((const char *)m->buffer + mol_layout(m->n_grid, m->n_ao, m->precision).off_w);
+}
+// The device word where a kernel's expired wait is recorded.
+static int *mol_err(const gdft_molecule *m) {
+  return (int *)((char *)m->buffer + mol_layout(m->n_grid, m->n_ao, m->precision).off_err);
 }
 
 static const float *mol_pm(const gdft_molecule *m) {
@@ -331,16 +335,17 @@ static int batch_layout(int n_mol, const gdft_molecule *mols, const gdft_network
 }
 
 // Density stage into ws.feat.  kin: the Laplacian or tau is read (otherwise the FP64 form leaves both at 0).
-static int run_density(const gdft_molecule *m, const double *rdm1, char *ws, cudaStream_t st, bool kin = true) {
+// err: where an expired wait is recorded (null: the molecule's own word).
+static int run_density(const gdft_molecule *m, const double *rdm1, char *ws, cudaStream_t st, bool kin = true,
+                       int *err = nullptr) {
   const WsLayout W = ws_layout(m);
+  if (err == nullptr) err = mol_err(m);
   double *feat = (double *)(ws + W.off_feat);
   if (m->precision == GDFT_FP64) {
     StageTimer tm(GDFT_STAGE_DENSITY, st);
     const int64_t np = m->n_grid_pad;
     unsigned char *fw = (unsigned char *)(ws + W.off_fx);
-    int rc = check_cuda(fx::launch_density(mol_tab(m), np, m->ld, m->n_ao, rdm1, kin, feat, fw,
-                                           (int *)(ws + W.off_err), st),
-                        "fx density");
+    int rc = check_cuda(fx::launch_density(mol_tab(m), np, m->ld, m->n_ao, rdm1, kin, feat, fw, err, st), "fx density");
     if (rc) return rc;
     const int *bad = fx::bad_word(fw, fx::xc_ws(np, m->n_ao));  // the plain kernel runs for operands that are not finite
     return check_cuda(launch_dens_f64(mol_tab(m), np, m->ld, m->n_ao, rdm1, feat, bad, st), "dens_f64");
@@ -353,7 +358,7 @@ static int run_density(const gdft_molecule *m, const double *rdm1, char *ws, cud
     if ((rc = check_cuda(launch_pack_rdm1(rdm1, m->n_ao, ldk, dpk, st), "pack_rdm1"))) return rc;
   }
   StageTimer tm(GDFT_STAGE_DENSITY, st);
-  return check_cuda(launch_dens_tc(mol_pm(m), dpk, m->n_grid_pad, ldk, feat, (int *)(ws + W.off_err), st),
+  return check_cuda(launch_dens_tc(mol_pm(m), dpk, m->n_grid_pad, ldk, feat, err, st),
                     "dens_tc");
 }
 
@@ -362,10 +367,11 @@ static int run_density(const gdft_molecule *m, const double *rdm1, char *ws, cud
 using namespace gdft;
 
 // V_xc contraction of the adjoint coefficients in ws.coef into d_vxc.
-// kin: coef's C_KIN rows may be non-zero.
+// kin: coef's C_KIN rows may be non-zero.  err: as in run_density.
 static int run_vxc(const gdft_molecule *mol, const double *coef, double *d_vxc, char *ws, cudaStream_t st,
-                   bool kin = true) {
+                   bool kin = true, int *err = nullptr) {
   const WsLayout W = ws_layout(mol);
+  if (err == nullptr) err = mol_err(mol);
   int rc;
   double *vpart = (double *)(ws + W.off_vpart);
   if (mol->precision == GDFT_FP64) {
@@ -374,8 +380,7 @@ static int run_vxc(const gdft_molecule *mol, const double *coef, double *d_vxc, 
     const int *bad = fx::bad_word(fw, fx::xc_ws(np, mol->n_ao));  // as in run_density
     {
       StageTimer tm(GDFT_STAGE_VXC, st);
-      if ((rc = check_cuda(fx::launch_vxc(mol_tab(mol), np, mol->ld, mol->n_ao, coef, kin, fw, d_vxc,
-                                          (int *)(ws + W.off_err), st),
+      if ((rc = check_cuda(fx::launch_vxc(mol_tab(mol), np, mol->ld, mol->n_ao, coef, kin, fw, d_vxc, err, st),
                            "fx vxc")))
         return rc;
       rc = check_cuda(launch_vxc_f64(mol_tab(mol), np, mol->ld, mol->n_ao, coef, W.n_vsplit, vpart, bad, st),
@@ -387,8 +392,7 @@ static int run_vxc(const gdft_molecule *mol, const double *coef, double *d_vxc, 
   }
   StageTimer tm(GDFT_STAGE_VXC, st);
   return check_cuda(launch_vxc_q_tc(mol_av(mol), mol_af(mol), coef, mol->n_grid_pad, (int)round_up(mol->n_ao, 128),
-                                    mol->n_ao, kin, (float *)(ws + W.off_q), vpart, d_vxc, (int *)(ws + W.off_err),
-                                    st),
+                                    mol->n_ao, kin, (float *)(ws + W.off_q), vpart, d_vxc, err, st),
                     "vxc_q_tc");
 }
 
@@ -503,6 +507,7 @@ int gdft_molecule_load(const gdft_molecule *mol, const double *d_ao, const doubl
   const MolLayout L = mol_layout(mol->n_grid, mol->n_ao, mol->precision);
   double *tab = (double *)((char *)mol->buffer + L.off_tab);
   double *w = (double *)((char *)mol->buffer + L.off_w);
+  if ((rc = check_cuda(cudaMemsetAsync(mol_err(mol), 0, sizeof(int), (cudaStream_t)stream), "error word"))) return rc;
   StageTimer tm(GDFT_STAGE_AO, (cudaStream_t)stream);
   if (mol->precision == GDFT_TF32X3)
     return check_cuda(launch_pack_tables(d_ao, d_grad_ao, d_grad2_ao, nullptr, nullptr, d_weights, mol->n_grid,
@@ -526,6 +531,7 @@ int gdft_molecule_eval_basis(const gdft_molecule *mol, const double *d_basis, co
   const MolLayout L = mol_layout(mol->n_grid, mol->n_ao, mol->precision);
   double *tab = (double *)((char *)mol->buffer + L.off_tab);
   double *w = (double *)((char *)mol->buffer + L.off_w);
+  if ((rc = check_cuda(cudaMemsetAsync(mol_err(mol), 0, sizeof(int), (cudaStream_t)stream), "error word"))) return rc;
   StageTimer tm(GDFT_STAGE_AO, (cudaStream_t)stream);
   if (mol->precision == GDFT_TF32X3)
     return check_cuda(launch_pack_tables(nullptr, nullptr, nullptr, d_basis, d_coords, d_weights, mol->n_grid,
@@ -602,6 +608,7 @@ int gdft_molecule_eval_shells(const gdft_molecule *mol, const gdft_basis *basis,
   if ((rc = check_aligned8(d_coords, "coords")) || (rc = check_aligned8(d_weights, "weights"))) return rc;
   const MolLayout L = mol_layout(mol->n_grid, mol->n_ao, mol->precision);
   double *w = (double *)((char *)mol->buffer + L.off_w);
+  if ((rc = check_cuda(cudaMemsetAsync(mol_err(mol), 0, sizeof(int), (cudaStream_t)stream), "error word"))) return rc;
   StageTimer tm(GDFT_STAGE_AO, (cudaStream_t)stream);
   if (mol->precision == GDFT_TF32X3)
     return check_cuda(launch_pack_tables(nullptr, nullptr, nullptr, nullptr, d_coords, d_weights, mol->n_grid,
@@ -745,7 +752,7 @@ static int kpt_density(const gdft_molecule *mols, int32_t K, const double *rdm1c
   int rc;
   for (int k = 0; k < K; ++k) {
     if ((rc = check_cuda(launch_kpt_build_m(rdm1c, K, k, n, h_kweights[k], M, st), "kpt_build_m"))) return rc;
-    if ((rc = run_density(&mols[k], M, ws, st, kin))) return rc;
+    if ((rc = run_density(&mols[k], M, ws, st, kin, mol_err(&mols[0])))) return rc;
     if ((rc = check_cuda(launch_feat_add((const double *)(ws + W.off_feat), fsum, nf, k == 0, st), "feat_add")))
       return rc;
   }
@@ -832,7 +839,7 @@ int gdft_kpoint_xc_energy_and_grads(const gdft_molecule *mols, int32_t n_kpt, co
   const int n = mols[0].n_ao / 2;
   double *V = (double *)(ws + KW.off_v);
   for (int k = 0; k < n_kpt; ++k) {
-    if ((rc = run_vxc(&mols[k], coef, V, ws, st, kin))) return rc;
+    if ((rc = run_vxc(&mols[k], coef, V, ws, st, kin, mol_err(&mols[0])))) return rc;
     if ((rc = check_cuda(launch_kpt_vxc(V, n_kpt, k, n, h_kweights[k], d_vxc, st), "kpt_vxc"))) return rc;
   }
   return GDFT_OK;
@@ -929,10 +936,10 @@ int gdft_neural_xc_energy_and_grads(const gdft_molecule *mol, const double *d_rd
     StageTimer tm(GDFT_STAGE_MLP, st);
     if (net->precision == GDFT_TF32X3)
       rc = mlp_run_tc(net_shape(net), d_params, d_dparams, feat, d_ehf, mol_w(mol), mol->n_grid, mol->n_grid_pad,
-                      net->clip, ws + W.bytes, d_exc, coef, (int *)(ws + W.off_err), st);
+                      net->clip, ws + W.bytes, d_exc, coef, mol_err(mol), st);
     else
       rc = mlp_run_f64(net_shape(net), d_params, d_dparams, feat, d_ehf, mol_w(mol), mol->n_grid, mol->n_grid_pad,
-                       net->clip, (double *)(ws + W.bytes), d_exc, coef, (int *)(ws + W.off_err), st);
+                       net->clip, (double *)(ws + W.bytes), d_exc, coef, mol_err(mol), st);
     if (rc) return rc;
   }
   if (d_vxc == nullptr) return GDFT_OK;
@@ -977,10 +984,10 @@ int gdft_neural_xc_hf_grads(const gdft_molecule *mol, const double *d_rdm1, cons
     StageTimer tm(GDFT_STAGE_MLP, st);
     if (net->precision == GDFT_TF32X3)
       rc = mlp_run_tc(net_shape(net), d_params, nullptr, feat, d_ehf, mol_w(mol), mol->n_grid, mol->n_grid_pad,
-                      net->clip, ws + W.bytes, d_exc, coef, (int *)(ws + W.off_err), st);
+                      net->clip, ws + W.bytes, d_exc, coef, mol_err(mol), st);
     else
       rc = mlp_run_f64(net_shape(net), d_params, nullptr, feat, d_ehf, mol_w(mol), mol->n_grid, mol->n_grid_pad,
-                       net->clip, mws, d_exc, coef, (int *)(ws + W.off_err), st);
+                       net->clip, mws, d_exc, coef, mol_err(mol), st);
     if (rc) return rc;
   }
   if (net->precision == GDFT_TF32X3) {
@@ -1110,10 +1117,10 @@ int gdft_neural_xc_hvp(const gdft_molecule *mol, const double *d_rdm1, const gdf
     StageTimer tm(GDFT_STAGE_MLP, st);
     if (tc)
       rc = mlp_hvp_tc(S, d_params, d_hparams, featp, feat, d_ehf, mol_w(mol), mol->n_grid, mol->n_grid_pad,
-                      net->clip, hws, d_value, coef, (int *)(ws + W.off_err), st);
+                      net->clip, hws, d_value, coef, mol_err(mol), st);
     else
       rc = mlp_hvp_f64(S, d_params, d_hparams, featp, feat, d_ehf, mol_w(mol), mol->n_grid, mol->n_grid_pad,
-                       net->clip, (double *)hws, d_value, coef, (int *)(ws + W.off_err), st);
+                       net->clip, (double *)hws, d_value, coef, mol_err(mol), st);
     if (rc) return rc;
   }
   if (d_hrdm1 == nullptr) return GDFT_OK;
@@ -1178,10 +1185,6 @@ int gdft_neural_batch_xc(int32_t n_mol, const gdft_molecule *mols, const double 
     return rc;
   int *batch_err = (int *)ws;
   char *wsm = ws + B.off_mol;  // the shared molecule region
-  // A molecule's error word sits where its own layout puts it in the shared
-  // region: cleared before the molecule's stage (a previous molecule's data may
-  // lie there) and folded into the batch's word after it.
-  auto mol_err = [&](const gdft_molecule *mol) { return (int *)(wsm + ws_layout(mol).off_err); };
   if (B.ragged) {
     // Every molecule's density in one persistent launch over all their tiles,
     // straight into the joint feature array.
@@ -1213,9 +1216,7 @@ int gdft_neural_batch_xc(int32_t n_mol, const gdft_molecule *mols, const double 
         return rc;
       continue;
     }
-    if ((rc = check_cuda(cudaMemsetAsync(mol_err(mol), 0, sizeof(int), st), "batch error word"))) return rc;
-    if ((rc = run_density(mol, h_rdm1[m], wsm, st))) return rc;
-    if ((rc = check_cuda(launch_err_fold(batch_err, mol_err(mol), st), "batch error fold"))) return rc;
+    if ((rc = run_density(mol, h_rdm1[m], wsm, st, true, batch_err))) return rc;
     if ((rc = check_cuda(cudaMemcpy2DAsync(feat + off, (size_t)npt * 8, wsm + W.off_feat, (size_t)np * 8,
                                            (size_t)np * 8, 2 * kFeat, cudaMemcpyDeviceToDevice, st),
                          "batch features")) ||
@@ -1238,13 +1239,11 @@ int gdft_neural_batch_xc(int32_t n_mol, const gdft_molecule *mols, const double 
     const gdft_molecule *mol = &mols[m];
     const WsLayout W = ws_layout(mol);
     const int64_t np = mol->n_grid_pad, off = B.seg[m];
-    if ((rc = check_cuda(cudaMemsetAsync(mol_err(mol), 0, sizeof(int), st), "batch error word")) ||
-        (rc = check_cuda(cudaMemcpy2DAsync(wsm + W.off_coef, (size_t)np * 8, coef + off, (size_t)npt * 8,
+    if ((rc = check_cuda(cudaMemcpy2DAsync(wsm + W.off_coef, (size_t)np * 8, coef + off, (size_t)npt * 8,
                                            (size_t)np * 8, 2 * kFeat, cudaMemcpyDeviceToDevice, st),
                          "batch coefficients")))
       return rc;
-    if ((rc = run_vxc(mol, (const double *)(wsm + W.off_coef), h_vxc[m], wsm, st))) return rc;
-    if ((rc = check_cuda(launch_err_fold(batch_err, mol_err(mol), st), "batch error fold"))) return rc;
+    if ((rc = run_vxc(mol, (const double *)(wsm + W.off_coef), h_vxc[m], wsm, st, true, batch_err))) return rc;
   }
   return GDFT_OK;
 }
@@ -1282,8 +1281,7 @@ int gdft_device_status(const gdft_molecule *mol, void *d_ws, size_t ws_bytes, in
     set_error("gdft_device_status: null output");
     return GDFT_ERR_INVALID;
   }
-  const WsLayout W = ws_layout(mol);
-  int *err = (int *)((char *)d_ws + W.off_err);
+  int *err = mol_err(mol);
   int h = 0;
   cudaStream_t st = (cudaStream_t)stream;
   if ((rc = check_cuda(cudaMemcpyAsync(&h, err, sizeof(int), cudaMemcpyDeviceToHost, st), "status read"))) return rc;
@@ -1305,8 +1303,7 @@ int gdft_selftest_wait_expiry(const gdft_molecule *mol, void *d_ws, size_t ws_by
     set_error("gdft_selftest_wait_expiry: limit %d outside 1..65536 polls", limit);
     return GDFT_ERR_INVALID;
   }
-  int *err = (int *)((char *)d_ws + ws_layout(mol).off_err);
-  return check_cuda(launch_wait_expiry_probe(err, (uint32_t)limit, GDFT_WAIT_EXPIRY_PROBE, (cudaStream_t)stream),
+  return check_cuda(launch_wait_expiry_probe(mol_err(mol), (uint32_t)limit, GDFT_WAIT_EXPIRY_PROBE, (cudaStream_t)stream),
                     "wait expiry probe");
 }
 
@@ -1487,7 +1484,7 @@ static int chunk_pass(const gdft_molecule *m, char *ws, const ChunkWs &C, char *
   const WsLayout W = ws_layout(m);
   int rc;
   // A shorter (last) chunk's layout puts its error word where the full chunks kept other data.
-  if ((rc = check_cuda(cudaMemsetAsync(ws + W.off_err, 0, sizeof(int), st), "chunk status clear"))) return rc;
+  if ((rc = check_cuda(cudaMemsetAsync(mol_err(m), 0, sizeof(int), st), "chunk status clear"))) return rc;
   const bool kin = net != nullptr || xc_reads_kinetic(*fn);
   if ((rc = run_density(m, rdm1, ws, st, kin))) return rc;
   const double *ehf_c = nullptr;
@@ -1507,10 +1504,10 @@ static int chunk_pass(const gdft_molecule *m, char *ws, const ChunkWs &C, char *
     StageTimer tm(GDFT_STAGE_MLP, st);
     if (net->precision == GDFT_TF32X3)
       rc = mlp_run_tc(net_shape(net), params, dp_c, feat, ehf_c, mol_w(m), m->n_grid, m->n_grid_pad, net->clip,
-                      ws + W.bytes, e_c, coef, (int *)(ws + W.off_err), st);
+                      ws + W.bytes, e_c, coef, mol_err(m), st);
     else
       rc = mlp_run_f64(net_shape(net), params, dp_c, feat, ehf_c, mol_w(m), m->n_grid, m->n_grid_pad, net->clip,
-                       (double *)(ws + W.bytes), e_c, coef, (int *)(ws + W.off_err), st);
+                       (double *)(ws + W.bytes), e_c, coef, mol_err(m), st);
     if (rc) return rc;
   } else {
     double *epart = (double *)(ws + W.off_epart);
@@ -1538,7 +1535,7 @@ static int chunk_pass(const gdft_molecule *m, char *ws, const ChunkWs &C, char *
     if ((rc = check_cuda(launch_feat_add(v_c, vxc, (size_t)2 * m->n_ao * m->n_ao, first, st), "chunk V")))
       return rc;
   }
-  return check_cuda(launch_err_fold((int *)base, (int *)(ws + W.off_err), st), "chunk status");
+  return check_cuda(launch_err_fold((int *)base, mol_err(m), st), "chunk status");
 }
 
 static int run_chunked(const char *who, const gdft_basis *shells, const double *rows, int32_t n_ao,

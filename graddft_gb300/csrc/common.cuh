@@ -63,15 +63,15 @@ struct MolLayout {
   int64_t np;   // padded grid points
   int ld;       // AO leading dimension of the FP64 planes
   int ldk;      // AO extent of the TF32x3 tables (multiple of 128)
-  size_t off_tab, off_w, off_pm, off_av, off_af, bytes;
+  size_t off_tab, off_w, off_pm, off_av, off_af, off_err, bytes;  // off_err: the error word of expired waits
   size_t plane_elems() const { return (size_t)np * ld; }
 };
 
 MolLayout mol_layout(int64_t n_grid, int n_ao, int precision);
 
-// Layout of the per-call workspace.
+// Layout of the per-call workspace.  Nothing in it outlives a call.
 struct WsLayout {
-  size_t off_feat, off_coef, off_epart, off_vpart, off_dpk, off_q, off_fx, off_err, bytes;
+  size_t off_feat, off_coef, off_epart, off_vpart, off_dpk, off_q, off_fx, bytes;
   int n_eblocks;   // blocks of the point kernel (energy partial sums)
   int n_vsplit;    // split-K factor of the V contraction
 };

@@ -63,11 +63,29 @@ class Resident:
                                      _ptr(self.buffer), nbytes.value))
         wbytes = ctypes.c_size_t()
         check(lib.gdft_workspace_bytes(ctypes.byref(self.desc), ctypes.byref(wbytes)))
-        self.ws = torch.zeros(wbytes.value, dtype=torch.uint8, device=self.device)  # error word starts at 0
+        self._ws_bytes = wbytes.value
+        if precision != "fp64":
+            self.ws = torch.zeros(wbytes.value, dtype=torch.uint8, device=self.device)
+
+    # The FP64 form's workspace holds the digits of a slab of the grid, up to a GB whatever the size of the
+    # tables, and nothing between calls: each call takes it from PyTorch's caching allocator, on the stream
+    # that it runs on, and gives it back, so that a set of molecules holds its tables and one workspace.  In
+    # a CUDA graph (``torch.cuda.graph``) it belongs to the graph's pool.  The mixed form keeps its own.
+    @property
+    def ws(self) -> torch.Tensor:
+        """The workspace for one call; hold it until the call has been made."""
+        own = self.__dict__.get("_own_ws")
+        return own if own is not None else torch.empty(self._ws_bytes, dtype=torch.uint8, device=self.device)
+
+    @ws.setter
+    def ws(self, t: torch.Tensor) -> None:
+        self.__dict__["_own_ws"] = t
 
     @property
     def nbytes(self) -> int:
-        return self.buffer.numel() + self.ws.numel()
+        """Device memory held between calls."""
+        own = self.__dict__.get("_own_ws")
+        return self.buffer.numel() + (0 if own is None else own.numel())
 
     @classmethod
     def from_tables(cls, ao, grad_ao, grad2_ao, weights, precision="fp64", device=None) -> "Resident":
@@ -139,8 +157,9 @@ class Resident:
             "lapl": torch.empty((n, 2), dtype=F64, device=self.device) if "lapl" in want else None,
             "tau": torch.empty((n, 2), dtype=F64, device=self.device) if "tau" in want else None,
         }
+        ws = self.ws
         check(_lib.load().gdft_density(ctypes.byref(self.desc), _ptr(rdm1), _ptr(out["rho"]), _ptr(out["grad_rho"]),
-                                       _ptr(out["lapl"]), _ptr(out["tau"]), _ptr(self.ws), self.ws.numel(),
+                                       _ptr(out["lapl"]), _ptr(out["tau"]), _ptr(ws), ws.numel(),
                                        _stream(self.device)))
         return out
 
@@ -157,9 +176,10 @@ class Resident:
         if want_vxc:
             vxc = vxc_out if vxc_out is not None else torch.empty((2, self.n_ao, self.n_ao), dtype=F64,
                                                                    device=self.device)
+        ws = self.ws
         check(_lib.load().gdft_xc_energy_and_grads(ctypes.byref(self.desc), _ptr(rdm1), ctypes.byref(fn),
-                                                   _ptr(ehf_t), n_omega, _ptr(exc), _ptr(vxc), _ptr(self.ws),
-                                                   self.ws.numel(), _stream(self.device)))
+                                                   _ptr(ehf_t), n_omega, _ptr(exc), _ptr(vxc), _ptr(ws),
+                                                   ws.numel(), _stream(self.device)))
         return exc, vxc
 
     def xc_energy_grads_hf(self, rdm1, fn: GdftFunctional, ehf, want_vxc=True):
@@ -171,9 +191,10 @@ class Resident:
         exc = torch.empty((), dtype=F64, device=self.device)
         vxc = torch.empty((2, self.n_ao, self.n_ao), dtype=F64, device=self.device) if want_vxc else None
         ghf = torch.empty(self.n_grid, dtype=F64, device=self.device)
+        ws = self.ws
         check(_lib.load().gdft_xc_energy_grads_hf(ctypes.byref(self.desc), _ptr(rdm1), ctypes.byref(fn), _ptr(ehf_t),
-                                                  ehf_t.shape[0], _ptr(exc), _ptr(vxc), _ptr(ghf), _ptr(self.ws),
-                                                  self.ws.numel(), _stream(self.device)))
+                                                  ehf_t.shape[0], _ptr(exc), _ptr(vxc), _ptr(ghf), _ptr(ws),
+                                                  ws.numel(), _stream(self.device)))
         return exc, vxc, ghf
 
     def vxc_from_potentials(self, pot, vxc_out=None):
@@ -182,8 +203,9 @@ class Resident:
         if pot.shape != (2, 6, self.n_grid):
             raise ValueError(f"potentials must be (2, 6, {self.n_grid}), got {tuple(pot.shape)}")
         vxc = vxc_out if vxc_out is not None else torch.empty((2, self.n_ao, self.n_ao), dtype=F64, device=self.device)
-        check(_lib.load().gdft_vxc_from_potentials(ctypes.byref(self.desc), _ptr(pot), _ptr(vxc), _ptr(self.ws),
-                                                   self.ws.numel(), _stream(self.device)))
+        ws = self.ws
+        check(_lib.load().gdft_vxc_from_potentials(ctypes.byref(self.desc), _ptr(pot), _ptr(vxc), _ptr(ws),
+                                                   ws.numel(), _stream(self.device)))
         return vxc
 
     def neural_xc_energy_and_grads(self, rdm1, net: "Network", flat_params, ehf, want_vxc=True,
@@ -250,7 +272,7 @@ class Resident:
                                              ws.numel(), _stream(self.device)))
         return val, hd, hp
 
-    # Workspaces of the network passes, one per network shape and form: callers that mix networks (the
+    # Workspaces of the mixed form's network passes, one per network shape: callers that mix networks (the
     # DM21 inputs of the default network beside a functional's own, say) would otherwise reallocate and
     # zero a workspace of gigabytes on every switch.  The cache drops its least recently used entry.
     _WS_KEEP = 4
@@ -263,9 +285,17 @@ class Resident:
             check(size_fn(ctypes.byref(self.desc), ctypes.byref(net.desc), ctypes.byref(nbytes)))
             if len(cache) >= self._WS_KEEP:
                 self._retire_ws(cache.pop(next(iter(cache))))
-            ws = torch.zeros(nbytes.value, dtype=torch.uint8, device=self.device)  # error word 0
+            ws = torch.zeros(nbytes.value, dtype=torch.uint8, device=self.device)
         cache[net.key] = ws
         return ws
+
+    def _net_ws(self, name: str, net: "Network", size_fn) -> torch.Tensor:
+        """The workspace of a network pass: where either form is FP64 one for the call, as ``ws``."""
+        if self.precision != "fp64" and net.precision != "fp64":
+            return self._cached_ws(name, net, size_fn)
+        nbytes = ctypes.c_size_t()
+        check(size_fn(ctypes.byref(self.desc), ctypes.byref(net.desc), ctypes.byref(nbytes)))
+        return torch.empty(nbytes.value, dtype=torch.uint8, device=self.device)
 
     def _retire_ws(self, ws: torch.Tensor) -> None:
         """Read a dropped workspace's error word before it goes: an expired bounded wait recorded there
@@ -279,16 +309,17 @@ class Resident:
             check(rc)
 
     def _hvp_ws(self, net: "Network") -> torch.Tensor:
-        return self._cached_ws("_hws", net, _lib.load().gdft_neural_hvp_workspace_bytes)
+        return self._net_ws("_hws", net, _lib.load().gdft_neural_hvp_workspace_bytes)
 
     def _neural_ws(self, net: "Network") -> torch.Tensor:
-        return self._cached_ws("_nws", net, _lib.load().gdft_neural_workspace_bytes)
+        return self._net_ws("_nws", net, _lib.load().gdft_neural_workspace_bytes)
 
     def status(self) -> int:
         """Synchronise and raise if a kernel recorded an expired bounded wait since the last query
         (including one recorded in a network workspace the cache has since dropped)."""
         st = ctypes.c_int32()
-        check(_lib.load().gdft_device_status(ctypes.byref(self.desc), _ptr(self.ws), self.ws.numel(),
+        ws = self.ws
+        check(_lib.load().gdft_device_status(ctypes.byref(self.desc), _ptr(ws), ws.numel(),
                                              ctypes.byref(st), _stream(self.device)))
         for name in ("_nws", "_hws"):
             for ws in self.__dict__.get(name, {}).values():
@@ -348,13 +379,14 @@ class ChunkedResident:
                 raise ValueError(f"basis rows must be (n_ao, 8), got {tuple(self._rows.shape)}")
             self.n_ao = int(self._rows.shape[0])
         self._ws = workspace_pool if workspace_pool is not None else {}
+        self._word = torch.zeros(1, dtype=torch.int32, device=self.device)  # of workspaces that were given back
 
     def _basis_args(self):
         return (None if self._desc is None else ctypes.byref(self._desc)), _ptr(self._rows)
 
     def use_workspace_pool(self, pool: dict) -> None:
-        """Take workspaces from ``pool`` from now on (molecules that share a pool must run one after another
-        on one stream; ``batch.ChunkedBatch`` gives each of its streams its own)."""
+        """Take the mixed form's workspaces from ``pool`` from now on (molecules that share a pool must run one
+        after another on one stream; ``batch.ChunkedBatch`` gives each of its streams its own)."""
         self._ws = pool
 
     def workspace_bytes(self, chunk: int, net: Optional["Network"] = None) -> int:
@@ -364,9 +396,23 @@ class ChunkedResident:
                                                        ctypes.byref(nbytes)))
         return nbytes.value
 
+    def _per_call(self, net: Optional["Network"]) -> bool:
+        return self.precision == "fp64" or (net is not None and net.precision == "fp64")
+
+    def _give_back(self, ws: torch.Tensor, net: Optional["Network"]) -> None:
+        """After a call: the error word of a workspace that is not kept goes to this molecule's."""
+        if self._per_call(net):
+            torch.maximum(self._word, ws[:4].view(torch.int32), out=self._word)
+
     def workspace(self, net: Optional["Network"] = None) -> torch.Tensor:
+        """The workspace for one call.  Where either form is FP64 it is taken for the call, as
+        ``Resident.ws``, and its error word is collected by ``_give_back``; the mixed form's come from the pool."""
         key = None if net is None else net.key
         need = self.workspace_bytes(self.chunk, net)
+        if self._per_call(net):
+            ws = torch.empty(need, dtype=torch.uint8, device=self.device)
+            ws[:4].zero_()
+            return ws
         ws = self._ws.get(key)
         if ws is None or ws.numel() < need:
             if ws is not None:  # report what the smaller workspace recorded before it goes
@@ -422,6 +468,7 @@ class ChunkedResident:
             shells, rows, self.n_ao, _ptr(self.coords), _ptr(self.weights), self.n_grid, self.chunk,
             PRECISIONS[self.precision], _ptr(rdm1), ctypes.byref(fn), _ptr(ehf_t), n_omega, _ptr(exc), _ptr(vxc),
             _ptr(ws), ws.numel(), _stream(self.device)))
+        self._give_back(ws, None)
         return exc, vxc
 
     def neural_xc_energy_and_grads(self, rdm1, net: "Network", flat_params, ehf, want_vxc=True,
@@ -446,6 +493,7 @@ class ChunkedResident:
             shells, rows, self.n_ao, _ptr(self.coords), _ptr(self.weights), self.n_grid, self.chunk,
             PRECISIONS[self.precision], _ptr(rdm1), ctypes.byref(net.desc), _ptr(flat), _ptr(ehf_t.contiguous()),
             _ptr(exc), _ptr(vxc), _ptr(dp), _ptr(ws), ws.numel(), _stream(self.device)))
+        self._give_back(ws, net)
         return exc, vxc, dp
 
     def status(self) -> int:
@@ -453,6 +501,10 @@ class ChunkedResident:
         st = ctypes.c_int32()
         for ws in self._ws.values():
             check(_lib.load().gdft_chunked_status(_ptr(ws), ws.numel(), ctypes.byref(st), _stream(self.device)))
+        code = int(self._word)
+        if code:
+            self._word.zero_()
+            raise _lib.GdftError(f"a device-side wait expired (code {code}); results of the last calls are invalid")
         return st.value
 
     def __getattr__(self, name):

@@ -74,9 +74,10 @@ def molecule_energy_densities(molecule, cols: Sequence[int], clip_cte: float = C
     out = torch.empty((r.n_grid, len(cols)), dtype=torch.float64, device=r.device)
     import ctypes
     n_omega = 0 if ehf_t is None else ehf_t.shape[0]
+    ws = r.ws
     _lib.check(_lib.load().gdft_energy_densities(ctypes.byref(r.desc), engine._ptr(molecule._rdm1()),
                                                  ctypes.byref(fn), engine._ptr(ehf_t), n_omega, engine._ptr(out),
-                                                 engine._ptr(r.ws), r.ws.numel(), engine._stream(r.device)))
+                                                 engine._ptr(ws), ws.numel(), engine._stream(r.device)))
     return out
 
 

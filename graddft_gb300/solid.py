@@ -83,7 +83,14 @@ class KPointResident:
         self.descs = (_lib.GdftMolecule * n_kpt)(*[m.desc for m in self.mols])
         nbytes = ctypes.c_size_t()
         _lib.check(_lib.load().gdft_kpoint_workspace_bytes(self.descs, n_kpt, ctypes.byref(nbytes)))
-        self.ws = torch.zeros(nbytes.value, dtype=torch.uint8, device=dev)
+        self._ws_bytes = nbytes.value
+        self._own_ws = torch.zeros(nbytes.value, dtype=torch.uint8, device=dev) if precision != "fp64" else None
+
+    @property
+    def ws(self) -> torch.Tensor:
+        """The workspace for one call: the FP64 form's is taken and given back for each (``engine.Resident.ws``)."""
+        return self._own_ws if self._own_ws is not None else torch.empty(self._ws_bytes, dtype=torch.uint8,
+                                                                         device=self.device)
 
     def _rdm1(self, rdm1) -> torch.Tensor:
         d = _as_c128(rdm1, self.device)
@@ -100,10 +107,10 @@ class KPointResident:
             "lapl": torch.empty((n, 2), dtype=F64, device=self.device) if "lapl" in want else None,
             "tau": torch.empty((n, 2), dtype=F64, device=self.device) if "tau" in want else None,
         }
-        P = engine._ptr
+        P, ws = engine._ptr, self.ws
         _lib.check(_lib.load().gdft_kpoint_density(self.descs, self.n_kpt, P(torch.view_as_real(d)), self.kw_host,
                                                    P(out["rho"]), P(out["grad_rho"]), P(out["lapl"]), P(out["tau"]),
-                                                   P(self.ws), self.ws.numel(), engine._stream(self.device)))
+                                                   P(ws), ws.numel(), engine._stream(self.device)))
         return out
 
     def xc_energy_and_grads(self, rdm1, fn, ehf=None, want_vxc=True):
@@ -113,10 +120,10 @@ class KPointResident:
         d = self._rdm1(rdm1)
         exc = torch.empty((), dtype=F64, device=self.device)
         vxc = torch.empty_like(d) if want_vxc else None
-        P = engine._ptr
+        P, ws = engine._ptr, self.ws
         _lib.check(_lib.load().gdft_kpoint_xc_energy_and_grads(
             self.descs, self.n_kpt, P(torch.view_as_real(d)), self.kw_host, ctypes.byref(fn), P(exc),
-            None if vxc is None else P(torch.view_as_real(vxc)), P(self.ws), self.ws.numel(),
+            None if vxc is None else P(torch.view_as_real(vxc)), P(ws), ws.numel(),
             engine._stream(self.device)))
         return exc, vxc
 

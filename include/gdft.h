@@ -14,7 +14,10 @@
  *    host except where a function says so.
  *  - The library allocates no device memory: molecules live in a
  *    caller-provided buffer (gdft_molecule_bytes) and every call takes a
- *    caller-provided workspace (gdft_workspace_bytes).
+ *    caller-provided workspace (gdft_workspace_bytes).  A molecule's workspace
+ *    may hold anything before a call and holds nothing that a later one needs,
+ *    so one can serve molecules that are used one after another on a stream
+ *    (batch, chunked and exact-exchange workspaces start with an error word).
  *  - Return value: GDFT_OK or an error code; gdft_last_error() gives the
  *    message of the calling thread's last failure.
  */
@@ -468,9 +471,10 @@ int gdft_fock(int32_t n_ao, const double *d_h1e, const double *d_vj, const doubl
 int gdft_coulomb(int32_t n_ao, const double *d_eri, const double *d_rdm1, const double *d_h1e,
                  double nuclear_repulsion, double *d_vj, double *d_enonxc, void *stream);
 
-/* Device-side status of the calls made with this workspace since the last
- * query: kernels never trap; a bounded wait that expired records a nonzero
- * code in the workspace.  Synchronises `stream`, returns GDFT_ERR_DEVICE (and
+/* Device-side status of the calls made on this molecule since it was loaded or
+ * last queried: kernels never trap; a bounded wait that expired records a
+ * nonzero code in the molecule's buffer (k-point calls: the first one's).
+ * Synchronises `stream`, returns GDFT_ERR_DEVICE (and
  * the code in *status) if set, and clears it.  No counterpart in the
  * reference (its errors are Python exceptions). */
 int gdft_device_status(const gdft_molecule *mol, void *d_ws, size_t ws_bytes, int32_t *status, void *stream);
@@ -513,7 +517,7 @@ int gdft_chunked_status(void *d_ws, size_t ws_bytes, int32_t *status, void *stre
 /* Test of the failure path above: one kernel waits on an mbarrier that
  * nothing arrives on, with `limit` (1..65536) polls instead of the pipeline
  * kernels' limit, so the wait runs out; it records GDFT_WAIT_EXPIRY_PROBE in
- * the workspace's error word and returns (no trap; nothing else is in flight,
+ * the molecule's error word and returns (no trap; nothing else is in flight,
  * the context stays usable).  The next gdft_device_status reports it.  No
  * counterpart in the reference. */
 #define GDFT_WAIT_EXPIRY_PROBE 99

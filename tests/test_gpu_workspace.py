@@ -132,3 +132,64 @@ def test_another_molecules_nan_stays_its_own(E):
     for (wl, d), (e0, v0) in list(zip(made, alone))[1:]:
         e, v = chunked(wl, pool).xc_energy_and_grads(d, fn)
         assert torch.equal(e, e0) and torch.equal(v, v0)
+
+
+@pytest.mark.parametrize("kind", ["resident", "chunked", "network"])
+def test_molecules_hold_no_workspace(E, kind):
+    """After its calls an FP64 molecule holds its tables (chunked: its grid), not a workspace of its own."""
+    from graddft_gb300 import _lib
+
+    fn = E.make_functional([_lib.COL_LSDA, _lib.COL_B88, _lib.COL_LYP], [1.0])
+    n_ao, n_grid = 24, 3600
+    wl, (ao, g1, g2) = _workload(n_ao, n_grid)
+    d = torch.as_tensor(wl.rdm1, device="cuda")
+    net = E.Network(n_layers=2, width=64)
+    flat = torch.zeros(net.n_params, dtype=torch.float64, device="cuda")
+    ehf = torch.as_tensor(synthetic.make_ehf(n_grid, 3, None, 2), device="cuda")
+    torch.cuda.synchronize()
+    before, made, held = torch.cuda.memory_allocated(), [], 0
+    for _ in range(4):
+        if kind == "chunked":
+            r = E.ChunkedResident(wl.basis.packed(), wl.coords, wl.weights, "fp64", 2048)
+            held += r.coords.numel() * 8 + r.weights.numel() * 8 + n_ao * 64
+        else:
+            r = E.Resident.from_tables(ao, g1, g2, wl.weights)
+            held += r.buffer.numel()
+            r.density(d)
+        r.xc_energy_and_grads(d, fn)
+        if kind == "network":
+            r.neural_xc_energy_and_grads(d, net, flat, ehf, want_dparams=True)
+            r.neural_xc_hvp(d, net, flat, ehf, d)
+        assert r.status() == 0
+        made.append(r)
+    assert torch.cuda.memory_allocated() - before <= held + len(made) * 4096
+    assert kind == "chunked" or sum(r.nbytes for r in made) == held
+
+
+def test_captured_calls_own_their_workspace(E):
+    """Calls captured in a CUDA graph, replayed with new density matrices between other molecules' calls."""
+    from graddft_gb300 import _lib
+
+    fn = E.make_functional([_lib.COL_LSDA, _lib.COL_B88, _lib.COL_LYP], [1.0])
+    made = []
+    for n_ao, n_grid in ((43, 700), (130, 900), (24, 300)):
+        wl, (ao, g1, g2) = _workload(n_ao, n_grid)
+        made.append((E.Resident.from_tables(ao, g1, g2, wl.weights), torch.as_tensor(wl.rdm1, device="cuda")))
+    ref = [r.xc_energy_and_grads(d * 0.5, fn) for r, d in made]
+    graphs = []
+    for r, d in made:
+        d = d.clone()
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            out = r.xc_energy_and_grads(d, fn)
+        graphs.append((g, d, out))
+    for g, d, _ in graphs:
+        d.mul_(0.5)
+    for i, (g, _, (e, v)) in enumerate(graphs):
+        other, d = made[(i + 1) % len(made)]
+        other.density(d)
+        g.replay()
+        other.density(torch.full_like(d, float("nan")))
+        assert torch.equal(e, ref[i][0]) and torch.equal(v, ref[i][1])
+    assert all(r.status() == 0 for r, _ in made)
