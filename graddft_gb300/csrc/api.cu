@@ -1040,7 +1040,7 @@ int gdft_network_apply_workspace_bytes(const gdft_network *net, int64_t n_rows, 
     set_error("gdft_network_apply_workspace_bytes: invalid arguments");
     return GDFT_ERR_INVALID;
   }
-  *bytes = align256(mlp_layout(net_shape(net), n_rows).doubles * sizeof(double));
+  *bytes = 256 + align256(mlp_layout(net_shape(net), n_rows).doubles * sizeof(double));
   return GDFT_OK;
 }
 
@@ -1052,14 +1052,15 @@ int gdft_network_apply(const gdft_network *net, const double *d_params, int64_t 
     set_error("gdft_network_apply: invalid arguments");
     return GDFT_ERR_INVALID;
   }
-  const size_t need = align256(mlp_layout(net_shape(net), n_rows).doubles * sizeof(double));
+  const size_t need = 256 + align256(mlp_layout(net_shape(net), n_rows).doubles * sizeof(double));  // error word first
   if (d_ws == nullptr || ws_bytes < need) {
     set_error("workspace of %zu bytes is smaller than the %zu bytes required", ws_bytes, need);
     return GDFT_ERR_WORKSPACE;
   }
   cudaStream_t st = (cudaStream_t)stream;
   StageTimer tm(GDFT_STAGE_MLP, st);
-  return mlp_apply_f64(net_shape(net), d_params, d_x, n_rows, (double *)d_ws, d_c, st);
+  if ((rc = check_cuda(cudaMemsetAsync(d_ws, 0, sizeof(int), st), "error word"))) return rc;
+  return mlp_apply_f64(net_shape(net), d_params, d_x, n_rows, (double *)((char *)d_ws + 256), d_c, (int *)d_ws, st);
 }
 
 int gdft_neural_hvp_workspace_bytes(const gdft_molecule *mol, const gdft_network *net, size_t *bytes) {

@@ -134,8 +134,9 @@ cudaError_t launch_gemm(const GemmArgs &a, cudaStream_t st);
 cudaError_t launch_rows(const double *src, int64_t plane_elems, int planes, int64_t rows, int64_t ld, int k_valid,
                         int chunks, const int *oct, unsigned char *out, int *exps, int *bad, cudaStream_t st);
 
-// FP64 GEMMs of fx_mat.cu, on row-major operands.  ws: scratch of gemm_rows_bytes / gemm_cols_bytes; err: a device
-// error word or null (an expired wait leaves NaN in the output either way); part: partials of the plain kernel that takes over where an operand is not finite (nsplit x M x N doubles).
+// FP64 GEMMs of fx_mat.cu, on row-major operands.  ws: scratch of gemm_rows_bytes / gemm_cols_bytes; err: the device
+// word that an expired wait is recorded in (it also leaves NaN in the output); part: partials of the plain kernel that
+// takes over where an operand is not finite (nsplit x M x N doubles).
 size_t gemm_rows_bytes(int64_t M, int N, int K);
 size_t gemm_cols_bytes(int M, int N, int64_t K);
 // C[m][n] = sum_k A[m][k] B[k][n] (B stored N x K when b_rows) + add[m][n] (laid out like C; null: nothing).  oct, or

@@ -149,7 +149,7 @@ RowsWs rows_ws(int64_t M, int N, int K) {
   w.slab = (int64_t)kSlabBytes / ((int64_t)kSetBytes * ch) * kTile;
   w.slab = w.slab < kTile ? kTile : w.slab;
   if (w.slab > tiles_of(M) * kTile) w.slab = tiles_of(M) * kTile;
-  size_t off = 256;  // the bad word and an error word
+  size_t off = 256;  // the bad word
   w.off_b = off;
   off = align256(off + (size_t)tiles_of(N) * ch * kSetBytes);
   w.off_eb = off;
@@ -214,7 +214,7 @@ cudaError_t gemm_rows(int64_t M, int N, int K, const double *A, int64_t lda, con
   cudaError_t e;
   for (int64_t m0 = 0; m0 < M; m0 += w.slab) {
     const int64_t rows = M - m0 < w.slab ? M - m0 : w.slab;
-    if ((e = cudaMemsetAsync(bad, 0, 2 * sizeof(int), st)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(bad, 0, sizeof(int), st)) != cudaSuccess) return e;
     if (b_rows)
       e = launch_rows(B, 0, 1, N, ldb, K, ch, nullptr, sw, ew, bad, st);
     else {
@@ -241,7 +241,7 @@ cudaError_t gemm_rows(int64_t M, int N, int K, const double *A, int64_t lda, con
     g.n_valid = rows;
     g.add = add != nullptr ? add + m0 * ldc : nullptr;
     g.bad = bad;
-    g.err = err != nullptr ? err : bad + 1;
+    g.err = err;
     if ((e = launch_gemm(g, st)) != cudaSuccess) return e;
     e = b_rows ? plain_gemm<kNT>((int)rows, N, K, A + m0 * lda, (int)lda, B, (int)ldb, C + m0 * ldc, (int)ldc,
                                  g.add, bad, st)
@@ -261,7 +261,7 @@ cudaError_t gemm_cols(int M, int N, int64_t K, const double *A, int64_t lda, con
   int *bad = (int *)ws, *ea = (int *)(ws + w.off_exp), *eb = ea + tm * kTile;
   uint32_t *ma = (uint32_t *)(ws + w.off_mx), *mb = ma + tm * kTile;
   double *fpart = (double *)(ws + w.off_part);
-  cudaError_t e = cudaMemsetAsync(bad, 0, 2 * sizeof(int), st);
+  cudaError_t e = cudaMemsetAsync(bad, 0, sizeof(int), st);
   if (e != cudaSuccess) return e;
   for (int64_t k0 = 0; k0 < K; k0 += w.slab) {
     const int64_t rows = K - k0 < w.slab ? K - k0 : w.slab;
@@ -301,7 +301,7 @@ cudaError_t gemm_cols(int M, int N, int64_t K, const double *A, int64_t lda, con
     g.n_valid = M;
     g.add = k0 > 0 ? fpart : nullptr;
     g.bad = bad;
-    g.err = err != nullptr ? err : bad + 1;
+    g.err = err;
     if ((e = launch_gemm(g, st)) != cudaSuccess) return e;
   }
   const size_t total = (size_t)M * N;

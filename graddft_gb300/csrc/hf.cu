@@ -242,9 +242,11 @@ int hf_splits(int64_t n_grid) {
   return (int)s;
 }
 
+// FP64 form's workspace: the error word, X or B at kHfX, the split partials of F, then the GEMMs' octaves and scratch.
+constexpr size_t kHfX = 256;
+size_t hf_part_off(int64_t n_grid, int n_ao) { return kHfX + align256((size_t)2 * n_grid * n_ao * sizeof(double)); }
 size_t hf_gemm_off(int64_t n_grid, int n_ao) {
-  return align256((size_t)2 * n_grid * n_ao * sizeof(double)) +
-         align256((size_t)hf_splits(n_grid) * n_ao * n_ao * sizeof(double));
+  return hf_part_off(n_grid, n_ao) + align256((size_t)hf_splits(n_grid) * n_ao * n_ao * sizeof(double));
 }
 // The octaves of an FP64 call (the workspace itself may be aligned to 8 bytes only); `len` of them, then the scratch.
 int *hf_octaves(void *ws, int64_t n_grid, int n_ao) {
@@ -376,7 +378,6 @@ int gdft_hf_workspace_bytes_form(int64_t n_grid, int32_t n_ao, int32_t n_omega, 
     *bytes = hf_tc_layout(n_grid, n_ao).bytes;
     return GDFT_OK;
   }
-  // X or B: [2][n_grid][n_ao]; split partials of F: [nsplit][n_ao][n_ao]; the GEMMs' octaves and scratch, aligned.
   const size_t rows = align256((size_t)fx::octaves_len(n_ao) * sizeof(int)) + fx::gemm_rows_bytes(n_grid, n_ao, n_ao);
   const size_t cols = align256((size_t)n_grid * sizeof(int)) + fx::gemm_cols_bytes(n_ao, n_ao, n_grid);
   *bytes = hf_gemm_off(n_grid, n_ao) + 256 + (rows > cols ? rows : cols);
@@ -399,13 +400,15 @@ int gdft_hf_energy_density_form(const double *d_ao, const double *d_rdm1, const 
   cudaStream_t st = (cudaStream_t)stream;
   if (form == GDFT_TF32X3) return hf_energy_density_tc(d_ao, d_rdm1, d_chi, n_grid, n_ao, n_omega, d_ehf,
                                                        (char *)d_ws, st);
-  double *X = (double *)d_ws;
+  double *X = (double *)((char *)d_ws + kHfX);
+  int *err = (int *)d_ws;
+  if ((rc = check_cuda(cudaMemsetAsync(err, 0, sizeof(int), st), "hf err clear"))) return rc;
   int *oct = hf_octaves(d_ws, n_grid, n_ao);
   if ((rc = check_cuda(fx::launch_octaves(d_rdm1, n_ao, oct, nullptr, st), "hf octaves"))) return rc;
   for (int s = 0; s < 2; ++s)
     if ((rc = check_cuda(fx::gemm_rows(n_grid, n_ao, n_ao, d_ao, n_ao, d_rdm1 + (size_t)s * n_ao * n_ao, n_ao, false,
                                        oct, X + (size_t)s * n_grid * n_ao, n_ao, nullptr,
-                                       hf_scratch(oct, fx::octaves_len(n_ao)), nullptr, st),
+                                       hf_scratch(oct, fx::octaves_len(n_ao)), err, st),
                          "hf ao.D")))
       return rc;
   const int64_t threads = 2 * n_grid * 32;
@@ -430,8 +433,10 @@ int gdft_hf_fock_form(const double *d_ao, const double *d_chi, const double *d_g
   }
   cudaStream_t st = (cudaStream_t)stream;
   if (form == GDFT_TF32X3) return hf_fock_tc(d_ao, d_chi, d_g, n_grid, n_ao, n_omega, d_fock_hf, (char *)d_ws, st);
-  double *B = (double *)d_ws;
-  double *part = (double *)((char *)d_ws + align256((size_t)2 * n_grid * n_ao * sizeof(double)));
+  double *B = (double *)((char *)d_ws + kHfX);
+  double *part = (double *)((char *)d_ws + hf_part_off(n_grid, n_ao));
+  int *err = (int *)d_ws;
+  if ((rc = check_cuda(cudaMemsetAsync(err, 0, sizeof(int), st), "hf err clear"))) return rc;
   const size_t total = (size_t)2 * n_grid * n_ao;
   launch_next(hf_bmat_kernel, (unsigned)((total + 255) / 256), 256, 0, st, d_chi, d_g, n_grid, n_ao, n_omega, B);
   int *oct = hf_octaves(d_ws, n_grid, n_ao);
@@ -440,7 +445,7 @@ int gdft_hf_fock_form(const double *d_ao, const double *d_chi, const double *d_g
   const int nsplit = hf_splits(n_grid);
   for (int s = 0; s < 2; ++s)
     if ((rc = check_cuda(fx::gemm_cols(n_ao, n_ao, n_grid, d_ao, n_ao, B + (size_t)s * n_grid * n_ao, n_ao,
-                                       oct, d_fock_hf + (size_t)s * n_ao * n_ao, hf_scratch(oct, n_grid), nullptr, nsplit,
+                                       oct, d_fock_hf + (size_t)s * n_ao * n_ao, hf_scratch(oct, n_grid), err, nsplit,
                                        part, st),
                          "hf ao^T B")))
       return rc;

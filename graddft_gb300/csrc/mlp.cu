@@ -402,12 +402,12 @@ int mlp_inputs_f64(const MlpShape &S, const double *feat, const double *ehf, int
 }
 
 int mlp_apply_f64(const MlpShape &S, const double *params, const double *x, int64_t rows, double *ws, double *c,
-                  cudaStream_t st) {
+                  int *err, cudaStream_t st) {
   const MlpLayout L = mlp_layout(S, rows);
   launch_next(squash_kernel, (unsigned)((rows + 255) / 256), 256, 0, st, x, rows, S.n_in, S.squash_offset, ws + L.u);
   int rc = check_cuda(cudaGetLastError(), "mlp squash");
   if (rc) return rc;
-  if ((rc = net_forward(S, params, L, ws, rows, nullptr, st))) return rc;
+  if ((rc = net_forward(S, params, L, ws, rows, err, st))) return rc;
   const double *bout = params + layer_offset(S, S.n_layers) + (size_t)S.width * S.n_out;
   launch_next(head_coeff_kernel, (unsigned)((rows * S.n_out + 255) / 256), 256, 0, st, ws + L.y, bout, rows, S.n_out,
               S.sigmoid_scale, c);

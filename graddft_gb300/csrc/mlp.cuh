@@ -154,6 +154,6 @@ int mlp_inputs_f64(const MlpShape &S, const double *feat, const double *ehf, int
 
 // Coefficients c (rows x n_out) of the network on given inputs x (rows x n_in).
 int mlp_apply_f64(const MlpShape &S, const double *params, const double *x, int64_t rows, double *ws, double *c,
-                  cudaStream_t st);
+                  int *err, cudaStream_t st);
 
 }  // namespace gdft

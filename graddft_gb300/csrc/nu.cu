@@ -246,12 +246,14 @@ int make_plan(const gdft_basis *b, PairPlan &plan, const char *who) {
 }
 
 struct NuWs {
-  size_t off_boys, off_pairs, off_pp, off_nu, off_x, off_oct, off_fx, bytes;  // off_oct, off_fx: of the GEMM X = ao D
+  size_t off_err, off_boys, off_pairs, off_pp, off_nu, off_x, off_oct, off_fx, bytes;  // off_oct, off_fx: of the GEMM X = ao D
 };
 
 NuWs nu_ws(const PairPlan &plan, int n_ao, int64_t chunk, bool want_chi, int n_omega) {
   NuWs W;
   size_t off = 0;
+  W.off_err = off;  // expired waits of the GEMM X = ao D
+  off = al256(off + sizeof(int));
   W.off_boys = off;
   off = al256(off + kBoysLen * sizeof(double));
   W.off_pairs = off;
@@ -428,7 +430,8 @@ int gdft_chi(const gdft_basis *basis, const double *d_coords, const double *d_ao
   char *ws = (char *)d_ws;
   double *nu = (double *)(ws + W.off_nu);
   double *X = (double *)(ws + W.off_x);
-  int *oct = (int *)(ws + W.off_oct);
+  int *oct = (int *)(ws + W.off_oct), *err = (int *)(ws + W.off_err);
+  if ((rc = check_cuda(cudaMemsetAsync(err, 0, sizeof(int), st), who))) return rc;
   if ((rc = check_cuda(fx::launch_octaves(d_rdm1, n, oct, nullptr, st), who))) return rc;
   for (int w = 0; w < n_omega; ++w)
     if ((rc = setup_nu(B, plan, W, ws, w, h_omegas[w], w == 0, who, st))) return rc;
@@ -437,7 +440,7 @@ int gdft_chi(const gdft_basis *basis, const double *d_coords, const double *d_ao
     // X_s = ao[p0 : p0 + np_] D_s, shared by the omegas
     for (int s = 0; s < 2; ++s)
       if ((rc = check_cuda(fx::gemm_rows(np_, n, n, d_ao + p0 * n, n, d_rdm1 + (size_t)s * n * n, n, false,
-                                         oct, X + (size_t)s * pc * n, n, nullptr, (unsigned char *)(ws + W.off_fx), nullptr,
+                                         oct, X + (size_t)s * pc * n, n, nullptr, (unsigned char *)(ws + W.off_fx), err,
                                          st),
                            who)))
         return rc;
@@ -449,7 +452,14 @@ int gdft_chi(const gdft_basis *basis, const double *d_coords, const double *d_ao
       if ((rc = check_cuda(cudaGetLastError(), who))) return rc;
     }
   }
-  return check_cuda(cudaStreamSynchronize(st), who);
+  int h = 0;
+  if ((rc = check_cuda(cudaMemcpyAsync(&h, err, sizeof(int), cudaMemcpyDeviceToHost, st), who))) return rc;
+  if ((rc = check_cuda(cudaStreamSynchronize(st), who))) return rc;
+  if (h != 0) {
+    set_error("%s: a device-side wait expired (code %d); chi is invalid", who, h);
+    return GDFT_ERR_DEVICE;
+  }
+  return GDFT_OK;
 }
 
 }  // extern "C"

@@ -620,7 +620,8 @@ def _hf_ws(n_grid: int, n_ao: int, n_omega: int, form: int, device) -> torch.Ten
 
 
 def _hf_status(ws: torch.Tensor, form: int) -> None:
-    """The bounded-wait error word of a mixed-form exchange call (synchronises the stream)."""
+    """The bounded-wait error word of a mixed-form exchange call (synchronises the stream).  FP64 calls are not
+    waited for: there an expired wait shows as NaN in the result (and in the C entry's status)."""
     if form == _lib.GDFT_TF32X3:
         status = ctypes.c_int32()
         check(_lib.load().gdft_hf_device_status(_ptr(ws), ws.numel(), ctypes.byref(status), _stream(ws.device)))

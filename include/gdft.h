@@ -231,7 +231,8 @@ int gdft_nu_integrals(const gdft_basis *basis, const double *d_coords, int64_t n
                       void *d_ws, size_t ws_bytes, void *stream);
 
 /* d_ao: (n_grid, n_ao) phi on the grid; d_rdm1: (2, n_ao, n_ao); h_omegas: n_omega
- * host values >= 0; d_chi: (n_grid, n_omega, 2, n_ao). */
+ * host values >= 0; d_chi: (n_grid, n_omega, 2, n_ao).  Synchronises the stream;
+ * GDFT_ERR_DEVICE where a bounded device wait expired. */
 int gdft_chi(const gdft_basis *basis, const double *d_coords, const double *d_ao, const double *d_rdm1,
              int64_t n_grid, const double *h_omegas, int32_t n_omega, int64_t chunk, double *d_chi, void *d_ws,
              size_t ws_bytes, void *stream);
@@ -268,7 +269,9 @@ int gdft_xc_energy_grads_hf(const gdft_molecule *mol, const double *d_rdm1, cons
 /* Exact-exchange terms from a supplied chi tensor (grid, omega, spin,
  * orbitals), FP64 device arrays in the reference's layouts; ao is (grid,
  * orbitals) row-major, rdm1 (2, n, n).  Workspace of
- * gdft_hf_workspace_bytes bytes (8-byte aligned).
+ * gdft_hf_workspace_bytes bytes (8-byte aligned); gdft_hf_device_status on it
+ * tells whether a bounded device wait of the call expired, which also leaves
+ * NaN in the result.
  *   gdft_hf_energy_density: ehf (omega, 2, grid) =
  *       -1/2 einsum("rwsc,sac,ra->wsr", chi, rdm1, ao)   (molecule.py:507-541)
  *   gdft_hf_fock: fock_hf (2, n, n) =
@@ -299,7 +302,7 @@ int gdft_hf_energy_density_form(const double *d_ao, const double *d_rdm1, const 
 int gdft_hf_fock_form(const double *d_ao, const double *d_chi, const double *d_g, int64_t n_grid, int32_t n_ao,
                       int32_t n_omega, int32_t form, double *d_fock_hf, void *d_ws, size_t ws_bytes, void *stream);
 /* Reads (synchronising the stream) the device error word of a workspace last
- * used by a GDFT_TF32X3 exact-exchange call: GDFT_ERR_DEVICE with *status the
+ * used by an exact-exchange call of either form: GDFT_ERR_DEVICE with *status the
  * code when a bounded wait expired. */
 int gdft_hf_device_status(void *d_ws, size_t ws_bytes, int32_t *status, void *stream);
 
@@ -413,7 +416,9 @@ int gdft_neural_inputs(const gdft_molecule *mol, const double *d_rdm1, const gdf
 int gdft_network_apply_workspace_bytes(const gdft_network *net, int64_t n_rows, size_t *bytes);
 
 /* The network alone on given inputs (NeuralFunctional.apply, the coefficients
- * of functional.py:797-822 + :407-419): d_x (n_rows, n_in) -> d_c (n_rows, n_out). */
+ * of functional.py:797-822 + :407-419): d_x (n_rows, n_in) -> d_c (n_rows, n_out).
+ * gdft_hf_device_status on the workspace tells whether a bounded device wait
+ * of the call expired, which also leaves NaN in the result. */
 int gdft_network_apply(const gdft_network *net, const double *d_params, int64_t n_rows, const double *d_x,
                        double *d_c, void *d_ws, size_t ws_bytes, void *stream);
 

@@ -84,3 +84,36 @@ def test_dlpack_inputs_through_energy_predictor(lib, golden):
     assert abs(float(E) - ref) <= 1e-11 * abs(ref)
     Fr = g["predict_F_B88"]
     assert np.max(np.abs(F.cpu().numpy() - Fr)) <= 1e-11 * np.max(np.abs(Fr))
+
+
+@pytest.mark.parametrize("kind", ["energy", "fock", "apply"])
+def test_calls_with_an_error_word_first(lib, kind):
+    """FP64 exact exchange and the network on given inputs clear the error word at the start of their workspace, whatever
+    it held, and the status entry reports a code that is there after the call."""
+    from graddft_gb300 import engine
+
+    L, n_grid, n = lib.load(), 300, 20
+    g = torch.Generator(device="cuda").manual_seed(1)
+    new = lambda *s: torch.randn(s, dtype=torch.float64, device="cuda", generator=g)  # noqa: E731
+    P, nbytes, st = engine._ptr, ctypes.c_size_t(), ctypes.c_int32()
+    net = engine.Network(n_layers=1, width=32)
+    if kind == "apply":
+        lib.check(L.gdft_network_apply_workspace_bytes(ctypes.byref(net.desc), n_grid, ctypes.byref(nbytes)))
+    else:
+        lib.check(L.gdft_hf_workspace_bytes(n_grid, n, 1, ctypes.byref(nbytes)))
+    ws = torch.full((nbytes.value,), 0xFF, dtype=torch.uint8, device="cuda")
+    stream = engine._stream(ws.device)
+    tail = (P(ws), ws.numel(), stream)
+    if kind == "apply":
+        x, out, params = new(n_grid, 11), new(n_grid, 3), new(net.n_params)
+        lib.check(L.gdft_network_apply(ctypes.byref(net.desc), P(params), n_grid, P(x), P(out), *tail))
+    elif kind == "energy":
+        ao, d, chi, out = new(n_grid, n), new(2, n, n), new(n_grid, 1, 2, n), new(1, 2, n_grid)
+        lib.check(L.gdft_hf_energy_density(P(ao), P(d), P(chi), n_grid, n, 1, P(out), *tail))
+    else:
+        ao, chi, w, out = new(n_grid, n), new(n_grid, 1, 2, n), new(1, 2, n_grid), new(2, n, n)
+        lib.check(L.gdft_hf_fock(P(ao), P(chi), P(w), n_grid, n, 1, P(out), *tail))
+    assert L.gdft_hf_device_status(P(ws), ws.numel(), ctypes.byref(st), stream) == lib.GDFT_OK
+    assert torch.isfinite(out).all()
+    ws[:4].copy_(torch.tensor([71, 0, 0, 0], dtype=torch.uint8))
+    assert L.gdft_hf_device_status(P(ws), ws.numel(), ctypes.byref(st), stream) == lib.GDFT_ERR_DEVICE and st.value == 71
