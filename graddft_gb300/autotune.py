@@ -4,7 +4,8 @@ The chunk size of ``engine.ChunkedResident`` trades device memory (one
 chunk's AO tables and workspace) against the per-chunk fixed costs (table
 packing launches, split-K tails, the last wave of each contraction).  For a
 problem bucket (AO count rounded up to the tile of 128, arithmetic form,
-network shape, GPU name) the tuner times the real call at each candidate
+network shape, GPU name, and the library's build: a size tuned for other kernels
+says nothing) the tuner times the real call at each candidate
 size that fits the memory budget, keeps the smallest size within ``tol`` of
 the fastest, and records it in a JSON cache (``$GDFT_AUTOTUNE_CACHE``, by
 default ``~/.cache/graddft_gb300/autotune.json``), so later processes reuse
@@ -12,11 +13,14 @@ the choice without timing.
 """
 from __future__ import annotations
 
+import hashlib
 import json
 import os
 from typing import Callable, Iterable, Optional
 
 import torch
+
+from . import _lib
 
 CANDIDATES = (1 << 14, 1 << 15, 1 << 16, 1 << 17, 1 << 18)
 
@@ -46,9 +50,15 @@ def _store(table: dict) -> None:
         pass  # a read-only home: the choice is still used by this process
 
 
+def build_tag() -> str:
+    """Eight hex digits of the library's contents."""
+    with open(_lib.LIB_PATH, "rb") as f:
+        return hashlib.sha1(f.read()).hexdigest()[:8]
+
+
 def bucket_key(n_ao: int, precision: str, net_key, device) -> str:
     name = torch.cuda.get_device_name(device)
-    return f"chunk|{name}|{precision}|ao{-(-int(n_ao) // 128) * 128}|net{net_key}"
+    return f"chunk|{name}|{precision}|ao{-(-int(n_ao) // 128) * 128}|net{net_key}|lib{build_tag()}"
 
 
 def time_call(fn: Callable[[], None], device, reps: int = 2) -> float:

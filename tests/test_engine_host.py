@@ -215,3 +215,17 @@ def test_longest_first_schedule():
     costs = [float(c) for c in range(1, 40)]
     loads = [sum(costs[i] for i in qq) for qq in schedule_longest_first(costs, 4)]
     assert max(loads) - min(loads) <= max(costs)
+
+
+def test_chunk_sizes_are_kept_for_one_build(monkeypatch, tmp_path):
+    """A chunk size that was timed with other kernels is not taken from the cache."""
+    from graddft_gb300 import _lib, autotune
+
+    monkeypatch.setattr(torch.cuda, "get_device_name", lambda device=None: "GPU")
+    keys = set()
+    for i, text in enumerate((b"kernels", b"other kernels", b"kernels")):
+        path = tmp_path / f"lib{i}.so"
+        path.write_bytes(text)
+        monkeypatch.setattr(_lib, "LIB_PATH", str(path))
+        keys.add(autotune.bucket_key(100, "fp64", None, None))
+    assert len(keys) == 2
