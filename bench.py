@@ -58,6 +58,23 @@ def _profiled_traffic(kernel: str, n_grid: int, n_ao: int):
     return None
 
 
+def _tensor_products(stage: str, form: str, n_ao: int) -> float:
+    """Tensor-core products that a contraction stage executes for each of its 8 N n^2 terms (2 spins x 4 planes).
+
+    Mixed: three TF32 products a term in the density and six in the V_xc GEMM, where from two tiles of 128 AOs on the
+    three d_j planes are formed on and above the diagonal only.  FP64: 28 pairs of BF16 digits; the d_j planes of the
+    density take the blocks of 64 AOs up to the diagonal, those of V_xc the 128 x 64 tiles that reach it.
+    """
+    m, n = -(-n_ao // 128), -(-n_ao // 64)
+    if form == "tf32x3":
+        if stage == "density":
+            return 3.0
+        return 6.0 * (1.0 if m == 1 else (1 + 3 * (m + 1) / (2 * m)) / 4)
+    if stage == "density":
+        return 28.0 * (1 + 3 * (n + 1) / (2 * n)) / 4
+    return 28.0 * (1 + 3 * sum(n - 2 * i for i in range(m)) / (m * n)) / 4
+
+
 def _peaks():
     try:
         with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
@@ -1232,10 +1249,9 @@ def main():
     t_dom, n_dom = stage[dom]
     flops_launch = 16.0 * args.n_grid * args.n_ao ** 2  # 2 spins x 4 planes x 2 N n^2 per contraction
     achieved = flops_launch / (t_dom / n_dom * 1e-3) / 1e12
-    if form == "fp64":
-        peak, bound, peak_src = 1.25, "fp64", "nominal GB300 FP64 rate (no measured FP64 peak)"
-    else:
-        peak, bound, peak_src = bf16, "tensor", f"{src} bf16 dense (the TF32 pipe nominally runs at half of it)"
+    peak, bound, peak_src = bf16, "tensor", f"{src} bf16 dense (the TF32 pipe nominally runs at half of it)"
+    executed = flops_launch * _tensor_products(dom, form, args.n_ao)
+    executed_tflops = executed / (t_dom / n_dom * 1e-3) / 1e12
     traffic = None
     if form == "tf32x3":
         traffic = _profiled_traffic({"density": "dens_tc", "vxc": "tcg_vxc"}[dom], args.n_grid, args.n_ao)
@@ -1244,14 +1260,12 @@ def main():
             "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of a 65,536-point capture "
                               "(profiles/), scaled by grid points" if traffic else None,
             "flops_per_launch": flops_launch,
-            # TF32 products per term: three in the density, six in the V_xc GEMM.
-            "executed_flops_per_launch": flops_launch * ((3 if dom == "density" else 6) if form == "tf32x3" else 1),
-            # The same stage measured as the tensor work it executes, against the
-            # TF32 rate (nominally half the dense BF16 one).
-            "executed_tflops": (flops_launch * ((3 if dom == "density" else 6) if form == "tf32x3" else 1)
-                                / (t_dom / n_dom * 1e-3) / 1e12),
-            "executed_frac_of_tf32": ((flops_launch * (3 if dom == "density" else 6) / (t_dom / n_dom * 1e-3) / 1e12)
-                                      / (peak / 2) if form == "tf32x3" else None),
+            # The same stage measured as the tensor work it executes (TF32 or BF16 products), against
+            # the TF32 rate (nominally half the dense BF16 one) or the BF16 rate.
+            "executed_flops_per_launch": executed,
+            "executed_tflops": executed_tflops,
+            "executed_frac_of_tf32": executed_tflops / (peak / 2) if form == "tf32x3" else None,
+            "executed_frac_of_bf16": executed_tflops / peak if form == "fp64" else None,
             "stage_ms_per_step": {k: v[0] / args.steps for k, v in stage.items()}}
 
     line = {
