@@ -224,8 +224,8 @@ __global__ void __launch_bounds__(256, 4) fx_features_kernel(const double *__res
 }
 
 // ---------------------------------------------------------------- V_xc operands
-// High words add like logarithms: hi(x) + hi(y) - hi(1) is at most the product's
-// and below it by less than 1/8 in the mantissa. 
+// High words add like logarithms: hi(x) + hi(y) - hi(1) is at most the product's, and
+// below it by at most 3 - 2 sqrt 2 = 0.172 of an octave (both mantissas sqrt 2), for which field_of adds 1/4.
 constexpr int kOneHi = 0x3FF00000;
 static_assert((int)T_PHI == (int)C_RHO && (int)T_DX == (int)C_GX && (int)T_DY == (int)C_GY && (int)T_DZ == (int)C_GZ &&
                   (int)T_LAP == (int)C_LAP,
