@@ -150,25 +150,10 @@ __device__ __forceinline__ Dual<K> operator/(double c, const Dual<K> &a) {
 __device__ __forceinline__ double xlog2(double x) { return log2(x); }
 __device__ __forceinline__ double xexp2(double x) { return exp2(x); }
 __device__ __forceinline__ double xlog(double x) { return log(x); }
-__device__ __forceinline__ double xexp(double x) { return exp(x); }
-__device__ __forceinline__ double xsqrt(double x) { return sqrt(x); }
-__device__ __forceinline__ double xasinh(double x) { return asinh(x); }
 __device__ __forceinline__ double xatan(double x) { return atan(x); }
-__device__ __forceinline__ double xpow(double x, double p) { return pow(x, p); }
-__device__ __forceinline__ double xpow3(double x, int n) {
-  if (!(x >= 0.0)) return pow(x, n / 3.0);  // NaN for negative or NaN x, as pow
-  if (n == -1) return rcbrt(x);
-  if (n == -5) {
-    const double r = rcbrt(x);
-    return (r * r) / x;
-  }
-  if (n == 4) return x * cbrt(x);
-  if (n == 8) {
-    const double c = cbrt(x);
-    return (x * x) * (c * c);
-  }
-  return pow(x, n / 3.0);
-}
+// x ** (4/3), the power of the exchange terms, from CUDA's cube root (within 1 ulp; pow
+// evaluates a logarithm and an exponential); NaN for negative or NaN x, as pow.
+__device__ __forceinline__ double xpow43(double x) { return x >= 0.0 ? x * cbrt(x) : pow(x, 4.0 / 3.0); }
 __device__ __forceinline__ double xsq(double x) { return x * x; }
 __device__ __forceinline__ double xclipmin(double x, double c) { return isnan(x) ? x : fmax(c, x); }
 __device__ __forceinline__ double xabs(double x) { return fabs(x); }
@@ -190,38 +175,12 @@ __device__ __forceinline__ Dual<K> xlog(const Dual<K> &x) {
   return chain(x, log(x.v), 1.0 / x.v);
 }
 template <int K>
-__device__ __forceinline__ Dual<K> xexp(const Dual<K> &x) {
-  const double f = exp(x.v);
-  return chain(x, f, f);
-}
-template <int K>
-__device__ __forceinline__ Dual<K> xsqrt(const Dual<K> &x) {
-  const double f = sqrt(x.v);
-  return chain(x, f, 0.5 / f);
-}
-template <int K>
-__device__ __forceinline__ Dual<K> xasinh(const Dual<K> &x) {
-  return chain(x, asinh(x.v), 1.0 / sqrt(1.0 + x.v * x.v));
-}
-template <int K>
 __device__ __forceinline__ Dual<K> xatan(const Dual<K> &x) {
   return chain(x, atan(x.v), 1.0 / (1.0 + x.v * x.v));
 }
-// x ** p with a constant real exponent (jax pow JVP: p * x ** (p - 1)).
 template <int K>
-__device__ __forceinline__ Dual<K> xpow(const Dual<K> &x, double p) {
-  return chain(x, pow(x.v, p), p * pow(x.v, p - 1.0));
-}
-// x ** (n/3) with an integer n from CUDA's cube roots (cbrt and rcbrt are
-// within 1 ulp; pow evaluates a logarithm and an exponential); pow for x < 0 or
-// NaN.  x ** (4/3), the power of the exchange terms: partial (4/3) cbrt(x).
-template <int K>
-__device__ __forceinline__ Dual<K> xpow3(const Dual<K> &x, int n) {
-  const double f = xpow3(x.v, n);
-  const double df = n == 4 && x.v >= 0.0               ? (4.0 / 3.0) * cbrt(x.v)
-                    : x.v > 0.0 && isfinite(f)         ? (n / 3.0) * f / x.v
-                                                       : (n / 3.0) * pow(x.v, n / 3.0 - 1.0);
-  return chain(x, f, df);
+__device__ __forceinline__ Dual<K> xpow43(const Dual<K> &x) {
+  return chain(x, xpow43(x.v), 4.0 / 3.0 * (x.v >= 0.0 ? cbrt(x.v) : pow(x.v, 1.0 / 3.0)));
 }
 // x ** 2 with an integer exponent (jax integer_pow JVP: 2 x).
 template <int K>

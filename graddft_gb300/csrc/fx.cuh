@@ -115,7 +115,7 @@ struct GemmArgs {
   int planes;                  // kDensity: 1 or 4; kVxc: 1 or 2
   int chunks;                  // K chunks of a tile (kVxc: of plane 0; plane 1 has three times as many)
   int a_stride, b_stride;      // sets between consecutive tiles
-  int splits, chunks_per_split;
+  int chunks_per_split;
   double *out;                 // row r, column c of half h (columns 64 h .. of a tile): out + split_stride split
   int64_t ldc;                 //   + plane_stride plane + half_stride h + nt_stride nt + ldc c + r (lanes are rows)
   int64_t half_stride, nt_stride, split_stride, plane_stride;

@@ -4,7 +4,7 @@
 // keeping its evaluation order, clip and where semantics; it is a template
 // over the scalar type (double for values, Dual<K> for values plus partials),
 // except B88 and LYP, whose partials are written out.
-// Powers of a third come from cube roots (xpow3), within a few ulp of pow, and
+// Powers of a third come from cube roots, within a few ulp of pow, and
 // B88 is evaluated without its logarithms (see b88_x_e).
 // Inputs per point: rho[2], s[2] = |grad rho_sigma|^2, st = |grad rho_a +
 // grad rho_b|^2, lap[2], tau[2].
@@ -24,7 +24,7 @@ template <class T>
 __device__ __forceinline__ T exch_pol(const T &e0, const T &e1, const T &r0, const T &r1) {
   const T zeta = (r0 - r1) / (r0 + r1);
   const double den = 2.0 * (pow(2.0, 1.0 / 3.0) - 1.0);
-  const T fz = (xpow3(1.0 - zeta, 4) + xpow3(1.0 + zeta, 4) - 2.0) / den;
+  const T fz = (xpow43(1.0 - zeta) + xpow43(1.0 + zeta) - 2.0) / den;
   return e0 + (e1 - e0) * fz;
 }
 
@@ -77,7 +77,7 @@ template <class T>
 __device__ __forceinline__ T lsda_x_e(const T rho_in[2], double clip) {
   const T r0 = xclipmin(rho_in[0], clip);
   const T r1 = xclipmin(rho_in[1], clip);
-  const T s43 = xpow3(r0 + r1, 4);
+  const T s43 = xpow43(r0 + r1);
   const T e0 = (-3.0 / 4.0 * pow(3.0 / kPi, 1.0 / 3.0)) * s43;
   const T e1 = (-3.0 / 4.0 * pow(6.0 / kPi, 1.0 / 3.0)) * s43;
   return exch_pol(e0, e1, r0, r1);
@@ -100,7 +100,7 @@ __device__ __forceinline__ double b88_x_e(const double rho_in[2], const double s
   for (int sp = 0; sp < 2; ++sp) {
     const double rho = xclipmin(rho_in[sp], clip), sc = xclipmin(s[sp], clip);
     const double g = sqrt(sc);
-    const double x = g / xpow3(rho, 4);
+    const double x = g / xpow43(rho);
     const double as = asinh(x);
     const double inv = 1.0 / (1.0 + 6.0 * beta * x * as);
     const double term = beta * (g * x) * inv;
