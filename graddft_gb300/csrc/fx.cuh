@@ -130,7 +130,7 @@ cudaError_t launch_gemm(const GemmArgs &a, cudaStream_t st);
 
 // Row-major FP64 rows (planes of them, k_valid values each) -> digit sets [plane][row tile][chunk], exponents
 // [plane][rows].  Rows past the last are left as they are: they only reach outputs that are not written.  oct, or
-// null: 64 chunks octaves t, aligned to 16 bytes; column k is taken times 2^t.
+// null: 64 chunks octaves t <= 0, aligned to 16 bytes; column k is taken times 2^t.
 cudaError_t launch_rows(const double *src, int64_t plane_elems, int planes, int64_t rows, int64_t ld, int k_valid,
                         int chunks, const int *oct, unsigned char *out, int *exps, int *bad, cudaStream_t st);
 
@@ -140,7 +140,7 @@ cudaError_t launch_rows(const double *src, int64_t plane_elems, int planes, int6
 size_t gemm_rows_bytes(int64_t M, int N, int K);
 size_t gemm_cols_bytes(int M, int N, int64_t K);
 // C[m][n] = sum_k A[m][k] B[k][n] (B stored N x K when b_rows) + add[m][n] (laid out like C; null: nothing).  oct, or
-// null (it has to be with b_rows): octaves_len(K) octaves t, aligned to 16 bytes; A's columns are taken times 2^t, B's
+// null (it has to be with b_rows): octaves_len(K) octaves t <= 0, aligned to 16 bytes; A's columns are taken times 2^t, B's
 // rows times 2^-t.
 cudaError_t gemm_rows(int64_t M, int N, int K, const double *A, int64_t lda, const double *B, int64_t ldb, bool b_rows,
                       const int *oct, double *C, int64_t ldc, const double *add, unsigned char *ws, int *err, cudaStream_t st);
@@ -150,10 +150,10 @@ cudaError_t gemm_cols(int M, int N, int64_t K, const double *A, int64_t lda, con
                       const int *oct, double *C, unsigned char *ws, int *err, int nsplit, double *part,
                       cudaStream_t st);
 
-// Octaves of the AOs for products of AO values with D (2, n, n), fx_xc.cu: octaves_len(n) of them.  bad: a word to clear,
-// or null.
+// Octaves of the AOs for products of AO values with D (2, n, n), fx_xc.cu: octaves_len(n) for both spins together, or
+// (each) for either.  mx: 2 octaves_len(n) integers of scratch; bad: a word to clear, or null.
 inline int octaves_len(int n) { return (n + 63) / 64 * 64; }
-cudaError_t launch_octaves(const double *D, int n, int *oct, int *bad, cudaStream_t st);
+cudaError_t launch_octaves(const double *D, int n, bool each, int *mx, int *oct, int *bad, cudaStream_t st);
 
 // Feature sets of fx_xc.cu: the FP64 form's density and V_xc contractions.
 struct XcWs {

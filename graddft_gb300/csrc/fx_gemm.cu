@@ -551,7 +551,7 @@ __global__ void __launch_bounds__(256) fx_rows_kernel(const double *__restrict__
     for (int j = 0; j < 8; ++j) {
       const uint32_t h = (uint32_t)__double2hiint(v[j]) & 0x7FFFFFFFu;
       m = max(m, h);
-      if (OCT) mt = max(mt, (int)min(h, 0x7FF00000u - (450u << 20)) + t[j] * (1 << 20));
+      if (OCT) mt = max(mt, (int)h + t[j] * (1 << 20));
     }
   }
 #pragma unroll

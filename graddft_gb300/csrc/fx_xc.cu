@@ -8,7 +8,8 @@
 // on the diagonal blocks), (n + 64) / 2n of the products.  A point's row of AOs is fixed
 // point on the largest, which may be one that D hardly occupies (a steep function near its
 // nucleus): phi_a is taken times 2^t and D_ab times 2^-t, t half the exponent of the
-// largest entry of D in row or column a (exact), so that rows are like phi_a sqrt(D_aa).
+// largest entry of D in row or column a, relative to D's largest (exact), so that rows are like
+// phi_a sqrt(D_aa).  The spins share the digits of phi: the larger of their two t counts.
 // s functions up to exponent 1e10, the two steepest not in D, errors relative to the sums of
 // the terms' sizes: rho 5e-15 -> 3e-16, tau 8e-11 -> 4e-16.
 //
@@ -19,7 +20,8 @@
 // value, and phi and Q are graded against one another: a steep function is large
 // where the weights, and so Q, are small.  Both are therefore taken times a power
 // of two for each point that shares the coefficients out evenly (phi 2^t and
-// Q 2^-t, t half the exponent of the point's largest coefficient; exact): rows are then
+// Q 2^-t, t half the exponent of the point's largest coefficient, relative to the spin's
+// largest in the slab, the larger of the spins' t; exact): rows are then
 // like sqrt(|c|) phi, square-integrable, and the error is relative to the product of
 // two such maxima instead of max |phi_a| max |Q_b|.  s functions of exponents A and 0.15
 // on one centre, 300 radial points, error relative to sum |phi_a Q_b|: A = 6,665
@@ -63,26 +65,49 @@ __device__ __forceinline__ int hi_of(double x) {
 constexpr int kNoRow = -(600 << 20);
 __device__ __forceinline__ int field_at(int m) { return m < kNoRow ? 1 : m >> 20; }
 
-// Octaves of the AOs, a warp each: half the exponent of the largest entry of either
-// spin's D in row or column a; also clears the non-finite word, if any.  kEmpty where there is
-// none (and past the last AO): the AO's digits are then below all others.
-constexpr int kEmpty = -1200;
-__global__ void __launch_bounds__(256) fx_octaves_kernel(const double *__restrict__ D, int n, int n_pad,
-                                                         int *__restrict__ oct, int *__restrict__ bad) {
+// Largest high word of D in row or column a of either spin, mx[2][n_pad], a warp each; also clears the non-finite
+// word, if any.
+__global__ void __launch_bounds__(256) fx_rdm1_max_kernel(const double *__restrict__ D, int n, int n_pad,
+                                                          int *__restrict__ mx, int *__restrict__ bad) {
   previous_done();
   if (blockIdx.x == 0 && threadIdx.x == 0 && bad != nullptr) *bad = 0;
-  const int a = (blockIdx.x * 256 + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (a >= n_pad) return;
+  const int i = (blockIdx.x * 256 + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (i >= 2 * n_pad) return;
+  const int a = i % n_pad;
+  const double *Ds = D + (size_t)(i / n_pad) * n * n;
   int m = kNone;
-  for (int b = lane; a < n && b < n; b += 32)
-#pragma unroll
-    for (int s = 0; s < 2; ++s) {
-      const double *Ds = D + (size_t)s * n * n;
-      m = max(m, max(hi_of(Ds[(size_t)a * n + b]), hi_of(Ds[(size_t)b * n + a])));
-    }
+  for (int b = lane; a < n && b < n; b += 32) m = max(m, max(hi_of(Ds[(size_t)a * n + b]), hi_of(Ds[(size_t)b * n + a])));
 #pragma unroll
   for (int o = 16; o > 0; o /= 2) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if (lane == 0) oct[a] = m == kNone ? kEmpty : ((m >> 20) - 1023) >> 1;
+  if (lane == 0) mx[i] = m;
+}
+
+// Octaves of the AOs from that, one block: half the exponent relative to the spin's
+// largest, of both spins together (the larger one) or of each.  kEmpty where D has no entry
+// (and past the last AO): the AO's digits are then below all others.
+constexpr int kEmpty = -1200;
+__global__ void __launch_bounds__(1024) fx_octaves_kernel(const int *__restrict__ mx, int n_pad, bool each,
+                                                          int *__restrict__ oct) {
+  previous_done();
+  __shared__ int top[2];
+  if (threadIdx.x < 2) top[threadIdx.x] = kNone;
+  __syncthreads();
+  for (int i = threadIdx.x; i < 2 * n_pad; i += blockDim.x) atomicMax(&top[i / n_pad], mx[i]);
+  __syncthreads();
+  for (int a = threadIdx.x; a < n_pad; a += blockDim.x) {
+    int t[2];
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      const int m = mx[s * n_pad + a];
+      t[s] = m == kNone ? kEmpty : (m - top[s]) >> 21;
+    }
+    if (each) {
+      oct[a] = t[0];
+      oct[n_pad + a] = t[1];
+    } else {
+      oct[a] = max(t[0], t[1]);
+    }
+  }
 }
 
 // Digits of D as the B operand: tile nt = columns 64 nt .. of spin 0, then of
@@ -237,6 +262,32 @@ __device__ __forceinline__ int field_of(int m, int octaves) {
   return f > 0x7FE ? 0x7FE : f;
 }
 
+// Largest high words of a slab's coefficients: g[0][s] of those of Q_s, g[1][s] of c_kin,s.
+__global__ void __launch_bounds__(256) fx_coef_max_kernel(const double *__restrict__ coef, int64_t np, int64_t p0,
+                                                          int64_t rows, int *__restrict__ g) {
+  previous_done();
+  __shared__ int sg[4];
+  if (threadIdx.x < 4) sg[threadIdx.x] = kNone;
+  __syncthreads();
+  const int64_t p = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  const int warp_lane = threadIdx.x & 31;
+#pragma unroll
+  for (int s = 0; s < 2; ++s) {
+    int m[2] = {kNone, kNone};
+    if (p < rows)
+#pragma unroll
+      for (int k = 0; k < kFeat; ++k)
+        m[k == C_KIN] = max(m[k == C_KIN], hi_of(coef[((size_t)s * kFeat + k) * np + p0 + p]));
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int w = __reduce_max_sync(0xffffffffu, m[i]);
+      if (warp_lane == 0) atomicMax(&sg[2 * i + s], w);
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < 4) atomicMax(g + threadIdx.x, sg[threadIdx.x]);
+}
+
 // The non-finite word, and n maxima below every high word (a kernel, not a
 // memset: launches before and after it stay chained).
 __global__ void fx_clear_kernel(int *bad, int *mx, int n) {
@@ -252,8 +303,8 @@ __global__ void fx_clear_kernel(int *bad, int *mx, int n) {
 // Lanes are AOs, a block takes 32 AOs and `per` points, its warps every eighth point.
 __global__ void __launch_bounds__(256) fx_vmax_kernel(const double *__restrict__ tab, size_t pe, int64_t np, int ld,
                                                       const double *__restrict__ coef, int64_t p0, int64_t rows,
-                                                      int per, bool kin, int n_max, int *__restrict__ mx,
-                                                      int *__restrict__ oct, int64_t oct_stride,
+                                                      int per, bool kin, int n_max, const int *__restrict__ g,
+                                                      int *__restrict__ mx, int *__restrict__ oct, int64_t oct_stride,
                                                       int *__restrict__ bad) {
   previous_done();
   __shared__ int sc[2][kFeat][128], so[2][128];  // high words over 1 (2^-t, for the octaves), octaves
@@ -274,9 +325,12 @@ __global__ void __launch_bounds__(256) fx_vmax_kernel(const double *__restrict__
     {
       const int p = threadIdx.x % 128, part = threadIdx.x / 128;  // part 1: the kinetic rows
       const int k0 = part ? C_KIN : 0, k1 = part ? C_KIN + 1 : C_KIN;
-      int m = kNone;
-      for (int k = k0; k < k1; ++k) m = max(m, max(sc[0][k][p], sc[1][k][p]));
-      const int t = m == kNone ? kDead : m >> 21;
+      int t = kDead;
+      for (int s = 0; s < 2; ++s) {
+        int m = kNone;
+        for (int k = k0; k < k1; ++k) m = max(m, sc[s][k][p]);
+        if (m != kNone) t = max(t, (m - (g[2 * part + s] - kOneHi)) >> 21);
+      }
       so[part][p] = t;
       for (int k = k0; k < k1; ++k)
         for (int s = 0; s < 2; ++s)  // kept at or above kNone: two of them still add without overflow
@@ -482,7 +536,7 @@ XcWs xc_ws(int64_t np, int n_ao) {
   w.off_dexp = off;
   off = align256(off + (size_t)2 * w.nb * kTile * sizeof(int));
   w.off_doct = off;
-  off = align256(off + (size_t)octaves_len(n_ao) * sizeof(int));
+  off = align256(off + (size_t)3 * octaves_len(n_ao) * sizeof(int));  // and the maxima they come from
   w.off_a = off;
   off = align256(off + (size_t)4 * (w.dens_slab / kTile) * w.nb * kSetBytes);
   w.off_ea = off;
@@ -496,7 +550,7 @@ XcWs xc_ws(int64_t np, int n_ao) {
   w.off_vb = off;
   off = align256(off + (size_t)w.nb * 4 * npc * kSetBytes);
   w.off_vexp = off;
-  off = align256(off + (size_t)(2 * w.mt * kTile + 2 * w.nb * kTile + 6 * n128 + 2 * w.v_slab) * sizeof(int));
+  off = align256(off + (size_t)(2 * w.mt * kTile + 2 * w.nb * kTile + 6 * n128 + 4 + 2 * w.v_slab) * sizeof(int));
   w.off_vpart = off;
   // s0 + s1 is at most this for any grid, so a shorter grid never needs more than a longer one.
   const int64_t most = 4 * 2 * 148 / ((int64_t)w.mt * w.nb + 3 * upper) + 2;
@@ -505,9 +559,10 @@ XcWs xc_ws(int64_t np, int n_ao) {
   return w;
 }
 
-cudaError_t launch_octaves(const double *D, int n, int *oct, int *bad, cudaStream_t st) {
+cudaError_t launch_octaves(const double *D, int n, bool each, int *mx, int *oct, int *bad, cudaStream_t st) {
   const int len = octaves_len(n);
-  launch_next(fx_octaves_kernel, len / 8, 256, 0, st, D, n, len, oct, bad);
+  launch_next(fx_rdm1_max_kernel, 2 * len / 8, 256, 0, st, D, n, len, mx, bad);
+  launch_next(fx_octaves_kernel, 1, len < 1024 ? len : 1024, 0, st, mx, len, each, oct);
   return cudaGetLastError();
 }
 
@@ -520,7 +575,7 @@ cudaError_t launch_density(const double *tab, int64_t np, int ld, int n_ao, cons
   int *dexp = (int *)(ws + w.off_dexp), *ea = (int *)(ws + w.off_ea), *oct = (int *)(ws + w.off_doct);
   double *X = (double *)(ws + w.off_x);
   cudaError_t e;
-  if ((e = launch_octaves(rdm1, n_ao, oct, bad, st)) != cudaSuccess) return e;
+  if ((e = launch_octaves(rdm1, n_ao, false, oct + octaves_len(n_ao), oct, bad, st)) != cudaSuccess) return e;
   launch_next(fx_rdm1_kernel, dim3((unsigned)(w.nb * 4), kin ? 2 : 1), 128, 0, st, rdm1, n_ao, w.nb, oct, dset, dexp,
               bad);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
@@ -568,21 +623,22 @@ cudaError_t launch_vxc(const double *tab, int64_t np, int ld, int n_ao, const do
   const size_t pe = (size_t)np * ld;
   int *bad = bad_word(ws, w);
   const int n_max = w.mt * kTile;
-  int *ea = (int *)(ws + w.off_vexp), *eb = ea + 2 * n_max, *mx = eb + 2 * w.nb * kTile, *oct = mx + 6 * n_max;
+  int *ea = (int *)(ws + w.off_vexp), *eb = ea + 2 * n_max, *mx = eb + 2 * w.nb * kTile, *g = mx + 6 * n_max, *oct = g + 4;
   unsigned char *va = ws + w.off_va, *vb = ws + w.off_vb;
   double *part = (double *)(ws + w.off_vpart);
   cudaError_t e;
   for (int64_t p0 = 0; p0 < np; p0 += w.v_slab) {
     const int64_t rows = np - p0 < w.v_slab ? np - p0 : w.v_slab;
     const int npc = (int)((rows + kChunkK - 1) / kChunkK);
-    launch_next(fx_clear_kernel, (6 * n_max + 255) / 256, 256, 0, st, p0 == 0 ? bad : nullptr, mx, 6 * n_max);
+    launch_next(fx_clear_kernel, (6 * n_max + 4 + 255) / 256, 256, 0, st, p0 == 0 ? bad : nullptr, mx, 6 * n_max + 4);
+    launch_next(fx_coef_max_kernel, (unsigned)((rows + 255) / 256), 256, 0, st, coef, np, p0, rows, g);
     const int blocks_a = (ld + 31) / 32;
     int64_t segs = (8 * 148 + blocks_a - 1) / blocks_a;
     int64_t per = (rows + segs - 1) / segs;
     per = per < 64 ? 64 : per;
     segs = (rows + per - 1) / per;
     launch_next(fx_vmax_kernel, dim3(blocks_a, (unsigned)segs), 256, 0, st, tab, pe, np, ld, coef, p0, rows, (int)per,
-                kin, n_max, mx, oct, w.v_slab, bad);
+                kin, n_max, g, mx, oct, w.v_slab, bad);
     launch_next(fx_vdigits_kernel, dim3(3, ld / 32, npc), 256, 0, st, tab, pe, np, ld, coef, p0, rows, npc, kin, w.mt,
                 w.nb, (n_ao + 7) / 8 * 8, mx, oct, w.v_slab, ea, eb, va, vb, bad);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;

@@ -68,14 +68,14 @@ __global__ void hf_bmat_kernel(const double *__restrict__ chi, const double *__r
   B[i] = -0.5 * acc;
 }
 
-// Octaves of a point for ao^T B: half the exponent of its largest |g|.
-__global__ void hf_octaves_kernel(const double *__restrict__ g, int64_t n_grid, int n_rows, int *__restrict__ oct) {
+// Octaves of a point for ao^T B_s, oct[s][r]: half the exponent of the spin's largest |g| there.
+__global__ void hf_octaves_kernel(const double *__restrict__ g, int64_t n_grid, int n_omega, int *__restrict__ oct) {
   previous_done();
-  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= n_grid) return;
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= 2 * n_grid) return;
   int m = 0;
-  for (int k = 0; k < n_rows; ++k) m = max(m, __double2hiint(g[(size_t)k * n_grid + r]) & 0x7FFFFFFF);
-  oct[r] = m == 0 ? fx::kDead : ((m >> 20) - 1023) >> 1;
+  for (int w = 0; w < n_omega; ++w) m = max(m, __double2hiint(g[(size_t)w * 2 * n_grid + i]) & 0x7FFFFFFF);
+  oct[i] = m == 0 ? fx::kDead : ((m >> 20) - 1023) >> 1;
 }
 
 // fock[s] = abs_clip(fock[s] + F[s] + F[s]^T)  (train.py:200-210).
@@ -378,8 +378,8 @@ int gdft_hf_workspace_bytes_form(int64_t n_grid, int32_t n_ao, int32_t n_omega, 
     *bytes = hf_tc_layout(n_grid, n_ao).bytes;
     return GDFT_OK;
   }
-  const size_t rows = align256((size_t)fx::octaves_len(n_ao) * sizeof(int)) + fx::gemm_rows_bytes(n_grid, n_ao, n_ao);
-  const size_t cols = align256((size_t)n_grid * sizeof(int)) + fx::gemm_cols_bytes(n_ao, n_ao, n_grid);
+  const size_t rows = align256((size_t)4 * fx::octaves_len(n_ao) * sizeof(int)) + fx::gemm_rows_bytes(n_grid, n_ao, n_ao);
+  const size_t cols = align256((size_t)2 * n_grid * sizeof(int)) + fx::gemm_cols_bytes(n_ao, n_ao, n_grid);
   *bytes = hf_gemm_off(n_grid, n_ao) + 256 + (rows > cols ? rows : cols);
   return GDFT_OK;
 }
@@ -403,12 +403,13 @@ int gdft_hf_energy_density_form(const double *d_ao, const double *d_rdm1, const 
   double *X = (double *)((char *)d_ws + kHfX);
   int *err = (int *)d_ws;
   if ((rc = check_cuda(cudaMemsetAsync(err, 0, sizeof(int), st), "hf err clear"))) return rc;
-  int *oct = hf_octaves(d_ws, n_grid, n_ao);
-  if ((rc = check_cuda(fx::launch_octaves(d_rdm1, n_ao, oct, nullptr, st), "hf octaves"))) return rc;
+  const int len = fx::octaves_len(n_ao);
+  int *oct = hf_octaves(d_ws, n_grid, n_ao);  // [2][len], then the maxima they come from
+  if ((rc = check_cuda(fx::launch_octaves(d_rdm1, n_ao, true, oct + 2 * len, oct, nullptr, st), "hf octaves"))) return rc;
   for (int s = 0; s < 2; ++s)
     if ((rc = check_cuda(fx::gemm_rows(n_grid, n_ao, n_ao, d_ao, n_ao, d_rdm1 + (size_t)s * n_ao * n_ao, n_ao, false,
-                                       oct, X + (size_t)s * n_grid * n_ao, n_ao, nullptr,
-                                       hf_scratch(oct, fx::octaves_len(n_ao)), err, st),
+                                       oct + s * len, X + (size_t)s * n_grid * n_ao, n_ao, nullptr,
+                                       hf_scratch(oct, 4 * len), err, st),
                          "hf ao.D")))
       return rc;
   const int64_t threads = 2 * n_grid * 32;
@@ -440,12 +441,12 @@ int gdft_hf_fock_form(const double *d_ao, const double *d_chi, const double *d_g
   const size_t total = (size_t)2 * n_grid * n_ao;
   launch_next(hf_bmat_kernel, (unsigned)((total + 255) / 256), 256, 0, st, d_chi, d_g, n_grid, n_ao, n_omega, B);
   int *oct = hf_octaves(d_ws, n_grid, n_ao);
-  launch_next(hf_octaves_kernel, (unsigned)((n_grid + 255) / 256), 256, 0, st, d_g, n_grid, 2 * n_omega, oct);
+  launch_next(hf_octaves_kernel, (unsigned)((2 * n_grid + 255) / 256), 256, 0, st, d_g, n_grid, n_omega, oct);
   if ((rc = check_cuda(cudaGetLastError(), "hf B"))) return rc;
   const int nsplit = hf_splits(n_grid);
   for (int s = 0; s < 2; ++s)
     if ((rc = check_cuda(fx::gemm_cols(n_ao, n_ao, n_grid, d_ao, n_ao, B + (size_t)s * n_grid * n_ao, n_ao,
-                                       oct, d_fock_hf + (size_t)s * n_ao * n_ao, hf_scratch(oct, n_grid), err, nsplit,
+                                       oct + s * n_grid, d_fock_hf + (size_t)s * n_ao * n_ao, hf_scratch(oct, 2 * n_grid), err, nsplit,
                                        part, st),
                          "hf ao^T B")))
       return rc;

@@ -267,7 +267,7 @@ NuWs nu_ws(const PairPlan &plan, int n_ao, int64_t chunk, bool want_chi, int n_o
     W.off_x = off;
     off = al256(off + (size_t)2 * chunk * n_ao * sizeof(double));
     W.off_oct = off;
-    off = al256(off + (size_t)fx::octaves_len(n_ao) * sizeof(int));
+    off = al256(off + (size_t)4 * fx::octaves_len(n_ao) * sizeof(int));  // [2][octaves], the maxima they come from
     W.off_fx = off;
     off = al256(off + fx::gemm_rows_bytes(chunk, n_ao, n_ao));
   }
@@ -432,7 +432,8 @@ int gdft_chi(const gdft_basis *basis, const double *d_coords, const double *d_ao
   double *X = (double *)(ws + W.off_x);
   int *oct = (int *)(ws + W.off_oct), *err = (int *)(ws + W.off_err);
   if ((rc = check_cuda(cudaMemsetAsync(err, 0, sizeof(int), st), who))) return rc;
-  if ((rc = check_cuda(fx::launch_octaves(d_rdm1, n, oct, nullptr, st), who))) return rc;
+  const int len = fx::octaves_len(n);
+  if ((rc = check_cuda(fx::launch_octaves(d_rdm1, n, true, oct + 2 * len, oct, nullptr, st), who))) return rc;
   for (int w = 0; w < n_omega; ++w)
     if ((rc = setup_nu(B, plan, W, ws, w, h_omegas[w], w == 0, who, st))) return rc;
   for (int64_t p0 = 0; p0 < n_grid; p0 += pc) {
@@ -440,7 +441,7 @@ int gdft_chi(const gdft_basis *basis, const double *d_coords, const double *d_ao
     // X_s = ao[p0 : p0 + np_] D_s, shared by the omegas
     for (int s = 0; s < 2; ++s)
       if ((rc = check_cuda(fx::gemm_rows(np_, n, n, d_ao + p0 * n, n, d_rdm1 + (size_t)s * n * n, n, false,
-                                         oct, X + (size_t)s * pc * n, n, nullptr, (unsigned char *)(ws + W.off_fx), err,
+                                         oct + s * len, X + (size_t)s * pc * n, n, nullptr, (unsigned char *)(ws + W.off_fx), err,
                                          st),
                            who)))
         return rc;

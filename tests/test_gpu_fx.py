@@ -188,3 +188,78 @@ def test_tiny_products(E):
         bound = 2 * _dot_bound(aX, chi[:, 0, s], 2 * n + 20) + n * (2.0 ** -57 * np.abs(ao).max(1) * np.abs(
             D[s]).max() + 2.0 ** -1022) * np.abs(chi[:, 0, s]).sum(1)
         assert np.all(np.abs(ehf[0, s] + 0.5 * (chi[:, 0, s] * (ao @ D[s])).sum(1)) <= bound)
+
+
+def test_gemms_past_one_slab(E):
+    """The tall GEMMs hold the digits of about 512 MB at a time: 150,000 rows of a layer of width 256, 75,000 points of an
+    exchange Fock term of 200 AOs.  Against float64 products on the GPU; rows and elements as above."""
+    import graddft_gb300 as G
+    import oracle as O
+    from graddft_gb300 import synthetic
+
+    rows, width = 160_001, 256
+    p = synthetic.glorot_params(layer_widths=(width,), seed=3)
+    x = torch.as_tensor(np.random.default_rng(4).standard_normal((rows, 11)), device="cuda")
+    got = G.DM21(layer_widths=(width,)).apply(p, x)
+    tp = {"params": {k: {kk: torch.as_tensor(v) for kk, v in d.items()} for k, d in p["params"].items()}}
+    for part in (slice(0, 300), slice(149_000, 151_000), slice(rows - 300, rows)):  # the first slab's end among them
+        assert torch.max(torch.abs(got[part].cpu() - O.dm21_network(tp, x[part].cpu(), n_layers=1))) <= 1e-13
+    N, n = 80_001, 200
+    g = torch.Generator(device="cuda").manual_seed(5)
+    new = lambda *s: torch.randn(s, dtype=torch.float64, device="cuda", generator=g)  # noqa: E731
+    ao, chi, w = new(N, n), new(N, 1, 2, n), new(1, 2, N)
+    fock = E.hf_fock(ao, chi, w)
+    for s in range(2):
+        B = -0.5 * w[0, s][:, None] * chi[:, 0, s]
+        # w's octaves move up to 2^3 from one operand to the other here: 2^-56 of the products of the scaled maxima.
+        t = torch.exp2(torch.floor(torch.floor(torch.log2(w[0].abs().amax(0))) / 2))[:, None]
+        lost = N * 2.0 ** -56 * (ao * t).abs().amax(0)[:, None] * (B / t).abs().amax(0)[None]
+        bound = (N + 200) * U * (ao.abs().T @ B.abs()) + lost
+        assert bool((torch.abs(fock[s] - ao.T @ B) <= bound).all())
+
+
+@pytest.mark.parametrize("value", [2.0 ** 460, np.inf, np.nan])
+def test_exchange_left_to_the_plain_kernels(E, value):
+    """One AO value past the digits' range (2^450) or not finite: the plain kernels' sums and IEEE's pattern."""
+    n, N = 70, 300
+    g = np.random.default_rng(8)
+    ao, D, chi, w = (g.standard_normal(s) for s in ((N, n), (2, n, n), (N, 1, 2, n), (1, 2, N)))
+    ao[17, 5] = value
+    c = lambda x: torch.as_tensor(x, device="cuda")  # noqa: E731
+    ehf, fock = E.hf_energy_density(c(ao), c(D), c(chi)).cpu().numpy(), E.hf_fock(c(ao), c(chi), c(w)).cpu().numpy()
+    for s in range(2):
+        B = -0.5 * w[0, s][:, None] * chi[:, 0, s]
+        with np.errstate(invalid="ignore"):
+            refs = (ehf[0, s], -0.5 * (chi[:, 0, s] * (ao @ D[s])).sum(1), (np.abs(chi[:, 0, s]) * (np.abs(ao) @ np.abs(
+                D[s]))).sum(1)), (fock[s], ao.T @ B, np.abs(ao).T @ np.abs(B))
+        for got, ref, size in refs:
+            ok = np.isfinite(size)
+            assert np.all(np.abs(got[ok] - ref[ok]) <= 2 * (N + n) * U * size[ok])
+            assert not np.isfinite(got[~ok]).any()
+
+
+@pytest.mark.parametrize("what", ["ao", "rdm1", "pot"])
+def test_past_the_digits_range(E, what):
+    """A finite value past 2^450: density and V_xc come from the plain kernels, finite and right."""
+    n, N = 40, 300
+    ao, g1, g2, D, pot = _tables(n, N, 11)
+    {"ao": ao, "rdm1": D[0], "pot": pot[0]}[what].flat[7] = 2.0 ** 460
+    r = _resident(E, ao, g1, g2)
+    rho = r.density(D)["rho"].cpu().numpy()
+    v = r.vxc_from_potentials(pot).cpu().numpy()
+    lap = g2.sum(-1)
+    for s in range(2):
+        size = ((np.abs(ao) @ np.abs(D[s])) * np.abs(ao)).sum(1)
+        lost = n * 2.0 ** -56 * np.abs(ao).max(1) * np.abs(D[s]).max() * np.abs(ao).sum(1)  # where the digits serve
+        assert np.all(np.abs(rho[:, s] - ((ao @ D[s]) * ao).sum(1)) <= 4 * n * U * size + lost + 1e-290)
+        c = pot[s][..., None]
+        Q = c[0] * ao + sum(c[1 + j] * g1[..., j] for j in range(3)) + c[4] * lap
+        aQ = np.abs(c[0] * ao) + sum(np.abs(c[1 + j] * g1[..., j]) for j in range(3)) + np.abs(c[4] * lap)
+        ref, size = ao.T @ Q, np.abs(ao).T @ aQ
+        lost = np.abs(ao).max(0)[:, None] * aQ.max(0)[None]
+        for j in range(3):
+            K = c[5] * g1[..., j]
+            ref += g1[..., j].T @ K
+            size += np.abs(g1[..., j]).T @ np.abs(K)
+            lost += np.abs(g1[..., j]).max(0)[:, None] * np.abs(K).max(0)[None]
+        assert np.all(np.abs(v[s] - ref) <= (N + 400) * U * size + N * 2.0 ** -52 * np.maximum(lost, lost.T) + 1e-290)

@@ -2,7 +2,7 @@
 largest where the integration weights are smallest, beside diffuse ones.
 
 Bound, element by element.  A row is fixed point on its largest value after each point's power of two (half the
-exponent of the point's largest coefficient), 61 bits, and the products left out are below 2^-58 of the product of the
+exponent of the point's largest coefficient, relative to the spin's largest; of the two spins' the larger), 61 bits, and the products left out are below 2^-58 of the product of the
 rows' powers of two.  Those are at most twice the largest phi 2^t and 2^5 times the largest term of Q 2^-t (three
 octaves for the sum of five terms, a quarter for the approximate product, one for the mantissa), so 2^-52 of the
 product of these maxima for each point.  Without the octaves the maxima are those of phi and Q themselves, thousands
@@ -20,8 +20,12 @@ ALPHAS = np.array([1e10, 1e8, 1e6, 6665.0, 30.0, 1.0, 0.15])
 
 
 def _octaves(c):
-    """2^t, t half the exponent of the largest |c| of a point (floor), c (k, N)."""
-    return 2.0 ** ((np.frexp(np.abs(c).max(0))[1] - 1) // 2)
+    """2^t of the points or AOs: t half the difference of the high words of the largest |c| there and of the spin's
+    largest, in octaves (floor), the larger of the spins'; c (spin, k, points); 0 where there is none."""
+    hi = (np.ascontiguousarray(np.abs(c).max(1)).view(np.int64) >> 32).astype(np.int64)
+    t = (hi - hi.max(1, keepdims=True)) >> 21
+    t = np.where(hi > 0, t, -1200).max(0)
+    return np.where(t > -1200, 2.0 ** np.maximum(t, -1023), 0.0)
 
 
 def _tables(N, seed):
@@ -54,7 +58,7 @@ def test_vxc(E, terms):  # noqa: F811
     got = r.vxc_from_potentials(pot).cpu().numpy()
     assert r.status() == 0
     lap = g2.sum(-1)
-    t0, t1 = _octaves(pot[:, :5].reshape(-1, N))[:, None], _octaves(np.maximum(pot[:, 5], 1e-300))[:, None]
+    t0, t1 = _octaves(pot[:, :5])[:, None], _octaves(pot[:, 5:])[:, None]
     for s in range(2):
         c = pot[s][..., None]
         each = [c[0] * phi, *(c[1 + j] * g1[..., j] for j in range(3)), c[4] * lap]
@@ -71,16 +75,16 @@ def test_vxc(E, terms):  # noqa: F811
 
 
 def test_exact_exchange_fock(E):  # noqa: F811
-    """F = ao^T B with B = -1/2 sum_w g chi: the octaves are those of g, and both rows' powers of two are at most twice
-    their largest values, 2^-56 of whose product is lost for each point."""
+    """F = ao^T B with B = -1/2 sum_w g chi: the octaves are those of each spin's g, and both rows' powers of two are at
+    most twice their largest values, 2^-56 of whose product is lost for each point."""
     N, n = 300, len(ALPHAS)
     phi, _, _, _, w, v = _tables(N, 2)
     chi = phi[:, None, None] * np.random.default_rng(3).uniform(0.5, 1.0, (N, 2, 2, 1))
     g = -(w * v)[None, None] * np.array([1.0, 0.6])[:, None, None] * np.array([1.0, 0.7])[None, :, None]
     c = lambda x: torch.as_tensor(x, device="cuda")  # noqa: E731
     got = E.hf_fock(c(phi), c(chi), c(g)).cpu().numpy()
-    t = _octaves(g.reshape(-1, N))[:, None]
     for s in range(2):
+        t = 2.0 ** ((np.frexp(np.abs(g[:, s]).max(0))[1] - 1) // 2)[:, None]
         B = -0.5 * sum(g[o, s][:, None] * chi[:, o, s] for o in range(2))
         size = np.abs(phi).T @ np.abs(B)
         bound = (N + 200) * U * size + N * 2.0 ** -56 * np.abs(phi * t).max(0)[:, None] * np.abs(B / t).max(0)
@@ -90,7 +94,7 @@ def test_exact_exchange_fock(E):  # noqa: F811
 @pytest.mark.parametrize("faint", [0.0, 1e-9, 1.0])
 def test_density(E, faint):  # noqa: F811
     """Features of density matrices that hold little of the two steepest functions.  phi_a is taken times 2^t, D_ab
-    times 2^-t, t half the exponent of D's largest entry in row or column a: X is off by 2^-56 of the product of these
+    times 2^-t, t from D's largest entry in row or column a as above: X is off by 2^-56 of the product of these
     rows' largest values for each of n products (2^-55 where D + D^T is contracted), tau by such sums over d_j phi."""
     N = 300
     phi, g1, g2, *_ = _tables(N, 4)
@@ -104,8 +108,7 @@ def test_density(E, faint):  # noqa: F811
     r = E.Resident.from_tables(phi, g1, g2, np.ones(N), "fp64", "cuda:0")
     out = {k: v.cpu().numpy() for k, v in r.density(D).items()}
     assert r.status() == 0
-    big = np.abs(D).max((0, 1))
-    t = np.where(big > 0, 2.0 ** ((np.frexp(np.maximum(big, 1e-300))[1] - 1) // 2), 0.0)
+    t = _octaves(np.concatenate([D, D.transpose(0, 2, 1)], 1))
     lap, k = g2.sum(-1), 2 * n + 20
     for s in range(2):
         X, aX = phi @ D[s], np.abs(phi) @ np.abs(D[s])
@@ -138,11 +141,33 @@ def test_exact_exchange_energy(E):  # noqa: F811
     D = np.random.default_rng(7).standard_normal((2, n, n))
     D[:, :4] = D[:, :, :4] = 0.0
     got = E.hf_energy_density(*(torch.as_tensor(x, device="cuda") for x in (phi, D, chi))).cpu().numpy()
-    big = np.maximum(np.abs(D).max((0, 1)), np.abs(D).max((0, 2)))[4:]
-    t = np.r_[np.zeros(4), 2.0 ** ((np.frexp(big)[1] - 1) // 2)]
     for s in range(2):
+        t = _octaves(np.concatenate([D[s], D[s].T])[None])
         c = np.abs(chi[:, 0, s])
         scaled = (np.abs(D[s, 4:]) / t[4:, None]).max(0)
         bound = (2 * n + 20) * U * (np.abs(phi) @ np.abs(D[s]) * c).sum(1)
         bound += n * 2.0 ** -56 * (np.abs(phi) * t).max(1) * (scaled * c).sum(1)
         assert np.all(np.abs(got[0, s] + 0.5 * (chi[:, 0, s] * (phi @ D[s])).sum(1)) <= bound)
+
+
+@pytest.mark.parametrize("spin", [0, 1])
+def test_spins_of_different_size(E, spin):  # noqa: F811
+    """The spins share the digits of phi: an entry of one spin's D or potentials that is larger by 2^440 takes nothing
+    from the other spin's results."""
+    n, N = 40, 300
+    g = np.random.default_rng(12)
+    ao, g1, g2 = (g.standard_normal((N, n) + s) for s in ((), (3,), (3,)))
+    D, pot = g.standard_normal((2, n, n)), g.standard_normal((2, 6, N))
+    D[spin, 3, 7], pot[spin, :, 11] = 2.0 ** 440, 2.0 ** 440
+    r = E.Resident.from_tables(ao, g1, g2, np.ones(N), "fp64", "cuda:0")
+    rho, v = r.density(D)["rho"].cpu().numpy(), r.vxc_from_potentials(pot).cpu().numpy()
+    s, lap = 1 - spin, g2.sum(-1)
+    size = ((np.abs(ao) @ np.abs(D[s])) * np.abs(ao)).sum(1)
+    assert np.all(np.abs(rho[:, s] - ((ao @ D[s]) * ao).sum(1)) <= 4 * n * U * size)
+    c = pot[s][..., None]
+    each = [c[0] * ao, *(c[1 + j] * g1[..., j] for j in range(3)), c[4] * lap]
+    ref, size = ao.T @ sum(each), np.abs(ao).T @ sum(np.abs(t) for t in each)
+    for j in range(3):
+        ref += g1[..., j].T @ (c[5] * g1[..., j])
+        size += np.abs(g1[..., j]).T @ np.abs(c[5] * g1[..., j])
+    assert np.all(np.abs(v[s] - ref) <= (N + 400) * U * size)  # 2^-52 of maxima of a few units is well inside
