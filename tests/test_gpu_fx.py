@@ -263,3 +263,40 @@ def test_past_the_digits_range(E, what):
             size += np.abs(g1[..., j]).T @ np.abs(K)
             lost += np.abs(g1[..., j]).max(0)[:, None] * np.abs(K).max(0)[None]
         assert np.all(np.abs(v[s] - ref) <= (N + 400) * U * size + N * 2.0 ** -52 * np.maximum(lost, lost.T) + 1e-290)
+
+
+@pytest.mark.parametrize("n,N", [(24, 400), (115, 300), (400, 120)])
+def test_error_against_longer_sums(E, n, N):
+    """The rounding error in itself, against sums in numpy's longer type (64 or 113 bits), as the root mean square over
+    the points of the error relative to the sum of the terms' sizes.
+
+    Independent roundings of up to half a unit (U / sqrt 3 in the mean square): one of each X, the n / 8 + 11 additions
+    of a feature, and for V the additions of its partial sums, of which there are at most ten at these sizes."""
+    g = np.random.default_rng(n)
+    ao, g1, g2 = (g.standard_normal((N, n) + s) for s in ((), (3,), (3,)))
+    q = np.linalg.qr(g.standard_normal((2, n, n)))[0][:, :, :max(1, n // 8)]
+    D = q @ q.transpose(0, 2, 1)
+    pot = g.standard_normal((2, 6, N))
+    r = _resident(E, ao, g1, g2)
+    out, v = r.density(D), r.vxc_from_potentials(pot).cpu().numpy()
+    L = np.longdouble
+    A, G, lap, limit = ao.astype(L), g1.astype(L), g2.sum(-1), U * (1 + np.sqrt((n / 8 + 12) / 3))
+    rms = lambda got, ref, size: float(np.sqrt(np.mean(((got - ref) / size) ** 2)))  # noqa: E731
+    for s in range(2):
+        Dl = D[s].astype(L)
+        X, aX = A @ Dl, np.abs(ao) @ np.abs(D[s])
+        kin = sum(((G[..., j] @ Dl) * G[..., j]).sum(1) for j in range(3))
+        akin = sum(((np.abs(g1[..., j]) @ np.abs(D[s])) * np.abs(g1[..., j])).sum(1) for j in range(3))
+        o = {k: t[:, s].cpu().numpy() for k, t in out.items()}
+        assert rms(o["rho"], (X * A).sum(1), (aX * np.abs(ao)).sum(1)) <= limit
+        for j in range(3):
+            assert rms(o["grad_rho"][:, j], 2 * (X * G[..., j]).sum(1), 2 * (aX * np.abs(g1[..., j])).sum(1)) <= limit
+        assert rms(o["tau"], kin / 2, akin / 2) <= limit
+        assert rms(o["lapl"], 2 * kin + 2 * (X * lap.astype(L)).sum(1), 2 * akin + 2 * (aX * np.abs(lap)).sum(1)) <= limit
+        c = pot[s].astype(L)[..., None]
+        each = [c[0] * A, *(c[1 + j] * G[..., j] for j in range(3)), c[4] * lap.astype(L)]
+        ref, size = A.T @ sum(each), np.abs(ao).T @ sum(np.abs(t).astype(float) for t in each)
+        for j in range(3):
+            ref = ref + G[..., j].T @ (c[5] * G[..., j])
+            size += np.abs(g1[..., j]).T @ np.abs(c[5] * G[..., j]).astype(float)
+        assert rms(v[s], ref, size) <= U * (1 + np.sqrt((5 + 10) / 3))
