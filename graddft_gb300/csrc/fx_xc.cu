@@ -35,7 +35,7 @@
 // faster one at every size (E_xc + V_xc, B88+LYP, plain kernels -> here: 4 AOs x
 // 128 points 779 -> 294 us, 24 x 3,600 928 -> 397 us, 100 x 10,000 5.4 -> 0.74 ms,
 // 400 x 150,001 827 -> 27.6 ms; with the point kernel's and launches' later forms 24 x
-// 3,600 147 us, 400 x 150,001 22.6 ms), and the more accurate one (features at 400 AOs
+// 3,600 146 us, 400 x 150,001 22.9 ms), and the more accurate one (features at 400 AOs
 // against quadruple precision: 1.4e-16 .. 2.7e-16, before 2.7e-16 .. 6.0e-16).
 #include "common.cuh"
 #include "fx.cuh"
@@ -371,7 +371,7 @@ __global__ void __launch_bounds__(256) fx_vmax_kernel(const double *__restrict__
 // for plane t.  One plane's values live at a time (the planes are read again from
 // L1): with all five in registers one block of 168 registers a thread fitted an SM
 // and the kernel ran at 3 TB/s, bound by its latencies (6,800 points x 400 AOs 187 us,
-// then 139).  The three blocks of a tile are neighbours in the launch, so that its
+// then 139; 72 bytes are spilled at 64 registers, and one block less an SM costs more).  The three blocks of a tile are neighbours in the launch, so that its
 // planes come from HBM once (128 us).  The blocks of chunk 0 write
 // the exponent fields of the operand rows: ea [2][128 mt] (phi, kinetic), eb
 // [2][128 nb] (Q, kinetic; tile rows 64 of each spin).

@@ -638,7 +638,7 @@ def _chi(chi, ao):
 def hf_energy_density(ao, rdm1, chi, form: str = "fp64") -> torch.Tensor:
     """molecule.py:507-541: ehf (omega, 2, grid) = -1/2 einsum("rwsc,sac,ra->wsr", chi, rdm1, ao).
 
-    ``form`` "fp64" contracts on the FP64 GEMM, "tf32x3" on the block-scaled three-slice tensor-core GEMM.
+    ``form`` "fp64" contracts on the FP64 form's digit products, "tf32x3" on the block-scaled three-slice tensor-core GEMM.
     """
     dev = require_cuda(ao.device if isinstance(ao, torch.Tensor) and ao.is_cuda else None)
     code = _hf_form(form)

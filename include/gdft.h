@@ -47,7 +47,10 @@ enum {
 
 /* Arithmetic forms of the path. */
 enum {
-  GDFT_FP64 = 0,    /* plain FP64 form: FP64 contractions and FP64 point work      */
+  GDFT_FP64 = 0,    /* FP64 form: contractions as exact 9-bit digit products on tcgen05,
+                       errors relative to the product of two operand rows' largest
+                       values (2^-56 for each term, V_xc 2^-52); FP64 point work;
+                       operands not finite or above 2^450: plain FP64 sums     */
   GDFT_TF32X3 = 1   /* mixed form: tcgen05 TF32 3-term split products, FP32
                        accumulation inside a K-chunk, FP64 across chunks       */
 };
