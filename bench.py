@@ -1154,9 +1154,9 @@ def main():
     # Kernels per step of the library's XC call (the stage timers count regions, some of which hold
     # several kernels): mixed pack_rdm1, dens_tc, xc_point, energy_reduce, build_q, tcg3 (twice from
     # two tiles of 128 AOs on), vxc_q_reduce; FP64, with one slab of the grid (more slabs launch
-    # more): fx clear, rdm1, rows, gemm, features, dens_f64, xc_point, energy_reduce, clear, vmax,
-    # vdigits, gemm, vreduce, vxc_f64, vxc_reduce.
-    launches = ((8 if args.n_ao > 128 else 7) if form == "tf32x3" else 15) * args.steps
+    # more): fx rdm1_max, octaves, rdm1, rows, gemm, features, dens_f64, xc_point, energy_reduce,
+    # clear, coef_max, vmax, vdigits, gemm, vreduce, vxc_f64, vxc_reduce.
+    launches = ((8 if args.n_ao > 128 else 7) if form == "tf32x3" else 17) * args.steps
     if world > 1:
         import torch.distributed as dist
 
