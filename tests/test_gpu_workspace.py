@@ -10,8 +10,6 @@ from graddft_gb300 import synthetic
 
 pytestmark = pytest.mark.gpu
 
-ERR = 256  # a workspace ends in the block that holds its error word, which a caller clears
-
 
 @pytest.fixture(scope="module")
 def E(built_lib):
@@ -25,12 +23,6 @@ def E(built_lib):
 def _workload(n_ao, n_grid, seed=1):
     wl = synthetic.make_workload(n_grid, n_ao, max(1, n_ao // 8), seed=seed, box_angstrom=7.0, centre_box_angstrom=4.0)
     return wl, O.eval_ao_planes(wl.basis, wl.coords)
-
-
-def _workspace(nbytes, value):
-    ws = torch.full((nbytes,), value, dtype=torch.uint8, device="cuda")
-    ws[-ERR:] = 0
-    return ws
 
 
 @pytest.mark.parametrize("precision", ["fp64", "tf32x3"])
@@ -55,7 +47,7 @@ def test_contents_do_not_matter(E, precision, n_ao, n_grid):
         p = [E._ptr(t) for t in out]
 
         def ws():  # fresh for each call
-            t = _workspace(nbytes.value, value)
+            t = torch.full((nbytes.value,), value, dtype=torch.uint8, device="cuda")
             return t, E._ptr(t), t.numel()
 
         keep = [ws() for _ in range(4)]
@@ -85,19 +77,13 @@ def test_network_contents_do_not_matter(E, net_form):
     ehf = torch.as_tensor(synthetic.make_ehf(n_grid, 3, None, 2), device="cuda")
     d = torch.as_tensor(wl.rdm1, device="cuda")
     mol, dn, st = ctypes.byref(r.desc), ctypes.byref(net.desc), E._stream(r.device)
-    nb, hb, xb = ctypes.c_size_t(), ctypes.c_size_t(), ctypes.c_size_t()
-    _lib.check(L.gdft_workspace_bytes(mol, ctypes.byref(xb)))
+    nb, hb = ctypes.c_size_t(), ctypes.c_size_t()
     _lib.check(L.gdft_neural_workspace_bytes(mol, dn, ctypes.byref(nb)))
     _lib.check(L.gdft_neural_hvp_workspace_bytes(mol, dn, ctypes.byref(hb)))
 
-    def ws(nbytes, value):
-        t = torch.full((nbytes,), value, dtype=torch.uint8, device="cuda")
-        t[xb.value - ERR:xb.value] = 0
-        return t
-
     def calls(value):
         new = lambda *s: torch.empty(s, dtype=torch.float64, device="cuda")  # noqa: E731
-        a, b, c = ws(nb.value, value), ws(hb.value, value), ws(nb.value, value)
+        a, b, c = (torch.full((x.value,), value, dtype=torch.uint8, device="cuda") for x in (nb, hb, nb))
         out = [new(), new(2, n_ao, n_ao), new(net.n_params), new(), new(2, n_ao, n_ao), new(net.n_params), new(),
                new(2, n_ao, n_ao), new(2, 2, n_grid), new(2, 2, n_grid)]
         q = [E._ptr(t) for t in out]
